@@ -231,7 +231,6 @@ struct pibem_handle
     d_parents, d_diag_col, d_m2p_pair_tgt, d_q_src, d_ch_start, d_ch_cnt, d_ch_op, d_up_box,
     d_down_box, d_up_q, d_down_q, d_up_child8, d_down_par, d_m2p_item_pair, d_m2l_yslot,
     d_down_m2l_beg, d_down_m2l_end, d_m2p_tnodes;
-  DBuf<uint8_t> d_down_oct;
   DBuf<NearEntry> d_entries;
   DBuf<double>  d_N, d_D, d_S, d_T1, d_T2, d_W, d_ops, d_Tc;
   // leaf-block Jacobi inverses, column-major: FP32 for the mixed path, FP64
@@ -336,7 +335,7 @@ struct pibem_handle
     add(d_row_leaf, d_nrows, d_ncols, d_pleaf_box, d_prow_dof, d_pcontrib_q, d_lleaf_box,
         d_gather_ptr, d_gather_ids, d_m2l_tgt, d_m2l_src, d_m2l_off, d_m2p_tgt, d_m2p_src,
         d_l2l_box, d_parents, d_diag_col, d_m2p_pair_tgt, d_q_src, d_ch_start, d_ch_cnt, d_ch_op,
-        d_up_box, d_down_box, d_up_q, d_down_q, d_up_child8, d_down_par, d_down_oct,
+        d_up_box, d_down_box, d_up_q, d_down_q, d_up_child8, d_down_par,
         d_m2p_item_pair, d_m2l_yslot, d_down_m2l_beg, d_down_m2l_end, d_m2p_tnodes);
     add(d_con_row, d_con_col, d_con_p, d_con_q, d_con_kind, d_con_nrm, d_con_sg);
     add(d_ilu_ptr, d_ilu_diag, d_ilu_col, d_ilu_rows_lo, d_ilu_rows_up, d_ilu_val);
@@ -1866,16 +1865,27 @@ namespace
       op.down_q_ptr    = h->d_down_q_ptr.p;
       op.up_child8     = h->d_up_child8.p;
       op.down_par      = h->d_down_par.p;
-      op.down_oct      = h->d_down_oct.p;
       op.m2l_yslot     = h->d_m2l_yslot.p;
       op.down_m2l_beg  = h->d_down_m2l_beg.p;
       op.down_m2l_end  = h->d_down_m2l_end.p;
       op.lv_op0        = int(pl.offsets.size() / 3);
-      op.down_l2l_level.assign(pl.down_box_ptr.size(), 0);
+      // the boxes with an L2L parent, by level and octant (listed in that order)
+      op.down_oct_ptr.assign(pl.down_box_ptr.empty() ? 0 : pl.down_box_ptr.size() - 1, LevelOctants());
       for (size_t l = 0; l + 1 < pl.down_box_ptr.size(); ++l)
-        for (int i = pl.down_box_ptr[l]; i < pl.down_box_ptr[l + 1]; ++i)
-          if (pl.down_par[i] >= 0)
-            op.down_l2l_level[l] = 1;
+        {
+          int i = pl.down_box_ptr[l];
+          while (i < pl.down_box_ptr[l + 1] && pl.down_par[i] < 0)
+            ++i;
+          for (int o = 0; o < 8; ++o)
+            {
+              op.down_oct_ptr[l].p[o] = i;
+              while (i < pl.down_box_ptr[l + 1] && pl.down_par[i] >= 0 && pl.down_oct[i] == o)
+                ++i;
+            }
+          op.down_oct_ptr[l].p[8] = i;
+          if (i != pl.down_box_ptr[l + 1])
+            throw Error(PIBEM_EINVAL, "internal plan check failed: L2L boxes not listed by octant");
+        }
       op.n_pairs       = int64_t(pl.q_src.size());
       op.Tc            = nullptr; // made by set_bc
       op.max_near_cols = 0;
@@ -2240,7 +2250,6 @@ namespace
     h->d_down_q_ptr.upload(pl.down_q_ptr, s);
     h->d_up_child8.upload(pl.up_child8, s);
     h->d_down_par.upload(pl.down_par, s);
-    h->d_down_oct.upload(pl.down_oct, s);
     h->d_m2l_yslot.upload(pl.m2l_yslot, s);
     h->d_down_m2l_beg.upload(pl.down_m2l_beg, s);
     h->d_down_m2l_end.upload(pl.down_m2l_end, s);

@@ -72,6 +72,13 @@ namespace pibem
   constexpr int NEAR_BLOCKS_PER_SM_F32  = 6;
   constexpr int NEAR_BLOCKS_PER_SM_WIDE = 5;
 
+  // a level's boxes with an L2L parent in the down_box list: octant o has the
+  // entries [p[o], p[o + 1])
+  struct LevelOctants
+  {
+    int p[9] = {};
+  };
+
   template <typename T>
   struct OperatorDev
   {
@@ -108,14 +115,13 @@ namespace pibem
     const int32_t *up_box = nullptr, *down_box = nullptr, *up_q = nullptr, *down_q = nullptr;
     const int64_t *up_q_ptr = nullptr, *down_q_ptr = nullptr;
     // fused level passes (levels.cu): children of each up_box entry by octant,
-    // L2L parent (-1: none) and octant of each down_box entry; the M2M
+    // L2L parent of each down_box entry (-1: none); the M2M
     // operators are ops[lv_op0 .. lv_op0 + 7], the L2L ones the next 8
     const int32_t *up_child8 = nullptr, *down_par = nullptr;
-    const uint8_t *down_oct  = nullptr;
     int            lv_op0    = 0;
     const T       *lv_ops    = nullptr; // the 16 level operators, each padded to 16 bytes
     int           *dev_err   = nullptr; // set by a bounded device wait that timed out
-    std::vector<char> down_l2l_level; // per level: its boxes receive L2L
+    std::vector<LevelOctants> down_oct_ptr; // per level
     // target-major M2L products (fused passes): slot of each M2L pair, and the
     // slot range of each down_box entry
     const int32_t *m2l_yslot = nullptr, *down_m2l_beg = nullptr, *down_m2l_end = nullptr;

@@ -11,19 +11,19 @@
 // round trip of the products through HBM.  Here a block computes complete
 // expansions of up to CPB columns (column = (box, right-hand side)).
 //
-// Threads: groups of KT = 32 ceil(K/32) (at most 128) threads; thread t of a
-// group owns output coefficients t, t + KT, ...  Every column's result is
-// computed by a fixed sequence of operations that depends on the column's own
-// data only (M2M: one octant per group, the eight partial sums added in a
-// fixed order; L2L: one thread per output coefficient, k ascending; M2L sums:
-// one warp per 32 coefficients, pairs in list order): the same bits whatever
-// the number of columns, their grouping into blocks or the other columns of
-// the batch.
+// Threads: LV_G groups of KT = 32 ceil(K/32) (at most 128) threads; thread t of a
+// group owns output coefficient t of the group's columns g, g + LV_G, ...  Every
+// column's result is computed by a fixed sequence of operations that depends on
+// the column's own data only (a K-term chain with k ascending per operator; M2M:
+// the eight octants' products added in a fixed order; M2L sums: one warp per 32
+// coefficients, pairs in list order): the same bits whatever the number of
+// columns, their grouping into blocks or the other columns of the batch.
 //
-// Where the eight operators of a pass fit in shared memory (K <= 81, p <= 8)
-// the M2M and L2L kernels are persistent (one block per SM) and read the
-// operators from shared memory, copied there once per launch; otherwise they
-// read them through the L1 cache.
+// A block holds one operator (26 KB at p = 8, 59 KB at p = 10) in shared memory.
+// The passes are short chains of small launches, so what bounds them is latency:
+// the operator's copy is started before the block waits for the launch ahead of
+// it (the operators are constants of the mesh), and one operator per block
+// leaves room for the next level's blocks beside the running ones.
 #include <algorithm>
 #include <cstdint>
 
@@ -37,94 +37,203 @@ namespace pibem
   {
     __host__ __device__ inline int lv_kx(int K) { return (K + 3) / 4 * 4; }
 
-    // acc[c] += sum_{k in [k0, k1)} T[k][ko] X[c][k], k ascending, eight
-    // operator loads in flight; T is one operator stored [in][out]
-    template <int CPB>
-    __device__ __forceinline__ void lv_dot(float (&acc)[CPB], const float *__restrict__ T, int K,
-                                           int ko, const float *X, int Kx, int k0, int k1)
+    constexpr int  LV_G          = 4; // column groups per block
+    constexpr long LV_SPIN_LIMIT = 1L << 24;
+
+    __host__ __device__ inline int lv_kk(int K) { return (K * K + 3) / 4 * 4; } // padded operator
+
+    // acc[i] = sum_k T[k][ko] X[g + LV_G i][k], k ascending; T one operator stored
+    // [in][out], both in shared memory
+    template <int C>
+    __device__ __forceinline__ void lv_dot(float (&acc)[C], const float *T, const float *X, int K,
+                                           int Kx, int ko)
     {
-      int k = k0;
-      for (; k + 8 <= k1; k += 8)
+#pragma unroll
+      for (int i = 0; i < C; ++i)
+        acc[i] = 0.0f;
+      int k = 0;
+#pragma unroll 4
+      for (; k + 4 <= K; k += 4)
         {
-          float t[8];
+          float tv[4];
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
-            t[u] = __ldg(T + size_t(k + u) * K + ko);
+          for (int u = 0; u < 4; ++u)
+            tv[u] = T[(k + u) * K + ko];
 #pragma unroll
-          for (int c = 0; c < CPB; ++c)
+          for (int i = 0; i < C; ++i)
             {
-              const float *x = X + c * Kx + k;
-#pragma unroll
-              for (int u = 0; u < 8; ++u)
-                acc[c] = fmaf(t[u], x[u], acc[c]);
+              const float4 xv = *reinterpret_cast<const float4 *>(X + i * LV_G * Kx + k);
+              acc[i]          = fmaf(tv[0], xv.x, acc[i]);
+              acc[i]          = fmaf(tv[1], xv.y, acc[i]);
+              acc[i]          = fmaf(tv[2], xv.z, acc[i]);
+              acc[i]          = fmaf(tv[3], xv.w, acc[i]);
             }
         }
-      for (; k < k1; ++k)
+      for (; k < K; ++k)
         {
-          const float t = __ldg(T + size_t(k) * K + ko);
+          const float tv = T[k * K + ko];
 #pragma unroll
-          for (int c = 0; c < CPB; ++c)
-            acc[c] = fmaf(t, X[c * Kx + k], acc[c]);
+          for (int i = 0; i < C; ++i)
+            acc[i] = fmaf(tv, X[i * LV_G * Kx + k], acc[i]);
         }
     }
 
-    // One level of the upward pass; 8 groups, group o applies the octant-o
-    // operator.  Columns c = i * R + r over the level's parents i (par[i],
-    // children child8[8 i + o], -1: none).  Shared memory: the children's
-    // expansions X[o][CPB][Kx] (zero where a child is missing), then the
-    // partial sums P[o][CPB][Kx].
-    template <int CPB>
-    __global__ void __launch_bounds__(1024)
-      m2m_level_kernel(int R, int K, int ncols, const int32_t *__restrict__ par,
-                       const int32_t *__restrict__ child8, const float *__restrict__ ops,
-                       float *__restrict__ M)
+    // Thread 0 starts the bulk copy of one operator (lv_kk(K) floats, 16-byte
+    // aligned) into shared memory, completing on the barrier.
+    __device__ inline void lv_start_op(float *dst, const float *src, int K, uint32_t bar)
     {
-      extern __shared__ float lv_sm[];
-      const int Kx = lv_kx(K);
-      float    *X  = lv_sm;
-      float    *P  = lv_sm + 8 * CPB * Kx;
-      const int KT = blockDim.x / 8;
-      const int g = threadIdx.x / KT, t = threadIdx.x - g * KT;
-      const int c0 = blockIdx.x * CPB, nc = min(CPB, ncols - c0);
-      for (int i = threadIdx.x; i < 8 * CPB * Kx; i += blockDim.x)
+      const uint32_t bytes = uint32_t(lv_kk(K)) * 4u;
+      mbar_arrive_expect_tx(bar, bytes);
+      bulk_copy(smem_u32(dst), src, bytes, bar);
+    }
+
+    // Every thread waits (bounded) for the operator; false after a timeout,
+    // which is recorded in *err.
+    __device__ inline bool lv_wait_op(uint32_t bar, uint32_t parity, int *err)
+    {
+      if (mbar_wait_bounded(bar, parity, LV_SPIN_LIMIT))
+        return true;
+      atomicExch(err, 1);
+      return false;
+    }
+
+    __device__ inline void prefetch_l1(const void *p)
+    {
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+    }
+
+    __device__ inline uint32_t cluster_rank()
+    {
+      uint32_t r;
+      asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+      return r;
+    }
+    __device__ inline void cluster_barrier()
+    {
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+    // 16 bytes at shared-memory address addr of the block with the given rank
+    __device__ inline float4 ld_cluster(uint32_t addr, uint32_t rank)
+    {
+      uint32_t a;
+      float4   v;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                   : "r"(a)
+                   : "memory");
+      return v;
+    }
+
+    // One level of the upward pass.  Columns c = i * R + r over the level's
+    // parents i (par[i], children child8[8 i + o], -1: none).  A cluster of
+    // eight blocks takes batches of LV_G C columns: the block of rank o applies
+    // the octant-o operator to the batch's octant-o children (zero where there
+    // is none) and leaves its products in its shared memory; after a cluster
+    // barrier each block adds the eight blocks' products of an eighth of the
+    // batch, read through distributed shared memory.  The products are double
+    // buffered, so a batch has one cluster barrier.
+    // Shared memory: T[lv_kk], X[LV_G C][Kx], P[2][LV_G C][Kx].
+    // What bounds it: latency (a level's arithmetic is below a microsecond).  Measured
+    // (kernel times, warm caches, GB300), against one block per SM holding all
+    // eight operators: 98k spheroid, p = 8, five levels 50 -> 46 us, and less in the
+    // step, where the copies overlap the launch ahead; 55k hull, p = 10, seven
+    // levels 85 -> 65 us (the operators read through L1 before).
+    template <int C>
+    __global__ void __launch_bounds__(LV_G * 128)
+      m2m_level_kernel(int R, int K, int ncols, const int32_t *__restrict__ par,
+                       const int32_t *__restrict__ child8, const float *__restrict__ lvops,
+                       float *__restrict__ M, int *__restrict__ err)
+    {
+      extern __shared__ __align__(16) float lv_sm[];
+      __shared__ uint64_t op_bar;
+      constexpr int NB = LV_G * C; // columns of a batch
+      const int Kx = lv_kx(K), n4 = Kx / 4;
+      float    *T = lv_sm, *X = T + lv_kk(K), *P = X + NB * Kx;
+      const int KT = blockDim.x / LV_G;
+      const int g = threadIdx.x / KT, ko = threadIdx.x - g * KT; // KT >= Kx: one coefficient
+      const int o = int(cluster_rank());
+      const uint32_t bar = smem_u32(&op_bar);
+      if (threadIdx.x == 0)
         {
-          const int k = i % Kx, oc = i / Kx, c = oc % CPB, o = oc / CPB;
-          float     v = 0.0f;
-          if (c < nc && k < K)
-            {
-              const int col = c0 + c, pi = col / R, r = col - pi * R;
-              const int ch  = child8[8 * pi + o];
-              if (ch >= 0)
-                v = M[(int64_t(ch) * R + r) * K + k];
-            }
-          X[i] = v;
+          mbar_init(bar, 1);
+          mbar_init_fence();
+          lv_start_op(T, lvops + size_t(o) * lv_kk(K), K, bar);
         }
-      bool has = false; // some column of the block has an octant-g child
-      for (int c = 0; c < nc; ++c)
-        has = has || child8[8 * ((c0 + c) / R) + g] >= 0;
-      __syncthreads();
-      for (int ko = t; ko < K; ko += KT)
+      const int cl = blockIdx.x >> 3, ncl = gridDim.x >> 3;
+      if (threadIdx.x < NB && cl * NB + int(threadIdx.x) < ncols)
         {
-          float acc[CPB];
-#pragma unroll
-          for (int c = 0; c < CPB; ++c)
-            acc[c] = 0.0f;
-          if (has)
-            lv_dot<CPB>(acc, ops + size_t(g) * K * K, K, ko, X + g * CPB * Kx, Kx, 0, K);
-#pragma unroll
-          for (int c = 0; c < CPB; ++c)
-            P[(g * CPB + c) * Kx + ko] = acc[c];
+          const int pi = (cl * NB + threadIdx.x) / R;
+          prefetch_l1(child8 + 8 * pi + o);
+          prefetch_l1(par + pi);
         }
-      __syncthreads();
-      if (g == 0)
-        for (int ko = t; ko < K; ko += KT)
-          for (int c = 0; c < nc; ++c)
+      pdl_entry();
+      bool      ops_ok = true, waited = false;
+      int       buf = 0;
+      for (int c0 = cl * NB; c0 < ncols; c0 += ncl * NB, buf ^= 1)
+        {
+          const int nc = min(NB, ncols - c0);
+          // thread (g, ko) brings coefficient ko of the columns it computes
+          float v[C];
+#pragma unroll
+          for (int i = 0; i < C; ++i)
             {
-              const int col = c0 + c, pi = col / R, r = col - pi * R;
-              auto      at  = [&](int o) { return P[(o * CPB + c) * Kx + ko]; };
-              const float v = ((at(0) + at(1)) + (at(2) + at(3))) + ((at(4) + at(5)) + (at(6) + at(7)));
-              M[(int64_t(par[pi]) * R + r) * K + ko] = v;
+              const int c = g + LV_G * i, col = c0 + c, pi = col / R;
+              const int ch = c < nc && ko < K ? child8[8 * pi + o] : -1;
+              v[i]         = ch >= 0 ? M[(int64_t(ch) * R + (col - pi * R)) * K + ko] : 0.0f;
             }
+          if (ko < Kx)
+#pragma unroll
+            for (int i = 0; i < C; ++i)
+              X[(g + LV_G * i) * Kx + ko] = v[i];
+          __syncthreads();
+          if (!waited)
+            {
+              ops_ok = lv_wait_op(bar, 0, err);
+              waited = true;
+            }
+          float *Pb = P + buf * NB * Kx;
+          if (ko < Kx)
+            {
+              float acc[C];
+              if (ko < K && ops_ok)
+                lv_dot<C>(acc, T, X + g * Kx, K, Kx, ko);
+              else
+#pragma unroll
+                for (int i = 0; i < C; ++i)
+                  acc[i] = 0.0f;
+#pragma unroll
+              for (int i = 0; i < C; ++i)
+                Pb[(g + LV_G * i) * Kx + ko] = acc[i];
+            }
+          cluster_barrier(); // the eight blocks' products are in place; X is no longer read
+          for (int i = o * blockDim.x + threadIdx.x; i < nc * n4; i += 8 * blockDim.x)
+            {
+              const int c = i / n4, q = i - c * n4;
+              float4    v[8];
+#pragma unroll
+              for (int b = 0; b < 8; ++b)
+                v[b] = ld_cluster(smem_u32(Pb) + uint32_t(c * Kx + 4 * q) * 4u, uint32_t(b));
+              const int   col = c0 + c, pi = col / R, r = col - pi * R;
+              float      *m = M + (int64_t(par[pi]) * R + r) * K + 4 * q;
+              const float s[4] = {
+                ((v[0].x + v[1].x) + (v[2].x + v[3].x)) + ((v[4].x + v[5].x) + (v[6].x + v[7].x)),
+                ((v[0].y + v[1].y) + (v[2].y + v[3].y)) + ((v[4].y + v[5].y) + (v[6].y + v[7].y)),
+                ((v[0].z + v[1].z) + (v[2].z + v[3].z)) + ((v[4].z + v[5].z) + (v[6].z + v[7].z)),
+                ((v[0].w + v[1].w) + (v[2].w + v[3].w)) + ((v[4].w + v[5].w) + (v[6].w + v[7].w))};
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                if (4 * q + u < K)
+                  m[u] = s[u];
+            }
+        }
+      if (!waited) // never leave with the copy in flight
+        {
+          __syncthreads();
+          lv_wait_op(bar, 0, err);
+        }
+      cluster_barrier(); // no block leaves while another reads its products
     }
 
     // M2L sums of the boxes of the downward lists, all levels.  The M2L
@@ -184,320 +293,141 @@ namespace pibem
     }
 
     // One level of the downward pass after the M2L sums: L[b] += T_oct L[parent]
-    // for the level's boxes with an L2L parent (par[i] >= 0); 4 groups, group g
-    // takes input coefficients [K g / 4, K (g + 1) / 4).  Columns c = i * R + r.
-    // Shared memory: the parents' expansions X[CPB][Kx], partial sums
-    // P[g][CPB][Kx].
-    template <int CPB>
-    __global__ void __launch_bounds__(512)
-      l2l_level_kernel(int R, int K, int ncols, const int32_t *__restrict__ box,
-                       const int32_t *__restrict__ par, const uint8_t *__restrict__ oct,
-                       const float *__restrict__ ops, float *__restrict__ Lx)
+    // for the level's boxes with an L2L parent.  They are listed by octant (oct:
+    // the bounds of the octants in the list); the columns c = i * R + r of an
+    // octant are cut into batches of LV_G C, numbered octant after octant, and a
+    // block takes a contiguous range of batches, so that a batch has one operator
+    // and most blocks copy one only.  What does not depend on the launch ahead
+    // (the operator, the box ids) is fetched before waiting for it.  Measured (as
+    // above; one block per SM with up to eight operators before): 98k spheroid
+    // 43 -> 33 us over five levels; 55k hull, p = 10, 76 -> 49 us over seven.  A
+    // mixed solve to 1e-12: 50.8 -> 47.2 ms (98k), 67.9 -> 58.6 ms (hull).
+    // Shared memory: T[lv_kk], X[LV_G C][Kx].
+    template <int C>
+    __global__ void __launch_bounds__(LV_G * 128)
+      l2l_level_kernel(int R, int K, LevelOctants oct, int n_batches, const int32_t *__restrict__ box,
+                       const int32_t *__restrict__ par, const float *__restrict__ lvops,
+                       float *__restrict__ Lx, int *__restrict__ err)
     {
-      extern __shared__ float lv_sm[];
+      extern __shared__ __align__(16) float lv_sm[];
+      __shared__ uint64_t op_bar;
+      constexpr int NB = LV_G * C; // columns of a batch
       const int Kx = lv_kx(K);
-      float    *X  = lv_sm;
-      float    *P  = lv_sm + CPB * Kx;
-      const int KT = blockDim.x / 4;
-      const int g = threadIdx.x / KT, t = threadIdx.x - g * KT;
-      const int c0 = blockIdx.x * CPB, nc = min(CPB, ncols - c0);
-      for (int i = threadIdx.x; i < CPB * Kx; i += blockDim.x)
+      float    *T = lv_sm, *X = T + lv_kk(K);
+      const int KT = blockDim.x / LV_G;
+      const int g = threadIdx.x / KT, ko = threadIdx.x - g * KT;
+      int       b_lo = int(int64_t(n_batches) * blockIdx.x / gridDim.x);
+      const int b_hi = int(int64_t(n_batches) * (blockIdx.x + 1) / gridDim.x);
+      if (b_lo >= b_hi)
+        return;
+      // octant of batch b_lo, its first column in the octant
+      int o = 0, c0 = b_lo;
+      for (; o < 7; ++o)
         {
-          const int k = i % Kx, c = i / Kx;
-          float     v = 0.0f;
-          if (c < nc && k < K)
-            {
-              const int col = c0 + c, bi = col / R, r = col - bi * R;
-              const int pb  = par[bi];
-              if (pb >= 0)
-                v = Lx[(int64_t(pb) * R + r) * K + k];
-            }
-          X[i] = v;
+          const int nb = ((oct.p[o + 1] - oct.p[o]) * R + NB - 1) / NB;
+          if (c0 < nb)
+            break;
+          c0 -= nb;
         }
-      // one operator for the whole block when its columns share the octant
-      // (the boxes of a level are listed by octant); the arithmetic per column
-      // is the same either way
-      const int o0      = oct[c0 / R];
-      bool      uniform = true;
-      for (int c = 1; c < nc; ++c)
-        uniform = uniform && oct[(c0 + c) / R] == o0;
-      __syncthreads();
-      const int k0 = K * g / 4, k1 = K * (g + 1) / 4;
-      for (int ko = t; ko < K; ko += KT)
-        {
-          float acc[CPB];
-#pragma unroll
-          for (int c = 0; c < CPB; ++c)
-            acc[c] = 0.0f;
-          if (uniform)
-            lv_dot<CPB>(acc, ops + size_t(o0) * K * K, K, ko, X, Kx, k0, k1);
-          else
-#pragma unroll
-            for (int c = 0; c < CPB; ++c)
-              if (c < nc)
-                {
-                  float a1[1] = {0.0f};
-                  lv_dot<1>(a1, ops + size_t(oct[(c0 + c) / R]) * K * K, K, ko, X + c * Kx, Kx, k0,
-                            k1);
-                  acc[c] = a1[0];
-                }
-#pragma unroll
-          for (int c = 0; c < CPB; ++c)
-            P[(g * CPB + c) * Kx + ko] = acc[c];
-        }
-      __syncthreads();
-      if (g == 0)
-        for (int ko = t; ko < K; ko += KT)
-          for (int c = 0; c < nc; ++c)
-            {
-              const int col = c0 + c, bi = col / R, r = col - bi * R;
-              if (par[bi] < 0)
-                continue;
-              auto        at = [&](int q) { return P[(q * CPB + c) * Kx + ko]; };
-              const float l  = (at(0) + at(1)) + (at(2) + at(3));
-              float      *o  = Lx + (int64_t(box[bi]) * R + r) * K + ko;
-              *o             = *o + l;
-            }
-    }
-
-    __host__ __device__ inline int lv_kk(int K) { return (K * K + 3) / 4 * 4; } // padded operator
-
-    constexpr long LV_SPIN_LIMIT = 1L << 24;
-
-    // Thread 0 starts one bulk copy of n operators (lv_kk(K) floats each,
-    // 16-byte aligned) into shared memory, completing on the barrier; the
-    // barrier is initialised here and visible after the next __syncthreads.
-    __device__ inline void lv_start_ops(float *dst, const float *src, int n, int K, uint64_t *bar)
-    {
+      c0 *= NB;
+      const uint32_t bar = smem_u32(&op_bar);
+      int            held = o, loads = 1, waited = 0; // operator held, copies started and waited for
       if (threadIdx.x == 0)
         {
-          const uint32_t b     = smem_u32(bar);
-          const uint32_t bytes = uint32_t(n) * uint32_t(lv_kk(K)) * 4u;
-          mbar_init(b, 1);
+          mbar_init(bar, 1);
           mbar_init_fence();
-          mbar_arrive_expect_tx(b, bytes);
-          bulk_copy(smem_u32(dst), src, bytes, b);
+          lv_start_op(T, lvops + size_t(o) * lv_kk(K), K, bar);
         }
-    }
-
-    // Every thread waits (bounded) for the operators; false after a timeout,
-    // which is recorded in *err.
-    __device__ inline bool lv_wait_ops(uint64_t *bar, int *err)
-    {
-      if (mbar_wait_bounded(smem_u32(bar), 0, LV_SPIN_LIMIT))
-        return true;
-      atomicExch(err, 1);
-      return false;
-    }
-
-    // M2M of one level with the eight operators in shared memory; persistent
-    // blocks take batches of CPB columns.  8 groups, group o applies octant o.
-    // Shared memory: T[8][lv_kk], X[8][CPB][Kx] (children), reused for the
-    // partial sums P[8][CPB][Kx].
-    template <int CPB>
-    __global__ void __launch_bounds__(768, 1)
-      m2m_level_smem_kernel(int R, int K, int ncols, const int32_t *__restrict__ par,
-                            const int32_t *__restrict__ child8, const float *__restrict__ lvops,
-                            float *__restrict__ M, int *__restrict__ err)
-    {
-      pdl_entry();
-      extern __shared__ __align__(16) float lv_sm[];
-      __shared__ uint64_t ops_bar;
-      const int Kx = lv_kx(K), KK = lv_kk(K);
-      float    *Ts = lv_sm;
-      float    *X  = lv_sm + 8 * KK;
-      const int KT = blockDim.x / 8, nw = blockDim.x >> 5;
-      const int g = threadIdx.x / KT, ko = threadIdx.x - g * KT; // KT >= K: one coefficient
-      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-      lv_start_ops(Ts, lvops, 8, K, &ops_bar);
-      const float *T     = Ts + g * KK;
-      bool         ops_ok = true, waited = false;
-      for (int c0 = blockIdx.x * CPB; c0 < ncols; c0 += gridDim.x * CPB)
+      if (threadIdx.x < NB && c0 + int(threadIdx.x) < (oct.p[o + 1] - oct.p[o]) * R)
         {
-          const int nc = min(CPB, ncols - c0);
-          for (int row = warp; row < 8 * CPB; row += nw)
-            {
-              const int o = row / CPB, c = row - o * CPB;
-              int64_t   src = -1;
-              if (c < nc)
-                {
-                  const int col = c0 + c, pi = col / R, r = col - pi * R;
-                  const int ch  = child8[8 * pi + o];
-                  if (ch >= 0)
-                    src = (int64_t(ch) * R + r) * K;
-                }
-              for (int k = lane; k < Kx; k += 32)
-                X[row * Kx + k] = (src >= 0 && k < K) ? M[src + k] : 0.0f;
-            }
-          bool has = false; // some column of the batch has an octant-g child
-          for (int c = 0; c < nc; ++c)
-            has = has || child8[8 * ((c0 + c) / R) + g] >= 0;
-          __syncthreads();
-          if (!waited)
-            {
-              ops_ok = lv_wait_ops(&ops_bar, err);
-              waited = true;
-            }
-          float acc[CPB];
-#pragma unroll
-          for (int c = 0; c < CPB; ++c)
-            acc[c] = 0.0f;
-          if (has && ops_ok && ko < K)
-            {
-              const float *x = X + g * CPB * Kx;
-              int          k = 0;
-              for (; k + 4 <= K; k += 4)
-                {
-                  float tv[4];
-#pragma unroll
-                  for (int u = 0; u < 4; ++u)
-                    tv[u] = T[(k + u) * K + ko];
-#pragma unroll
-                  for (int c = 0; c < CPB; ++c)
-                    {
-                      const float4 xv = *reinterpret_cast<const float4 *>(x + c * Kx + k);
-                      acc[c]          = fmaf(tv[0], xv.x, acc[c]);
-                      acc[c]          = fmaf(tv[1], xv.y, acc[c]);
-                      acc[c]          = fmaf(tv[2], xv.z, acc[c]);
-                      acc[c]          = fmaf(tv[3], xv.w, acc[c]);
-                    }
-                }
-              for (; k < K; ++k)
-                {
-                  const float tv = T[k * K + ko];
-#pragma unroll
-                  for (int c = 0; c < CPB; ++c)
-                    acc[c] = fmaf(tv, x[c * Kx + k], acc[c]);
-                }
-            }
-          __syncthreads(); // X no longer read: it becomes P
-          if (ko < K)
-#pragma unroll
-            for (int c = 0; c < CPB; ++c)
-              X[(g * CPB + c) * Kx + ko] = acc[c];
-          __syncthreads();
-          if (g == 0 && ko < K)
-            for (int c = 0; c < nc; ++c)
-                {
-                  const int col = c0 + c, pi = col / R, r = col - pi * R;
-                  auto      at  = [&](int o) { return X[(o * CPB + c) * Kx + ko]; };
-                  const float v = ((at(0) + at(1)) + (at(2) + at(3))) + ((at(4) + at(5)) + (at(6) + at(7)));
-                  M[(int64_t(par[pi]) * R + r) * K + ko] = v;
-                }
-          __syncthreads();
+          prefetch_l1(par + oct.p[o] + (c0 + threadIdx.x) / R);
+          prefetch_l1(box + oct.p[o] + (c0 + threadIdx.x) / R);
         }
-      if (!waited) // never leave with the copy in flight
-        lv_wait_ops(&ops_bar, err);
-    }
-
-    // L2L of one level with its operators in shared memory, after the M2L
-    // sums: L[b] += T_oct L[parent] for the boxes with an L2L parent.  Persistent
-    // blocks take contiguous column ranges (the boxes are listed by octant, so
-    // a range needs the operators of a few octants, copied once); batches of
-    // 16 columns, 8 groups, group g computes columns g and g + 8 of a batch,
-    // one thread per output coefficient, k ascending.  Shared memory:
-    // T[8][lv_kk] (the octants [o_lo, o_hi] of the range), X[16][Kx].
-    __global__ void __launch_bounds__(768, 1)
-      l2l_level_smem_kernel(int R, int K, int ncols, const int32_t *__restrict__ box,
-                            const int32_t *__restrict__ par, const uint8_t *__restrict__ oct,
-                            const float *__restrict__ lvops, float *__restrict__ Lx,
-                            int *__restrict__ err)
-    {
       pdl_entry();
-      extern __shared__ __align__(16) float lv_sm[];
-      __shared__ uint64_t ops_bar;
-      const int Kx = lv_kx(K), KK = lv_kk(K);
-      const int lo = int(int64_t(ncols) * blockIdx.x / gridDim.x);
-      const int hi = int(int64_t(ncols) * (blockIdx.x + 1) / gridDim.x);
-      if (lo >= hi)
-        return;
-      float    *Ts = lv_sm;
-      float    *X  = lv_sm + 8 * KK;
-      const int KT = blockDim.x / 8, nw = blockDim.x >> 5;
-      const int g = threadIdx.x / KT, t = threadIdx.x - g * KT;
-      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-      const int o_lo = oct[lo / R], o_hi = oct[(hi - 1) / R];
-      lv_start_ops(Ts, lvops + size_t(o_lo) * KK, o_hi - o_lo + 1, K, &ops_bar);
-      bool ops_ok = true, waited = false;
-      for (int c0 = lo; c0 < hi; c0 += 16)
+      bool ops_ok = true;
+      for (; b_lo < b_hi; ++b_lo)
         {
-          const int nc = min(16, hi - c0);
-          for (int c = warp; c < nc; c += nw)
+          const int32_t *pb = par + oct.p[o], *bb = box + oct.p[o];
+          const int      n = (oct.p[o + 1] - oct.p[o]) * R, nc = min(NB, n - c0);
+          if (o != held)
             {
-              const int col = c0 + c, bi = col / R, r = col - bi * R;
-              const int pb  = par[bi];
-              for (int k = lane; k < Kx; k += 32)
-                X[c * Kx + k] = (pb >= 0 && k < K) ? Lx[(int64_t(pb) * R + r) * K + k] : 0.0f;
-            }
-          __syncthreads();
-          if (!waited)
-            {
-              ops_ok = lv_wait_ops(&ops_bar, err);
-              waited = true;
-            }
-          for (int c = g; c < nc; c += 8)
-            {
-              const int col = c0 + c, bi = col / R, r = col - bi * R;
-              if (par[bi] < 0 || !ops_ok)
-                continue;
-              const float *T = Ts + (oct[bi] - o_lo) * KK;
-              const float *x = X + c * Kx;
-              for (int ko = t; ko < K; ko += KT)
+              if (threadIdx.x == 0 && ops_ok)
                 {
-                  float a = 0.0f;
-                  int   k = 0;
-                  for (; k + 4 <= K; k += 4)
-                    {
-                      const float4 xv = *reinterpret_cast<const float4 *>(x + k);
-                      a               = fmaf(T[k * K + ko], xv.x, a);
-                      a               = fmaf(T[(k + 1) * K + ko], xv.y, a);
-                      a               = fmaf(T[(k + 2) * K + ko], xv.z, a);
-                      a               = fmaf(T[(k + 3) * K + ko], xv.w, a);
-                    }
-                  for (; k < K; ++k)
-                    a = fmaf(T[k * K + ko], x[k], a);
-                  float *o = Lx + (int64_t(box[bi]) * R + r) * K + ko;
-                  *o       = *o + a;
+                  // the reads of T by the last batch ended before the barrier below
+                  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                  lv_start_op(T, lvops + size_t(o) * lv_kk(K), K, bar);
+                }
+              held = o;
+              ++loads;
+            }
+          // thread (g, ko) brings coefficient ko of the parents' expansions and of the
+          // boxes' M2L sums (needed last) of the columns it computes
+          float *l[C], sum[C], v[C];
+#pragma unroll
+          for (int i = 0; i < C; ++i)
+            {
+              const int c = g + LV_G * i, col = c0 + c, bi = col / R, r = col - bi * R;
+              l[i]        = nullptr;
+              sum[i] = v[i] = 0.0f;
+              if (c < nc && ko < K)
+                {
+                  v[i]   = Lx[(int64_t(pb[bi]) * R + r) * K + ko];
+                  l[i]   = Lx + (int64_t(bb[bi]) * R + r) * K + ko;
+                  sum[i] = *l[i];
                 }
             }
+          if (ko < Kx)
+#pragma unroll
+            for (int i = 0; i < C; ++i)
+              X[(g + LV_G * i) * Kx + ko] = v[i];
           __syncthreads();
+          if (waited < loads)
+            {
+              if (ops_ok)
+                ops_ok = lv_wait_op(bar, uint32_t(loads - 1) & 1u, err);
+              ops_ok = __syncthreads_and(ops_ok);
+              waited = loads;
+            }
+          if (ko < K && ops_ok)
+            {
+              float acc[C];
+              lv_dot<C>(acc, T, X + g * Kx, K, Kx, ko);
+#pragma unroll
+              for (int i = 0; i < C; ++i)
+                if (l[i])
+                  *l[i] = sum[i] + acc[i];
+            }
+          __syncthreads(); // X and T no longer read
+          c0 += NB;
+          while (o < 7 && c0 >= (oct.p[o + 1] - oct.p[o]) * R) // on to the next octant with boxes
+            {
+              ++o;
+              c0 = 0;
+            }
         }
-      if (!waited)
-        lv_wait_ops(&ops_bar, err);
     }
 
     int lv_kt(int K) { return std::min(128, (K + 31) / 32 * 32); }
 
-    // Columns per block: the most (up to cap) that still give every SM a
-    // block; shared memory = floats_per_col * CPB * Kx floats.
-    int lv_cpb(int K, int64_t ncols, int floats_per_col, int cap)
+    int lv_n_sm()
     {
       int dev = 0, n_sm = 1;
       PIBEM_CUDA(cudaGetDevice(&dev));
       PIBEM_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-      int cpb = cap;
-      while (cpb > 1 && (ncols < int64_t(cpb) * n_sm ||
-                         size_t(floats_per_col) * cpb * lv_kx(K) * sizeof(float) > 48 * 1024))
-        cpb /= 2;
-      return cpb;
+      return n_sm;
+    }
+
+    // Columns per thread (1, 2, 4 or 8): the fewest with which `blocks` blocks
+    // (clusters) take the level in one batch each, so that a small level spreads
+    // over the chip and a large one reads its operators fewest times.
+    int lv_cols(int64_t ncols, int64_t blocks)
+    {
+      int c = 1;
+      while (c < 8 && int64_t(LV_G) * c * blocks < ncols)
+        c *= 2;
+      return c;
     }
   } // namespace
-
-  // the operator pass in shared memory: 8 operators + the larger of the
-  // M2M X (8 x 4 columns) and the L2L X (16 columns)
-  static size_t lv_smem_bytes(int K)
-  {
-    return (size_t(8) * lv_kk(K) + size_t(32) * lv_kx(K)) * sizeof(float);
-  }
-  static bool lv_smem_ok(int K) { return K <= 96 && lv_smem_bytes(K) <= 227 * 1024; }
-
-  static int lv_n_sm()
-  {
-    int dev = 0, n_sm = 1;
-    PIBEM_CUDA(cudaGetDevice(&dev));
-    PIBEM_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-    return n_sm;
-  }
 
   bool fused_levels_ok(int K, int R)
   {
@@ -514,36 +444,20 @@ namespace pibem
       return;
     const int K     = op.K;
     const int ncols = (b - a) * R;
-    if (op.lv_ops && op.dev_err && lv_smem_ok(K))
-      {
-        const int    cpb  = ncols >= 4 * lv_n_sm() ? 4 : (ncols >= 2 * lv_n_sm() ? 2 : 1);
-        const size_t smem = (size_t(8) * lv_kk(K) + size_t(8) * cpb * lv_kx(K)) * sizeof(float);
-        const dim3   grid(unsigned(std::min<int64_t>(lv_n_sm(), (ncols + cpb - 1) / cpb)));
-        auto launch = [&](auto kern) {
-          raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
-          launch_pdl(kern, grid, 8 * lv_kt(K), smem, s, R, K, ncols, op.up_box + a,
-                     op.up_child8 + size_t(8) * a, op.lv_ops, M, op.dev_err);
-        };
-        switch (cpb)
-          {
-            case 4: launch(m2m_level_smem_kernel<4>); break;
-            case 2: launch(m2m_level_smem_kernel<2>); break;
-            default: launch(m2m_level_smem_kernel<1>); break;
-          }
-        PIBEM_CUDA(cudaGetLastError());
-        note_launch();
-        return;
-      }
-    const int    cpb   = lv_cpb(K, ncols, 16, 4);
-    const size_t smem  = size_t(16) * cpb * lv_kx(K) * sizeof(float);
-    const float *ops   = op.ops + size_t(op.lv_op0) * K * K;
-    const dim3   grid(unsigned((ncols + cpb - 1) / cpb));
+    // two blocks per SM, in clusters of eight
+    const int    max_cl = std::max(1, 2 * lv_n_sm() / 8);
+    const int    C      = lv_cols(ncols, max_cl);
+    const int    ncl    = std::min(max_cl, (ncols + LV_G * C - 1) / (LV_G * C));
+    const size_t smem   = (size_t(lv_kk(K)) + size_t(3) * LV_G * C * lv_kx(K)) * sizeof(float);
     auto launch = [&](auto kern) {
-      kern<<<grid, 8 * lv_kt(K), smem, s>>>(R, K, ncols, op.up_box + a,
-                                            op.up_child8 + size_t(8) * a, ops, M);
+      if (smem > 48 * 1024)
+        raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
+      launch_pdl_cluster(kern, unsigned(8 * ncl), LV_G * lv_kt(K), 8, smem, s, R, K, ncols,
+                         op.up_box + a, op.up_child8 + size_t(8) * a, op.lv_ops, M, op.dev_err);
     };
-    switch (cpb)
+    switch (C)
       {
+        case 8: launch(m2m_level_kernel<8>); break;
         case 4: launch(m2m_level_kernel<4>); break;
         case 2: launch(m2m_level_kernel<2>); break;
         default: launch(m2m_level_kernel<1>); break;
@@ -569,31 +483,26 @@ namespace pibem
   void launch_l2l_level_fused(const OperatorDev<float> &op, int R, int level, float *Lx,
                               cudaStream_t s)
   {
-    const int a = op.down_box_ptr[level], b = op.down_box_ptr[level + 1];
-    if (b <= a || op.down_l2l_level.empty() || !op.down_l2l_level[level])
+    if (level >= int(op.down_oct_ptr.size()))
+      return;
+    const LevelOctants &oct   = op.down_oct_ptr[level];
+    const int           ncols = (oct.p[8] - oct.p[0]) * R;
+    if (ncols <= 0)
       return;
     const int K     = op.K;
-    const int ncols = (b - a) * R;
-    if (op.lv_ops && op.dev_err && lv_smem_ok(K))
-      {
-        const size_t smem = lv_smem_bytes(K);
-        raise_smem_limit(reinterpret_cast<const void *>(l2l_level_smem_kernel), smem);
-        launch_pdl(l2l_level_smem_kernel, unsigned(std::min(lv_n_sm(), ncols)), 8 * lv_kt(K), smem, s,
-          R, K, ncols, op.down_box + a, op.down_par + a, op.down_oct + a,
-          op.lv_ops + size_t(8) * lv_kk(K), Lx, op.dev_err);
-        PIBEM_CUDA(cudaGetLastError());
-        note_launch();
-        return;
-      }
-    const int    cpb   = lv_cpb(K, ncols, 5, 8);
-    const size_t smem  = size_t(5) * cpb * lv_kx(K) * sizeof(float);
-    const float *ops   = op.ops + size_t(op.lv_op0 + 8) * K * K;
-    const dim3   grid(unsigned((ncols + cpb - 1) / cpb));
+    const int max_b = 2 * lv_n_sm();
+    const int C     = lv_cols(ncols, max_b);
+    int       nb    = 0;
+    for (int o = 0; o < 8; ++o)
+      nb += ((oct.p[o + 1] - oct.p[o]) * R + LV_G * C - 1) / (LV_G * C);
+    const size_t smem = (size_t(lv_kk(K)) + size_t(LV_G) * C * lv_kx(K)) * sizeof(float);
     auto launch = [&](auto kern) {
-      kern<<<grid, 4 * lv_kt(K), smem, s>>>(R, K, ncols, op.down_box + a, op.down_par + a,
-                                            op.down_oct + a, ops, Lx);
+      if (smem > 48 * 1024)
+        raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
+      launch_pdl(kern, unsigned(std::min(nb, max_b)), LV_G * lv_kt(K), smem, s, R, K, oct, nb,
+                 op.down_box, op.down_par, op.lv_ops + size_t(8) * lv_kk(K), Lx, op.dev_err);
     };
-    switch (cpb)
+    switch (C)
       {
         case 8: launch(l2l_level_kernel<8>); break;
         case 4: launch(l2l_level_kernel<4>); break;

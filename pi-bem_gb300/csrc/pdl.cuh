@@ -48,6 +48,28 @@ namespace pibem
     PdlScope &operator=(const PdlScope &) = delete;
   };
 
+  // As launch_pdl, in thread-block clusters of `cluster` blocks.
+  template <typename... P, typename... A>
+  inline void launch_pdl_cluster(void (*kern)(P...), dim3 grid, dim3 block, unsigned cluster,
+                                 size_t smem, cudaStream_t s, A &&...args)
+  {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim            = grid;
+    cfg.blockDim           = block;
+    cfg.dynamicSmemBytes   = smem;
+    cfg.stream             = s;
+    cudaLaunchAttribute at[2];
+    at[0].id               = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs                                        = at;
+    cfg.numAttrs                                     = (pdl_on() && t_pdl_allowed) ? 2 : 1;
+    PIBEM_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
+  }
+
   template <typename... P, typename... A>
   inline void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                          A &&...args)
