@@ -188,7 +188,7 @@ namespace pibem
     bool                 mixed = false, prec = false;
     std::vector<ColHost> col;
     DBuf<double>         V, z, w, u, b, x, r, d, tmp, cz, cw, hb, partial, H, cs, sn, g, y, bn, tol, nrm;
-    DBuf<int>            ticket, kdone, jvec, its, maxit, sel, act, ctl;
+    DBuf<int>            jcur, kdone, jvec, its, maxit, sel, act, ctl;
     PinnedBuf<int>       ipin;
     std::vector<double>  h_bn, h_tol;
     std::vector<int>     h_its, h_maxit, h_jvec, h_ctl;
@@ -347,7 +347,7 @@ struct pibem_handle
     add(sv_b, sv_x, sv_r, sv_d, sv_w, sv_part, sv_nrm, sh_part, sh_nrm);
     add(eng.V, eng.z, eng.w, eng.u, eng.b, eng.x, eng.r, eng.d, eng.tmp, eng.cz, eng.cw, eng.hb,
         eng.partial, eng.H, eng.cs, eng.sn, eng.g, eng.y, eng.bn, eng.tol, eng.nrm);
-    add(eng.ticket, eng.kdone, eng.jvec, eng.its, eng.maxit, eng.sel, eng.act, eng.ctl);
+    add(eng.jcur, eng.kdone, eng.jvec, eng.its, eng.maxit, eng.sel, eng.act, eng.ctl);
     for (const auto &b : io_buf)
       t += b.bytes();
     return t;
@@ -879,7 +879,7 @@ namespace
   // application is shared by the columns that need it at that moment (they are
   // gathered into one contiguous batch), and the Arnoldi steps of every column
   // inside a GMRES cycle run on the device -- CGS2 in FP64, the Hessenberg
-  // column's Givens rotation and the stopping test (gmres_givens_kernel) -- as
+  // column's Givens rotation and the stopping test (arnoldi_finish_kernel) -- as
   // one CUDA graph, a conditional while node around one step, until some column
   // ends its cycle (it met its tolerance, took m steps or reached its iteration
   // limit).  While phase timing is on, or the caller's stream is itself being
@@ -896,34 +896,38 @@ namespace
                                  size_t(n) * sizeof(double), size_t(R), cudaMemcpyDeviceToDevice, s));
   }
 
+  template <typename P>
+  BlockPrec<P> block_prec(pibem_handle *h, const P *Pinv)
+  {
+    BlockPrec<P> bp;
+    bp.n_leaves = int(h->blk_ptr.size()) - 1;
+    bp.max_rows = std::max(h->max_leaf_rows, 1);
+    bp.row_ptr  = h->d_nrow_ptr.p;
+    bp.blk_ptr  = h->d_blk_ptr.p;
+    bp.rows     = h->d_nrows.p;
+    bp.Pinv     = Pinv;
+    return bp;
+  }
+
   // z = P^-1 v for R columns (v column stride ldv).  Leaf-block Jacobi: the
   // FP64 inverses where the handle keeps them (GMRES on an FP64-accurate
   // operator), else the FP32 ones.  ILU(0): z = v, then the level-scheduled
-  // forward and backward substitutions in place (FP64).  With nrm2, v / |v|
-  // is also written to vout (column stride ldo, at column jvec[r] + 1).
+  // forward and backward substitutions in place (FP64).
   void apply_prec(pibem_handle *h, int R, const double *v, int64_t ldv, double *z, cudaStream_t s,
-                  const double *nrm2 = nullptr, double *vout = nullptr, int64_t ldo = 0,
-                  const int *jvec = nullptr, const int *sel = nullptr)
+                  const int *sel = nullptr)
   {
     const int64_t N = h->N();
     if (h->ilu_on)
       {
-        if (nrm2)
-          launch_normalize(N, R, v, nrm2, vout, ldo, s, jvec, z, sel);
-        else
-          launch_copy_sel(N, R, v, ldv, z, sel, s);
+        launch_copy_sel(N, R, v, ldv, z, sel, s);
         launch_ilu_apply(h->ilu_lptr_lo, h->d_ilu_rows_lo.p, h->ilu_lptr_up, h->d_ilu_rows_up.p, R, N,
                          h->d_ilu_ptr.p, h->d_ilu_col.p, h->d_ilu_val.p, h->d_ilu_diag.p, z, sel,
-                         jvec, s);
-        return;
+                         nullptr, s);
       }
-    const int nl = int(h->blk_ptr.size()) - 1;
-    if (h->d_Pinv64.p)
-      launch_block_apply(nl, h->max_leaf_rows, R, N, h->d_nrow_ptr.p, h->d_blk_ptr.p, h->d_nrows.p,
-                         h->d_Pinv64.p, v, ldv, z, s, nrm2, vout, ldo, jvec, sel);
+    else if (h->d_Pinv64.p)
+      launch_block_apply(block_prec(h, h->d_Pinv64.p), R, N, v, ldv, z, sel, s);
     else
-      launch_block_apply(nl, h->max_leaf_rows, R, N, h->d_nrow_ptr.p, h->d_blk_ptr.p, h->d_nrows.p,
-                         h->d_Pinv.p, v, ldv, z, s, nrm2, vout, ldo, jvec, sel);
+      launch_block_apply(block_prec(h, h->d_Pinv.p), R, N, v, ldv, z, sel, s);
   }
 
   // n values from the device into out, through the handle's page-locked buffer
@@ -936,7 +940,7 @@ namespace
     std::copy(h->g_small.p, h->g_small.p + n, out);
   }
 
-  constexpr int ENG_NBLK = 2 * 152; // partial-sum blocks of the GMRES norms and Gram-Schmidt passes
+  constexpr int ENG_NBLK = 2 * 152; // partial-sum blocks of the GMRES norms
   constexpr int ENG_NBLK_REFINE = 64; // of the refinement residual norms
 
   // (re)size the engine for S columns and Krylov dimension m; keeps nothing
@@ -962,8 +966,8 @@ namespace
     for (DBuf<double> *v : {&E.z, &E.w, &E.cz, &E.cw})
       v->alloc(size_t(2 * S) * N);
     PIBEM_CUDA(cudaMemsetAsync(E.z.p + size_t(S) * N, 0, sizeof(double) * size_t(S) * N, h->stream));
-    E.hb.alloc(size_t(S) * (2 * L + 1));
-    E.partial.alloc(size_t(S) * ENG_NBLK * L);
+    E.hb.alloc(size_t(S) * 2 * L);
+    E.partial.alloc(size_t(S) * std::max(ENG_NBLK, (2 * L + 1) * arnoldi_blocks(N)));
     E.H.alloc(size_t(S) * L * m);
     E.cs.alloc(size_t(S) * m);
     E.sn.alloc(size_t(S) * m);
@@ -972,9 +976,7 @@ namespace
     E.bn.alloc(S);
     E.tol.alloc(S);
     E.nrm.alloc(S);
-    E.ticket.alloc(S);
-    E.ticket.zero(h->stream);
-    for (DBuf<int> *v : {&E.kdone, &E.jvec, &E.its, &E.maxit, &E.sel})
+    for (DBuf<int> *v : {&E.jcur, &E.kdone, &E.jvec, &E.its, &E.maxit, &E.sel})
       v->alloc(S);
     E.act.alloc(2 * S);
     std::vector<int> minus(S, -1);
@@ -1080,48 +1082,88 @@ namespace
     return b;
   }
 
-  // One Arnoldi step of every column in a cycle (E.act holds them, R' of them):
-  // w = A z (through the contiguous batch), CGS2 into hb, V_{j+1} = w / |w| and
-  // the next z, then the Givens step.
+  // the step runs straight on the FP32 operator's buffers d_x32 -> d_y32 (mixed
+  // path without constraint lines or the pure-Neumann shift), else on cz -> cw
+  bool eng_direct32(const pibem_handle *h)
+  {
+    return h->eng.mixed && h->have_dirichlet && h->con_row.empty();
+  }
+
+  // the first step's operator input from the slots' z
+  void eng_gather(pibem_handle *h, int Ra)
+  {
+    Engine       &E = h->eng;
+    const int64_t N = h->N();
+    if (eng_direct32(h))
+      launch_gather_d2f(N, Ra, E.act.p, E.z.p, h->d_x32.p, h->stream);
+    else
+      launch_gather_cols(N, Ra, E.act.p, E.z.p, N, E.cz.p, h->stream);
+  }
+
+  // the next step's operator input back into the slots' z, for columns whose cycle
+  // goes on at a later call (the batch may be another one by then)
+  void eng_scatter(pibem_handle *h, int Ra)
+  {
+    Engine       &E = h->eng;
+    const int64_t N = h->N();
+    if (h->ilu_on) // z is in the slots already
+      return;
+    if (eng_direct32(h))
+      launch_f2d_scatter(N, Ra, E.act.p, h->d_x32.p, E.z.p, h->stream);
+    else
+      launch_scatter_cols(N, Ra, E.act.p, E.cz.p, E.z.p, N, h->stream);
+  }
+
+  // One Arnoldi step of every column in a cycle (E.act holds them, padded to Ra):
+  // the operator on the batch, CGS2, V_{j+1} = w / |w|, the next step's operator
+  // input P^-1 V_{j+1} into the batch, and the Givens step.
   void eng_step(pibem_handle *h, int Ra, const std::function<void(const double *, double *, int)> &A,
                 cudaGraphConditionalHandle cond, bool use_cond)
   {
-    Engine       &E   = h->eng;
-    const int64_t N   = h->N();
-    cudaStream_t  s   = h->stream;
-    const int     L   = E.m + 1;
-    const int64_t ldr = int64_t(L) * N;
-    double *h1 = E.hb.p, *h2 = h1 + size_t(E.S) * L, *nr = h2 + size_t(E.S) * L;
-    if (E.mixed && h->have_dirichlet && h->con_row.empty())
+    Engine       &E = h->eng;
+    const int64_t N = h->N();
+    cudaStream_t  s = h->stream;
+    ArnoldiArgs   a;
+    a.n       = N;
+    a.S       = E.S;
+    a.m       = E.m;
+    a.Ra      = Ra;
+    a.act     = E.act.p;
+    a.V       = E.V.p;
+    a.w       = E.w.p;
+    a.partial = E.partial.p;
+    a.jcur    = E.jcur.p;
+    a.g.m = E.m, a.g.hb = E.hb.p, a.g.H = E.H.p, a.g.cs = E.cs.p, a.g.sn = E.sn.p, a.g.g = E.g.p;
+    a.g.kdone = E.kdone.p, a.g.jvec = E.jvec.p, a.g.its = E.its.p, a.g.maxit = E.maxit.p;
+    a.g.bn = E.bn.p, a.g.tol = E.tol.p, a.g.ctl = E.ctl.p;
+    a.g.cond = cond, a.g.use_cond = use_cond ? 1 : 0;
+    const bool direct = eng_direct32(h);
+    if (direct)
       {
-        // the FP32 operator straight on the gathered columns: gather + FP32
-        // conversion and FP64 conversion + scatter fused (as system_apply32)
-        h->d_x32.alloc(size_t(Ra) * N);
-        h->d_y32.alloc(size_t(Ra) * N);
-        launch_gather_d2f(N, Ra, E.act.p, E.z.p, h->d_x32.p, s);
         operator32(h, Ra);
         finish_timing(h, 1);
-        launch_f2d_scatter(N, Ra, E.act.p, h->d_y32.p, E.w.p, s);
         h->cnt32 += Ra;
+        launch_arnoldi_cgs(a, h->d_y32.p, s);
       }
     else
       {
-        launch_gather_cols(N, Ra, E.act.p, E.z.p, N, E.cz.p, s);
         A(E.cz.p, E.cw.p, Ra);
-        launch_scatter_cols(N, Ra, E.act.p, E.cw.p, E.w.p, N, s);
+        launch_arnoldi_cgs(a, E.cw.p, s);
       }
-    launch_cgs_step(0, N, E.S, 0, N, ldr, E.V.p, nullptr, 0, E.w.p, ENG_NBLK, E.partial.p,
-                    E.ticket.p, h1, s, E.jvec.p, L);
-    launch_cgs_step(1, N, E.S, 0, N, ldr, E.V.p, h1, L, E.w.p, ENG_NBLK, E.partial.p, E.ticket.p, h2,
-                    s, E.jvec.p, L);
-    launch_cgs_step(2, N, E.S, 0, N, ldr, E.V.p, h2, L, E.w.p, ENG_NBLK, E.partial.p, E.ticket.p, nr,
-                    s, E.jvec.p, 1);
-    if (E.prec) // V_{j+1} = w / |w| and the next step's z = P^-1 V_{j+1} in one pass
-      apply_prec(h, E.S, E.w.p, N, E.z.p, s, nr, E.V.p, ldr, E.jvec.p);
+    if (h->ilu_on)
+      {
+        launch_arnoldi_finish(a, BlockPrec<double>(), E.z.p, true, s);
+        launch_ilu_apply(h->ilu_lptr_lo, h->d_ilu_rows_lo.p, h->ilu_lptr_up, h->d_ilu_rows_up.p, E.S, N,
+                         h->d_ilu_ptr.p, h->d_ilu_col.p, h->d_ilu_val.p, h->d_ilu_diag.p, E.z.p,
+                         nullptr, E.jcur.p, s);
+        eng_gather(h, Ra);
+      }
+    else if (direct)
+      launch_arnoldi_finish(a, block_prec(h, E.prec ? h->d_Pinv.p : nullptr), h->d_x32.p, false, s);
+    else if (h->d_Pinv64.p)
+      launch_arnoldi_finish(a, block_prec(h, E.prec ? h->d_Pinv64.p : nullptr), E.cz.p, false, s);
     else
-      launch_normalize(N, E.S, E.w.p, nr, E.V.p, ldr, s, E.jvec.p, E.z.p);
-    launch_gmres_givens(E.S, E.m, h1, E.H.p, E.cs.p, E.sn.p, E.g.p, E.kdone.p, E.jvec.p, E.its.p,
-                        E.maxit.p, E.bn.p, E.tol.p, E.ctl.p, cond, use_cond, s);
+      launch_arnoldi_finish(a, block_prec(h, E.prec ? h->d_Pinv.p : nullptr), E.cz.p, false, s);
   }
 
   // Runs the Arnoldi steps of the columns in a cycle until one of them ends its
@@ -1150,6 +1192,12 @@ namespace
     // join, and finished columns leave, at the next call)
     E.h_ctl = {0, 0, quantum > 0 ? quantum : std::numeric_limits<int>::max(), 0};
     E.ctl.upload(E.h_ctl, s);
+    PIBEM_CUDA(cudaMemsetAsync(E.jcur.p, 0xff, sizeof(int) * E.S, s)); // -1: not in a cycle
+    if (eng_direct32(h))
+      {
+        h->d_x32.alloc(size_t(Ra) * h->N());
+        h->d_y32.alloc(size_t(Ra) * h->N());
+      }
     bool graph = !h->timing;
     if (graph)
       {
@@ -1160,6 +1208,7 @@ namespace
     if (!graph)
       {
         int steps = 0;
+        eng_gather(h, Ra);
         while (true)
           {
             eng_step(h, Ra, A, 0, false);
@@ -1169,6 +1218,8 @@ namespace
             if (!E.ipin.p[0])
               break;
           }
+        if (quantum > 0)
+          eng_scatter(h, Ra);
         return steps;
       }
     // the operator reads d_modes: COMBINED for the Ra columns (other calls
@@ -1177,7 +1228,7 @@ namespace
       set_modes(h, Ra, MODE_COMBINED);
     // every buffer a step touches (a reallocation changes an address)
     auto bufs_now = [&](int i) -> const void * {
-      const void *b[] = {E.V.p,    E.z.p,     E.w.p,      E.hb.p,    E.partial.p, E.ticket.p,
+      const void *b[] = {E.V.p,    E.z.p,     E.w.p,      E.hb.p,    E.partial.p, E.jcur.p,
                          E.H.p,    E.cs.p,    E.sn.p,     E.g.p,     E.kdone.p,   E.jvec.p,
                          E.its.p,  E.maxit.p, E.bn.p,     E.tol.p,   E.ctl.p,     E.act.p,
                          E.cz.p,   E.cw.p,    h->d_x32.p, h->d_y32.p, h->d_M32.p, h->d_L32.p,
@@ -1277,7 +1328,10 @@ namespace
         h->cycle_graphs.push_back(c);
         cg = &h->cycle_graphs.back();
       }
+    eng_gather(h, Ra);
     PIBEM_CUDA(cudaGraphLaunch(cg->exec, s));
+    if (quantum > 0)
+      eng_scatter(h, Ra);
     PIBEM_CUDA(cudaMemcpyAsync(E.ipin.p, E.ctl.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     PIBEM_CUDA(cudaStreamSynchronize(s));
     const int steps = E.ipin.p[1];
@@ -1360,7 +1414,7 @@ namespace
             double *tgt = E.mixed ? E.d.p : E.x.p;
             if (E.prec)
               {
-                apply_prec(h, E.S, E.u.p, N, E.z.p, s, nullptr, nullptr, 0, nullptr, E.sel.p);
+                apply_prec(h, E.S, E.u.p, N, E.z.p, s, E.sel.p);
                 launch_axpby_sel(N, E.S, E.sel.p, 1.0, E.z.p, 1.0, tgt, s);
               }
             else
@@ -1491,10 +1545,10 @@ namespace
               {
                 upload_sel(h, cyc);
                 // V[c][0] = w / |w| (and z = V_0 without preconditioner)
-                launch_normalize(N, E.S, E.w.p, E.nrm.p, E.V.p, ldr, s, nullptr,
-                                 E.prec ? nullptr : E.z.p, E.sel.p);
+                launch_normalize(N, E.S, E.w.p, E.nrm.p, E.V.p, ldr, s, E.prec ? nullptr : E.z.p,
+                                 E.sel.p);
                 if (E.prec)
-                  apply_prec(h, E.S, E.V.p, ldr, E.z.p, s, nullptr, nullptr, 0, nullptr, E.sel.p);
+                  apply_prec(h, E.S, E.V.p, ldr, E.z.p, s, E.sel.p);
                 launch_gmres_cycle_init(E.S, E.m, E.sel.p, E.nrm.p, E.g.p, E.kdone.p, E.jvec.p, s);
                 for (int c : cyc)
                   {

@@ -3,6 +3,7 @@
 // system matrix).  Reductions are two-stage with a fixed order, so results do
 // not depend on scheduling.
 #include <algorithm>
+#include <cmath>
 
 #include "krylov.h"
 #include "pdl.cuh"
@@ -11,7 +12,8 @@ namespace pibem
 {
   namespace
   {
-    constexpr int kDotBlock = 256;
+    constexpr int kDotBlock  = 256;
+    constexpr int AR_THREADS = 512; // Arnoldi kernels
 
     // partial[(r * nblk + blk) * ncols + i] = sum over the block's rows of V[r][i][t] w[r][t].
     // Warp k of the block takes columns k, k + 8, ...; its lanes stride over the
@@ -85,121 +87,229 @@ namespace pibem
       w[idx] -= sign * s;
     }
 
-    // One Gram-Schmidt step of the Arnoldi process in one launch per pass, with
-    // the same arithmetic as dots_partial + dots_final and gemv_sub:
-    //   MODE 0: out[r][i]  = V[r][i] . w[r]                      (i < ncols)
-    //   MODE 1: w[r] -= sum_i V[r][i] hin[r][i], then out[r][i] = V[r][i] . w[r]
-    //   MODE 2: w[r] -= sum_i V[r][i] hin[r][i], then out[r][0] = w[r] . w[r]
-    // Block blk of row r owns rows [blk chunk, (blk + 1) chunk) of every vector:
-    // it updates them (threads stride over the rows, the sum over i in order),
-    // then forms its partial dots (warp k takes outputs k, k + 8, ...; lanes
-    // stride over the rows; fixed shuffle tree).  The last block of row r to
-    // finish (a ticket taken after a fence) adds the nblk partials of each
-    // output in the fixed order of dots_final and resets the ticket, so the
-    // result does not depend on which block is last.
-    //   jvec (may be null): per-column Arnoldi step j = jvec[r] read on the
-    //   device (the pass takes ncols = j + 1 basis vectors; j < 0: the column
-    //   is idle and its blocks return); out holds ldo values per column r.
-    template <int MODE>
-    __global__ void __launch_bounds__(256)
-      cgs_step_kernel(int64_t n, int ncols, int64_t ldv, int64_t ldr, const double *__restrict__ V,
-                      const double *__restrict__ hin, int ldh, double *__restrict__ w, int nblk,
-                      double *__restrict__ partial, int *__restrict__ ticket,
-                      double *__restrict__ out, const int *__restrict__ jvec, int ldo)
+    // ---- one Arnoldi step, four launches ---------------------------------------
+    // Classical Gram-Schmidt applied twice (FP64) on the batch's columns, then the
+    // normalisation, the preconditioner and the Givens step:
+    //   arnoldi_dots    w = the operator's result, dots V_i . w
+    //   arnoldi_sub<0>  h1 = the dots' sums; w -= V h1; dots V_i . w
+    //   arnoldi_sub<1>  h2 likewise; w -= V h2; |w|^2
+    //   arnoldi_finish  V_{j+1} = w / |w|, z = P^-1 V_{j+1}, Givens (below)
+    // Column k of the batch is slot act[k] (act[k] >= S: an idle padding column).
+    // A column's rows are cut into G chunks, one block each; a block leaves its
+    // partial sums in global memory and every block of the next launch adds the G
+    // partials itself, in a fixed order: the launch boundary is the only barrier,
+    // so nothing waits on a flag and no block is last.  G depends on n alone, so a
+    // column's arithmetic depends on nothing but the column.
+    //   What bounds it: on large meshes the FP64 units (2 FMA per clock and SM: 4 n j
+    // FMA a step), on small ones the four launches' latency.  G = ceil(sqrt(n) / 2),
+    // up to one block per SM, balances the chunk's 2 n / G FMA per basis vector against
+    // the G additions of the partials (mixed solves at 1.5k / 98k nodes and 16 columns
+    // at 24k: 5.83 / 45.0 / 154.7 ms with sqrt(n), 5.86 / 45.0 / 150.9 with half of
+    // it, 5.88 / 46.0 / 148.2 with 0.35).  Sums run over groups of eight lanes, so
+    // that a warp works on four basis vectors and a sum ends after three shuffles.
+    //   Measured (kernel times of a step, warm caches, GB300) against one launch per
+    // pass with a last-block reduction, the scatter / gather of the columns, the
+    // preconditioner and a one-thread Givens step: 1.5k nodes 45 -> 26 us, 98k
+    // nodes 68 -> 47 us; mixed solves to 1e-12 6.95 -> 5.86 ms and 47.2 -> 45.0 ms.
+
+    // partial dots of the block's rows [t0, t1) with the ncols vectors V_i (n
+    // apart): out[i * G + blk]; warp = (row part, group of four vectors)
+    __device__ __forceinline__ void ar_dots(int64_t n, int ncols, const double *V, const double *w,
+                                            int64_t t0, int64_t t1, double (*red)[64], double *out,
+                                            int G, int blk)
     {
-      pdl_entry();
-      if (jvec)
+      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      const int part = warp & 3, quad = warp >> 2;
+      for (int i0 = 0; i0 < ncols; i0 += 64)
         {
-          const int j = jvec[blockIdx.y];
-          if (j < 0)
-            return;
-          ncols = j + 1;
-        }
-      const int     r     = blockIdx.y;
-      const int     blk   = blockIdx.x;
-      const double *Vr    = V + int64_t(r) * ldr;
-      double       *wr    = w + int64_t(r) * n;
-      const int64_t chunk = (n + nblk - 1) / nblk;
-      const int64_t t0 = int64_t(blk) * chunk, t1 = min(n, t0 + chunk);
-      const int     warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-      if constexpr (MODE > 0)
-        {
-          const double *hr = hin + int64_t(r) * ldh;
-          for (int64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x)
+#pragma unroll 1
+          for (int q = 0; q < 4 && i0 + 16 * q < ncols; ++q)
             {
-              double s = 0;
-#pragma unroll 8
-              for (int i = 0; i < ncols; ++i)
-                s += Vr[int64_t(i) * ldv + t] * hr[i];
-              wr[t] -= s;
+              const int l = 16 * q + 4 * quad + (lane >> 3), i = i0 + l;
+              double    s = 0;
+              if (i < ncols)
+                {
+                  const double *v = V + int64_t(i) * n;
+                  for (int64_t t = t0 + 8 * part + (lane & 7); t < t1; t += 8 * 32)
+                    {
+                      double a[8], b[8];
+#pragma unroll
+                      for (int u = 0; u < 8; ++u)
+                        if (t + 32 * u < t1)
+                          {
+                            a[u] = v[t + 32 * u];
+                            b[u] = w[t + 32 * u];
+                          }
+#pragma unroll
+                      for (int u = 0; u < 8; ++u)
+                        if (t + 32 * u < t1)
+                          s = fma(a[u], b[u], s);
+                    }
+                }
+              __syncwarp();
+              for (int o = 4; o > 0; o >>= 1)
+                s += __shfl_xor_sync(0xffffffffu, s, o);
+              if ((lane & 7) == 0)
+                red[part][l] = s;
             }
-          __syncthreads(); // the block's w rows are updated (visible to the block)
+          __syncthreads();
+          const int i = i0 + threadIdx.x;
+          if (threadIdx.x < 64 && i < ncols)
+            out[int64_t(i) * G + blk] = (red[0][threadIdx.x] + red[1][threadIdx.x]) +
+                                        (red[2][threadIdx.x] + red[3][threadIdx.x]);
+          __syncthreads();
         }
-      const int nout = MODE == 2 ? 1 : ncols;
-      // partial sums of column r: per block pstride values (with jvec the
-      // columns have different output counts, so a fixed stride, ldo, keeps
-      // their regions apart)
-      const int pstride = jvec ? ldo : nout;
-      for (int i = warp; i < nout; i += nw)
-        {
-          const double *v = MODE == 2 ? wr : Vr + int64_t(i) * ldv;
-          double        s = 0;
-#pragma unroll 8
-          for (int64_t t = t0 + lane; t < t1; t += 32)
-            s += v[t] * wr[t];
-          for (int o = 16; o > 0; o >>= 1)
-            s += __shfl_xor_sync(0xffffffffu, s, o);
-          if (lane == 0)
-            partial[(int64_t(r) * nblk + blk) * pstride + i] = s;
-        }
-      __threadfence();
-      __syncthreads();
-      __shared__ int last;
-      if (threadIdx.x == 0)
-        last = atomicAdd(ticket + r, 1) == nblk - 1;
-      __syncthreads();
-      if (!last)
-        return;
-      __threadfence();
-      for (int i = warp; i < nout; i += nw)
-        {
-          double s = 0;
-          for (int b = lane; b < nblk; b += 32)
-            s += __ldcg(partial + (int64_t(r) * nblk + b) * pstride + i);
-          for (int o = 16; o > 0; o >>= 1)
-            s += __shfl_xor_sync(0xffffffffu, s, o);
-          if (lane == 0)
-            out[int64_t(r) * ldo + i] = s;
-        }
-      if (threadIdx.x == 0)
-        ticket[r] = 0;
     }
 
-    // V[r][j+1] = w[r] / hn[r]  (hn > 0), else 0; with jvec the output column
-    // is basis vector jvec[r] + 1 of out (jvec[r] < 0: column skipped); with sel
-    // only the columns with sel[r] != 0; with z the value is also written to z[r]
-    __global__ void normalize_kernel(int64_t n, int R, const double *__restrict__ w,
-                                     const double *__restrict__ nrm, double *__restrict__ out,
-                                     int64_t ldr, const int *__restrict__ jvec,
-                                     double *__restrict__ z, const int *__restrict__ sel)
+    // w = the operator's result on the batch (FP32 or FP64), the first dots, and
+    // jcur = the columns' step for the rest of this step's launches
+    template <typename T>
+    __global__ void __launch_bounds__(AR_THREADS)
+      arnoldi_dots_kernel(int64_t n, int S, int G, int L, int64_t ldr, const int *__restrict__ act,
+                          const T *__restrict__ in, const double *__restrict__ V,
+                          double *__restrict__ w, const int *__restrict__ jvec,
+                          int *__restrict__ jcur, double *__restrict__ partial)
     {
       pdl_entry();
+      __shared__ double red[4][64];
+      const int k = blockIdx.y, r = act[k], blk = blockIdx.x;
+      if (r >= S)
+        return;
+      const int j = jvec[r];
+      if (blk == 0 && threadIdx.x == 0)
+        jcur[r] = j;
+      if (j < 0)
+        return;
+      const int64_t chunk = (n + G - 1) / G;
+      const int64_t t0 = int64_t(blk) * chunk, t1 = min(n, t0 + chunk);
+      double       *wr = w + int64_t(r) * n;
+      for (int64_t t = t0 + threadIdx.x; t < t1; t += AR_THREADS)
+        wr[t] = double(in[int64_t(k) * n + t]);
+      __syncthreads();
+      ar_dots(n, j + 1, V + int64_t(r) * ldr, wr, t0, t1, red, partial + int64_t(k) * L * G, G, blk);
+    }
+
+    // h_i = the sum of the G partials (block 0 keeps it in hout), w -= V h, then
+    // the dots of the next pass (LAST: the partial squared norms).  With chunks of
+    // fewer than AR_THREADS rows four warps share a row's sum over i.
+    template <bool LAST>
+    __global__ void __launch_bounds__(AR_THREADS)
+      arnoldi_sub_kernel(int64_t n, int S, int G, int L, int64_t ldr, const int *__restrict__ act,
+                         const double *__restrict__ V, double *__restrict__ w,
+                         const int *__restrict__ jcur, const double *__restrict__ pin,
+                         double *__restrict__ hout, double *__restrict__ pout)
+    {
+      pdl_entry();
+      extern __shared__ double sh[]; // [L]
+      __shared__ double red[4][AR_THREADS];
+      const int k = blockIdx.y, r = act[k], blk = blockIdx.x;
+      if (r >= S)
+        return;
+      const int j = jcur[r];
+      if (j < 0)
+        return;
+      const int     ncols = j + 1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      const int64_t chunk = (n + G - 1) / G;
+      const int64_t t0 = int64_t(blk) * chunk, t1 = min(n, t0 + chunk);
+      const double *Vr = V + int64_t(r) * ldr;
+      double       *wr = w + int64_t(r) * n;
+      for (int i0 = 0; i0 < ncols; i0 += AR_THREADS / 8)
+        {
+          const int i = i0 + int(threadIdx.x >> 3);
+          double    s = 0;
+          if (i < ncols)
+            {
+              const double *p = pin + (int64_t(k) * L + i) * G;
+#pragma unroll 4
+              for (int b = lane & 7; b < G; b += 8)
+                s += p[b];
+            }
+          __syncwarp();
+          for (int o = 4; o > 0; o >>= 1)
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+          if (i < ncols && (lane & 7) == 0)
+            {
+              sh[i] = s;
+              if (blk == 0)
+                hout[int64_t(r) * L + i] = s;
+            }
+        }
+      __syncthreads();
+      double nrm = 0;
+      // sum over i = i0, i0 + step, ... of V_i[t] h_i, eight loads in flight
+      auto dot_h = [&](int64_t t, int i0, int step) {
+        double s = 0;
+        for (int i = i0; i < ncols; i += 8 * step)
+          {
+            double a[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (i + u * step < ncols)
+                a[u] = Vr[int64_t(i + u * step) * n + t];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (i + u * step < ncols)
+                s = fma(a[u], sh[i + u * step], s);
+          }
+        return s;
+      };
+      if (chunk >= AR_THREADS)
+        for (int64_t t = t0 + threadIdx.x; t < t1; t += AR_THREADS)
+          {
+            const double v = wr[t] - dot_h(t, 0, 1);
+            wr[t]          = v;
+            nrm            = LAST ? fma(v, v, nrm) : 0;
+          }
+      else
+        {
+          const int part = warp & 3, rg = warp >> 2;
+          for (int64_t t = t0 + 32 * rg + lane; t < t1; t += 128)
+            red[part][t - t0] = dot_h(t, part, 4);
+          __syncthreads();
+          const int l = threadIdx.x;
+          if (t0 + l < t1)
+            {
+              const double v = wr[t0 + l] - ((red[0][l] + red[1][l]) + (red[2][l] + red[3][l]));
+              wr[t0 + l]     = v;
+              nrm            = LAST ? v * v : 0;
+            }
+        }
+      __syncthreads(); // w is updated (visible to the block); red is free
+      if constexpr (!LAST)
+        ar_dots(n, ncols, Vr, wr, t0, t1, reinterpret_cast<double(*)[64]>(&red[0][0]),
+                pout + int64_t(k) * L * G, G, blk);
+      else
+        {
+          for (int o = 16; o > 0; o >>= 1)
+            nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+          if (lane == 0)
+            red[0][warp] = nrm;
+          __syncthreads();
+          if (threadIdx.x == 0)
+            {
+              double s = 0;
+              for (int q = 0; q < AR_THREADS / 32; ++q)
+                s += red[0][q];
+              pout[int64_t(k) * G + blk] = s;
+            }
+        }
+    }
+
+    // out[r] = w[r] / sqrt(nrm[r]) (0 for a zero norm) of the columns with sel[r]
+    // (column stride ldr); with z also into z[r]
+    __global__ void normalize_kernel(int64_t n, int R, const double *__restrict__ w,
+                                     const double *__restrict__ nrm, double *__restrict__ out,
+                                     int64_t ldr, double *__restrict__ z, const int *__restrict__ sel)
+    {
       int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
       if (idx >= n * R)
         return;
       int64_t r = idx / n, t = idx % n;
-      if (sel && !sel[r])
+      if (!sel[r])
         return;
-      int64_t off = 0;
-      if (jvec)
-        {
-          if (jvec[r] < 0)
-            return;
-          off = int64_t(jvec[r] + 1) * n;
-        }
       double       h = sqrt(nrm[r]);
       const double v = h > 0 ? w[idx] / h : 0.0;
-      out[r * ldr + off + t] = v;
+      out[r * ldr + t] = v;
       if (z)
         z[idx] = v;
     }
@@ -210,8 +320,8 @@ namespace pibem
     // Arnoldi step; -1: the column takes no part), kdone[r] (-1, or the step
     // count after which the column met its tolerance), its[r] / maxit[r]
     // (iterations so far / limit), bn[r], tol[r] (stopping test |g_{j+1}| /
-    // bn <= tol).  hb: [h1 (R x L) | h2 (R x L) | |w|^2 (R)], L = m + 1, the two
-    // Gram-Schmidt passes' coefficients and the norm of a step.  ctl[0]: 1 while
+    // bn <= tol).  hb: [h1 (R x L) | h2 (R x L)], L = m + 1, the two Gram-Schmidt
+    // passes' coefficients of a step.  ctl[0]: 1 while
     // the steps go on; ctl[1]: steps run; ctl[2]: most steps before the host is
     // back (a quantum); ctl[3]: 1 to stop at the first column that ends its
     // cycle, 0 to go on until every column has ended its cycle.
@@ -229,85 +339,6 @@ namespace pibem
             kdone[r]          = -1;
             jvec[r]           = 0;
           }
-    }
-
-    // Step j = jvec[r] of every active column: the Hessenberg column, its Givens
-    // rotation and the stopping test (|g_{j+1}| / bn <= tol, or a zero
-    // subdiagonal); then jvec and the iteration count advance.  A column ends its
-    // cycle when it meets its tolerance, after m steps or at its iteration
-    // limit (jvec = -2 - steps: no more steps); when the steps stop (see ctl),
-    // ctl[0] = 0 and, in a graph, the loop's condition is cleared.
-    __global__ void gmres_givens_kernel(int R, int m, const double *__restrict__ hb,
-                                        double *__restrict__ H, double *__restrict__ cs,
-                                        double *__restrict__ sn, double *__restrict__ g,
-                                        int *__restrict__ kdone, int *__restrict__ jvec,
-                                        int *__restrict__ its, const int *__restrict__ maxit,
-                                        const double *__restrict__ bn,
-                                        const double *__restrict__ tol, int *__restrict__ ctl,
-                                        cudaGraphConditionalHandle cond, int use_cond)
-    {
-      pdl_entry();
-      const int L = m + 1;
-      __shared__ int ended, active, alive;
-      if (threadIdx.x == 0)
-        ended = active = alive = 0;
-      __syncthreads();
-      for (int r = threadIdx.x; r < R; r += blockDim.x)
-        {
-          const int j = jvec[r];
-          if (j < 0)
-            continue;
-          active = 1;
-          double       *Hc = H + int64_t(r) * L * m;
-          const double *h1 = hb + int64_t(r) * L, *h2 = hb + int64_t(R) * L + int64_t(r) * L;
-          for (int i = 0; i <= j; ++i)
-            Hc[int64_t(i) * m + j] = h1[i] + h2[i];
-          Hc[int64_t(j + 1) * m + j] = sqrt(hb[2 * int64_t(R) * L + r]);
-          double *c = cs + int64_t(r) * m, *sv = sn + int64_t(r) * m, *gg = g + int64_t(r) * L;
-          for (int i = 0; i < j; ++i)
-            {
-              const double a0 = Hc[int64_t(i) * m + j], a1 = Hc[int64_t(i + 1) * m + j];
-              Hc[int64_t(i) * m + j]     = c[i] * a0 + sv[i] * a1;
-              Hc[int64_t(i + 1) * m + j] = -sv[i] * a0 + c[i] * a1;
-            }
-          const double a = Hc[int64_t(j) * m + j], bb = Hc[int64_t(j + 1) * m + j];
-          const double d = hypot(a, bb);
-          c[j]           = d > 0 ? a / d : 1.0;
-          sv[j]          = d > 0 ? bb / d : 0.0;
-          Hc[int64_t(j) * m + j]     = d;
-          Hc[int64_t(j + 1) * m + j] = 0;
-          gg[j + 1]                  = -sv[j] * gg[j];
-          gg[j]                      = c[j] * gg[j];
-          const int it               = its[r] + 1;
-          its[r]                     = it;
-          if (fabs(gg[j + 1]) / bn[r] <= tol[r] || bb == 0.0)
-            kdone[r] = j + 1;
-          if (kdone[r] >= 0 || j + 1 >= m || it >= maxit[r])
-            {
-              // the column ends its cycle: it takes no more steps (jvec
-              // -2 - steps until the host has used it)
-              jvec[r] = -2 - (j + 1);
-              ended   = 1;
-            }
-          else
-            {
-              jvec[r] = j + 1;
-              alive   = 1;
-            }
-        }
-      __syncthreads();
-      if (threadIdx.x == 0)
-        {
-          const int steps = ctl[1] + 1; // steps run since the host set ctl
-          // the steps go on while some column is in its cycle, for at most
-          // ctl[2] steps, and with ctl[3] set only until the first column ends
-          // its cycle (every active column ends its cycle within m steps)
-          const int stop = !alive || (ended && ctl[3]) || steps >= ctl[2];
-          ctl[0]          = !stop;
-          ctl[1]          = steps;
-          if (use_cond && stop)
-            cudaGraphSetConditional(cond, 0);
-        }
     }
 
     // End of a column's cycle: y[r] solves its triangular system of k steps (k =
@@ -364,9 +395,8 @@ namespace pibem
       dst[int64_t(cols[k]) * ldd + t] = src[idx];
     }
 
-    // dst[k] = float(src[cols[k]]) and dst[cols[k]] = double(src[k]): the
-    // gather / scatter of the active columns fused with the FP32 operator's
-    // input and output conversions
+    // dst[k] = float(src[cols[k]]) and dst[cols[k]] = double(src[k]): the FP32
+    // operator's input from the slots and back
     __global__ void gather_d2f_kernel(int64_t n, int Rc, const int *__restrict__ cols,
                                       const double *__restrict__ src, float *__restrict__ dst)
     {
@@ -380,7 +410,6 @@ namespace pibem
     __global__ void f2d_scatter_kernel(int64_t n, int Rc, const int *__restrict__ cols,
                                        const float *__restrict__ src, double *__restrict__ dst)
     {
-      pdl_entry();
       const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
       if (idx >= n * Rc)
         return;
@@ -530,85 +559,277 @@ namespace pibem
       x[idx] += -sqrt(nrm2[idx / n]);
     }
 
-    // z[node] = sum_c Pinv[leaf][r][c] v[rows_c]  (leaf-block Jacobi, right
-    // preconditioner), in the precision P of the stored inverses: FP32 for the
-    // mixed path's inner solves (GB300's FP64 rate is 1/58 of its FP32 rate),
-    // FP64 for the plain FP64 path (whose GMRES would otherwise see the FP32
-    // rounding as a nonlinearity near its 1e-8 target).  One warp per leaf, 8
-    // per block: the leaf's v entries are gathered into the warp's shared
-    // slice, lane i computes rows i, i + 32, ... with c ascending; the blocks
-    // are stored column-major (entry (r, c) at c * nr + r), so a column is read
-    // across the lanes.
+    // Leaf-block Jacobi (right preconditioner), z[node] = sum_c Pinv[leaf][r][c]
+    // v[rows_c], in the precision P of the stored inverses: FP32 for the mixed
+    // path's inner solves (GB300's FP64 rate is 1/58 of its FP32 rate), FP64 for
+    // the plain FP64 path (whose GMRES would otherwise see the FP32 rounding as a
+    // nonlinearity near its 1e-8 target).  One warp per leaf: the leaf's v entries
+    // of CB columns are in the warp's shared slice sv, lane i computes rows i,
+    // i + 32, ... with c ascending (the same chain for every CB); the blocks are
+    // stored column-major (entry (r, c) at c * nr + r), so a column is read across
+    // the lanes, once for the CB columns.  put(column, row, value) takes the result.
+    template <int CB, typename P, typename F>
+    __device__ __forceinline__ void block_rows(int nr, const int32_t *rows, const P *B, const P *sv,
+                                               int max_rows, F put)
+    {
+      const int lane = threadIdx.x & 31;
+      for (int i = lane; i < nr; i += 32)
+        {
+          P s[CB];
+#pragma unroll
+          for (int q = 0; q < CB; ++q)
+            s[q] = P(0);
+          int c = 0;
+          for (; c + 8 <= nr; c += 8)
+            {
+              P p[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u)
+                p[u] = B[int64_t(c + u) * nr + i];
+#pragma unroll
+              for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int q = 0; q < CB; ++q)
+                  s[q] = fma(p[u], sv[q * max_rows + c + u], s[q]);
+            }
+          for (; c < nr; ++c)
+            {
+              const P p = B[int64_t(c) * nr + i];
+#pragma unroll
+              for (int q = 0; q < CB; ++q)
+                s[q] = fma(p, sv[q * max_rows + c], s[q]);
+            }
+          const int row = rows[i];
+#pragma unroll
+          for (int q = 0; q < CB; ++q)
+            put(q, row, s[q]);
+        }
+    }
+
     template <typename P>
     __global__ void __launch_bounds__(256)
       block_apply_kernel(int n_leaves, int max_rows, int R, int64_t n, int64_t ldv,
                          const int64_t *__restrict__ row_ptr, const int64_t *__restrict__ blk_ptr,
                          const int32_t *__restrict__ rows, const P *__restrict__ Pinv,
                          const double *__restrict__ v, double *__restrict__ z,
-                         const double *__restrict__ nrm2, double *__restrict__ vout, int64_t ldo,
-                         const int *__restrict__ jvec, const int *__restrict__ sel)
+                         const int *__restrict__ sel)
     {
-      pdl_entry();
       extern __shared__ __align__(8) unsigned char sv_raw[];
-      P        *sv_all = reinterpret_cast<P *>(sv_raw);
       const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
       const int leaf = blockIdx.x * 8 + warp;
       if (leaf >= n_leaves)
         return;
-      P            *sv = sv_all + int64_t(warp) * max_rows;
+      P            *sv = reinterpret_cast<P *>(sv_raw) + int64_t(warp) * max_rows;
       const int64_t r0 = row_ptr[leaf];
       const int     nr = int(row_ptr[leaf + 1] - r0);
-      const P      *B  = Pinv + blk_ptr[leaf];
       for (int rr = 0; rr < R; ++rr)
         {
           if (sel && !sel[rr])
             continue;
-          int64_t vo = int64_t(rr) * ldo; // output column (basis vector jvec[rr] + 1 with jvec)
-          if (jvec)
+          for (int c = lane; c < nr; c += 32)
+            sv[c] = P(v[int64_t(rr) * ldv + rows[r0 + c]]);
+          __syncwarp();
+          block_rows<1, P>(nr, rows + r0, Pinv + blk_ptr[leaf], sv, max_rows,
+                           [&](int, int row, P s) { z[int64_t(rr) * n + row] = double(s); });
+          __syncwarp();
+        }
+    }
+
+    // The Givens step of the batch's columns (one block): the Hessenberg column
+    // h1 + h2, the previous rotations, the new one and the stopping test (|g_{j+1}|
+    // / bn <= tol, or a zero subdiagonal); then jvec and the iteration count
+    // advance.  A column ends its cycle when it meets its tolerance, after m steps
+    // or at its iteration limit (jvec = -2 - steps: no more steps); when the steps
+    // stop (see ctl), ctl[0] = 0 and, in a graph, the loop's condition is cleared.
+    // A warp per column: lane l holds rotation l of a group of 32, the chain a <-
+    // -s_l a + c_l h_{l+1} runs in every lane (one FMA a rotation), and lane l
+    // forms its entry from the a it saw.
+    __device__ __forceinline__ void givens_step(const GivensArgs &a, int Ra, int S, const int *act,
+                                                const int *sj, const double *snr)
+    {
+      __shared__ int ended, alive;
+      if (threadIdx.x == 0)
+        ended = alive = 0;
+      __syncthreads();
+      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+      const int m = a.m, L = m + 1;
+      for (int k = warp; k < Ra; k += nw)
+        {
+          const int j = sj[k];
+          if (j < 0)
+            continue;
+          const int     r  = act[k];
+          double       *Hc = a.H + int64_t(r) * L * m;
+          const double *h1 = a.hb + int64_t(r) * L, *h2 = h1 + int64_t(S) * L;
+          double       *c = a.cs + int64_t(r) * m, *sv = a.sn + int64_t(r) * m;
+          double        x = h1[0] + h2[0];
+          for (int i0 = 0; i0 < j; i0 += 32)
             {
-              if (jvec[rr] < 0)
+              const int i = i0 + lane;
+              double    ci = 0, si = 0, hn = 0, mine = 0;
+              if (i < j)
+                {
+                  ci = c[i];
+                  si = sv[i];
+                  hn = h1[i + 1] + h2[i + 1];
+                }
+              const double ch = ci * hn;
+              for (int l = 0; l < 32 && i0 + l < j; ++l)
+                {
+                  mine = lane == l ? x : mine;
+                  x    = fma(-__shfl_sync(0xffffffffu, si, l), x, __shfl_sync(0xffffffffu, ch, l));
+                }
+              if (i < j)
+                Hc[int64_t(i) * m + j] = fma(ci, mine, si * hn);
+            }
+          if (lane == 0)
+            {
+              const double bb = sqrt(snr[k]), d = hypot(x, bb);
+              const double cj = d > 0 ? x / d : 1.0, sj2 = d > 0 ? bb / d : 0.0;
+              double      *gg = a.g + int64_t(r) * L;
+              c[j]            = cj;
+              sv[j]           = sj2;
+              Hc[int64_t(j) * m + j]       = d;
+              Hc[int64_t(j + 1) * m + j]   = 0;
+              const double gj = gg[j], g1 = -sj2 * gj;
+              gg[j + 1]       = g1;
+              gg[j]           = cj * gj;
+              const int it    = a.its[r] + 1;
+              a.its[r]        = it;
+              int done        = a.kdone[r];
+              if (fabs(g1) / a.bn[r] <= a.tol[r] || bb == 0.0)
+                a.kdone[r] = done = j + 1;
+              if (done >= 0 || j + 1 >= m || it >= a.maxit[r])
+                {
+                  a.jvec[r] = -2 - (j + 1);
+                  ended     = 1;
+                }
+              else
+                {
+                  a.jvec[r] = j + 1;
+                  alive     = 1;
+                }
+            }
+        }
+      __syncthreads();
+      if (threadIdx.x == 0)
+        {
+          const int steps = a.ctl[1] + 1; // steps run since the host set ctl
+          // the steps go on while some column is in its cycle, for at most
+          // ctl[2] steps, and with ctl[3] set only until the first column ends
+          // its cycle (every active column ends its cycle within m steps)
+          const int stop = !alive || (ended && a.ctl[3]) || steps >= a.ctl[2];
+          a.ctl[0]       = !stop;
+          a.ctl[1]       = steps;
+          if (a.use_cond && stop)
+            cudaGraphSetConditional(a.cond, 0);
+        }
+    }
+
+    // End of an Arnoldi step.  Every block adds the columns' squared norms; block 0
+    // takes the Givens step, the others V_{j+1} = w / |w| and, into out (the
+    // operator's next input: batch column k, or slot act[k] with SLOT), BJ: the
+    // leaf-block Jacobi result z = P^-1 V_{j+1}, a warp per leaf and CB columns at
+    // a time; otherwise V_{j+1} itself.  Columns with jcur < 0 are skipped.
+    // Shared memory: |w|^2 and 1 / |w| [Ra], steps [Ra], sv[warps][CB][max_rows].
+    template <typename P, typename OUT, bool BJ, int CB, bool SLOT>
+    __global__ void __launch_bounds__(AR_THREADS)
+      arnoldi_finish_kernel(int64_t n, int S, int G, int Ra, int64_t ldr, const int *__restrict__ act,
+                            const int *__restrict__ jcur, const double *__restrict__ pn,
+                            const double *__restrict__ w, double *__restrict__ V,
+                            OUT *__restrict__ out, BlockPrec<P> bp, GivensArgs ga)
+    {
+      pdl_entry();
+      extern __shared__ __align__(16) unsigned char fin_raw[];
+      double   *snr = reinterpret_cast<double *>(fin_raw), *sinv = snr + Ra;
+      int      *sj   = reinterpret_cast<int *>(sinv + Ra);
+      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+      for (int k = warp; k < Ra; k += nw)
+        {
+          const int r = act[k], j = r < S ? jcur[r] : -1;
+          double    s = 0;
+          if (j >= 0)
+            for (int b = lane; b < G; b += 32)
+              s += pn[int64_t(k) * G + b];
+          for (int o = 16; o > 0; o >>= 1)
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+          if (lane == 0)
+            {
+              snr[k]  = s;
+              sinv[k] = s > 0 ? 1.0 / sqrt(s) : 0.0;
+              sj[k]   = j;
+            }
+        }
+      __syncthreads();
+      if (blockIdx.x == 0)
+        {
+          givens_step(ga, Ra, S, act, sj, snr);
+          return;
+        }
+      auto col_of = [&](int k) { return int64_t(SLOT ? act[k] : k) * n; };
+      if constexpr (!BJ)
+        {
+          for (int k = 0; k < Ra; ++k)
+            {
+              const int j = sj[k];
+              if (j < 0)
                 continue;
-              vo += int64_t(jvec[rr] + 1) * n;
-            }
-          if (nrm2)
-            {
-              // the Arnoldi normalisation fused in (as normalize_kernel):
-              // vout = v / |v|, then z = P^-1 vout
-              const double h = sqrt(nrm2[rr]);
-              for (int c = lane; c < nr; c += 32)
+              const int64_t r = act[k];
+              double       *v = V + r * ldr + int64_t(j + 1) * n;
+              for (int64_t t = int64_t(blockIdx.x - 1) * blockDim.x + threadIdx.x; t < n;
+                   t += int64_t(gridDim.x - 1) * blockDim.x)
                 {
-                  const int64_t row = rows[r0 + c];
-                  const double  vn  = h > 0 ? v[int64_t(rr) * ldv + row] / h : 0.0;
-                  vout[vo + row] = vn;
-                  sv[c]          = P(vn);
+                  const double x      = w[r * n + t] * sinv[k];
+                  v[t]                = x;
+                  out[col_of(k) + t]  = OUT(x);
                 }
             }
-          else
-            for (int c = lane; c < nr; c += 32)
-              sv[c] = P(v[int64_t(rr) * ldv + rows[r0 + c]]);
-          __syncwarp();
-          for (int i = lane; i - lane < nr; i += 32)
+        }
+      else
+        {
+          P *sv = reinterpret_cast<P *>(fin_raw + (size_t(Ra) * 20 + 15) / 16 * 16) +
+                  int64_t(warp) * CB * bp.max_rows;
+          for (int leaf = int(blockIdx.x - 1) * nw + warp; leaf < bp.n_leaves;
+               leaf += int(gridDim.x - 1) * nw)
             {
-              P s = P(0);
-              if (i < nr)
+              const int64_t  r0   = bp.row_ptr[leaf];
+              const int      nr   = int(bp.row_ptr[leaf + 1] - r0);
+              const int32_t *rows = bp.rows + r0;
+              const P       *B    = bp.Pinv + bp.blk_ptr[leaf];
+              for (int k0 = 0; k0 < Ra; k0 += CB)
                 {
-                  int c = 0;
-                  for (; c + 8 <= nr; c += 8)
+                  bool any = false;
+#pragma unroll
+                  for (int q = 0; q < CB; ++q)
                     {
-                      P p[8];
-#pragma unroll
-                      for (int u = 0; u < 8; ++u)
-                        p[u] = B[int64_t(c + u) * nr + i];
-#pragma unroll
-                      for (int u = 0; u < 8; ++u)
-                        s = fma(p[u], sv[c + u], s);
+                      const int k = k0 + q, j = k < Ra ? sj[k] : -1;
+                      if (j < 0)
+                        {
+                          for (int c = lane; c < nr; c += 32)
+                            sv[q * bp.max_rows + c] = P(0);
+                          continue;
+                        }
+                      any             = true;
+                      const int64_t r = act[k];
+                      double       *v = V + r * ldr + int64_t(j + 1) * n;
+                      for (int c = lane; c < nr; c += 32)
+                        {
+                          const int64_t row       = rows[c];
+                          const double  x         = w[r * n + row] * sinv[k];
+                          v[row]                  = x;
+                          sv[q * bp.max_rows + c] = P(x);
+                        }
                     }
-                  for (; c < nr; ++c)
-                    s = fma(B[int64_t(c) * nr + i], sv[c], s);
-                  z[int64_t(rr) * n + rows[r0 + i]] = double(s);
+                  __syncwarp();
+                  if (any)
+                    block_rows<CB, P>(nr, rows, B, sv, bp.max_rows, [&](int q, int row, P s) {
+                      const int k = k0 + q;
+                      if (k < Ra && sj[k] >= 0)
+                        out[col_of(k) + row] = OUT(s);
+                    });
+                  __syncwarp();
                 }
             }
-          __syncwarp();
         }
     }
 
@@ -831,26 +1052,80 @@ namespace pibem
     note_launch(2);
   }
 
-  void launch_cgs_step(int mode, int64_t n, int R, int ncols, int64_t ldv, int64_t ldr,
-                       const double *V, const double *hin, int ldh, double *w, int nblk,
-                       double *partial, int *ticket, double *out, cudaStream_t s, const int *jvec,
-                       int ldo)
+  int arnoldi_blocks(int64_t n)
   {
-    dim3 grid(nblk, R);
-    if (ldo <= 0)
-      ldo = mode == 2 ? 1 : ncols;
-    if (mode == 0)
-      launch_pdl(cgs_step_kernel<0>, grid, kDotBlock, 0, s, n, ncols, ldv, ldr, V, hin, ldh, w, nblk, partial,
-                                                     ticket, out, jvec, ldo);
-    else if (mode == 1)
-      launch_pdl(cgs_step_kernel<1>, grid, kDotBlock, 0, s, n, ncols, ldv, ldr, V, hin, ldh, w, nblk, partial,
-                                                     ticket, out, jvec, ldo);
+    return std::max(1, std::min(AR_MAX_BLOCKS, int(std::ceil(0.5 * std::sqrt(double(n))))));
+  }
+
+  template <typename T>
+  void launch_arnoldi_cgs(const ArnoldiArgs &a, const T *in, cudaStream_t s)
+  {
+    const int     G = arnoldi_blocks(a.n), L = a.m + 1;
+    const dim3    grid(G, a.Ra);
+    const size_t  smem = size_t(L) * sizeof(double);
+    const int64_t ldr  = int64_t(L) * a.n;
+    double       *pa = a.partial, *pb = pa + int64_t(a.S) * L * G, *pn = pb + int64_t(a.S) * L * G;
+    if (smem > 16 * 1024)
+      {
+        raise_smem_limit(reinterpret_cast<const void *>(arnoldi_sub_kernel<false>), smem);
+        raise_smem_limit(reinterpret_cast<const void *>(arnoldi_sub_kernel<true>), smem);
+      }
+    launch_pdl(arnoldi_dots_kernel<T>, grid, AR_THREADS, 0, s, a.n, a.S, G, L, ldr, a.act, in, a.V, a.w,
+               a.g.jvec, a.jcur, pa);
+    launch_pdl(arnoldi_sub_kernel<false>, grid, AR_THREADS, smem, s, a.n, a.S, G, L, ldr, a.act, a.V,
+               a.w, a.jcur, pa, a.g.hb, pb);
+    launch_pdl(arnoldi_sub_kernel<true>, grid, AR_THREADS, smem, s, a.n, a.S, G, L, ldr, a.act, a.V,
+               a.w, a.jcur, pb, a.g.hb + int64_t(a.S) * L, pn);
+    PIBEM_CUDA(cudaGetLastError());
+    note_launch(3);
+  }
+  template void launch_arnoldi_cgs<float>(const ArnoldiArgs &, const float *, cudaStream_t);
+  template void launch_arnoldi_cgs<double>(const ArnoldiArgs &, const double *, cudaStream_t);
+
+  template <typename P, typename OUT>
+  void launch_arnoldi_finish(const ArnoldiArgs &a, const BlockPrec<P> &bp, OUT *out, bool slot,
+                             cudaStream_t s)
+  {
+    const int     G = arnoldi_blocks(a.n), L = a.m + 1;
+    const int64_t ldr  = int64_t(L) * a.n;
+    double       *pn   = a.partial + int64_t(2) * a.S * L * G;
+    const size_t  head = (size_t(a.Ra) * 20 + 15) / 16 * 16;
+    auto launch = [&](auto kern, int threads, int64_t blocks, size_t smem) {
+      if (smem > 40 * 1024)
+        raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
+      launch_pdl(kern, unsigned(1 + std::max<int64_t>(1, blocks)), threads, smem, s, a.n, a.S, G, a.Ra,
+                 ldr, a.act, a.jcur, pn, a.w, a.V, out, bp, a.g);
+    };
+    if (!bp.Pinv)
+      {
+        const int64_t nb = std::min<int64_t>(2 * AR_MAX_BLOCKS, (a.n + AR_THREADS - 1) / AR_THREADS);
+        if (slot)
+          launch(arnoldi_finish_kernel<P, OUT, false, 1, true>, AR_THREADS, nb, head);
+        else
+          launch(arnoldi_finish_kernel<P, OUT, false, 1, false>, AR_THREADS, nb, head);
+      }
     else
-      launch_pdl(cgs_step_kernel<2>, grid, kDotBlock, 0, s, n, ncols, ldv, ldr, V, hin, ldh, w, nblk, partial,
-                                                     ticket, out, jvec, ldo);
+      {
+        // four columns at a time when several share the batch and their slices fit
+        // beside two blocks per SM; else one, with fewer warps for very large leaves
+        const size_t one = size_t(bp.max_rows) * sizeof(P);
+        const bool   big = 16 * one + head > 200 * 1024;
+        const int    nw  = big ? 8 : 16;
+        const int64_t nb = std::min<int64_t>(2 * AR_MAX_BLOCKS, (bp.n_leaves + nw - 1) / nw);
+        if (a.Ra > 1 && 64 * one + head <= 100 * 1024)
+          launch(arnoldi_finish_kernel<P, OUT, true, 4, false>, AR_THREADS, nb, head + 64 * one);
+        else
+          launch(arnoldi_finish_kernel<P, OUT, true, 1, false>, 32 * nw, nb, head + nw * one);
+      }
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
+  template void launch_arnoldi_finish<float, float>(const ArnoldiArgs &, const BlockPrec<float> &, float *,
+                                                    bool, cudaStream_t);
+  template void launch_arnoldi_finish<float, double>(const ArnoldiArgs &, const BlockPrec<float> &,
+                                                     double *, bool, cudaStream_t);
+  template void launch_arnoldi_finish<double, double>(const ArnoldiArgs &, const BlockPrec<double> &,
+                                                      double *, bool, cudaStream_t);
 
   void launch_gemv_sub(int64_t n, int R, int ncols, int64_t ldv, int64_t ldr, const double *V,
                        const double *h, int ldh, double *w, double sign, cudaStream_t s,
@@ -863,9 +1138,9 @@ namespace pibem
   }
 
   void launch_normalize(int64_t n, int R, const double *w, const double *nrm2, double *out,
-                        int64_t ldr, cudaStream_t s, const int *jvec, double *z, const int *sel)
+                        int64_t ldr, cudaStream_t s, double *z, const int *sel)
   {
-    launch_pdl(normalize_kernel, nblocks(n * R), 256, 0, s, n, R, w, nrm2, out, ldr, jvec, z, sel);
+    normalize_kernel<<<nblocks(n * R), 256, 0, s>>>(n, R, w, nrm2, out, ldr, z, sel);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
@@ -874,17 +1149,6 @@ namespace pibem
                                int *jvec, cudaStream_t s)
   {
     gmres_cycle_init_kernel<<<1, 256, 0, s>>>(R, m + 1, sel, nrm2, g, kdone, jvec);
-    PIBEM_CUDA(cudaGetLastError());
-    note_launch();
-  }
-
-  void launch_gmres_givens(int R, int m, const double *hb, double *H, double *cs, double *sn,
-                           double *g, int *kdone, int *jvec, int *its, const int *maxit,
-                           const double *bn, const double *tol, int *ctl,
-                           cudaGraphConditionalHandle cond, bool use_cond, cudaStream_t s)
-  {
-    launch_pdl(gmres_givens_kernel, 1, 256, 0, s, R, m, hb, H, cs, sn, g, kdone, jvec, its, maxit, bn, tol,
-                                          ctl, cond, use_cond ? 1 : 0);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
@@ -932,7 +1196,7 @@ namespace pibem
   {
     if (Rc == 0)
       return;
-    launch_pdl(f2d_scatter_kernel, nblocks(n * Rc), 256, 0, s, n, Rc, cols, src, dst);
+    f2d_scatter_kernel<<<nblocks(n * Rc), 256, 0, s>>>(n, Rc, cols, src, dst);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
@@ -1048,32 +1312,23 @@ namespace pibem
   }
 
   template <typename P>
-  void launch_block_apply(int n_leaves, int max_rows, int R, int64_t n, const int64_t *row_ptr,
-                          const int64_t *blk_ptr, const int32_t *rows, const P *Pinv,
-                          const double *v, int64_t ldv, double *z, cudaStream_t s,
-                          const double *nrm2, double *vout, int64_t ldo, const int *jvec,
-                          const int *sel)
+  void launch_block_apply(const BlockPrec<P> &bp, int R, int64_t n, const double *v, int64_t ldv,
+                          double *z, const int *sel, cudaStream_t s)
   {
-    if (n_leaves == 0)
+    if (bp.n_leaves == 0)
       return;
-    const int    mr   = std::max(max_rows, 1);
-    const size_t smem = size_t(8) * mr * sizeof(P);
+    const size_t smem = size_t(8) * bp.max_rows * sizeof(P);
     if (smem > 48 * 1024)
       raise_smem_limit(reinterpret_cast<const void *>(block_apply_kernel<P>), smem);
-    launch_pdl(block_apply_kernel<P>, (n_leaves + 7) / 8, 256, smem, s, n_leaves, mr, R, n, ldv, row_ptr,
-                                                                blk_ptr, rows, Pinv, v, z, nrm2,
-                                                                vout, ldo, jvec, sel);
+    block_apply_kernel<P><<<(bp.n_leaves + 7) / 8, 256, smem, s>>>(
+      bp.n_leaves, bp.max_rows, R, n, ldv, bp.row_ptr, bp.blk_ptr, bp.rows, bp.Pinv, v, z, sel);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
-  template void launch_block_apply<float>(int, int, int, int64_t, const int64_t *, const int64_t *,
-                                          const int32_t *, const float *, const double *, int64_t,
-                                          double *, cudaStream_t, const double *, double *, int64_t,
-                                          const int *, const int *);
-  template void launch_block_apply<double>(int, int, int, int64_t, const int64_t *, const int64_t *,
-                                           const int32_t *, const double *, const double *, int64_t,
-                                           double *, cudaStream_t, const double *, double *, int64_t,
-                                           const int *, const int *);
+  template void launch_block_apply<float>(const BlockPrec<float> &, int, int64_t, const double *, int64_t,
+                                          double *, const int *, cudaStream_t);
+  template void launch_block_apply<double>(const BlockPrec<double> &, int, int64_t, const double *,
+                                           int64_t, double *, const int *, cudaStream_t);
 
   void launch_ilu_fill(int64_t n, const int64_t *ptr, const int32_t *pos, const int32_t *row_leaf,
                        const int64_t *nrow_ptr, const int64_t *ncol_ptr, const int64_t *nval_ptr,

@@ -14,34 +14,61 @@ namespace pibem
   void launch_gemv_sub(int64_t n, int R, int ncols, int64_t ldv, int64_t ldr, const double *V,
                        const double *h, int ldh, double *w, double sign, cudaStream_t s,
                        const int *jvec = nullptr, const int *sel = nullptr);
-  // one Arnoldi Gram-Schmidt pass in one launch (mode 0: dots; 1: subtract then
-  // dots; 2: subtract then the squared norm); ticket: R ints, zero between
-  // calls; out: ldo values per column (ldo <= 0: the pass's output count);
-  // jvec non-null: column r takes ncols = jvec[r] + 1 (read on the device;
-  // jvec[r] < 0: the column is skipped)
-  void launch_cgs_step(int mode, int64_t n, int R, int ncols, int64_t ldv, int64_t ldr,
-                       const double *V, const double *hin, int ldh, double *w, int nblk,
-                       double *partial, int *ticket, double *out, cudaStream_t s,
-                       const int *jvec = nullptr, int ldo = 0);
-  // out[r] = w[r] / sqrt(nrm2[r]) (column stride ldr; jvec non-null: at basis
-  // vector jvec[r] + 1 of out, columns with jvec[r] < 0 skipped; sel non-null:
-  // selected columns only), also into z (stride n) when z is non-null
+  // leaf-block Jacobi: inverses of the childless boxes' diagonal blocks, column-
+  // major (Pinv null: no preconditioner)
+  template <typename P>
+  struct BlockPrec
+  {
+    int            n_leaves = 0, max_rows = 1;
+    const int64_t *row_ptr = nullptr, *blk_ptr = nullptr;
+    const int32_t *rows = nullptr;
+    const P       *Pinv = nullptr;
+  };
+  // the Givens state of the columns (layout in krylov.cu)
+  struct GivensArgs
+  {
+    int     m  = 0;
+    double *hb = nullptr, *H = nullptr, *cs = nullptr, *sn = nullptr, *g = nullptr;
+    int    *kdone = nullptr, *jvec = nullptr, *its = nullptr, *maxit = nullptr;
+    double *bn = nullptr, *tol = nullptr;
+    int    *ctl = nullptr;
+    cudaGraphConditionalHandle cond{};
+    int                        use_cond = 0;
+  };
+  // One Arnoldi step of the Ra batch columns (column k: slot act[k] of S, >= S
+  // idle) with jvec >= 0, after the operator: w <- in, CGS2 against V_0..V_j (cgs);
+  // V_{j+1}, the preconditioned input of the next step in out (batch column k, or
+  // slot act[k] with slot) and the Givens step (finish).  jcur: S ints of work;
+  // partial: S (2 (m + 1) + 1) arnoldi_blocks(n) doubles.
+  struct ArnoldiArgs
+  {
+    int64_t    n = 0;
+    int        S = 0, m = 0, Ra = 0;
+    const int *act = nullptr;
+    double    *V = nullptr, *w = nullptr, *partial = nullptr;
+    int       *jcur = nullptr;
+    GivensArgs g;
+  };
+  constexpr int AR_MAX_BLOCKS = 152; // blocks per column: one per SM
+  int           arnoldi_blocks(int64_t n);
+  template <typename T>
+  void launch_arnoldi_cgs(const ArnoldiArgs &a, const T *in, cudaStream_t s);
+  template <typename P, typename OUT>
+  void launch_arnoldi_finish(const ArnoldiArgs &a, const BlockPrec<P> &bp, OUT *out, bool slot,
+                             cudaStream_t s);
+  // out[r] = w[r] / sqrt(nrm2[r]) (column stride ldr) of the selected columns, also
+  // into z (stride n) when z is non-null
   void launch_normalize(int64_t n, int R, const double *w, const double *nrm2, double *out,
-                        int64_t ldr, cudaStream_t s, const int *jvec = nullptr,
-                        double *z = nullptr, const int *sel = nullptr);
+                        int64_t ldr, cudaStream_t s, double *z, const int *sel);
   // device-driven GMRES cycles, one state per column (layout in krylov.cu)
   void launch_gmres_cycle_init(int R, int m, const int *sel, const double *nrm2, double *g, int *kdone,
                                int *jvec, cudaStream_t s);
-  void launch_gmres_givens(int R, int m, const double *hb, double *H, double *cs, double *sn,
-                           double *g, int *kdone, int *jvec, int *its, const int *maxit,
-                           const double *bn, const double *tol, int *ctl,
-                           cudaGraphConditionalHandle cond, bool use_cond, cudaStream_t s);
   void launch_gmres_lsq(int R, int m, const int *sel, const double *H, const double *g,
                         const int *kdone, const int *jvec, double *y, cudaStream_t s);
   // compaction of selected columns for the operator: dst[k] = src[cols[k]] and back
   void launch_gather_cols(int64_t n, int Rc, const int *cols, const double *src, int64_t lds,
                           double *dst, cudaStream_t s);
-  // x32[k] = float(src[cols[k]]) / dst[cols[k]] = double(y32[k]) (column stride n)
+  // dst[k] = float(src[cols[k]]) / dst[cols[k]] = double(src[k]) (column stride n)
   void launch_gather_d2f(int64_t n, int Rc, const int *cols, const double *src, float *dst,
                          cudaStream_t s);
   void launch_f2d_scatter(int64_t n, int Rc, const int *cols, const float *src, double *dst,
@@ -88,14 +115,8 @@ namespace pibem
   void launch_constraint_rhs(int n_con, int R, int64_t n, const int32_t *rows, const uint8_t *kind,
                              const int32_t *p, const int32_t *q, const double *tmp,
                              const double *nrm, const double *sg, double *b, cudaStream_t s);
-  // z = P^-1 v (leaf-block Jacobi); with nrm2: v is first normalised, column
-  // r by sqrt(nrm2[r]), and written to vout (column stride ldo; jvec non-null:
-  // at basis vector jvec[r] + 1 of vout, vectors n apart, columns with
-  // jvec[r] < 0 skipped); sel non-null: the selected columns only
+  // z = P^-1 v (leaf-block Jacobi); sel non-null: the selected columns only
   template <typename P>
-  void launch_block_apply(int n_leaves, int max_rows, int R, int64_t n, const int64_t *row_ptr,
-                          const int64_t *blk_ptr, const int32_t *rows, const P *Pinv,
-                          const double *v, int64_t ldv, double *z, cudaStream_t s,
-                          const double *nrm2 = nullptr, double *vout = nullptr, int64_t ldo = 0,
-                          const int *jvec = nullptr, const int *sel = nullptr);
+  void launch_block_apply(const BlockPrec<P> &bp, int R, int64_t n, const double *v, int64_t ldv,
+                          double *z, const int *sel, cudaStream_t s);
 } // namespace pibem
