@@ -131,69 +131,6 @@ namespace pibem
     __device__ static float rb(int n, int m) { return c_leg.frb[n][m]; }
   };
 
-  // Table-driven evaluation (same sum as eval_expansion below, no square roots
-  // in the loop): value = sum_k coef[k] basis_k(r).
-  template <typename T, typename E>
-  __device__ inline T eval_expansion_fast(const E *__restrict__ coef, int p, T rx, T ry, T rz,
-                                          bool multipole)
-  {
-    using LT = LegT<T>;
-    const T r2  = rx * rx + ry * ry + rz * rz;
-    const T rho = sqrt(r2);
-    const T inv = T(1) / rho;
-    const T x   = rz * inv;
-    const T s   = sqrt(fmax(T(0), T(1) - x * x));
-    const T rxy = sqrt(rx * rx + ry * ry);
-    T       cb = T(1), sb = T(0);
-    if (rxy > T(0))
-      {
-        cb = rx / rxy;
-        sb = ry / rxy;
-      }
-    const T step = multipole ? inv : rho;
-    T       acc  = T(0);
-    T       pmm  = T(1);
-    T       rpm  = multipole ? inv : T(1);
-    T       cm = T(1), sm = T(0);
-    for (int m = 0; m <= p; ++m)
-      {
-        if (m > 0)
-          {
-            pmm *= -LT::cmm(m) * s;
-            rpm *= step;
-            const T c2 = cm * cb - sm * sb;
-            sm         = sm * cb + cm * sb;
-            cm         = c2;
-          }
-        const T cr = m == 0 ? T(1) : T(2) * cm;
-        const T ci = m == 0 ? T(0) : -T(2) * sm;
-        T       p0 = pmm, rp = rpm;
-        int     k0 = m * m + (m == 0 ? 0 : 2 * m - 1);
-        T       v  = T(coef[k0]) * cr + (m > 0 ? T(coef[k0 + 1]) * ci : T(0));
-        acc += v * p0 * rp;
-        if (m + 1 <= p)
-          {
-            T p1 = x * LT::cm1(m) * pmm;
-            rp *= step;
-            int n  = m + 1;
-            k0     = n * n + (m == 0 ? 0 : 2 * m - 1);
-            v      = T(coef[k0]) * cr + (m > 0 ? T(coef[k0 + 1]) * ci : T(0));
-            acc += v * p1 * rp;
-            for (n = m + 2; n <= p; ++n)
-              {
-                const T p2 = LT::ra(n, m) * x * p1 - LT::rb(n, m) * p0;
-                p0         = p1;
-                p1         = p2;
-                rp *= step;
-                k0 = n * n + (m == 0 ? 0 : 2 * m - 1);
-                v  = T(coef[k0]) * cr + (m > 0 ? T(coef[k0 + 1]) * ci : T(0));
-                acc += v * p1 * rp;
-              }
-          }
-      }
-    return acc;
-  }
-
   // Evaluation of a scaled expansion at relative position r (in box units):
   //   kind 0 (local):     sum_k E[k] * basis_k with r^n
   //   kind 1 (multipole): with r^(-n-1)

@@ -32,9 +32,18 @@ namespace pibem
       return v;
     }
 
+    __device__ __forceinline__ float  shfl_xor(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+    __device__ __forceinline__ double shfl_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+    __device__ __forceinline__ float2 shfl_xor(float2 v, int o)
+    {
+      return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+    }
+
     // a * b + c with one rounding (no dependence on the compiler's contraction)
     __device__ __forceinline__ float  fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
     __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+    __device__ __forceinline__ float  mul_rn(float a, float b) { return __fmul_rn(a, b); }
+    __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
     // s + a . x for 4 values, with the rounding steps spelled out so that every
     // code path (one column or several) computes a column bit-for-bit alike.
@@ -74,87 +83,100 @@ namespace pibem
       v[3] = b.y;
     }
 
-    // Near-field leaf-block SpMV: one block per childless box.  The x entries of
-    // the block's columns are gathered once into shared memory (rb rhs at a
-    // time, zero in the row padding), then each warp streams whole rows of the
-    // dense leaf block with 16-byte loads (rows padded to 4 values).
-    template <typename T, bool ONE_COL>
-    __global__ void __launch_bounds__(256)
-      near_leaf_kernel(int R, int rb, int N, const int64_t *__restrict__ nrow_ptr,
-                       const int64_t *__restrict__ ncol_ptr, const int64_t *__restrict__ nval_ptr,
-                       const int32_t *__restrict__ nrows, const int32_t *__restrict__ ncols,
-                       const T *__restrict__ vals, const T *__restrict__ x, T *__restrict__ y,
-                       bool acc)
+    // Sums over the warp of M values per lane (M = 2, 4, 8 or 16) with the additions
+    // of warp_sum's butterfly: after each of the first log2(M) steps a lane keeps half
+    // of the values, so M + 4 - log2(M) shuffles instead of 5 M.  Lane l ends with the
+    // sum of value l / (32 / M).
+    template <int M, typename T, typename ADD>
+    __device__ __forceinline__ T warp_sums(T (&v)[M], ADD add)
+    {
+      const int lane = threadIdx.x & 31;
+      int       o    = 16;
+#pragma unroll
+      for (int n = M / 2; n > 0; n >>= 1, o >>= 1)
+        {
+          const bool up = (lane & o) != 0;
+#pragma unroll
+          for (int i = 0; i < n; ++i)
+            v[i] = add(up ? v[i + n] : v[i], shfl_xor(up ? v[i] : v[i + n], o));
+        }
+      for (; o > 0; o >>= 1)
+        v[0] = add(v[0], shfl_xor(v[0], o));
+      return v[0];
+    }
+
+    // Near-field leaf-block SpMV for several columns: one block per childless box.
+    // The x entries of the block's columns are gathered into shared memory (rb
+    // right-hand sides at a time, zero in the paddings); a warp takes RR rows and RC
+    // columns at a time, so that a row's 16-byte loads serve RC columns and an x
+    // load RR rows.  A (row, column) sum has the chunks per lane, the order and the
+    // butterfly of the one-column kernels.
+    // What bounds it: the x gathers (4 bytes each) and shared-memory loads.
+    template <typename T, int RC, int RR>
+    __global__ void __launch_bounds__(128)
+      near_leaf_multi_kernel(int R, int rb, int N, const int64_t *__restrict__ nrow_ptr,
+                             const int64_t *__restrict__ ncol_ptr, const int64_t *__restrict__ nval_ptr,
+                             const int32_t *__restrict__ nrows, const int32_t *__restrict__ ncols,
+                             const T *__restrict__ vals, const T *__restrict__ x, T *__restrict__ y,
+                             bool acc)
     {
       pdl_entry();
       extern __shared__ __align__(16) unsigned char smem_raw[];
       T            *sx   = reinterpret_cast<T *>(smem_raw); // [rb][ld]
       const int     leaf = blockIdx.x;
-      const int64_t c0 = ncol_ptr[leaf], nc = ncol_ptr[leaf + 1] - c0;
-      const int64_t ld = (nc + 3) / 4 * 4;
-      const int64_t r0 = nrow_ptr[leaf], nr = nrow_ptr[leaf + 1] - r0;
+      const int64_t c0   = ncol_ptr[leaf];
+      const int     nc = int(ncol_ptr[leaf + 1] - c0), ld = (nc + 3) / 4 * 4, n4 = ld / 4;
+      const int64_t r0 = nrow_ptr[leaf];
+      const int     nr = int(nrow_ptr[leaf + 1] - r0);
       const T      *V    = vals + nval_ptr[leaf];
-      const int     warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-      const int     n4   = int(ld / 4);
+      const int     warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
       for (int ra = 0; ra < R; ra += rb)
         {
-          const int rc = min(rb, R - ra);
+          const int rc = min(rb, R - ra), rcp = (rc + RC - 1) / RC * RC;
           __syncthreads();
-          for (int64_t i = threadIdx.x; i < rc * ld; i += blockDim.x)
+          for (int c = threadIdx.x; c < ld; c += blockDim.x)
             {
-              const int64_t r = i / ld, c = i - r * ld;
-              sx[i]           = c < nc ? x[(ra + r) * int64_t(N) + ncols[c0 + c]] : T(0);
+              const T *xc = x + ra * int64_t(N) + (c < nc ? ncols[c0 + c] : 0);
+#pragma unroll 8
+              for (int r = 0; r < rcp; ++r)
+                sx[r * ld + c] = c < nc && r < rc ? xc[r * int64_t(N)] : T(0);
             }
           __syncthreads();
-          for (int64_t row = warp; row < nr; row += nw)
-            {
-              const T  *v    = V + row * ld;
-              const int node = nrows[r0 + row];
-              if (ONE_COL)
-                {
-                  // one column: several 16-byte loads of the row in flight per lane
-                  T s0 = T(0);
-#pragma unroll 4
-                  for (int j = lane; j < n4; j += 32)
-                    {
-                      T a[4];
-                      load4(v + 4 * j, a);
-                      s0 = dot4_acc(s0, a, sx + 4 * j);
-                    }
-                  const T t = warp_sum(s0);
-                  if (lane == 0)
-                    {
-                      T &o = y[ra * int64_t(N) + node];
-                      o    = acc ? o + t : t;
-                    }
-                  continue;
-                }
-              for (int rq = 0; rq < rc; rq += 4)
-                {
-                  T s[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll 2
-                  for (int j = lane; j < n4; j += 32)
-                    {
-                      T a[4];
-                      load4(v + 4 * j, a);
+          for (int row = warp * RR; row < nr; row += 4 * RR)
+            for (int rq = 0; rq < rcp; rq += RC)
+              {
+                T s[RR * RC];
 #pragma unroll
-                      for (int rr = 0; rr < 4; ++rr)
-                        if (rq + rr < rc)
-                          s[rr] = dot4_acc(s[rr], a, sx + (rq + rr) * ld + 4 * j);
-                    }
+                for (int i = 0; i < RR * RC; ++i)
+                  s[i] = T(0);
+                const T *v[RR];
 #pragma unroll
-                  for (int rr = 0; rr < 4; ++rr)
-                    if (rq + rr < rc)
-                      {
-                        const T t = warp_sum(s[rr]);
-                        if (lane == 0)
-                          {
-                            T &o = y[(ra + rq + rr) * int64_t(N) + node];
-                            o    = acc ? o + t : t;
-                          }
-                      }
-                }
-            }
+                for (int i = 0; i < RR; ++i) // a row beyond the leaf's repeats the last one
+                  v[i] = V + int64_t(min(row + i, nr - 1)) * ld;
+                for (int j = lane; j < n4; j += 32)
+                  {
+                    T a[RR][4], b[RC][4];
+#pragma unroll
+                    for (int i = 0; i < RR; ++i)
+                      load4(v[i] + 4 * j, a[i]);
+#pragma unroll
+                    for (int r = 0; r < RC; ++r)
+                      load4(sx + (rq + r) * ld + 4 * j, b[r]);
+#pragma unroll
+                    for (int i = 0; i < RR; ++i)
+#pragma unroll
+                      for (int r = 0; r < RC; ++r)
+                        s[i * RC + r] = dot4_acc(s[i * RC + r], a[i], b[r]);
+                  }
+                const T t = warp_sums<RR * RC>(s, [](T p, T q) { return p + q; });
+                constexpr int W = 32 / (RR * RC); // lanes per value
+                const int     i = row + lane / (W * RC), r = rq + (lane / W) % RC;
+                if (lane % W == 0 && i < nr && r < rc)
+                  {
+                    T &o = y[(ra + r) * int64_t(N) + nrows[r0 + i]];
+                    o    = acc ? o + t : t;
+                  }
+              }
         }
     }
 
@@ -187,7 +209,7 @@ namespace pibem
     // leaves from an atomic counter 89 us); while the warps stream the rows of a
     // leaf, the x entries of the block's next leaf are gathered into the other
     // half of a double buffer with cp.async.  A row is computed exactly as in
-    // near_leaf_kernel (same chunks per lane, same order, same butterfly).
+    // near_leaf_multi_kernel (same chunks per lane, same order, same butterfly).
     // Shared memory: 2 x ld_max values.
     template <typename T>
     __global__ void __launch_bounds__(256)
@@ -309,7 +331,7 @@ namespace pibem
     // the schedule record of leaf t+3, so that inside a leaf only the row
     // values are waited for.  Rows: two per warp at a time, the 16-byte loads of NB
     // chunks per lane and row issued before any is used (NA: loads that do not
-    // allocate in L1).  A row is computed exactly as in near_leaf_kernel (same
+    // allocate in L1).  A row is computed exactly as in near_leaf_multi_kernel (same
     // chunks per lane, same order, same butterfly), so the leaf order and the
     // block shape do not change a bit of y.
     // Shared memory: 128 bytes of records, 2 x ld_max column ids, 2 x ld_max x.
@@ -526,6 +548,89 @@ namespace pibem
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
 
+    // near_leaf_ff_kernel for several columns: RC columns' x pairs in shared memory,
+    // a warp takes RR rows and RC columns at a time, so that the values (8 bytes each)
+    // are read once per RC columns.  Per (row, column) the chunks, order and butterfly
+    // of the one-column kernel, whose sums it therefore repeats bit for bit.
+    // What bounds it: the FP32 pipes (11 instructions per value and column).
+    template <int RC, int RR>
+    __global__ void __launch_bounds__(128)
+      near_leaf_ff_multi_kernel(int R, int N, const int64_t *__restrict__ nrow_ptr,
+                                const int64_t *__restrict__ ncol_ptr, const int64_t *__restrict__ nval_ptr,
+                                const int32_t *__restrict__ nrows, const int32_t *__restrict__ ncols,
+                                const float2 *__restrict__ vals, const float2 *__restrict__ x,
+                                double *__restrict__ y, bool acc)
+    {
+      extern __shared__ __align__(16) unsigned char smem_raw[];
+      float2       *sx   = reinterpret_cast<float2 *>(smem_raw); // [RC][ld]
+      const int     leaf = blockIdx.x, ra = blockIdx.y * RC, rc = min(RC, R - ra);
+      const int64_t c0   = ncol_ptr[leaf];
+      const int     nc = int(ncol_ptr[leaf + 1] - c0), ld = (nc + 3) / 4 * 4, n4 = ld / 4;
+      const int64_t r0 = nrow_ptr[leaf];
+      const int     nr = int(nrow_ptr[leaf + 1] - r0);
+      const float2 *V    = vals + nval_ptr[leaf];
+      const int     warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      for (int c = threadIdx.x; c < ld; c += blockDim.x)
+        {
+          const float2 *xc = x + ra * int64_t(N) + (c < nc ? ncols[c0 + c] : 0);
+#pragma unroll
+          for (int r = 0; r < RC; ++r)
+            sx[r * ld + c] = c < nc && r < rc ? xc[r * int64_t(N)] : make_float2(0.f, 0.f);
+        }
+      __syncthreads();
+      for (int row = warp * RR; row < nr; row += 4 * RR)
+        {
+          float h[RR][RC], l[RR][RC];
+#pragma unroll
+          for (int i = 0; i < RR; ++i)
+#pragma unroll
+            for (int r = 0; r < RC; ++r)
+              h[i][r] = l[i][r] = 0.f;
+          const float4 *v[RR];
+#pragma unroll
+          for (int i = 0; i < RR; ++i) // a row beyond the leaf's repeats the last one
+            v[i] = reinterpret_cast<const float4 *>(V + int64_t(min(row + i, nr - 1)) * ld);
+          for (int j = lane; j < n4; j += 32)
+            {
+              float4 a[RR][2];
+#pragma unroll
+              for (int i = 0; i < RR; ++i)
+                {
+                  a[i][0] = v[i][2 * j];
+                  a[i][1] = v[i][2 * j + 1];
+                }
+#pragma unroll
+              for (int r = 0; r < RC; ++r)
+                {
+                  const float4 *xr = reinterpret_cast<const float4 *>(sx + r * ld) + 2 * j;
+                  const float4  p = xr[0], q = xr[1];
+#pragma unroll
+                  for (int i = 0; i < RR; ++i)
+                    {
+                      ff_mac(h[i][r], l[i][r], make_float2(a[i][0].x, a[i][0].y), make_float2(p.x, p.y));
+                      ff_mac(h[i][r], l[i][r], make_float2(a[i][0].z, a[i][0].w), make_float2(p.z, p.w));
+                      ff_mac(h[i][r], l[i][r], make_float2(a[i][1].x, a[i][1].y), make_float2(q.x, q.y));
+                      ff_mac(h[i][r], l[i][r], make_float2(a[i][1].z, a[i][1].w), make_float2(q.z, q.w));
+                    }
+                }
+            }
+          float2 t[RR * RC];
+#pragma unroll
+          for (int i = 0; i < RR; ++i)
+#pragma unroll
+            for (int r = 0; r < RC; ++r)
+              t[i * RC + r] = ff_norm(h[i][r], l[i][r]);
+          const float2  u = warp_sums<RR * RC>(t, [](float2 p, float2 q) { return ff_add(p, q); });
+          constexpr int W = 32 / (RR * RC);
+          const int     i = row + lane / (W * RC), r = (lane / W) % RC;
+          if (lane % W == 0 && i < nr && r < rc)
+            {
+              double &o = y[(ra + r) * int64_t(N) + nrows[r0 + i]];
+              o         = acc ? __dadd_rn(o, ff_join(u)) : ff_join(u);
+            }
+        }
+    }
+
     // P2M apply: M^[leaf][r][k] = sum_rows w(row, r) T[row][k] x_r[dof(row)],
     // w selecting the double layer (Ker1), the single layer (Ker2) or the
     // combined system strengths.  One warp per leaf, 8 leaves per block: lane l
@@ -535,7 +640,8 @@ namespace pibem
     // COMBINED: every column uses the combined strengths, read from the table
     // Tc = (Dirichlet dof ? -T2 : T1) made at set_bc (one table row per row
     // instead of two); T1 is then Tc and T2 is unused.
-    // RC: columns per pass (1 for one right-hand side, else 4).
+    // RC: columns per block (1 for one right-hand side, else 4; the groups of columns
+    // over blockIdx.y: a few hundred leaves alone would leave most of the chip idle).
     template <typename T, bool COMBINED, int RC>
     __global__ void __launch_bounds__(256)
       p2m_apply_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ prow_ptr,
@@ -552,7 +658,7 @@ namespace pibem
       const int64_t box = pleaf_box[leaf];
       const int64_t rb = prow_ptr[leaf], re = prow_ptr[leaf + 1];
       const bool    act = 4 * lane < K4;
-      for (int rq = 0; rq < R; rq += RC)
+      const int rq = blockIdx.y * RC;
         {
           const int rc = min(RC, R - rq);
           T         acc[RC][4];
@@ -819,20 +925,19 @@ namespace pibem
       const int64_t RK = int64_t(R) * K;
       for (int i = threadIdx.x; i < R * K; i += blockDim.x)
         {
-          float2  acc = make_float2(0.0f, 0.0f);
-          int64_t e   = e0;
-          for (; e + 8 <= e1; e += 8)
+          float2 acc = make_float2(0.0f, 0.0f);
+          for (int64_t e = e0; e < e1; e += 8)
             {
               float2 v[8];
 #pragma unroll
               for (int u = 0; u < 8; ++u)
-                v[u] = Y[int64_t(q[e + u]) * RK + i];
+                if (e + u < e1)
+                  v[u] = Y[int64_t(q[e + u]) * RK + i];
 #pragma unroll
               for (int u = 0; u < 8; ++u)
-                acc = ff_add(acc, v[u]);
+                if (e + u < e1)
+                  acc = ff_add(acc, v[u]);
             }
-          for (; e < e1; ++e)
-            acc = ff_add(acc, Y[int64_t(q[e]) * RK + i]);
           out[b * RK + i] = acc;
         }
     }
@@ -863,33 +968,99 @@ namespace pibem
       const int64_t RK = int64_t(R) * K;
       for (int i = threadIdx.x; i < R * K; i += blockDim.x)
         {
-          T       acc = T(0);
-          int64_t e   = e0;
-          for (; e + 8 <= e1; e += 8)
+          T acc = T(0);
+          for (int64_t e = e0; e < e1; e += 8)
             {
               T v[8];
 #pragma unroll
               for (int u = 0; u < 8; ++u)
-                v[u] = Y[int64_t(q[e + u]) * RK + i];
+                if (e + u < e1)
+                  v[u] = Y[int64_t(q[e + u]) * RK + i];
 #pragma unroll
               for (int u = 0; u < 8; ++u)
-                acc += v[u];
+                if (e + u < e1)
+                  acc += v[u];
             }
-          for (; e < e1; ++e)
-            acc += Y[int64_t(q[e]) * RK + i];
           out[b * RK + i] = acc;
         }
     }
 
+    // Multipole values of nc <= NC columns (K apart) at the offset r in box units:
+    // sum_k coef[k] basis_k(r) with the table-driven recurrences, m-major.  The basis
+    // is formed once for the columns, two FMA per term and column; the order of the
+    // additions and the roundings of a column do not depend on NC.
+    template <int NC, typename T>
+    __device__ __forceinline__ void eval_multipole_cols(const T *__restrict__ coef, int K, int nc, int p,
+                                                        T rx, T ry, T rz, T (&acc)[NC])
+    {
+      using LT    = LegT<T>;
+      const T r2  = rx * rx + ry * ry + rz * rz;
+      const T rho = sqrt(r2);
+      const T inv = T(1) / rho;
+      const T x   = rz * inv;
+      const T s   = sqrt(fmax(T(0), T(1) - x * x));
+      const T rxy = sqrt(rx * rx + ry * ry);
+      T       cb = T(1), sb = T(0);
+      if (rxy > T(0))
+        {
+          cb = rx / rxy;
+          sb = ry / rxy;
+        }
+      T pmm = T(1), rpm = inv, cm = T(1), sm = T(0);
+#pragma unroll
+      for (int r = 0; r < NC; ++r)
+        acc[r] = T(0);
+      // term (n, m): the basis value q (Legendre times power of r) times (cos, sin) m
+      auto term = [&](int n, int m, T q) {
+        const int k0 = n * n + (m == 0 ? 0 : 2 * m - 1);
+        const T   a  = m == 0 ? q : mul_rn(T(2) * cm, q);
+        const T   b  = m == 0 ? T(0) : mul_rn(-T(2) * sm, q);
+#pragma unroll
+        for (int r = 0; r < NC; ++r)
+          if (r < nc)
+            {
+              acc[r] = fma_rn(coef[r * K + k0], a, acc[r]);
+              if (m > 0)
+                acc[r] = fma_rn(coef[r * K + k0 + 1], b, acc[r]);
+            }
+      };
+      for (int m = 0; m <= p; ++m)
+        {
+          if (m > 0)
+            {
+              pmm        = mul_rn(pmm, mul_rn(-LT::cmm(m), s));
+              rpm        = mul_rn(rpm, inv);
+              const T c2 = fma_rn(cm, cb, -mul_rn(sm, sb));
+              sm         = fma_rn(sm, cb, mul_rn(cm, sb));
+              cm         = c2;
+            }
+          T p0 = pmm, rp = rpm;
+          term(m, m, mul_rn(p0, rp));
+          if (m + 1 <= p)
+            {
+              T p1 = mul_rn(mul_rn(x, LT::cm1(m)), pmm);
+              rp   = mul_rn(rp, inv);
+              term(m + 1, m, mul_rn(p1, rp));
+              for (int n = m + 2; n <= p; ++n)
+                {
+                  const T p2 = fma_rn(mul_rn(LT::ra(n, m), x), p1, -mul_rn(LT::rb(n, m), p0));
+                  p0         = p1;
+                  p1         = p2;
+                  rp         = mul_rn(rp, inv);
+                  term(n, m, mul_rn(p1, rp));
+                }
+            }
+        }
+    }
+
     // M2P phase 1: one thread per (pair, collocation node of the pair's target
-    // box): scratch[r][item] = multipole of the source box evaluated at the
-    // node.  tnodes lists each target box's collocation nodes (tnode_ptr).
-    template <typename T>
+    // box) and NC columns: scratch[r][item] = multipole of the source box evaluated
+    // at the node.  tnodes lists each target box's collocation nodes (tnode_ptr).
+    template <typename T, int NC>
     __global__ void m2p_eval_kernel(int64_t n_items, int R, int K, int p,
                                     const int64_t *__restrict__ item_ptr,
                                     const int32_t *__restrict__ item_pair,
                                     const int32_t *__restrict__ pair_tgt,
-                                    const int32_t *__restrict__ tgt,
                                     const int32_t *__restrict__ src,
                                     const int64_t *__restrict__ tnode_ptr,
                                     const int32_t *__restrict__ tnodes,
@@ -923,18 +1094,23 @@ namespace pibem
           rz = (xyz[3 * int64_t(node) + 2] - center[3 * s + 2]) / h;
           ih = 1.0 / h;
         }
-      for (int r = 0; r < R; ++r)
-        scratch[int64_t(r) * n_items + it] =
-          eval_expansion_fast<T, T>(M + (s * R + r) * K, p, rx, ry, rz, true) * ih;
+      const int r0 = blockIdx.y * NC, nc = min(NC, R - r0);
+      T         v[NC];
+      eval_multipole_cols<NC>(M + (s * R + r0) * K, K, nc, p, rx, ry, rz, v);
+#pragma unroll
+      for (int r = 0; r < NC; ++r)
+        if (r < nc)
+          scratch[int64_t(r0 + r) * n_items + it] = v[r] * ih;
     }
 
-    // The table-driven evaluation of eval_expansion_fast (same recurrences, same
-    // order of terms) in float-float arithmetic for the FP64-accurate operator:
-    // r is the offset from the box centre in box units (pairs), coef the
-    // expansion as pairs.  About 90 FP32 instructions per term against the
-    // FP64 pipe's 1/58 rate.
-    __device__ float2 eval_multipole_ff(const float2 *__restrict__ coef, int p, float2 rx, float2 ry,
-                                        float2 rz)
+    // eval_multipole_cols in float-float arithmetic for the FP64-accurate operator: r
+    // is the offset from the box centre in box units (pairs), coef the expansions as
+    // pairs (K apart), the sums carried with TwoProduct / TwoSum (ff_mac): 22 FP32
+    // instructions per term and column and about 40 shared by the columns, against
+    // the FP64 pipe's 1/58 rate.
+    template <int NC>
+    __device__ __forceinline__ void eval_multipole_ff(const float2 *__restrict__ coef, int K, int nc, int p,
+                                                      float2 rx, float2 ry, float2 rz, float2 (&out)[NC])
     {
       const float2 rxy2 = ff_add(ff_mul(rx, rx), ff_mul(ry, ry));
       const float2 rho  = ff_sqrt(ff_add(rxy2, ff_mul(rz, rz)));
@@ -949,52 +1125,64 @@ namespace pibem
           cb              = ff_mul(rx, ir);
           sb              = ff_mul(ry, ir);
         }
-      const float2 step = inv;
-      float2       acc = make_float2(0.f, 0.f), pmm = make_float2(1.f, 0.f), rpm = inv;
-      float2       cm = make_float2(1.f, 0.f), sm = make_float2(0.f, 0.f);
+      float  h[NC], l[NC];
+      float2 pmm = make_float2(1.f, 0.f), rpm = inv;
+      float2 cm = make_float2(1.f, 0.f), sm = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int r = 0; r < NC; ++r)
+        h[r] = l[r] = 0.f;
+      // term (n, m): the basis value q (Legendre times power of r) times (cos, sin) m
+      auto term = [&](int n, int m, float2 q) {
+        const int k0 = n * n + (m == 0 ? 0 : 2 * m - 1);
+        // 2 cm and -2 sm: exact scalings
+        const float2 a = m == 0 ? q : ff_mul(make_float2(2.f * cm.x, 2.f * cm.y), q);
+        const float2 b = m == 0 ? q : ff_mul(make_float2(-2.f * sm.x, -2.f * sm.y), q);
+#pragma unroll
+        for (int r = 0; r < NC; ++r)
+          if (r < nc)
+            {
+              ff_mac(h[r], l[r], coef[r * K + k0], a);
+              if (m > 0)
+                ff_mac(h[r], l[r], coef[r * K + k0 + 1], b);
+            }
+      };
       for (int m = 0; m <= p; ++m)
         {
           if (m > 0)
             {
               pmm             = ff_mul(pmm, ff_mul(ff_neg(c_leg.ffcmm[m]), s));
-              rpm             = ff_mul(rpm, step);
+              rpm             = ff_mul(rpm, inv);
               const float2 c2 = ff_sub(ff_mul(cm, cb), ff_mul(sm, sb));
               sm              = ff_add(ff_mul(sm, cb), ff_mul(cm, sb));
               cm              = c2;
             }
-          // 2 cm and -2 sm: exact scalings
-          const float2 cr = m == 0 ? make_float2(1.f, 0.f) : make_float2(2.f * cm.x, 2.f * cm.y);
-          const float2 ci = m == 0 ? make_float2(0.f, 0.f) : make_float2(-2.f * sm.x, -2.f * sm.y);
-          auto term = [&](int n) {
-            const int    k0 = n * n + (m == 0 ? 0 : 2 * m - 1);
-            const float2 v  = m > 0 ? ff_add(ff_mul(coef[k0], cr), ff_mul(coef[k0 + 1], ci))
-                                    : ff_mul(coef[k0], cr);
-            return v;
-          };
           float2 p0 = pmm, rp = rpm;
-          acc       = ff_add(acc, ff_mul(ff_mul(term(m), p0), rp));
+          term(m, m, ff_mul(p0, rp));
           if (m + 1 <= p)
             {
               float2 p1 = ff_mul(ff_mul(x, c_leg.ffcm1[m]), pmm);
-              rp        = ff_mul(rp, step);
-              acc       = ff_add(acc, ff_mul(ff_mul(term(m + 1), p1), rp));
+              rp        = ff_mul(rp, inv);
+              term(m + 1, m, ff_mul(p1, rp));
               for (int n = m + 2; n <= p; ++n)
                 {
                   const float2 p2 = ff_sub(ff_mul(ff_mul(c_leg.ffra[n][m], x), p1),
                                            ff_mul(c_leg.ffrb[n][m], p0));
                   p0 = p1;
                   p1 = p2;
-                  rp = ff_mul(rp, step);
-                  acc = ff_add(acc, ff_mul(ff_mul(term(n), p1), rp));
+                  rp = ff_mul(rp, inv);
+                  term(n, m, ff_mul(p1, rp));
                 }
             }
         }
-      return acc;
+#pragma unroll
+      for (int r = 0; r < NC; ++r)
+        out[r] = ff_norm(h[r], l[r]);
     }
 
     // M2P phase 1 of the FP64-accurate operator: as m2p_eval_kernel, from the
     // (hi, lo) multipoles; the offset from the centre is formed in FP64 and
     // split, the scaling by 1 / h in float-float; the value stored in FP64.
+    template <int NC>
     __global__ void m2p_eval_ff_kernel(int64_t n_items, int R, int K, int p,
                                        const int64_t *__restrict__ item_ptr,
                                        const int32_t *__restrict__ item_pair,
@@ -1017,20 +1205,24 @@ namespace pibem
       const float2  rx   = ff_mul(ff_split(__dsub_rn(xyz[3 * int64_t(node)], center[3 * s])), ih);
       const float2  ry   = ff_mul(ff_split(__dsub_rn(xyz[3 * int64_t(node) + 1], center[3 * s + 1])), ih);
       const float2  rz   = ff_mul(ff_split(__dsub_rn(xyz[3 * int64_t(node) + 2], center[3 * s + 2])), ih);
-      for (int r = 0; r < R; ++r)
-        scratch[int64_t(r) * n_items + it] =
-          ff_join(ff_mul(eval_multipole_ff(M + (s * R + r) * K, p, rx, ry, rz), ih));
+      const int     r0 = blockIdx.y * NC, nc = min(NC, R - r0);
+      float2        v[NC];
+      eval_multipole_ff<NC>(M + (s * R + r0) * K, K, nc, p, rx, ry, rz, v);
+#pragma unroll
+      for (int r = 0; r < NC; ++r)
+        if (r < nc)
+          scratch[int64_t(r0 + r) * n_items + it] = ff_join(ff_mul(v[r], ih));
     }
 
-    // M2P phase 2: one warp per target box, one lane per node of the box: the
-    // node's values over the box's sources, added in list order to y.  The
+    // M2P phase 2: one warp per target box and column (blockIdx.y), one lane per node
+    // of the box: the node's values over the box's sources, added in list order to y.  The
     // items of a target box are contiguous, source-major (item_ptr[e] =
     // item_ptr[e0] + (e - e0) nn), so a node's values sit nn apart; 16 loads
-    // in flight.
+    // in flight, the last group's too.
     template <typename T>
     __global__ void __launch_bounds__(256)
-      m2p_sum_kernel(int n_tgt, int R, int N, int64_t n_items, const int64_t *__restrict__ tnode_ptr,
-                     const int32_t *__restrict__ tgt, const int64_t *__restrict__ src_ptr,
+      m2p_sum_kernel(int n_tgt, int N, int64_t n_items, const int64_t *__restrict__ tnode_ptr,
+                     const int64_t *__restrict__ src_ptr,
                      const int64_t *__restrict__ item_ptr, const int32_t *__restrict__ tnodes,
                      const T *__restrict__ scratch, T *__restrict__ y)
     {
@@ -1042,37 +1234,42 @@ namespace pibem
       const int64_t  e0 = src_ptr[ti], ns = src_ptr[ti + 1] - e0;
       const int64_t  base = e0 < src_ptr[n_tgt] ? item_ptr[e0] : 0;
       const int32_t *nodes = tnodes + tnode_ptr[ti];
+      const int64_t  r     = blockIdx.y;
       for (int64_t i = lane; i < nn; i += 32)
         {
           const int node = nodes[i];
-          for (int r = 0; r < R; ++r)
+          const T  *sc   = scratch + r * n_items + base + i;
+          T         acc  = T(0), v[16];
+          int64_t   j    = 0;
+          for (; j + 16 <= ns; j += 16)
             {
-              const T *sc  = scratch + int64_t(r) * n_items + base + i;
-              T        acc = T(0);
-              int64_t  j   = 0;
-              for (; j + 16 <= ns; j += 16)
-                {
-                  T v[16];
 #pragma unroll
-                  for (int u = 0; u < 16; ++u)
-                    v[u] = sc[(j + u) * nn];
+              for (int u = 0; u < 16; ++u)
+                v[u] = sc[(j + u) * nn];
 #pragma unroll
-                  for (int u = 0; u < 16; ++u)
-                    acc += v[u];
-                }
-              for (; j < ns; ++j)
-                acc += sc[j * nn];
-              y[int64_t(r) * N + node] += acc;
+              for (int u = 0; u < 16; ++u)
+                acc += v[u];
             }
+#pragma unroll
+          for (int u = 0; u < 15; ++u)
+            if (j + u < ns)
+              v[u] = sc[(j + u) * nn];
+#pragma unroll
+          for (int u = 0; u < 15; ++u)
+            if (j + u < ns)
+              acc += v[u];
+          y[r * N + node] += acc;
         }
     }
 
     // L2P: y[r][node] += W[row] . L^[leaf][r] for every row (node of a
-    // childless box).  One warp per leaf, 8 leaves per block: lane l multiplies
-    // coefficients 4l..4l+3 (W rows padded to K4 values), eight rows in flight;
-    // the lanes' products are added by a fixed butterfly, and lane u updates
-    // the node of row u of each group of eight.
-    template <typename T>
+    // childless box).  One warp per leaf and RC columns (blockIdx.y): lane l
+    // multiplies coefficients 4l..4l+3 (W rows padded to K4 values) of RR rows and
+    // the columns; the lanes' products are added by warp_sum's butterfly.  A (row,
+    // column) value has the same roundings for every RC and RR.
+    // One column: 8 rows (16-byte loads) in flight.  Several: a row of W is read once
+    // for RC columns.
+    template <typename T, int RC, int RR>
     __global__ void __launch_bounds__(256)
       l2p_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ row_ptr,
                  const int32_t *__restrict__ lleaf_box, const int32_t *__restrict__ nrows,
@@ -1084,39 +1281,54 @@ namespace pibem
         return;
       const int     K4  = (K + 3) / 4 * 4;
       const int64_t box = lleaf_box[leaf];
-      const int64_t r0 = row_ptr[leaf], r1 = row_ptr[leaf + 1];
+      const int64_t i0 = row_ptr[leaf], i1 = row_ptr[leaf + 1];
+      const int     ra = blockIdx.y * RC, rc = min(RC, R - ra);
       const bool    act = 4 * lane < K4;
-      for (int r = 0; r < R; ++r)
+      T             l[RC][4];
+#pragma unroll
+      for (int r = 0; r < RC; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          l[r][c] = r < rc && 4 * lane + c < K ? Lx[(box * R + ra + r) * K + 4 * lane + c] : T(0);
+      for (int64_t i = i0; i < i1; i += RR)
         {
-          T l[4] = {T(0), T(0), T(0), T(0)};
-          if (act)
-            {
-              const T *lp = Lx + (box * R + r) * K;
+          T w[RR][4];
 #pragma unroll
-              for (int c = 0; c < 4; ++c)
-                if (4 * lane + c < K)
-                  l[c] = lp[4 * lane + c];
-            }
-          for (int64_t i0 = r0; i0 < r1; i0 += 8)
+          for (int u = 0; u < RR; ++u)
+            if (act && i + u < i1)
+              load4(W + (i + u) * K4 + 4 * lane, w[u]);
+            else
+              w[u][0] = w[u][1] = w[u][2] = w[u][3] = T(0);
+          auto dot = [&](int u, int r) {
+            return fma_rn(w[u][0], l[r][0], mul_rn(w[u][1], l[r][1])) +
+                   fma_rn(w[u][2], l[r][2], mul_rn(w[u][3], l[r][3]));
+          };
+          if constexpr (RC == 1)
             {
-              T w[8][4];
-#pragma unroll
-              for (int u = 0; u < 8; ++u)
-                if (act && i0 + u < r1)
-                  load4(W + (i0 + u) * K4 + 4 * lane, w[u]);
-                else
-                  w[u][0] = w[u][1] = w[u][2] = w[u][3] = T(0);
               T mine = T(0);
 #pragma unroll
-              for (int u = 0; u < 8; ++u)
+              for (int u = 0; u < RR; ++u)
                 {
-                  T s = (w[u][0] * l[0] + w[u][1] * l[1]) + (w[u][2] * l[2] + w[u][3] * l[3]);
-                  s   = warp_sum(s);
+                  const T t = warp_sum(dot(u, 0));
                   if (lane == u)
-                    mine = s;
+                    mine = t;
                 }
-              if (lane < 8 && i0 + lane < r1)
-                y[int64_t(r) * N + nrows[i0 + lane]] += mine;
+              if (lane < RR && i + lane < i1)
+                y[int64_t(ra) * N + nrows[i + lane]] += mine;
+            }
+          else
+            {
+              T v[RR * RC];
+#pragma unroll
+              for (int u = 0; u < RR; ++u)
+#pragma unroll
+                for (int r = 0; r < RC; ++r)
+                  v[u * RC + r] = dot(u, r);
+              const T       t  = warp_sums<RR * RC>(v, [](T p, T q) { return p + q; });
+              constexpr int Wn = 32 / (RR * RC); // lanes per value
+              const int     u = lane / (Wn * RC), r = (lane / Wn) % RC;
+              if (lane % Wn == 0 && i + u < i1 && r < rc)
+                y[int64_t(ra + r) * N + nrows[i + u]] += t;
             }
         }
     }
@@ -1138,7 +1350,7 @@ namespace pibem
       const int64_t box = lleaf_box[leaf];
       const int64_t r0 = row_ptr[leaf], r1 = row_ptr[leaf + 1];
       const bool    act = 4 * lane < K4;
-      for (int r = 0; r < R; ++r)
+      const int r = blockIdx.y;
         {
           float2 l[4];
 #pragma unroll
@@ -1192,8 +1404,6 @@ namespace pibem
         }
     }
 
-    inline int tpb_for(int RK) { return RK >= 256 ? 256 : (RK >= 128 ? 128 : 64); }
-
     int near_sm_count()
     {
       int dev = 0, n_sm = 1;
@@ -1209,7 +1419,7 @@ namespace pibem
   {
     if (op.n_rows == 0 || op.n_near_leaves == 0)
       return;
-    l2p_ff_kernel<<<unsigned((op.n_near_leaves + 7) / 8), 256, 0, s>>>(
+    l2p_ff_kernel<<<dim3(unsigned((op.n_near_leaves + 7) / 8), unsigned(R)), 256, 0, s>>>(
       op.n_near_leaves, R, op.K, N, op.nrow_ptr, op.lleaf_box, op.nrows, op.Wff, Lff, y);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
@@ -1222,9 +1432,6 @@ namespace pibem
     if (op.n_near_leaves == 0)
       return;
     const int64_t maxnc = (std::max<int64_t>(op.max_near_cols, 1) + 3) / 4 * 4;
-    int           rb    = int(std::max<int64_t>(1, (96 * 1024) / (maxnc * int64_t(sizeof(T)))));
-    rb                  = std::min(rb, R);
-    const size_t smem   = size_t(rb) * maxnc * sizeof(T);
     const size_t smem_s = 128 + size_t(2) * maxnc * (4 + sizeof(T));
     if (R == 1 && op.near_sched && smem_s <= 227 * 1024)
       {
@@ -1266,11 +1473,27 @@ namespace pibem
         note_launch();
         return;
       }
-    auto kern = near_leaf_kernel<T, false>;
-    if (smem > 48 * 1024)
-      raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
-    launch_pdl(kern, op.n_near_leaves, 256, smem, s, R, rb, N, op.nrow_ptr, op.ncol_ptr, op.nval_ptr,
-                                             op.nrows, op.ncols, vals, x, y, accumulate);
+    // several columns: up to 96 KB of x at a time, a multiple of the columns a warp
+    // takes (two for two right-hand sides, else four)
+    auto launch = [&](auto kern, int rcw) {
+      const int64_t fit = (96 * 1024) / (maxnc * int64_t(sizeof(T)) * rcw) * rcw;
+      const int     rb  = int(std::min<int64_t>(std::max<int64_t>(fit, rcw), (R + rcw - 1) / rcw * rcw));
+      const size_t  smem = size_t(rb) * maxnc * sizeof(T);
+      if (smem > 48 * 1024)
+        raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
+      launch_pdl(kern, op.n_near_leaves, 128, smem, s, R, rb, N, op.nrow_ptr, op.ncol_ptr, op.nval_ptr,
+                 op.nrows, op.ncols, vals, x, y, accumulate);
+    };
+    constexpr int RR4 = sizeof(T) == 4 ? 4 : 2;
+    if (R == 2 || 4 * maxnc * int64_t(sizeof(T)) > 200 * 1024)
+      {
+        if (2 * maxnc * int64_t(sizeof(T)) > 200 * 1024) // one column's x for very wide leaves
+          launch(near_leaf_multi_kernel<T, 1, 4>, 1);
+        else
+          launch(near_leaf_multi_kernel<T, 2, 4>, 2);
+      }
+    else
+      launch(near_leaf_multi_kernel<T, 4, RR4>, 4);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
@@ -1290,16 +1513,28 @@ namespace pibem
     const size_t smem1 = size_t(2) * maxnc * sizeof(float2);
     if (smem1 > 48 * 1024)
       raise_smem_limit(reinterpret_cast<const void *>(near_leaf_ff_kernel), smem1);
-    // one launch per column: a column's result does not depend on R
-    for (int r = 0; r < R; ++r)
+    if (R == 1)
+      near_leaf_ff_kernel<<<std::min(op.n_near_leaves, NEAR_BLOCKS_PER_SM_WIDE * near_sm_count()), 256,
+                            smem1, s>>>(op.n_near_leaves, int(maxnc), op.nrow_ptr, op.ncol_ptr,
+                                        op.nval_ptr, op.nrows, op.ncols, vals, xff, y, accumulate);
+    else
       {
-        near_leaf_ff_kernel<<<std::min(op.n_near_leaves, NEAR_BLOCKS_PER_SM_WIDE * near_sm_count()),
-                              256, smem1, s>>>(
-          op.n_near_leaves, int(maxnc), op.nrow_ptr, op.ncol_ptr, op.nval_ptr, op.nrows, op.ncols, vals,
-          xff + int64_t(r) * N, y + int64_t(r) * N, accumulate);
-        PIBEM_CUDA(cudaGetLastError());
-        note_launch();
+        // two columns at a time for two and for leaves whose four columns would not
+        // leave two blocks per SM, else four
+        auto launch = [&](auto kern, int rc) {
+          const size_t smem = size_t(rc) * maxnc * sizeof(float2);
+          if (smem > 48 * 1024)
+            raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
+          kern<<<dim3(op.n_near_leaves, (R + rc - 1) / rc), 128, smem, s>>>(
+            R, N, op.nrow_ptr, op.ncol_ptr, op.nval_ptr, op.nrows, op.ncols, vals, xff, y, accumulate);
+        };
+        if (R == 2 || 4 * maxnc * sizeof(float2) > 100 * 1024)
+          launch(near_leaf_ff_multi_kernel<2, 2>, 2);
+        else
+          launch(near_leaf_ff_multi_kernel<4, 2>, 4);
       }
+    PIBEM_CUDA(cudaGetLastError());
+    note_launch();
   }
 
   template <typename T>
@@ -1308,8 +1543,8 @@ namespace pibem
   {
     if (op.n_p2m_leaves == 0)
       return;
-    const unsigned grid = unsigned((op.n_p2m_leaves + 7) / 8);
-    const bool     comb = combined && op.Tc;
+    const dim3 grid(unsigned((op.n_p2m_leaves + 7) / 8), unsigned(R == 1 ? 1 : (R + 3) / 4));
+    const bool comb = combined && op.Tc;
     auto launch = [&](auto kern) {
       launch_pdl(kern, grid, 256, 0, s, op.n_p2m_leaves, R, op.K, N, op.prow_ptr, op.pleaf_box, op.prow_dof,
                                 comb ? op.Tc : op.T1, op.T2, dir, modes, x, M);
@@ -1541,15 +1776,23 @@ namespace pibem
   {
     if (op.n_m2p_tgt == 0)
       return;
-    launch_pdl(m2p_eval_kernel<T>, unsigned((op.n_m2p_items + 127) / 128), 128, 0, s, 
-      op.n_m2p_items, R, op.K, op.p, op.m2p_item_ptr, op.m2p_item_pair, op.m2p_pair_tgt,
-      op.m2p_tgt, op.m2p_src, op.m2p_tnode_ptr, op.m2p_tnodes, td.xyz, td.center, td.delta, M,
-      op.m2p_scratch);
+    auto eval = [&](auto kern, int nc) {
+      launch_pdl(kern, dim3(unsigned((op.n_m2p_items + 127) / 128), unsigned((R + nc - 1) / nc)), 128, 0, s,
+                 op.n_m2p_items, R, op.K, op.p, op.m2p_item_ptr, op.m2p_item_pair, op.m2p_pair_tgt,
+                 op.m2p_src, op.m2p_tnode_ptr, op.m2p_tnodes, td.xyz, td.center, td.delta, M,
+                 op.m2p_scratch);
+    };
+    if (R == 1)
+      eval(m2p_eval_kernel<T, 1>, 1);
+    else if (R <= 4)
+      eval(m2p_eval_kernel<T, 4>, 4);
+    else
+      eval(m2p_eval_kernel<T, 8>, 8);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
-    launch_pdl(m2p_sum_kernel<T>, unsigned((op.n_m2p_tgt + 7) / 8), 256, 0, s, 
-      op.n_m2p_tgt, R, N, op.n_m2p_items, op.m2p_tnode_ptr, op.m2p_tgt, op.m2p_src_ptr,
-      op.m2p_item_ptr, op.m2p_tnodes, op.m2p_scratch, y);
+    launch_pdl(m2p_sum_kernel<T>, dim3(unsigned((op.n_m2p_tgt + 7) / 8), unsigned(R)), 256, 0, s, 
+      op.n_m2p_tgt, N, op.n_m2p_items, op.m2p_tnode_ptr, op.m2p_src_ptr, op.m2p_item_ptr,
+      op.m2p_tnodes, op.m2p_scratch, y);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
@@ -1559,14 +1802,20 @@ namespace pibem
   {
     if (op.n_m2p_tgt == 0)
       return;
-    m2p_eval_ff_kernel<<<unsigned((op.n_m2p_items + 127) / 128), 128, 0, s>>>(
-      op.n_m2p_items, R, op.K, op.p, op.m2p_item_ptr, op.m2p_item_pair, op.m2p_pair_tgt, op.m2p_src,
-      op.m2p_tnode_ptr, op.m2p_tnodes, td.xyz, td.center, td.delta, Mff, op.m2p_scratch);
+    auto eval = [&](auto kern, int nc) {
+      kern<<<dim3(unsigned((op.n_m2p_items + 127) / 128), unsigned((R + nc - 1) / nc)), 128, 0, s>>>(
+        op.n_m2p_items, R, op.K, op.p, op.m2p_item_ptr, op.m2p_item_pair, op.m2p_pair_tgt, op.m2p_src,
+        op.m2p_tnode_ptr, op.m2p_tnodes, td.xyz, td.center, td.delta, Mff, op.m2p_scratch);
+    };
+    if (R == 1)
+      eval(m2p_eval_ff_kernel<1>, 1);
+    else
+      eval(m2p_eval_ff_kernel<4>, 4);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
-    m2p_sum_kernel<double><<<unsigned((op.n_m2p_tgt + 7) / 8), 256, 0, s>>>(
-      op.n_m2p_tgt, R, N, op.n_m2p_items, op.m2p_tnode_ptr, op.m2p_tgt, op.m2p_src_ptr,
-      op.m2p_item_ptr, op.m2p_tnodes, op.m2p_scratch, y);
+    m2p_sum_kernel<double><<<dim3(unsigned((op.n_m2p_tgt + 7) / 8), unsigned(R)), 256, 0, s>>>(
+      op.n_m2p_tgt, N, op.n_m2p_items, op.m2p_tnode_ptr, op.m2p_src_ptr, op.m2p_item_ptr,
+      op.m2p_tnodes, op.m2p_scratch, y);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
@@ -1590,8 +1839,14 @@ namespace pibem
   {
     if (op.n_rows == 0 || op.n_near_leaves == 0)
       return;
-    launch_pdl(l2p_kernel<T>, unsigned((op.n_near_leaves + 7) / 8), 256, 0, s, 
-      op.n_near_leaves, R, op.K, N, op.nrow_ptr, op.lleaf_box, op.nrows, op.W, Lx, y);
+    auto launch = [&](auto kern, int rc) {
+      launch_pdl(kern, dim3(unsigned((op.n_near_leaves + 7) / 8), unsigned((R + rc - 1) / rc)), 256, 0, s,
+                 op.n_near_leaves, R, op.K, N, op.nrow_ptr, op.lleaf_box, op.nrows, op.W, Lx, y);
+    };
+    if (R == 1)
+      launch(l2p_kernel<T, 1, 8>, 1);
+    else
+      launch(l2p_kernel<T, 4, 4>, 4);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }

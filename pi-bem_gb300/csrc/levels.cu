@@ -259,29 +259,22 @@ namespace pibem
         {
           const float4 *y      = reinterpret_cast<const float4 *>(Y) + (int64_t(e0) * R + r) * n4 + lane;
           const int64_t stride = int64_t(R) * n4;
-          int           e      = e0;
-          for (; e + 16 <= e1; e += 16)
+          for (int e = e0; e < e1; e += 16, y += 16 * stride)
             {
               float4 v[16];
 #pragma unroll
               for (int u = 0; u < 16; ++u)
-                v[u] = __ldg(y + int64_t(e - e0 + u) * stride);
+                if (e + u < e1)
+                  v[u] = __ldg(y + u * stride);
 #pragma unroll
               for (int u = 0; u < 16; ++u)
-                {
-                  s.x += v[u].x;
-                  s.y += v[u].y;
-                  s.z += v[u].z;
-                  s.w += v[u].w;
-                }
-            }
-          for (; e < e1; ++e)
-            {
-              const float4 v = __ldg(y + int64_t(e - e0) * stride);
-              s.x += v.x;
-              s.y += v.y;
-              s.z += v.z;
-              s.w += v.w;
+                if (e + u < e1)
+                  {
+                    s.x += v[u].x;
+                    s.y += v[u].y;
+                    s.z += v[u].z;
+                    s.w += v[u].w;
+                  }
             }
           float *o = Lx + (int64_t(box[bi]) * R + r) * K + 4 * lane;
           const float sv[4] = {s.x, s.y, s.z, s.w};
