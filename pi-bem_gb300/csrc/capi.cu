@@ -219,6 +219,13 @@ struct pibem_handle
   DBuf<double>  d_xyz, d_qpts, d_qnrm, d_qjxw, d_qshape, d_gpts, d_gw;
   DBuf<int32_t> d_cells, d_dbl_off, d_dbl_ids, d_elem_off, d_elem_ids;
   DBuf<double>  d_proj; // L2-projection work (grow-only)
+  // row layout of the projections' mass matrix, made by the first one on a mesh
+  DBuf<int64_t>  d_proj_slices;
+  DBuf<int32_t>  d_proj_long;
+  int64_t        proj_slots  = 0; // 0: not made
+  int            proj_n_long = 0;
+  PinnedBuf<int> proj_flags;
+  cudaEvent_t    ev_proj[2] = {};
   // tree
   DBuf<int32_t> d_parent, d_child_first, d_nchild, d_digit, d_nbeg, d_nend, d_node_sorted;
   DBuf<double>  d_center, d_delta;
@@ -326,7 +333,7 @@ struct pibem_handle
     size_t t = 0;
     auto   add = [&t](const auto &...b) { ((t += b.bytes()), ...); };
     add(d_xyz, d_qpts, d_qnrm, d_qjxw, d_qshape, d_gpts, d_gw, d_cells, d_dbl_off, d_dbl_ids,
-        d_elem_off, d_elem_ids, d_proj);
+        d_elem_off, d_elem_ids, d_proj, d_proj_slices, d_proj_long);
     add(d_parent, d_child_first, d_nchild, d_digit, d_nbeg, d_nend, d_node_sorted, d_center,
         d_delta);
     add(d_nrow_ptr, d_ncol_ptr, d_nval_ptr, d_nent_ptr, d_prow_ptr, d_pcontrib_ptr, d_m2l_src_ptr,
@@ -2141,6 +2148,7 @@ namespace
     std::fill(h->setup_phase, h->setup_phase + PIBEM_SETUP_PHASES, 0.0);
     drop_graph(h); // its kernels carry the previous mesh's sizes
     h->d_con_nrm.release();
+    h->proj_slots = 0;
     if (n_nodes <= 0 || n_cells <= 0 || !xyz || !cells)
       throw Error(PIBEM_EINVAL, "empty mesh");
     if ((doff == nullptr) != (dids == nullptr))
@@ -2705,8 +2713,29 @@ namespace
                       double *dout)
   {
     const int64_t N = h->N();
-    h->d_proj.alloc(l2_projection_work(N, h->mesh.n_cells_body, R));
+    if (!h->proj_slots)
+      {
+        std::vector<int64_t> slices;
+        std::vector<int32_t> long_rows;
+        proj_row_layout(N, h->mesh.elem_off, slices, long_rows);
+        h->d_proj_slices.upload(slices, h->stream);
+        h->d_proj_long.upload(long_rows, h->stream);
+        PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+        h->proj_slots  = slices.back();
+        h->proj_n_long = int(long_rows.size());
+        for (auto &e : h->ev_proj)
+          if (!e)
+            PIBEM_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      }
+    h->proj_flags.alloc(size_t(6) * R);
+    h->d_proj.alloc(l2_projection_work(N, h->mesh.n_cells_body, R, h->proj_slots));
     ProjectionArgs a;
+    a.slice_ptr = h->d_proj_slices.p;
+    a.n_slots   = h->proj_slots;
+    a.long_rows = h->d_proj_long.p;
+    a.n_long    = h->proj_n_long;
+    a.flags     = h->proj_flags.p;
+    std::copy(h->ev_proj, h->ev_proj + 2, a.looked);
     a.mode     = mode;
     a.n_nodes  = N;
     a.n_cells  = h->mesh.n_cells_body; // a double body's reflected cells come after these
@@ -2906,7 +2935,7 @@ extern "C"
     for (auto &e : h->ev)
       if (e)
         cudaEventDestroy(e);
-    for (cudaEvent_t e : {h->ev_fork, h->ev_up, h->ev_side, h->ev_main})
+    for (cudaEvent_t e : {h->ev_fork, h->ev_up, h->ev_side, h->ev_main, h->ev_proj[0], h->ev_proj[1]})
       if (e)
         cudaEventDestroy(e);
     for (cudaStream_t st : {h->side, h->main_hp})

@@ -245,14 +245,23 @@ namespace pibem
     const int32_t *cells = nullptr, *elem_off = nullptr, *elem_ids = nullptr;
     const double  *xyz = nullptr, *gpts = nullptr, *qshape = nullptr, *qjxw = nullptr,
                   *qnrm = nullptr, *u = nullptr, *dudn = nullptr;
+    // rows of the mass matrix in slices of 32 nodes (proj_row_layout): slice starts,
+    // their total, and the nodes of many cells
+    const int64_t *slice_ptr = nullptr;
+    int64_t        n_slots   = 0;
+    const int32_t *long_rows = nullptr;
+    int            n_long    = 0;
     double        *work = nullptr; // l2_projection_work() doubles
     double        *out  = nullptr; // R x N x 3, node-major
     int            max_iterations = 1000;
     double         tolerance      = 1e-13;
-    int           *iterations     = nullptr;
+    int           *flags          = nullptr; // 2 x 3 R page-locked ints
+    cudaEvent_t    looked[2]      = {};
   };
+  void   proj_row_layout(int64_t N, const std::vector<int32_t> &elem_off,
+                         std::vector<int64_t> &slice_ptr, std::vector<int32_t> &long_rows);
   void   l2_projection(const ProjectionArgs &a, cudaStream_t s);
-  size_t l2_projection_work(int64_t n_nodes, int64_t n_cells, int R);
+  size_t l2_projection_work(int64_t n_nodes, int64_t n_cells, int R, int64_t n_slots);
 
   // ---- vector kernels (krylov.cu) -------------------------------------------
   void launch_convert_d2f(int64_t n, const double *a, float *b, cudaStream_t s);

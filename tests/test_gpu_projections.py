@@ -38,3 +38,18 @@ def test_projections_match_oracle(name, pibem_mod, synthetic):
     np.testing.assert_array_equal(g.gradients(u[1], dn[1]), gr[1])
     np.testing.assert_array_equal(g.surface_gradients(u[0]), sg[0])
     g.close()
+
+
+@pytest.mark.parametrize("shape", ["spheroid_115", "wigley_fan"])
+def test_projection_row_shapes(shape, pibem_mod, synthetic):
+    """More rows than one pass of the grid takes, and a bow and stern node with more cells than a
+    thread's row holds (a warp per such row): the same 1e-10."""
+    mesh = synthetic.spheroid(115) if shape == "spheroid_115" else synthetic.wigley_hull(21, 5, 33)
+    g = pibem_mod.BEMSolver(fma_truncation_order=3, max_nodes_per_childless_block=60)
+    g.set_mesh(mesh.xyz, mesh.cells)
+    u = np.cos(mesh.xyz @ np.array([1.0, -0.5, 2.0]))
+    assert rel(g.normals(), P.project(mesh.xyz, mesh.cells, "normals")) < 1e-10
+    gr = g.gradients(np.stack([u, 2.0 * u, u]), np.stack([u, u, u]))
+    assert rel(gr[2], P.project(mesh.xyz, mesh.cells, "gradients", u, u)) < 1e-10
+    np.testing.assert_array_equal(gr[0], gr[2])
+    g.close()
