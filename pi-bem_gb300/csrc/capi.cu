@@ -257,11 +257,10 @@ struct pibem_handle
   // order (values: L below the diagonal, unit diagonal implied; U from it),
   // the position of each row's diagonal, and the rows by level of the lower
   // and of the upper triangle (the rows of a level depend on earlier levels
-  // only); level bounds on the host
+  // only)
   DBuf<int64_t> d_ilu_ptr, d_ilu_diag;
   DBuf<int32_t> d_ilu_col, d_ilu_rows_lo, d_ilu_rows_up;
-  DBuf<double>  d_ilu_val;
-  std::vector<int64_t> ilu_lptr_lo, ilu_lptr_up;
+  DBuf<double>  d_ilu_val, d_ilu_y; // d_ilu_y: work of the substitutions
   bool          ilu_on = false;
   bool          use_tc = true;
   std::vector<int64_t> blk_ptr;
@@ -345,7 +344,7 @@ struct pibem_handle
         d_up_box, d_down_box, d_up_q, d_down_q, d_up_child8, d_down_par,
         d_m2p_item_pair, d_m2l_yslot, d_down_m2l_beg, d_down_m2l_end, d_m2p_tnodes);
     add(d_con_row, d_con_col, d_con_p, d_con_q, d_con_kind, d_con_nrm, d_con_sg);
-    add(d_ilu_ptr, d_ilu_diag, d_ilu_col, d_ilu_rows_lo, d_ilu_rows_up, d_ilu_val);
+    add(d_ilu_ptr, d_ilu_diag, d_ilu_col, d_ilu_rows_lo, d_ilu_rows_up, d_ilu_val, d_ilu_y);
     add(d_Sff, d_Srff, d_xff, d_Wff, d_Tcr);
     add(d_entries, d_N, d_D, d_S, d_T1, d_T2, d_W, d_ops, d_Pinv, d_Pinv64, d_Tc, d_Tcf, d_S32, d_T1f, d_T2f, d_Wf,
         d_opsf, d_opsff, d_tcimg, d_lvopsf, d_err, d_dir, d_modes, d_modes32, d_alpha);
@@ -916,6 +915,13 @@ namespace
     return bp;
   }
 
+  void ilu_apply(pibem_handle *h, int R, double *z, const int *sel, const int *jvec, cudaStream_t s)
+  {
+    h->d_ilu_y.alloc(size_t(R) * h->N()); // sized by engine_open inside a capture
+    launch_ilu_apply(h->N(), R, h->d_ilu_rows_lo.p, h->d_ilu_rows_up.p, h->d_ilu_ptr.p, h->d_ilu_col.p,
+                     h->d_ilu_val.p, h->d_ilu_diag.p, z, h->d_ilu_y.p, sel, jvec, h->d_err.p, s);
+  }
+
   // z = P^-1 v for R columns (v column stride ldv).  Leaf-block Jacobi: the
   // FP64 inverses where the handle keeps them (GMRES on an FP64-accurate
   // operator), else the FP32 ones.  ILU(0): z = v, then the level-scheduled
@@ -927,9 +933,7 @@ namespace
     if (h->ilu_on)
       {
         launch_copy_sel(N, R, v, ldv, z, sel, s);
-        launch_ilu_apply(h->ilu_lptr_lo, h->d_ilu_rows_lo.p, h->ilu_lptr_up, h->d_ilu_rows_up.p, R, N,
-                         h->d_ilu_ptr.p, h->d_ilu_col.p, h->d_ilu_val.p, h->d_ilu_diag.p, z, sel,
-                         nullptr, s);
+        ilu_apply(h, R, z, sel, nullptr, s);
       }
     else if (h->d_Pinv64.p)
       launch_block_apply(block_prec(h, h->d_Pinv64.p), R, N, v, ldv, z, sel, s);
@@ -986,6 +990,8 @@ namespace
     for (DBuf<int> *v : {&E.jcur, &E.kdone, &E.jvec, &E.its, &E.maxit, &E.sel})
       v->alloc(S);
     E.act.alloc(2 * S);
+    if (h->ilu_on)
+      h->d_ilu_y.alloc(size_t(S) * N);
     std::vector<int> minus(S, -1);
     E.jvec.upload(minus, h->stream);
     E.ctl.alloc(4);
@@ -1160,9 +1166,7 @@ namespace
     if (h->ilu_on)
       {
         launch_arnoldi_finish(a, BlockPrec<double>(), E.z.p, true, s);
-        launch_ilu_apply(h->ilu_lptr_lo, h->d_ilu_rows_lo.p, h->ilu_lptr_up, h->d_ilu_rows_up.p, E.S, N,
-                         h->d_ilu_ptr.p, h->d_ilu_col.p, h->d_ilu_val.p, h->d_ilu_diag.p, E.z.p,
-                         nullptr, E.jcur.p, s);
+        ilu_apply(h, E.S, E.z.p, nullptr, E.jcur.p, s);
         eng_gather(h, Ra);
       }
     else if (direct)
@@ -1243,10 +1247,10 @@ namespace
                          h->d_m2p64.p, h->d_t4.p, h->d_Mff.p, h->d_Lff.p, h->d_xff.p,
                          h->d_ozslc.p, h->d_modes.p, h->d_modes32.p, h->sh_part.p,
                          h->d_ilu_val.p, h->d_ilu_col.p, h->d_ilu_ptr.p, h->d_ilu_diag.p,
-                         h->d_ilu_rows_lo.p, h->d_ilu_rows_up.p};
+                         h->d_ilu_rows_lo.p, h->d_ilu_rows_up.p, h->d_ilu_y.p};
       return b[i];
     };
-    constexpr int             nb = 44;
+    constexpr int             nb = 45;
     std::array<uintptr_t, 48> key{};
     key[0] = uintptr_t(Ra) | (uintptr_t(E.S) << 16) | (uintptr_t(E.m) << 32) |
              (uintptr_t(E.prec) << 48) | (uintptr_t(E.mixed) << 49) | (uintptr_t(h->ilu_on) << 50);
@@ -1867,8 +1871,9 @@ namespace
         rows[at[lev[i]]++] = int32_t(i);
     };
     std::vector<int32_t> rows_lo, rows_up;
-    group(lev_lo, h->ilu_lptr_lo, rows_lo);
-    group(lev_up, h->ilu_lptr_up, rows_up);
+    std::vector<int64_t> lptr_lo, lptr_up;
+    group(lev_lo, lptr_lo, rows_lo);
+    group(lev_up, lptr_up, rows_up);
     h->d_ilu_ptr.upload(ptr, s);
     h->d_ilu_diag.upload(diag, s);
     h->d_ilu_rows_lo.upload(rows_lo, s);
@@ -1881,7 +1886,7 @@ namespace
     launch_ilu_fill(n, h->d_ilu_ptr.p, d_pos.p, h->d_row_leaf.p, h->d_nrow_ptr.p, h->d_ncol_ptr.p,
                     h->d_nval_ptr.p, h->d_ncols.p, h->d_S.p, d_con.p, h->d_ilu_col.p, h->d_ilu_val.p,
                     s);
-    launch_ilu_factor(h->ilu_lptr_lo, h->d_ilu_rows_lo.p, h->d_ilu_ptr.p, h->d_ilu_col.p,
+    launch_ilu_factor(lptr_lo, h->d_ilu_rows_lo.p, h->d_ilu_ptr.p, h->d_ilu_col.p,
                       h->d_ilu_val.p, h->d_ilu_diag.p, max_row, s);
     PIBEM_CUDA(cudaStreamSynchronize(s));
     h->ilu_on = true;
@@ -3019,6 +3024,7 @@ extern "C"
         PIBEM_CUDA(cudaMemcpyAsync(dz, dv, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
       else
         apply_prec(h, R, dv, N, dz, h->stream);
+      check_device_error(h);
       PIBEM_CUDA(cudaMemcpyAsync(z, dz, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
       PIBEM_CUDA(cudaStreamSynchronize(h->stream));
     });

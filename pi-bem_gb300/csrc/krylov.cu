@@ -949,32 +949,211 @@ namespace pibem
       z[idx] = v[r * ldv + t];
     }
 
-    // forward (lower, unit diagonal) or backward (upper) substitution for the
-    // rows of one level, in place on the selected columns of z (stride n):
-    // warp per (row, column), lanes over the row's entries, fixed butterfly
-    template <bool FWD>
-    __global__ void ilu_solve_kernel(int nrows, const int32_t *__restrict__ rows, int R, int64_t n,
-                                     const int64_t *__restrict__ ptr, const int32_t *__restrict__ col,
-                                     const double *__restrict__ val, const int64_t *__restrict__ diag,
-                                     double *__restrict__ z, const int *__restrict__ sel,
-                                     const int *__restrict__ jvec)
+    // z = U^-1 L^-1 z in place: one block per column (blockIdx.x) runs both
+    // substitutions.  Its warps take the rows in level order, one after another in
+    // turn; a warp waits for the solution values of its row's columns in the vector
+    // itself, which starts as a NaN pattern that no arithmetic result is stored as,
+    // so a value is its own flag.  A row only waits for rows before it in the list
+    // and each warp takes its rows in order, so the first unfinished row can always
+    // proceed; every wait is bounded.  A row's sum: lanes stride over its entries,
+    // fixed butterfly.
+    //   What bounds it: the chain of dependent rows (some 650 levels of 4 rows at 2.4k
+    // nodes, 17,000 of 6 at 98k): no parallelism for more than an SM, so the
+    // hand-over between rows decides.  Inside one block it goes through shared memory
+    // (SMEM: up to some 25,000 nodes) or the L1 cache, 1.2-1.6 us a level (FP64 latency:
+    // the last FMA, five shuffled additions, the pivot), where one launch per level
+    // took 4.7 us.  The next row's indices are loaded a row ahead.  One application
+    // (p = 8, leaf 40): 2.4k nodes 13.4 -> 3.3 ms, 13.8k 29 -> 7.0, 31k 65 -> 21.
+    constexpr int                ILU_THREADS = 512;
+    constexpr int                ILU_E       = 16; // entries per lane loaded at once
+    constexpr unsigned long long ILU_UNSET   = ~0ull;
+    constexpr long               ILU_SPIN    = 1L << 22;
+
+    template <bool SMEM>
+    __device__ __forceinline__ double ilu_peek(const double *p)
     {
-      const int w    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-      const int lane = threadIdx.x & 31;
-      if (w >= nrows * R)
-        return;
-      const int r = w / nrows, i = rows[w - r * nrows];
+      double v;
+      if constexpr (SMEM)
+        v = *reinterpret_cast<const volatile double *>(p);
+      else
+        asm volatile("ld.relaxed.cta.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+      return v;
+    }
+    template <bool SMEM>
+    __device__ __forceinline__ void ilu_put(double *p, double v)
+    {
+      if (__double_as_longlong(v) == (long long)ILU_UNSET)
+        v = __longlong_as_double(0x7ff8000000000000ll); // another NaN
+      if constexpr (SMEM)
+        *reinterpret_cast<volatile double *>(p) = v;
+      else
+        asm volatile("st.relaxed.cta.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+    }
+
+    template <bool FWD, bool SMEM>
+    __device__ __forceinline__ void ilu_sweep(int n, const int32_t *__restrict__ rows,
+                                              const int64_t *__restrict__ ptr,
+                                              const int32_t *__restrict__ col,
+                                              const double *__restrict__ val,
+                                              const int64_t *__restrict__ diag, const double *rhs,
+                                              double *out, int *err, volatile int *abort)
+    {
+      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = ILU_THREADS / 32;
+      auto row_at = [&](int k) { return k < n ? rows[k] : -1; };
+      auto begin  = [&](int i) { return i < 0 ? int64_t(0) : (FWD ? ptr[i] : diag[i] + 1); };
+      auto end    = [&](int i) { return i < 0 ? int64_t(0) : (FWD ? diag[i] : ptr[i + 1]); };
+      auto right  = [&](int i) { return i < 0 ? 0.0 : rhs[i]; };
+      auto pivot  = [&](int i) { return i < 0 || FWD ? 1.0 : val[diag[i]]; };
+      int     i = row_at(warp), i1 = row_at(warp + nw);
+      int64_t a0 = begin(i), a1 = end(i);
+      double  b = right(i), d = pivot(i);
+      for (int k = warp; k < n; k += nw)
+        {
+          const int     i2 = row_at(k + 2 * nw);
+          const int64_t n0 = begin(i1), n1 = end(i1);
+          const double  nb = right(i1), nd = pivot(i1);
+          double        s = 0, di = 1.0 / d;
+          for (int64_t e0 = a0; e0 < a1; e0 += 32 * ILU_E)
+            {
+              int    c[ILU_E];
+              double v[ILU_E];
+              int    cnt = 0, next = 0; // entries of this lane, entries already added
+#pragma unroll
+              for (int u = 0; u < ILU_E; ++u)
+                {
+                  const int64_t e = e0 + lane + 32 * u;
+                  if (e < a1)
+                    {
+                      c[u] = col[e];
+                      v[u] = val[e];
+                      cnt  = u + 1;
+                    }
+                }
+              // Add the entries in order, each once its value is there; the late ones are
+              // the last columns, so little is left to add when they arrive.
+              auto ready = [](double x) { return __double_as_longlong(x) != (long long)ILU_UNSET; };
+              auto give_up = [&](long it) {
+                if ((it & 255) != 255 || (!*abort && it < ILU_SPIN))
+                  return;
+                if (!*abort)
+                  {
+                    *abort = 1;
+                    atomicExch(err, 1);
+                  }
+                next = cnt;
+              };
+              if constexpr (SMEM)
+                // shared memory: every pass looks at all entries that are due
+                for (long it = 0; __any_sync(0xffffffffu, next < cnt); ++it)
+                  {
+#pragma unroll
+                    for (int u = 0; u < ILU_E; ++u)
+                      if (u == next && u < cnt)
+                        {
+                          const double x = ilu_peek<SMEM>(out + c[u]);
+                          if (ready(x))
+                            {
+                              s = fma(v[u], x, s);
+                              ++next;
+                            }
+                        }
+                    give_up(it);
+                  }
+              else
+                {
+                  // L1: one look at all entries together, then at the first missing one
+                  // only (24 -> 21 ms per application at 31k nodes; every pass over all
+                  // entries 32 ms.  In shared memory this one is the slower, 4.5 against
+                  // 3.3 ms at 2.4k nodes)
+                  double x[ILU_E], vv = 0;
+                  int    cc   = 0;
+                  auto   take = [&] {
+#pragma unroll
+                    for (int u = 0; u < ILU_E; ++u)
+                      if (u == next)
+                        {
+                          cc = c[u];
+                          vv = v[u];
+                        }
+                  };
+#pragma unroll
+                  for (int u = 0; u < ILU_E; ++u)
+                    if (u < cnt)
+                      x[u] = ilu_peek<SMEM>(out + c[u]);
+#pragma unroll
+                  for (int u = 0; u < ILU_E; ++u)
+                    if (u == next && u < cnt && ready(x[u]))
+                      {
+                        s = fma(v[u], x[u], s);
+                        ++next;
+                      }
+                  take();
+                  for (long it = 0; __any_sync(0xffffffffu, next < cnt); ++it)
+                    {
+                      if (next < cnt)
+                        {
+                          const double xc = ilu_peek<SMEM>(out + cc);
+                          if (ready(xc))
+                            {
+                              s = fma(vv, xc, s);
+                              ++next;
+                              take();
+                            }
+                        }
+                      give_up(it);
+                    }
+                }
+            }
+          for (int o = 16; o > 0; o >>= 1)
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+          if (lane == 0)
+            ilu_put<SMEM>(out + i, FWD ? b - s : (b - s) * di);
+          i  = i1;
+          i1 = i2;
+          a0 = n0;
+          a1 = n1;
+          b  = nb;
+          d  = nd;
+        }
+    }
+
+    template <bool SMEM>
+    __global__ void __launch_bounds__(ILU_THREADS, 1)
+      ilu_apply_kernel(int n, const int32_t *__restrict__ rows_lo, const int32_t *__restrict__ rows_up,
+                       const int64_t *__restrict__ ptr, const int32_t *__restrict__ col,
+                       const double *__restrict__ val, const int64_t *__restrict__ diag, double *z,
+                       double *y, const int *__restrict__ sel, const int *__restrict__ jvec, int *err)
+    {
+      extern __shared__ double ilu_zs[];
+      __shared__ volatile int  abort;
+      const int64_t r = blockIdx.x;
       if ((sel && !sel[r]) || (jvec && jvec[r] < 0))
         return;
-      double       *zr = z + int64_t(r) * n;
-      const int64_t a0 = FWD ? ptr[i] : diag[i] + 1, a1 = FWD ? diag[i] : ptr[i + 1];
-      double        s  = 0;
-      for (int64_t e = a0 + lane; e < a1; e += 32)
-        s += val[e] * zr[col[e]];
-      for (int o = 16; o > 0; o >>= 1)
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0)
-        zr[i] = FWD ? zr[i] - s : (zr[i] - s) / val[diag[i]];
+      double *zr = z + r * n, *yr = y + r * n;
+      double *f  = SMEM ? ilu_zs : yr; // forward solution
+      const double unset = __longlong_as_double((long long)ILU_UNSET);
+      for (int t = threadIdx.x; t < n; t += ILU_THREADS)
+        f[t] = unset;
+      if (threadIdx.x == 0)
+        abort = 0;
+      __syncthreads();
+      ilu_sweep<true, SMEM>(n, rows_lo, ptr, col, val, diag, zr, f, err, &abort);
+      __syncthreads();
+      double *g = SMEM ? ilu_zs : zr; // backward solution
+      for (int t = threadIdx.x; t < n; t += ILU_THREADS)
+        {
+          if (SMEM)
+            yr[t] = f[t];
+          g[t] = unset;
+        }
+      __syncthreads();
+      ilu_sweep<false, SMEM>(n, rows_up, ptr, col, val, diag, yr, g, err, &abort);
+      if constexpr (SMEM)
+        {
+          __syncthreads();
+          for (int t = threadIdx.x; t < n; t += ILU_THREADS)
+            zr[t] = g[t];
+        }
     }
 
     template <typename T>
@@ -1372,31 +1551,26 @@ namespace pibem
     note_launch();
   }
 
-  void launch_ilu_apply(const std::vector<int64_t> &lptr_lo, const int32_t *rows_lo,
-                        const std::vector<int64_t> &lptr_up, const int32_t *rows_up, int R, int64_t n,
+  void launch_ilu_apply(int64_t n, int R, const int32_t *rows_lo, const int32_t *rows_up,
                         const int64_t *ptr, const int32_t *col, const double *val,
-                        const int64_t *diag, double *z, const int *sel, const int *jvec,
-                        cudaStream_t s)
+                        const int64_t *diag, double *z, double *y, const int *sel, const int *jvec,
+                        int *err, cudaStream_t s)
   {
-    for (size_t l = 0; l + 1 < lptr_lo.size(); ++l)
+    if (n == 0 || R == 0)
+      return;
+    const size_t smem = size_t(n) * sizeof(double);
+    if (smem <= 200 * 1024)
       {
-        const int nr = int(lptr_lo[l + 1] - lptr_lo[l]);
-        if (nr == 0)
-          continue;
-        ilu_solve_kernel<true><<<nblocks(int64_t(nr) * R * 32), 256, 0, s>>>(
-          nr, rows_lo + lptr_lo[l], R, n, ptr, col, val, diag, z, sel, jvec);
-        note_launch();
+        if (smem > 40 * 1024)
+          raise_smem_limit(reinterpret_cast<const void *>(ilu_apply_kernel<true>), smem);
+        ilu_apply_kernel<true><<<R, ILU_THREADS, smem, s>>>(int(n), rows_lo, rows_up, ptr, col, val, diag,
+                                                            z, y, sel, jvec, err);
       }
-    for (size_t l = 0; l + 1 < lptr_up.size(); ++l)
-      {
-        const int nr = int(lptr_up[l + 1] - lptr_up[l]);
-        if (nr == 0)
-          continue;
-        ilu_solve_kernel<false><<<nblocks(int64_t(nr) * R * 32), 256, 0, s>>>(
-          nr, rows_up + lptr_up[l], R, n, ptr, col, val, diag, z, sel, jvec);
-        note_launch();
-      }
+    else
+      ilu_apply_kernel<false><<<R, ILU_THREADS, 0, s>>>(int(n), rows_lo, rows_up, ptr, col, val, diag, z,
+                                                        y, sel, jvec, err);
     PIBEM_CUDA(cudaGetLastError());
+    note_launch();
   }
 
   template <typename T>
