@@ -167,7 +167,7 @@ namespace pibem
                   cudaStream_t s);
   // FP64-accurate translation GEMM on the tensor cores (ozaki_tc.cu): digits of
   // the operators (host, once) and of the expansions (device, per product),
-  // then Y = T E as (hi, lo) pairs; for K <= 96 (p <= 8)
+  // then Y = T E as (hi, lo) pairs; for K <= 128 (p <= 10)
   bool ozaki_ok(int K);
   void build_ozaki_images(const std::vector<double> &ops_out_in, int nops, int K,
                           std::vector<uint16_t> &img, std::vector<int16_t> &e_col);

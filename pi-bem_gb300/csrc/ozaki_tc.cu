@@ -15,15 +15,31 @@
 // accumulators; the pairs with g = 4, 5 share a fifth (its FP32 rounding is
 // below 2^-42 of the result); pairs with g > 5 (below 2^-48) are dropped.
 // The epilogue adds the five accumulators in float-float arithmetic and
-// scales the (hi, lo) pair by 2^(e_r + e_n).  Per 16 K values: 21 MMAs of
-// M = 128 rows, N = 96, K = 16.
+// scales the (hi, lo) pair by 2^(e_r + e_n).
 //
-// Block (160 threads, one per SM, persistent over a contiguous range of
-// chunks): warps 0-3 fill a 4-deep ring of A stages (one K chunk of 64 values
-// of one slice for the tile's 128 rows, 128-byte-swizzled K-major) from the
-// pre-sliced expansions and then run the epilogue; warp 4 copies the
-// operator's 12 B slice tiles (2 K chunks x 6 slices, pre-swizzled on the
-// host) with one bulk copy when the operator changes and issues the MMAs.
+// A unit of work is 128 rows (pairs of one operator) times 48 operator rows (a part:
+// two at p <= 8, three at p = 9, 10): five 48-column accumulators, so that two units
+// fit in tensor memory and a unit's epilogue runs beside the next one's MMAs.  Per 16
+// K values 11 MMAs (N = 48 to 240) take the 21 slice pairs; K steps beyond K are
+// neither loaded nor issued.
+//
+// Block (416 threads, one per SM, persistent over a contiguous range of chunks, part
+// after part within a run of chunks of one operator):
+//   warps 0-3  producers: a 6-deep ring of A stages (one K chunk of 64 values of one
+//              slice for the unit's 128 rows, 128-byte-swizzled K-major), filled with
+//              16-byte cp.async, eight lanes to a row's 128-byte line;
+//   warps 4-11 epilogue: tensor-memory loads, float-float sums, staging in shared
+//              memory and coalesced row segments;
+//   warp 12    copies the part's 12 operator slice tiles (pre-swizzled on the host)
+//              with one bulk copy when operator or part change, and issues the MMAs.
+// What bounds it: the tensor unit's operand reads (sm__pipe_tc 42 % active, the
+// products themselves 23 %), the epilogue's FP32 instructions and the hand-overs
+// between the roles.  Measured (GB300; before: one accumulator set of 96 columns, the
+// epilogue after the MMAs, a row loaded and stored by one thread, and the CUDA-core
+// float-float GEMM beyond K = 96): 98k spheroid (p = 8, 272,776 pairs) 441 -> 281 us,
+// 198k hull (p = 10) 5,920 -> 840 us, 16 columns at 23,816 nodes 1,754 -> 1,016 us.
+// (One MMA per slice pair 426 / 1,191 us for the first two, four epilogue warps
+// 318 / 895.)
 // All waits are bounded; a timeout is recorded in *err and the host reports
 // PIBEM_ETIMEDOUT.
 #include <algorithm>
@@ -44,22 +60,30 @@ namespace pibem
     constexpr int      OZ_G        = 5;   // accumulators: i + j = 0, 1, 2, 3 and 4..5
     constexpr int      OZ_KC       = 64;  // K values per chunk: one 128-byte line of BF16
     constexpr int      OZ_NKC      = 2;   // K chunks (K <= 128)
-    constexpr int      OZ_NP       = 96;  // operator rows per tile (N of the MMA; K <= 96)
-    constexpr int      OZ_ROWS     = 128; // tile rows (M of the MMA)
-    constexpr int      OZ_RING     = 4;   // A stages in flight
-    constexpr int      OZ_THREADS  = 160; // warps 0-3 producers / epilogue, warp 4 MMA
+    constexpr int      OZ_NP       = 48;  // operator rows per part (N of the MMA)
+    constexpr int      OZ_ROWS     = 128; // unit rows (M of the MMA)
+    constexpr int      OZ_RING     = 6;   // A stages
+    constexpr int      OZ_LAG      = 3;   // stages a producer has in flight
+    constexpr int      OZ_THREADS  = 416; // warps 0-3 producers, 4-11 epilogue, 12 MMA
+    constexpr int      OZ_MMA_WARP = 12;
+    constexpr int      OZ_EC       = OZ_NP / 2; // columns per epilogue warp
     constexpr uint32_t OZ_A_BYTES  = OZ_ROWS * 128;         // 16 KB
-    constexpr uint32_t OZ_BT_BYTES = OZ_NP * 128;           // 12 KB per (K chunk, slice)
-    constexpr uint32_t OZ_B_BYTES  = OZ_NKC * OZ_S * OZ_BT_BYTES; // 144 KB per operator
-    constexpr uint32_t OZ_TMEM_COLS = 512;
-    constexpr long     OZ_SPIN     = 1L << 22;
+    constexpr uint32_t OZ_BT_BYTES = OZ_NP * 128;           // 6 KB per (K chunk, slice)
+    constexpr uint32_t OZ_B_BYTES  = OZ_NKC * OZ_S * OZ_BT_BYTES; // 72 KB per (operator, part)
+    constexpr uint32_t OZ_ACC_COLS  = OZ_G * OZ_NP;         // one unit's accumulators
+    constexpr uint32_t OZ_TMEM_COLS = 512;                  // two units (480), a power of two
+    constexpr int      OZ_STG_LD    = OZ_EC + 1;            // staging row stride (float2)
+    constexpr uint32_t OZ_STG_BYTES = 32 * OZ_STG_LD * 8;   // per epilogue warp
+    constexpr long     OZ_SPIN      = 1L << 22;
 
-    // shared memory: B (144 KB) | A ring (64 KB) | barriers
+    // shared memory: B (72 KB) | A ring (96 KB) | staging (50 KB) | barriers
     constexpr uint32_t OZ_OFF_A    = OZ_B_BYTES;
-    constexpr uint32_t OZ_OFF_BAR  = OZ_OFF_A + OZ_RING * OZ_A_BYTES;
-    constexpr uint32_t OZ_SMEM     = OZ_OFF_BAR + 128 + 1024; // 11 barriers; alignment slack
+    constexpr uint32_t OZ_OFF_STG  = OZ_OFF_A + OZ_RING * OZ_A_BYTES;
+    constexpr uint32_t OZ_OFF_BAR  = OZ_OFF_STG + 8 * OZ_STG_BYTES;
+    constexpr int      OZ_NBAR     = 2 * OZ_RING + 7;
+    constexpr uint32_t OZ_SMEM     = OZ_OFF_BAR + 8 * OZ_NBAR + 1024; // + alignment slack
 
-    __host__ __device__ inline int oz_group(int i, int j) { return i + j < 4 ? i + j : 4; }
+    __host__ __device__ inline int oz_parts(int K) { return (K + OZ_NP - 1) / OZ_NP; }
 
     // Bounded wait; after a timeout anywhere in the block (abort raised) no
     // further waiting, so a broken pipeline ends quickly (results then wrong,
@@ -147,8 +171,8 @@ namespace pibem
     {
       int            R, K, chunk0, n_chunks;
       const int32_t *ch_start, *ch_cnt, *ch_op, *q_src;
-      const uint16_t *bimg;   // [op][kc][slice][96 x 64 swizzled]
-      const int16_t  *e_col;  // [op][96]
+      const uint16_t *bimg;   // [op][part][kc][slice][48 x 64 swizzled]
+      const int16_t  *e_col;  // [op][48 parts]
       const uint16_t *aslc;   // [slice][box row][128]
       const int      *e_row;  // [box row]
       int64_t         a_rows; // box rows (n_boxes * R)
@@ -156,23 +180,60 @@ namespace pibem
       int            *err;
     };
 
+    // The block's units in order, f(operator, part, first pair, rows of the chunk,
+    // first row): every role walks the same list.
+    template <typename F>
+    __device__ __forceinline__ void oz_units(const OzArgs &a, F f)
+    {
+      const int ch_lo = a.chunk0 + int(int64_t(a.n_chunks) * blockIdx.x / gridDim.x);
+      const int ch_hi = a.chunk0 + int(int64_t(a.n_chunks) * (blockIdx.x + 1) / gridDim.x);
+      const int parts = oz_parts(a.K);
+      for (int ch = ch_lo, end; ch < ch_hi; ch = end)
+        {
+          const int op = a.ch_op[ch];
+          for (end = ch + 1; end < ch_hi && a.ch_op[end] == op;)
+            ++end;
+          for (int part = 0; part < parts; ++part)
+            for (int c = ch; c < end; ++c)
+              {
+                const int start = a.ch_start[c], rows = a.ch_cnt[c] * a.R;
+                for (int t0 = 0; t0 < rows; t0 += OZ_ROWS)
+                  f(op, part, start, rows, t0);
+              }
+        }
+    }
+
+    // 16 bytes global -> shared, asynchronous; zeros when !ok
+    __device__ __forceinline__ void oz_cp16(uint32_t dst, const void *src, bool ok)
+    {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0)
+                   : "memory");
+    }
+    template <int N>
+    __device__ __forceinline__ void oz_cp_wait()
+    {
+      asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+    }
+
     __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(OzArgs a)
     {
       extern __shared__ uint8_t smem_raw[];
       __shared__ uint32_t     tmem_slot;
       __shared__ volatile int abort_flag;
+      __shared__ int          rows_src[2][OZ_ROWS]; // a unit's source rows (-1: padding)
       const uint32_t raw  = smem_u32(smem_raw);
       const uint32_t base = (raw + 1023u) & ~1023u;
       const int      tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
       const uint32_t bar0   = base + OZ_OFF_BAR;
       auto a_full  = [&](int s) { return bar0 + 8u * uint32_t(s); };
       auto a_empty = [&](int s) { return bar0 + 8u * uint32_t(OZ_RING + s); };
-      const uint32_t b_full = bar0 + 8u * uint32_t(2 * OZ_RING);
-      const uint32_t done   = b_full + 8u;
-      const uint32_t drain  = done + 8u;
-      const int ch_lo = a.chunk0 + int(int64_t(a.n_chunks) * blockIdx.x / gridDim.x);
-      const int ch_hi = a.chunk0 + int(int64_t(a.n_chunks) * (blockIdx.x + 1) / gridDim.x);
+      auto t_full  = [&](int b) { return bar0 + 8u * uint32_t(2 * OZ_RING + b); };
+      auto t_empty = [&](int b) { return bar0 + 8u * uint32_t(2 * OZ_RING + 2 + b); };
+      const uint32_t b_full = bar0 + 8u * uint32_t(2 * OZ_RING + 4);
+      const uint32_t b_free = b_full + 8u, drain = b_full + 16u;
       const int R = a.R, K = a.K;
+      const int nkc   = K > OZ_KC ? 2 : 1;
+      auto      steps = [&](int kc) { return min(OZ_KC / 16, (K - kc * OZ_KC + 15) / 16); };
       if (tid == 0)
         {
           abort_flag = 0;
@@ -181,12 +242,17 @@ namespace pibem
               mbar_init(a_full(s), 128);
               mbar_init(a_empty(s), 1);
             }
+          for (int b = 0; b < 2; ++b)
+            {
+              mbar_init(t_full(b), 1);
+              mbar_init(t_empty(b), 256);
+            }
           mbar_init(b_full, 1);
-          mbar_init(done, 1);
+          mbar_init(b_free, 1);
           mbar_init(drain, 1);
           mbar_init_fence();
         }
-      if (warp == 4)
+      if (warp == OZ_MMA_WARP)
         {
           asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                        :
@@ -198,181 +264,206 @@ namespace pibem
       __syncthreads();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem = tmem_slot;
-      // D f32, A and B bf16, both K-major, N = 96, M = 128
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(OZ_NP >> 3) << 17) |
-                             (uint32_t(OZ_ROWS >> 4) << 24);
-      int  loaded_op = -1, b_loads = 0, tiles = 0;
-      long stage = 0; // A stages over all tiles of this block
-      bool issued = false, b_pending = false;
-      for (int ch = ch_lo; ch < ch_hi; ++ch)
+
+      if (warp < 4)
         {
-          const int start = a.ch_start[ch], rows_total = a.ch_cnt[ch] * R, op = a.ch_op[ch];
-          for (int t0 = 0; t0 < rows_total; t0 += OZ_ROWS, ++tiles)
+          // ---------------- producers ----------------
+          long g = 0; // A stages started
+          int  unit = 0;
+          auto done = [&](long st) { // this thread's copies of stage st have landed
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_arrive(a_full(int(st % OZ_RING)));
+          };
+          oz_units(a, [&](int, int, int start, int rows, int t0) {
+            int *src = rows_src[unit & 1];
             {
-              if (warp == 4)
-                {
-                  if (lane == 0)
-                    {
-                      if (op != loaded_op)
-                        {
-                          mbar_arrive_expect_tx(b_full, OZ_B_BYTES);
-                          bulk_copy(base, a.bimg + size_t(op) * (OZ_B_BYTES / 2), OZ_B_BYTES, b_full);
-                          b_pending = !oz_wait(b_full, uint32_t(b_loads) & 1u, a.err, &abort_flag);
-                          ++b_loads;
-                          loaded_op = op;
-                        }
-                      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                      int started = 0; // accumulators written in this tile
-                      for (int s = 0; s < OZ_NKC * OZ_S; ++s)
-                        {
-                          const long g_st = stage + s;
-                          const int  slot = int(g_st % OZ_RING);
-                          oz_wait(a_full(slot), uint32_t(g_st / OZ_RING) & 1u, a.err, &abort_flag);
-                          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                          const int      kc = s / OZ_S, i = s % OZ_S;
-                          const uint32_t at = base + OZ_OFF_A + uint32_t(slot) * OZ_A_BYTES;
-                          for (int j = 0; i + j < OZ_S; ++j)
-                            {
-                              const int      g  = oz_group(i, j);
-                              const uint32_t bt = base + uint32_t(kc * OZ_S + j) * OZ_BT_BYTES;
+              const int row = t0 + tid;
+              src[tid]      = row < rows ? a.q_src[start + row / R] * R + row % R : -1;
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory"); // the producers' table
+            for (int kc = 0; kc < nkc; ++kc)
+              {
+                const int nch = 2 * steps(kc); // 16-byte pieces of a row that are used
+                for (int i = 0; i < OZ_S; ++i, ++g)
+                  {
+                    const int slot = int(g % OZ_RING);
+                    if (g >= OZ_RING)
+                      oz_wait(a_empty(slot), uint32_t(g / OZ_RING - 1) & 1u, a.err, &abort_flag);
+                    const uint32_t  at = base + OZ_OFF_A + uint32_t(slot) * OZ_A_BYTES;
+                    const uint16_t *E  = a.aslc + int64_t(i) * a.a_rows * 128 + kc * OZ_KC;
+                    const int       ch = tid & 7;
+                    if (ch < nch)
 #pragma unroll
-                              for (int ks = 0; ks < OZ_KC / 16; ++ks)
-                                {
-                                  const uint32_t acc = (((started >> g) & 1) != 0 || ks > 0) ? 1u : 0u;
-                                  mma_bf16(tmem + uint32_t(g * OZ_NP), smem_desc_sw128(at + ks * 32),
-                                           smem_desc_sw128(bt + ks * 32), idesc, acc);
-                                }
-                              started |= 1 << g;
-                            }
-                          mma_commit(a_empty(slot)); // frees the stage once these MMAs are done
-                          issued = true;
+                      for (int u = 0; u < 8; ++u)
+                        {
+                          const int row = 16 * u + (tid >> 3), sr = src[row];
+                          oz_cp16(at + sw128_off_b16(row, 8 * ch), E + int64_t(max(sr, 0)) * 128 + 8 * ch,
+                                  sr >= 0);
                         }
-                      mma_commit(done); // the tile's accumulators are complete
-                    }
-                  __syncwarp();
-                }
-              else
-                {
-                  // ---------------- producers: one tile row per thread ----------------
-                  const int row = t0 + tid;
-                  int64_t   src = -1;
-                  if (row < rows_total)
-                    {
-                      const int q = start + row / R, r = row - (row / R) * R;
-                      src         = int64_t(a.q_src[q]) * R + r;
-                    }
-                  // stage s = (K chunk s / 6, slice s % 6); the loads of stage s + 2
-                  // are issued before stage s is stored (three stages of the row in
-                  // registers), so the L2 latency overlaps the ring waits
-                  uint4 buf[3][8];
-                  auto  load = [&](int s, uint4(&v)[8]) {
-                    const int kc = s / OZ_S, i = s % OZ_S;
-                    if (src >= 0)
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                    if (g >= OZ_LAG)
                       {
-                        const uint4 *p = reinterpret_cast<const uint4 *>(
-                          a.aslc + (int64_t(i) * a.a_rows + src) * 128 + kc * OZ_KC);
+                        oz_cp_wait<OZ_LAG>();
+                        done(g - OZ_LAG);
+                      }
+                  }
+              }
+            ++unit;
+          });
+          oz_cp_wait<0>();
+          for (long st = g > OZ_LAG ? g - OZ_LAG : 0; st < g; ++st)
+            done(st);
+        }
+      else if (warp == OZ_MMA_WARP)
+        {
+          // ---------------- operator copies and MMAs ----------------
+          if (lane == 0)
+            {
+              // D f32, A and B bf16, both K-major, M = 128; idesc1: N = 48
+              const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(OZ_ROWS >> 4) << 24);
+              const uint32_t idesc1 = idesc | (uint32_t(OZ_NP >> 3) << 17);
+              int  held_op = -1, held_part = -1, b_loads = 0, unit = 0;
+              long g      = 0;
+              bool issued = false, b_pending = false;
+              oz_units(a, [&](int op, int part, int, int, int) {
+                if (op != held_op || part != held_part)
+                  {
+                    if (issued) // the MMAs that read the held tiles
+                      {
+                        mma_commit(b_free);
+                        oz_wait(b_free, uint32_t(b_loads - 1) & 1u, a.err, &abort_flag);
+                      }
+                    mbar_arrive_expect_tx(b_full, OZ_B_BYTES);
+                    bulk_copy(base, a.bimg + (size_t(op) * oz_parts(K) + part) * (OZ_B_BYTES / 2),
+                              OZ_B_BYTES, b_full);
+                    b_pending = !oz_wait(b_full, uint32_t(b_loads) & 1u, a.err, &abort_flag);
+                    ++b_loads;
+                    held_op   = op;
+                    held_part = part;
+                  }
+                const int buf = unit & 1;
+                if (unit >= 2)
+                  oz_wait(t_empty(buf), uint32_t((unit >> 1) - 1) & 1u, a.err, &abort_flag);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t d       = tmem + uint32_t(buf) * OZ_ACC_COLS;
+                for (int kc = 0; kc < nkc; ++kc)
+                  {
+                    const int      nks = steps(kc);
+                    const uint64_t db  = smem_desc_sw128(base + uint32_t(kc * OZ_S) * OZ_BT_BYTES);
+                    for (int i = 0; i < OZ_S; ++i, ++g)
+                      {
+                        const int slot = int(g % OZ_RING);
+                        oz_wait(a_full(slot), uint32_t(g / OZ_RING) & 1u, a.err, &abort_flag);
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint32_t at = base + OZ_OFF_A + uint32_t(slot) * OZ_A_BYTES;
+                        // Slice i with the operator slices j = 0 .. 4 - i: the groups i + j and
+                        // the slices' tiles follow one another, so that one MMA of N = 48 (5 - i)
+                        // reads A once for all of them; then j = 5 - i, also of group 4.
+                        // (Descriptors differ in their start address, 16-byte units, only.)
+                        const uint64_t da = smem_desc_sw128(at);
+                        const uint64_t dl = db + uint64_t((OZ_S - 1 - i) * (OZ_BT_BYTES >> 4));
+                        const int      nj = OZ_G - i; // 5 .. 0
+                        const uint32_t di = idesc + (uint32_t(nj * OZ_NP >> 3) << 17);
+                        const uint32_t first = kc == 0 && i == 0 ? 1u : 0u;
 #pragma unroll
-                        for (int c = 0; c < 8; ++c)
-                          v[c] = __ldg(p + c);
+                        for (int ks = 0; ks < OZ_KC / 16; ++ks)
+                          if (ks < nks)
+                            {
+                              if (nj > 0)
+                                mma_bf16(d + uint32_t(i * OZ_NP), da + uint64_t(2 * ks), db + uint64_t(2 * ks),
+                                         di, ks > 0 ? 1u : 1u - first);
+                              mma_bf16(d + uint32_t((OZ_G - 1) * OZ_NP), da + uint64_t(2 * ks),
+                                       dl + uint64_t(2 * ks), idesc1, 1u);
+                            }
+                        mma_commit(a_empty(slot)); // frees the stage once these MMAs are done
+                        issued = true;
+                      }
+                  }
+                mma_commit(t_full(buf)); // the unit's accumulators are complete
+                ++unit;
+              });
+              if (b_pending) // a copy whose wait gave up: let it land before the block ends
+                mbar_wait_bounded(b_full, uint32_t(b_loads - 1) & 1u, OZ_SPIN);
+              if (issued)
+                {
+                  mma_commit(drain); // every MMA issued above has completed
+                  mbar_wait_bounded(drain, 0, OZ_SPIN);
+                }
+            }
+          __syncwarp();
+        }
+      else
+        {
+          // -------- epilogue: rows 32 q .. 32 q + 31, half the columns of the unit --------
+          const int q = warp & 3, c_lo = (warp - 4) / 4 * OZ_EC;
+          float2   *stg  = reinterpret_cast<float2 *>(smem_raw + (base - raw) + OZ_OFF_STG +
+                                                   size_t(warp - 4) * OZ_STG_BYTES);
+          const int n_ec = oz_parts(K) * OZ_NP;
+          int       unit = 0;
+          oz_units(a, [&](int op, int part, int start, int rows, int t0) {
+            const int buf = unit & 1, row0 = t0 + 32 * q, nvalid = min(32, rows - row0);
+            int       er = 0;
+            if (lane < nvalid)
+              er = a.e_row[int64_t(a.q_src[start + (row0 + lane) / R]) * R + (row0 + lane) % R];
+            const int16_t *ec = a.e_col + size_t(op) * n_ec + part * OZ_NP + c_lo;
+            oz_wait(t_full(buf), uint32_t(unit >> 1) & 1u, a.err, &abort_flag);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t d = tmem + (uint32_t(32 * q) << 16) + uint32_t(buf) * OZ_ACC_COLS + uint32_t(c_lo);
+#pragma unroll 1
+            for (int c0 = 0; c0 < OZ_EC; c0 += 8)
+              {
+                // the five group sums of 8 columns (five loads, one wait): g0, g1 and
+                // g2, g3 pairwise by TwoSum, the two pairs by TwoSum, the errors and
+                // g4 added last (each below 2^-40 of the result), one renormalisation
+                uint32_t v[OZ_G][8];
+#pragma unroll
+                for (int b = 0; b < OZ_G; ++b)
+                  tmem_ld8_nowait(d + uint32_t(b * OZ_NP + c0), v[b]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int jj = 0; jj < 8; ++jj)
+                  {
+                    const float g0 = __uint_as_float(v[0][jj]), g1 = __uint_as_float(v[1][jj]);
+                    const float g2 = __uint_as_float(v[2][jj]), g3 = __uint_as_float(v[3][jj]);
+                    const float g4 = __uint_as_float(v[4][jj]);
+                    const float t1 = __fadd_rn(g0, g1), z1 = __fsub_rn(t1, g0);
+                    const float e1 = __fadd_rn(__fsub_rn(g0, __fsub_rn(t1, z1)), __fsub_rn(g1, z1));
+                    const float t2 = __fadd_rn(g2, g3), z2 = __fsub_rn(t2, g2);
+                    const float e2 = __fadd_rn(__fsub_rn(g2, __fsub_rn(t2, z2)), __fsub_rn(g3, z2));
+                    const float t  = __fadd_rn(t1, t2), z = __fsub_rn(t, t1);
+                    const float dd = __fadd_rn(__fsub_rn(t1, __fsub_rn(t, z)), __fsub_rn(t2, z));
+                    const float lo = __fadd_rn(__fadd_rn(e1, __fadd_rn(e2, dd)), g4);
+                    const float2 r = ff_norm(t, lo);
+                    // times 2^(e_r + e_n): a power of two built from its bits
+                    // when it is a normal float, else ldexpf
+                    const int e = er + ec[c0 + jj];
+                    float2    y;
+                    if (e > -127 && e < 128)
+                      {
+                        const float sc = __int_as_float((e + 127) << 23);
+                        y              = make_float2(__fmul_rn(r.x, sc), __fmul_rn(r.y, sc));
                       }
                     else
-#pragma unroll
-                      for (int c = 0; c < 8; ++c)
-                        v[c] = make_uint4(0u, 0u, 0u, 0u);
-                  };
-                  load(0, buf[0]);
-                  load(1, buf[1]);
-#pragma unroll
-                  for (int s = 0; s < OZ_NKC * OZ_S; ++s)
-                    {
-                      if (s + 2 < OZ_NKC * OZ_S)
-                        load(s + 2, buf[(s + 2) % 3]);
-                      const long g_st = stage + s;
-                      const int  slot = int(g_st % OZ_RING);
-                      if (g_st >= OZ_RING)
-                        oz_wait(a_empty(slot), uint32_t(g_st / OZ_RING - 1) & 1u, a.err, &abort_flag);
-                      uint8_t *at = smem_raw + (base - raw) + OZ_OFF_A + size_t(slot) * OZ_A_BYTES;
-#pragma unroll
-                      for (int c = 0; c < 8; ++c)
-                        *reinterpret_cast<uint4 *>(at + sw128_off_b16(tid, 8 * c)) = buf[s % 3][c];
-                      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                      mbar_arrive(a_full(slot));
-                    }
-                  // ---------------- epilogue: row tid of the tile ----------------
-                  oz_wait(done, uint32_t(tiles) & 1u, a.err, &abort_flag);
-                  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                  const int  q_row = t0 + 32 * warp + lane;
-                  const bool valid = q_row < rows_total;
-                  int        er    = 0;
-                  if (valid)
-                    {
-                      const int q = start + q_row / R, r = q_row - (q_row / R) * R;
-                      er          = a.e_row[int64_t(a.q_src[q]) * R + r];
-                    }
-                  const int16_t *ec   = a.e_col + size_t(op) * OZ_NP;
-                  float2        *yrow = a.Y + (int64_t(start) * R + q_row) * K;
-                  for (int c0 = 0; c0 < OZ_NP; c0 += 32)
-                    {
-                      // the five group sums of 32 columns (five loads, one wait):
-                      // g0, g1 and g2, g3 pairwise by TwoSum, the two pairs by
-                      // TwoSum, the errors and g4 added last (each below 2^-40 of
-                      // the result), one renormalisation
-                      uint32_t g[5][32];
-#pragma unroll
-                      for (int q = 0; q < OZ_G; ++q)
-                        tmem_ld32_nowait(tmem + (uint32_t(32 * warp) << 16) + uint32_t(q * OZ_NP + c0), g[q]);
-                      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                      if (valid)
-#pragma unroll
-                        for (int jj = 0; jj < 32; ++jj)
-                          {
-                            const int n = c0 + jj;
-                            if (n >= K)
-                              continue;
-                            const float g0 = __uint_as_float(g[0][jj]), g1 = __uint_as_float(g[1][jj]);
-                            const float g2 = __uint_as_float(g[2][jj]), g3 = __uint_as_float(g[3][jj]);
-                            const float g4 = __uint_as_float(g[4][jj]);
-                            const float t1 = __fadd_rn(g0, g1), z1 = __fsub_rn(t1, g0);
-                            const float e1 = __fadd_rn(__fsub_rn(g0, __fsub_rn(t1, z1)), __fsub_rn(g1, z1));
-                            const float t2 = __fadd_rn(g2, g3), z2 = __fsub_rn(t2, g2);
-                            const float e2 = __fadd_rn(__fsub_rn(g2, __fsub_rn(t2, z2)), __fsub_rn(g3, z2));
-                            const float t  = __fadd_rn(t1, t2), z = __fsub_rn(t, t1);
-                            const float d  = __fadd_rn(__fsub_rn(t1, __fsub_rn(t, z)), __fsub_rn(t2, z));
-                            const float lo = __fadd_rn(__fadd_rn(e1, __fadd_rn(e2, d)), g4);
-                            const float2 r = ff_norm(t, lo);
-                            // times 2^(e_r + e_n): a power of two built from its bits
-                            // when it is a normal float, else ldexpf
-                            const int e = er + ec[n];
-                            if (e > -127 && e < 128)
-                              {
-                                const float sc = __int_as_float((e + 127) << 23);
-                                yrow[n] = make_float2(__fmul_rn(r.x, sc), __fmul_rn(r.y, sc));
-                              }
-                            else
-                              yrow[n] = make_float2(ldexpf(r.x, e), ldexpf(r.y, e));
-                          }
-                    }
-                }
-              stage += OZ_NKC * OZ_S;
-              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-              __syncthreads(); // accumulators read: the next tile may overwrite them
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            }
-        }
-      if (warp == 4 && lane == 0)
-        {
-          if (b_pending) // a copy whose wait gave up: let it land before the block ends
-            mbar_wait_bounded(b_full, uint32_t(b_loads - 1) & 1u, OZ_SPIN);
-          if (issued)
-            {
-              mma_commit(drain); // every MMA issued above has completed
-              mbar_wait_bounded(drain, 0, OZ_SPIN);
-            }
+                      y = make_float2(ldexpf(r.x, e), ldexpf(r.y, e));
+                    stg[lane * OZ_STG_LD + c0 + jj] = y;
+                  }
+              }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(t_empty(buf)); // the accumulators may be overwritten
+            __syncwarp();
+            const int n0 = part * OZ_NP + c_lo, nc = min(OZ_EC, K - n0);
+            float2   *y  = a.Y + (int64_t(start) * R + row0) * K + n0;
+            for (int r = 0; r < nvalid; ++r, y += K)
+              if (lane < nc)
+                y[lane] = stg[r * OZ_STG_LD + lane];
+            __syncwarp(); // the staging rows are read
+            ++unit;
+          });
         }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncthreads();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (warp == 4)
+      if (warp == OZ_MMA_WARP)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
                      :
                      : "r"(tmem), "r"(OZ_TMEM_COLS)
@@ -380,15 +471,19 @@ namespace pibem
     }
   } // namespace
 
-  bool ozaki_ok(int K) { return K >= 1 && K <= OZ_NP; }
+  bool ozaki_ok(int K) { return K >= 1 && K <= OZ_NKC * OZ_KC; }
 
   // Host: digits of every operator row (output coefficient), B images and
   // column exponents.  ops_out_in: nops row-major [out][in] K x K operators.
   void build_ozaki_images(const std::vector<double> &ops_out_in, int nops, int K,
                           std::vector<uint16_t> &img, std::vector<int16_t> &e_col)
   {
-    img.assign(size_t(nops) * (OZ_B_BYTES / 2), 0);
-    e_col.assign(size_t(nops) * OZ_NP, 0);
+    const int parts = oz_parts(K);
+    img.assign(size_t(nops) * parts * (OZ_B_BYTES / 2), 0);
+    e_col.assign(size_t(nops) * parts * OZ_NP, 0);
+    double weight[OZ_S]; // of digit i: 2^-(7 + 8 i)
+    for (int i = 0; i < OZ_S; ++i)
+      weight[i] = std::ldexp(1.0, -(7 + 8 * i));
 #pragma omp parallel for schedule(dynamic, 4)
     for (int o = 0; o < nops; ++o)
       for (int n = 0; n < K; ++n)
@@ -400,7 +495,9 @@ namespace pibem
           int e = 0;
           if (mx > 0.0)
             std::frexp(mx, &e); // mx < 2^e
-          e_col[size_t(o) * OZ_NP + n] = int16_t(e);
+          e_col[size_t(o) * parts * OZ_NP + n] = int16_t(e);
+          uint16_t *tile = &img[(size_t(o) * parts + n / OZ_NP) * (OZ_B_BYTES / 2)];
+          const int row  = n % OZ_NP;
           for (int k = 0; k < K; ++k)
             {
               double v = std::ldexp(t[k], -e);
@@ -409,11 +506,8 @@ namespace pibem
                   v *= (i == 0 ? 128.0 : 256.0);
                   const double d = std::nearbyint(v);
                   v -= d;
-                  const int    kc = k / OZ_KC;
-                  const size_t at = size_t(o) * (OZ_B_BYTES / 2) +
-                                    size_t(kc * OZ_S + i) * (OZ_BT_BYTES / 2) +
-                                    sw128_off_b16(n, k % OZ_KC) / 2;
-                  img[at] = bf16_bits(float(std::ldexp(d, -(7 + 8 * i))));
+                  tile[size_t(k / OZ_KC * OZ_S + i) * (OZ_BT_BYTES / 2) + sw128_off_b16(row, k % OZ_KC) / 2] =
+                    bf16_bits(float(d * weight[i])); // exact
                 }
             }
         }

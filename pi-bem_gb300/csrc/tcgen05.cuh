@@ -58,19 +58,13 @@ namespace pibem
       v[j] = __uint_as_float(r[j]);
   }
 
-  // 32 columns of the warp's 32 lanes, without waiting (tcgen05.wait::ld
+  // 8 columns of the warp's 32 lanes, without waiting (tcgen05.wait::ld
   // before the registers are used)
-  __device__ inline void tmem_ld32_nowait(uint32_t taddr, uint32_t (&r)[32])
+  __device__ inline void tmem_ld8_nowait(uint32_t taddr, uint32_t (&r)[8])
   {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-                   "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                   "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
-                   "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
-                   "=r"(r[30]), "=r"(r[31])
+                   "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr)
                  : "memory");
   }
