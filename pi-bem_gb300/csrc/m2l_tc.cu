@@ -155,7 +155,6 @@ namespace pibem
                      float *__restrict__ Y, const int32_t *__restrict__ yslot, int ldy,
                      int *__restrict__ err)
     {
-      pdl_entry();
       extern __shared__ uint8_t smem_raw[];
       __shared__ uint32_t       tmem_slot;
       __shared__ volatile int   abort_flag;
@@ -172,10 +171,6 @@ namespace pibem
       auto tfull  = [&](int a) { return bar0 + 8u * uint32_t(2 * TC_STAGES + a); };
       auto tempty = [&](int a) { return bar0 + 8u * uint32_t(2 * TC_STAGES + 2 + a); };
       const uint32_t drain = bar0 + 8u * uint32_t(2 * TC_STAGES + 4);
-      // each block takes a contiguous range of chunks: consecutive chunks mostly
-      // share their operator, so a stage can keep its B tile (see the producers)
-      const int ch_lo = chunk0 + int(int64_t(n_chunks) * blockIdx.x / gridDim.x);
-      const int ch_hi = chunk0 + int(int64_t(n_chunks) * (blockIdx.x + 1) / gridDim.x);
       const size_t   op_img_floats = size_t(nkc) * Np * TC_KC; // one half of an operator image
 
       if (tid == 0)
@@ -202,6 +197,14 @@ namespace pibem
                        : "memory");
           asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
+      // the block's tiles: a contiguous range, whose chunks mostly share their operator,
+      // so that a stage can keep its B tile (see the producers).  The chunk tables do
+      // not depend on the launch ahead.
+      const TileRange range = tile_range(ch_cnt + chunk0, n_chunks, R);
+      const int       ch_lo = chunk0 + range.c_lo, ch_hi = chunk0 + range.c_hi; // inclusive
+      auto first_row = [&](int ch) { return ch == ch_lo ? range.t_lo * TC_ROWS : 0; };
+      auto end_row   = [&](int ch, int rows) { return ch == ch_hi ? min(rows, range.t_hi * TC_ROWS) : rows; };
+      pdl_entry();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncthreads();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -242,12 +245,12 @@ namespace pibem
               inflight[s]     = false;
               inflight_par[s] = 0;
             }
-          for (int ch = ch_lo; ok && ch < ch_hi; ++ch)
+          for (int ch = ch_lo; ok && ch <= ch_hi; ++ch)
             {
               const int    start = ch_start[ch], rows_total = ch_cnt[ch] * R, op = ch_op[ch];
               const float *Bhi   = images + size_t(op) * 2 * op_img_floats;
               const float *Blo   = Bhi + op_img_floats;
-              for (int t0 = 0; ok && t0 < rows_total; t0 += TC_ROWS)
+              for (int t0 = first_row(ch); ok && t0 < end_row(ch, rows_total); t0 += TC_ROWS)
                 {
                   // source offset of row t0 + 32 gw + lane (-1: padding row); the
                   // host checks that every offset fits in 32 bits
@@ -342,10 +345,10 @@ namespace pibem
                                      (uint32_t(Np >> 3) << 17) | (uint32_t(TC_ROWS >> 4) << 24);
               int  it = 0, tile = 0;
               bool issued = false;
-              for (int ch = ch_lo; ok && ch < ch_hi; ++ch)
+              for (int ch = ch_lo; ok && ch <= ch_hi; ++ch)
                 {
                   const int rows_total = ch_cnt[ch] * R;
-                  for (int t0 = 0; ok && t0 < rows_total; t0 += TC_ROWS, ++tile)
+                  for (int t0 = first_row(ch); ok && t0 < end_row(ch, rows_total); t0 += TC_ROWS, ++tile)
                     {
                       const int a = tile & 1, use_a = tile >> 1;
                       if (use_a > 0 &&
@@ -366,19 +369,18 @@ namespace pibem
                             }
                           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                           const uint32_t st = base + uint32_t(s) * lay.stage_bytes;
-                          const uint32_t ah = st, al = st + TC_A_BYTES, bh = st + 2 * TC_A_BYTES,
-                                         bl = bh + lay.b_bytes;
+                          // descriptors differ in their start address (16-byte units)
+                          const uint64_t dah = smem_desc_sw128(st),
+                                         dal = smem_desc_sw128(st + TC_A_BYTES),
+                                         dbh = smem_desc_sw128(st + 2 * TC_A_BYTES),
+                                         dbl = smem_desc_sw128(st + 2 * TC_A_BYTES + lay.b_bytes);
 #pragma unroll
                           for (int ks = 0; ks < TC_KC / 8; ++ks)
                             {
-                              const uint32_t off = uint32_t(ks) * 32;
-                              const uint64_t dah = smem_desc_sw128(ah + off),
-                                             dal = smem_desc_sw128(al + off),
-                                             dbh = smem_desc_sw128(bh + off),
-                                             dbl = smem_desc_sw128(bl + off);
-                              mma_tf32(d, dah, dbh, idesc, (kc > 0 || ks > 0) ? 1u : 0u);
-                              mma_tf32(d, dal, dbh, idesc, 1u);
-                              mma_tf32(d, dah, dbl, idesc, 1u);
+                              const uint64_t o = uint64_t(2 * ks);
+                              mma_tf32(d, dah + o, dbh + o, idesc, (kc > 0 || ks > 0) ? 1u : 0u);
+                              mma_tf32(d, dal + o, dbh + o, idesc, 1u);
+                              mma_tf32(d, dah + o, dbl + o, idesc, 1u);
                             }
                           mma_commit(empty(s)); // frees the stage once these MMAs are done
                           issued = true;
@@ -411,10 +413,10 @@ namespace pibem
           const bool     bulk  = (K & 1) != 0;
           bool           pending = false; // a bulk store of this warp may still read stg
           int            tile    = 0;
-          for (int ch = ch_lo; ok && ch < ch_hi; ++ch)
+          for (int ch = ch_lo; ok && ch <= ch_hi; ++ch)
             {
               const int start = ch_start[ch], rows_total = ch_cnt[ch] * R;
-              for (int t0 = 0; ok && t0 < rows_total; t0 += TC_ROWS, ++tile)
+              for (int t0 = first_row(ch); ok && t0 < end_row(ch, rows_total); t0 += TC_ROWS, ++tile)
                 {
                   const int a = tile & 1;
                   if (!mbar_wait(tfull(a), uint32_t(tile >> 1) & 1u, &abort_flag))

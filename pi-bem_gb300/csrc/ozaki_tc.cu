@@ -37,7 +37,7 @@
 // between the roles.  Measured (GB300; before: one accumulator set of 96 columns, the
 // epilogue after the MMAs, a row loaded and stored by one thread, and the CUDA-core
 // float-float GEMM beyond K = 96): 98k spheroid (p = 8, 272,776 pairs) 441 -> 281 us,
-// 198k hull (p = 10) 5,920 -> 840 us, 16 columns at 23,816 nodes 1,754 -> 1,016 us.
+// 198k hull (p = 10) 5,920 -> 840 us, 16 columns at 23,816 nodes 1,754 -> 814 us.
 // (One MMA per slice pair 426 / 1,191 us for the first two, four epilogue warps
 // 318 / 895.)
 // All waits are bounded; a timeout is recorded in *err and the host reports
@@ -183,21 +183,21 @@ namespace pibem
     // The block's units in order, f(operator, part, first pair, rows of the chunk,
     // first row): every role walks the same list.
     template <typename F>
-    __device__ __forceinline__ void oz_units(const OzArgs &a, F f)
+    __device__ __forceinline__ void oz_units(const OzArgs &a, const TileRange &tr, F f)
     {
-      const int ch_lo = a.chunk0 + int(int64_t(a.n_chunks) * blockIdx.x / gridDim.x);
-      const int ch_hi = a.chunk0 + int(int64_t(a.n_chunks) * (blockIdx.x + 1) / gridDim.x);
       const int parts = oz_parts(a.K);
-      for (int ch = ch_lo, end; ch < ch_hi; ch = end)
+      for (int ch = tr.c_lo, end; ch <= tr.c_hi; ch = end)
         {
           const int op = a.ch_op[ch];
-          for (end = ch + 1; end < ch_hi && a.ch_op[end] == op;)
+          for (end = ch + 1; end <= tr.c_hi && a.ch_op[end] == op;)
             ++end;
           for (int part = 0; part < parts; ++part)
             for (int c = ch; c < end; ++c)
               {
                 const int start = a.ch_start[c], rows = a.ch_cnt[c] * a.R;
-                for (int t0 = 0; t0 < rows; t0 += OZ_ROWS)
+                const int first = c == tr.c_lo ? tr.t_lo * OZ_ROWS : 0;
+                const int last  = c == tr.c_hi ? min(rows, tr.t_hi * OZ_ROWS) : rows;
+                for (int t0 = first; t0 < last; t0 += OZ_ROWS)
                   f(op, part, start, rows, t0);
               }
         }
@@ -260,6 +260,9 @@ namespace pibem
                        : "memory");
           asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
+      TileRange range = tile_range(a.ch_cnt + a.chunk0, a.n_chunks, R);
+      range.c_lo += a.chunk0;
+      range.c_hi += a.chunk0;
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncthreads();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -274,7 +277,7 @@ namespace pibem
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive(a_full(int(st % OZ_RING)));
           };
-          oz_units(a, [&](int, int, int start, int rows, int t0) {
+          oz_units(a, range, [&](int, int, int start, int rows, int t0) {
             int *src = rows_src[unit & 1];
             {
               const int row = t0 + tid;
@@ -325,7 +328,7 @@ namespace pibem
               int  held_op = -1, held_part = -1, b_loads = 0, unit = 0;
               long g      = 0;
               bool issued = false, b_pending = false;
-              oz_units(a, [&](int op, int part, int, int, int) {
+              oz_units(a, range, [&](int op, int part, int, int, int) {
                 if (op != held_op || part != held_part)
                   {
                     if (issued) // the MMAs that read the held tiles
@@ -400,7 +403,7 @@ namespace pibem
                                                    size_t(warp - 4) * OZ_STG_BYTES);
           const int n_ec = oz_parts(K) * OZ_NP;
           int       unit = 0;
-          oz_units(a, [&](int op, int part, int start, int rows, int t0) {
+          oz_units(a, range, [&](int op, int part, int start, int rows, int t0) {
             const int buf = unit & 1, row0 = t0 + 32 * q, nvalid = min(32, rows - row0);
             int       er = 0;
             if (lane < nvalid)
