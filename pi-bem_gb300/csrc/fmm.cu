@@ -743,174 +743,156 @@ namespace pibem
     // Batched translation GEMM.  Scaled operators do not depend on the level:
     // M2L depends only on the integer source-target offset, M2M / L2L only on
     // the child octant.  Pairs sharing an operator are cut into chunks of <= 128;
-    // block (c, t) computes  Y[q] = T_op(c) E[src(q)]  for columns 64t..64t+63 of
-    // chunk c (column = (pair, rhs)), with the operator staged in shared memory
-    // (CUDA-core FMA, 16x16 threads, KI x 4 outputs per thread, KI = ceil(K/16)
-    // so that no thread computes rows beyond K).
-    constexpr int GB_COLS = 64;
-    constexpr int GB_LDB  = GB_COLS + 1;
-
-    template <typename T, int KI>
-    __global__ void __launch_bounds__(256, 2)
-      trans_gemm_kernel(int R, int K, int chunk0, const int32_t *__restrict__ chunk_start,
-                        const int32_t *__restrict__ chunk_cnt, const int32_t *__restrict__ chunk_off,
-                        const int32_t *__restrict__ q_src, const T *__restrict__ ops,
-                        const T *__restrict__ M, T *__restrict__ Y,
-                        const int32_t *__restrict__ yslot, int ldy)
-    {
-      extern __shared__ unsigned char smem_raw[];
-      T        *sT    = reinterpret_cast<T *>(smem_raw); // [K][K] in-major
-      T        *sB    = sT + K * K;                      // [K][GB_LDB]
-      const int ch    = chunk0 + blockIdx.x;
-      const int start = chunk_start[ch], ncols = chunk_cnt[ch] * R;
-      const int c0    = blockIdx.y * GB_COLS;
-      if (c0 >= ncols)
-        return;
-      const int nc = min(GB_COLS, ncols - c0);
-      const T  *op = ops + int64_t(chunk_off[ch]) * K * K;
-      for (int i = threadIdx.x; i < K * K; i += blockDim.x)
-        sT[i] = op[i];
-      for (int idx = threadIdx.x; idx < nc * K; idx += blockDim.x)
-        {
-          const int     c  = idx / K, ki = idx - c * K;
-          const int     cg = c0 + c;
-          const int64_t q  = start + cg / R;
-          const int     r  = cg % R;
-          sB[ki * GB_LDB + c] = M[(int64_t(q_src[q]) * R + r) * K + ki];
-        }
-      __syncthreads();
-      // rows ko = row0 + tx + 16 i of this block (row0 > 0 when the rows are split
-      // over blockIdx.z for launches with few blocks)
-      const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, row0 = blockIdx.z * 16 * KI;
-      T         acc[KI][4];
-#pragma unroll
-      for (int i = 0; i < KI; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          acc[i][j] = T(0);
-      for (int ki = 0; ki < K; ++ki)
-        {
-          T a[KI], b[4];
-#pragma unroll
-          for (int i = 0; i < KI; ++i)
-            {
-              const int ko = row0 + tx + 16 * i;
-              a[i]         = ko < K ? sT[ki * K + ko] : T(0);
-            }
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            b[j] = sB[ki * GB_LDB + ty + 16 * j];
-#pragma unroll
-          for (int i = 0; i < KI; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              acc[i][j] = fma_rn(a[i], b[j], acc[i][j]);
-        }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        {
-          const int c = ty + 16 * j;
-          if (c >= nc)
-            continue;
-          const int     cg = c0 + c;
-          const int64_t q  = start + cg / R;
-          const int     r  = cg % R;
-          const int64_t yr = (yslot ? int64_t(yslot[q]) : q) * R + r; // row of (pair, rhs)
-#pragma unroll
-          for (int i = 0; i < KI; ++i)
-            {
-              const int ko = row0 + tx + 16 * i;
-              if (ko < K)
-                Y[yr * ldy + ko] = acc[i][j];
-            }
-        }
-    }
-
+    // block (c, t, z) computes  Y[q] = T_op(c) E[src(q)]  for TY CJ columns of chunk c
+    // (column = (pair, rhs)) from the t-th group on and rows z TX RI ... + TX RI - 1,
+    // the operator's rows and the columns staged in shared memory.  Thread (tx, ty) of
+    // TX x TY computes rows tx + TX i (i < RI) and columns ty + TY j (j < CJ), k ascending.
+    // Arithmetic: the type's FMA, or float-float on the FP32 pipes (OP = float2, the
+    // operator pre-split into (hi, lo) pairs; the expansions in that form too or, IO =
+    // double, split on load and joined on store).
+    //   What bounds it: the arithmetic, above all FP64's two FMA per clock and SM.  So
+    // no thread computes rows beyond the block's (TX = ceil(K / RI)), and the columns a
+    // chunk does not have are left out (most chunks of small meshes and of the small
+    // levels hold a few pairs): the columns per thread are rounded up to 1, 2, 4 or 8,
+    // and threads without a column leave.  Measured (GB300, one column,
+    // against 64-column tiles computed whole): FP64 M2L at 13,826 nodes 749 -> 570 us and
+    // M2M / L2L levels 38 -> 13; float-float levels at 198k nodes 77 -> 30, at 98k 28 -> 18;
+    // FP64 M2L at 386 nodes 155 -> 78.
     __device__ __forceinline__ float2 ff_load(const double *p) { return ff_split(*p); }
     __device__ __forceinline__ float2 ff_load(const float2 *p) { return *p; }
     __device__ __forceinline__ void   ff_store(double *p, float h, float l) { *p = __dadd_rn(double(h), double(l)); }
     __device__ __forceinline__ void   ff_store(float2 *p, float h, float l) { *p = ff_norm(h, l); }
 
-    // The translation GEMM of the FP64 operator in float-float arithmetic on
-    // the FP32 pipes: operator pre-split into (hi, lo) pairs; expansions and
-    // products either FP64 (split on load, joined on store) or already in
-    // (hi, lo) form (IO = float2: no FP64 instruction at all).  Thread (tx, ty)
-    // of TX x (64 / CJ) computes rows row0 + tx + TX i (i < RI) and columns
-    // ty + (64 / CJ) j (j < CJ) of a 64-column block of chunk c; TX RI >= K
-    // rows with TX = ceil(K / RI), so at most RI - 1 rows are padding.
-    template <int RI, int CJ, typename IO>
-    __global__ void __launch_bounds__(256, 2)
-      ff_gemm_kernel(int R, int K, int TX, int chunk0, const int32_t *__restrict__ chunk_start,
-                     const int32_t *__restrict__ chunk_cnt, const int32_t *__restrict__ chunk_off,
-                     const int32_t *__restrict__ q_src, const float2 *__restrict__ ops,
-                     const IO *__restrict__ M, IO *__restrict__ Y)
+    // one running sum: plain (OP = IO) or float-float
+    template <typename OP>
+    struct GemmSum
     {
+      OP s = OP(0);
+      __device__ __forceinline__ void mac(OP a, OP b) { s = fma_rn(a, b, s); }
+      __device__ __forceinline__ void store(OP *p) const { *p = s; }
+      __device__ static OP            load(const OP *p) { return *p; }
+      __device__ static OP            zero() { return OP(0); }
+    };
+    template <>
+    struct GemmSum<float2>
+    {
+      float h = 0.0f, l = 0.0f;
+      __device__ __forceinline__ void mac(float2 a, float2 b) { ff_mac(h, l, a, b); }
+      template <typename IO>
+      __device__ __forceinline__ void store(IO *p) const
+      {
+        ff_store(p, h, l);
+      }
+      template <typename IO>
+      __device__ static float2 load(const IO *p)
+      {
+        return ff_load(p);
+      }
+      __device__ static float2 zero() { return make_float2(0.0f, 0.0f); }
+    };
+
+    template <typename IO, typename OP, int RI, int CJ, int TY>
+    __global__ void __launch_bounds__(256, 2)
+      trans_gemm_kernel(int R, int K, int TX, int chunk0, const int32_t *__restrict__ chunk_start,
+                        const int32_t *__restrict__ chunk_cnt, const int32_t *__restrict__ chunk_off,
+                        const int32_t *__restrict__ q_src, const OP *__restrict__ ops,
+                        const IO *__restrict__ M, IO *__restrict__ Y,
+                        const int32_t *__restrict__ yslot, int ldy)
+    {
+      using Sum = GemmSum<OP>;
+      constexpr int COLS = TY * CJ, LDB = COLS + 1;
       extern __shared__ __align__(16) unsigned char smem_raw[];
-      float2   *sT    = reinterpret_cast<float2 *>(smem_raw); // [K][K] in-major
-      float2   *sB    = sT + K * K;                           // [K][GB_LDB]
+      const int W     = TX * RI;                        // rows of this block
+      OP       *sT    = reinterpret_cast<OP *>(smem_raw); // [K][W] in-major
+      OP       *sB    = sT + K * W;                       // [K][LDB]
       const int ch    = chunk0 + blockIdx.x;
       const int start = chunk_start[ch], ncols = chunk_cnt[ch] * R;
-      const int c0    = blockIdx.y * GB_COLS;
+      const int c0    = blockIdx.y * COLS;
       if (c0 >= ncols)
         return;
-      const int     nc = min(GB_COLS, ncols - c0);
-      const float2 *op = ops + int64_t(chunk_off[ch]) * K * K;
-      for (int i = threadIdx.x; i < K * K; i += blockDim.x)
-        sT[i] = op[i];
-      for (int idx = threadIdx.x; idx < nc * K; idx += blockDim.x)
+      const int nc = min(COLS, ncols - c0), row0 = blockIdx.z * W;
+      const OP *op = ops + int64_t(chunk_off[ch]) * K * K;
+      for (int i0 = threadIdx.x; i0 < K * W; i0 += 8 * blockDim.x)
         {
-          const int     c  = idx / K, ki = idx - c * K;
-          const int     cg = c0 + c;
-          const int64_t q  = start + cg / R;
-          const int     r  = cg % R;
-          sB[ki * GB_LDB + c] = ff_load(M + (int64_t(q_src[q]) * R + r) * K + ki);
+          OP v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            {
+              const int i = i0 + u * blockDim.x, ki = i / W, ko = row0 + i - ki * W;
+              v[u]        = i < K * W && ko < K ? op[ki * K + ko] : Sum::zero();
+            }
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (i0 + u * blockDim.x < K * W)
+              sT[i0 + u * blockDim.x] = v[u];
+        }
+      for (int i0 = threadIdx.x; i0 < nc * K; i0 += 4 * blockDim.x)
+        {
+          OP v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            {
+              const int i = i0 + u * blockDim.x, c = i / K, cg = c0 + c;
+              if (i < nc * K)
+                v[u] = Sum::load(M + (int64_t(q_src[start + cg / R]) * R + cg % R) * K + (i - c * K));
+            }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            {
+              const int i = i0 + u * blockDim.x, c = i / K;
+              if (i < nc * K)
+                sB[(i - c * K) * LDB + c] = v[u];
+            }
         }
       __syncthreads();
-      constexpr int TY = 64 / CJ;
-      const int     tx = threadIdx.x % TX, ty = threadIdx.x / TX, row0 = blockIdx.z * TX * RI;
-      if (ty >= TY)
+      const int     tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+      if (ty >= TY || ty >= nc)
         return;
-      float sh[RI][CJ], sl[RI][CJ];
+      auto run = [&](auto nj) {
+        constexpr int NJ = decltype(nj)::value;
+        Sum           acc[RI][NJ];
+        for (int ki = 0; ki < K; ++ki)
+          {
+            OP a[RI], b[NJ];
 #pragma unroll
-      for (int i = 0; i < RI; ++i)
+            for (int i = 0; i < RI; ++i)
+              a[i] = sT[ki * W + tx + TX * i];
 #pragma unroll
-        for (int j = 0; j < CJ; ++j)
-          sh[i][j] = sl[i][j] = 0.0f;
-      for (int ki = 0; ki < K; ++ki)
-        {
-          float2 a[RI], b[CJ];
+            for (int j = 0; j < NJ; ++j)
+              b[j] = sB[ki * LDB + ty + TY * j];
 #pragma unroll
-          for (int i = 0; i < RI; ++i)
-            {
-              const int ko = row0 + tx + TX * i;
-              a[i]         = ko < K ? sT[ki * K + ko] : make_float2(0.0f, 0.0f);
-            }
+            for (int i = 0; i < RI; ++i)
 #pragma unroll
-          for (int j = 0; j < CJ; ++j)
-            b[j] = sB[ki * GB_LDB + ty + TY * j];
+              for (int j = 0; j < NJ; ++j)
+                acc[i][j].mac(a[i], b[j]);
+          }
 #pragma unroll
-          for (int i = 0; i < RI; ++i)
+        for (int j = 0; j < NJ; ++j)
+          {
+            const int c = ty + TY * j;
+            if (c >= nc)
+              continue;
+            const int     cg = c0 + c;
+            const int64_t q  = start + cg / R;
+            const int64_t yr = (yslot ? int64_t(yslot[q]) : q) * R + cg % R; // row of (pair, rhs)
 #pragma unroll
-            for (int j = 0; j < CJ; ++j)
-              ff_mac(sh[i][j], sl[i][j], a[i], b[j]);
-        }
-#pragma unroll
-      for (int j = 0; j < CJ; ++j)
-        {
-          const int c = ty + TY * j;
-          if (c >= nc)
-            continue;
-          const int     cg = c0 + c;
-          const int64_t q  = start + cg / R;
-          const int     r  = cg % R;
-#pragma unroll
-          for (int i = 0; i < RI; ++i)
-            {
-              const int ko = row0 + tx + TX * i;
-              if (ko < K)
-                ff_store(Y + (q * R + r) * K + ko, sh[i][j], sl[i][j]);
-            }
-        }
+            for (int i = 0; i < RI; ++i)
+              {
+                const int ko = row0 + tx + TX * i;
+                if (ko < K)
+                  acc[i][j].store(Y + yr * ldy + ko);
+              }
+          }
+      };
+      const int nj = (nc + TY - 1) / TY; // columns per thread, the block's most
+      if (CJ == 1 || nj <= 1)
+        run(std::integral_constant<int, 1>());
+      else if (CJ == 2 || nj <= 2)
+        run(std::integral_constant<int, CJ < 2 ? CJ : 2>());
+      else if (CJ == 4 || nj <= 4)
+        run(std::integral_constant<int, CJ < 4 ? CJ : 4>());
+      else
+        run(std::integral_constant<int, CJ>());
     }
 
     // out[box] = sum of the box's (hi, lo) translation products, in list order,
@@ -1564,44 +1546,57 @@ namespace pibem
     return op.down_par && op.down_m2l_beg && fused_levels_ok(op.K, R);
   }
 
-  // The float-float translation GEMM for chunks [c0, c1); IO = double (FP64
-  // expansions) or float2 ((hi, lo) expansions).  A launch with fewer blocks
-  // than ~2 per SM splits the rows over blockIdx.z (16 per block).
+  // The CUDA-core translation GEMM for chunks [c0, c1): K / 32 rows per thread, at most
+  // 4, and eight threads across 64 columns (32 in FP64, whose blocks take so long that
+  // the last wave of 64-column ones left a third of the chip idle).  A launch with fewer
+  // than 256 blocks of 64 columns (the tree's small levels) splits the rows over
+  // blockIdx.z, 16 per block, and takes 16 (FP64) or 32 columns per block.
+  template <typename IO, typename OP>
+  static void launch_cuda_core_gemm(int K, int max_chunk_pairs, int R, int c0,
+                                    int c1, const int32_t *ch_start, const int32_t *ch_cnt,
+                                    const int32_t *ch_op, const int32_t *q_src, const OP *ops, const IO *E,
+                                    IO *Y, const int32_t *yslot, int ldy, cudaStream_t s)
+  {
+    if (c1 <= c0)
+      return;
+    if (K > 128)
+      throw Error(PIBEM_EINVAL, "translations: K = (p+1)^2 above 128");
+    constexpr bool fp64  = std::is_same<OP, double>::value;
+    const unsigned gx    = unsigned(c1 - c0);
+    const int      most  = max_chunk_pairs * R; // columns of a chunk
+    const bool     split = int64_t(gx) * ((most + 63) / 64) < 256;
+    const int      RI    = split ? 1 : std::min(4, (K + 31) / 32);
+    const int      TX    = split ? 16 : (K + RI - 1) / RI;
+    auto launch = [&](auto kern, int CJ, int TY) {
+      const int    cols = CJ * TY;
+      const size_t smem = (size_t(K) * TX * RI + size_t(K) * (cols + 1)) * sizeof(OP);
+      const dim3   grid(gx, unsigned((most + cols - 1) / cols), split ? unsigned((K + 15) / 16) : 1u);
+      if (smem > 48 * 1024)
+        raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
+      kern<<<grid, TY * TX, smem, s>>>(R, K, TX, c0, ch_start, ch_cnt, ch_op, q_src, ops, E, Y, yslot, ldy);
+    };
+    constexpr int CJ = fp64 ? 4 : 8, CJS = fp64 ? 1 : 2;
+    if (split)
+      launch(trans_gemm_kernel<IO, OP, 1, CJS, 16>, CJS, 16);
+    else
+      switch (RI)
+        {
+          case 1: launch(trans_gemm_kernel<IO, OP, 1, CJ, 8>, CJ, 8); break;
+          case 2: launch(trans_gemm_kernel<IO, OP, 2, CJ, 8>, CJ, 8); break;
+          case 3: launch(trans_gemm_kernel<IO, OP, 3, CJ, 8>, CJ, 8); break;
+          default: launch(trans_gemm_kernel<IO, OP, 4, CJ, 8>, CJ, 8); break;
+        }
+    PIBEM_CUDA(cudaGetLastError());
+    note_launch();
+  }
+
+  // in float-float: IO = double (FP64 expansions) or float2 ((hi, lo) expansions)
   template <typename IO>
   void launch_ff_gemm(const OperatorDev<double> &op, int R, int c0, int c1, const IO *E, IO *Y,
                       cudaStream_t s)
   {
-    if (c1 <= c0)
-      return;
-    const int      K  = op.K;
-    const unsigned gx = unsigned(c1 - c0),
-                   gy = unsigned((op.max_chunk_pairs * R + GB_COLS - 1) / GB_COLS);
-    const bool     split = int64_t(gx) * gy < 256;
-    const int      RI    = split ? 1 : std::min(4, (K + 31) / 32);
-    const int      TX    = split ? 16 : (K + RI - 1) / RI;
-    const int      CJ    = split ? 4 : 8; // columns per thread (split: 16 x 16 threads)
-    const dim3     grid(gx, gy, split ? unsigned((K + 15) / 16) : 1u);
-    const size_t   smem = (size_t(K) * K + size_t(K) * GB_LDB) * sizeof(float2);
-    if (K > 128)
-      throw Error(PIBEM_EINVAL, "float-float translations: K = (p+1)^2 above 128");
-    auto launch = [&](auto kern) {
-      if (smem > 48 * 1024)
-        raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
-      kern<<<grid, (64 / CJ) * TX, smem, s>>>(R, K, TX, c0, op.ch_start, op.ch_cnt, op.ch_op,
-                                              op.q_src, op.ops_ff, E, Y);
-    };
-    if (CJ == 4)
-      launch(ff_gemm_kernel<1, 4, IO>);
-    else
-      switch (RI)
-        {
-          case 1: launch(ff_gemm_kernel<1, 8, IO>); break;
-          case 2: launch(ff_gemm_kernel<2, 8, IO>); break;
-          case 3: launch(ff_gemm_kernel<3, 8, IO>); break;
-          default: launch(ff_gemm_kernel<4, 8, IO>); break;
-        }
-    PIBEM_CUDA(cudaGetLastError());
-    note_launch();
+    launch_cuda_core_gemm<IO, float2>(op.K, op.max_chunk_pairs, R, c0, c1, op.ch_start, op.ch_cnt,
+                                      op.ch_op, op.q_src, op.ops_ff, E, Y, nullptr, op.K, s);
   }
   template void launch_ff_gemm<double>(const OperatorDev<double> &, int, int, int, const double *,
                                        double *, cudaStream_t);
@@ -1671,40 +1666,14 @@ namespace pibem
           launch_tc_gemm(op, R, c0, c1, E, Y, yslot, ldy, op.tc_err, s);
           return;
         }
-    // largest column count of the chunks in [c0, c1): R x (<= 128 pairs).  A
-    // launch with fewer blocks than ~2 per SM (the tree's small levels) splits
-    // each block's rows over blockIdx.z (16 rows per block) for parallelism.
-    const unsigned gx = unsigned(c1 - c0),
-                   gy = unsigned((op.max_chunk_pairs * R + GB_COLS - 1) / GB_COLS);
-    const bool     split = int64_t(gx) * gy < 256;
-    const int      KI    = split ? 1 : (op.K + 15) / 16;
-    const dim3     grid(gx, gy, split ? unsigned((op.K + 15) / 16) : 1u);
     if constexpr (std::is_same<T, double>::value)
       if (op.ops_ff)
         {
           launch_ff_gemm<double>(op, R, c0, c1, E, Y, s);
           return;
         }
-    const size_t smem = (size_t(op.K) * op.K + size_t(op.K) * GB_LDB) * sizeof(T);
-    auto launch = [&](auto kern) {
-      if (smem > 48 * 1024)
-        raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
-      kern<<<grid, 256, smem, s>>>(R, op.K, c0, op.ch_start, op.ch_cnt, op.ch_op, op.q_src, op.ops,
-                                   E, Y, yslot, ldy);
-    };
-    switch (KI)
-      {
-        case 1: launch(trans_gemm_kernel<T, 1>); break;
-        case 2: launch(trans_gemm_kernel<T, 2>); break;
-        case 3: launch(trans_gemm_kernel<T, 3>); break;
-        case 4: launch(trans_gemm_kernel<T, 4>); break;
-        case 5: launch(trans_gemm_kernel<T, 5>); break;
-        case 6: launch(trans_gemm_kernel<T, 6>); break;
-        case 7: launch(trans_gemm_kernel<T, 7>); break;
-        default: launch(trans_gemm_kernel<T, 8>); break;
-      }
-    PIBEM_CUDA(cudaGetLastError());
-    note_launch();
+    launch_cuda_core_gemm<T, T>(op.K, op.max_chunk_pairs, R, c0, c1, op.ch_start, op.ch_cnt, op.ch_op,
+                                op.q_src, op.ops, E, Y, yslot, ldy, s);
   }
 
   template <typename T>
