@@ -642,16 +642,17 @@ namespace pibem
     // instead of two); T1 is then Tc and T2 is unused.
     // RC: columns per block (1 for one right-hand side, else 4; the groups of columns
     // over blockIdx.y: a few hundred leaves alone would leave most of the chip idle).
-    template <typename T, bool COMBINED, int RC>
+    template <bool COMBINED, int RC>
     __global__ void __launch_bounds__(256)
       p2m_apply_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ prow_ptr,
                        const int32_t *__restrict__ pleaf_box, const int32_t *__restrict__ prow_dof,
-                       const T *__restrict__ T1, const T *__restrict__ T2,
+                       const float *__restrict__ T1, const float *__restrict__ T2,
                        const uint8_t *__restrict__ dir, const uint8_t *__restrict__ modes,
-                       const T *__restrict__ x, T *__restrict__ M)
+                       const float *__restrict__ x, float *__restrict__ M)
     {
+      using T = float;
       pdl_entry();
-      const int leaf = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
       if (leaf >= n_leaves)
         return;
       const int     K4  = (K + 3) / 4 * 4;
@@ -737,6 +738,169 @@ namespace pibem
                 for (int c = 0; c < 4; ++c)
                   if (4 * lane + c < K)
                     M[(box * R + rq + rr) * K + 4 * lane + c] = acc[rr][c];
+        }
+    }
+
+    // P2M apply in FP64: the same sums (rows in order), but lane l owns coefficients l,
+    // l + 32, ... (NPL of them): the FP64 pipe takes a warp's FMA in the same time however
+    // many lanes have work, and ceil(K / 32) FMA a row replace 4.  A column of one layer
+    // only (KER1 / KER2) skips the other layer's table and products.  Bounded by those FMA and,
+    // on small meshes, by the rows' serial chain.  GB300, two columns at 386 nodes: 36 us with
+    // four coefficients a lane and eight warps a block -> 11.8.
+    template <bool COMBINED, int RC, int NPL>
+    __global__ void __launch_bounds__(256)
+      p2m_apply64_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ prow_ptr,
+                         const int32_t *__restrict__ pleaf_box, const int32_t *__restrict__ prow_dof,
+                         const double *__restrict__ T1, const double *__restrict__ T2,
+                         const uint8_t *__restrict__ dir, const uint8_t *__restrict__ modes,
+                         const double *__restrict__ x, double *__restrict__ M)
+    {
+      pdl_entry();
+      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      if (leaf >= n_leaves)
+        return;
+      const int     K4  = (K + 3) / 4 * 4;
+      const int64_t box = pleaf_box[leaf];
+      const int64_t rb = prow_ptr[leaf], re = prow_ptr[leaf + 1];
+      const int     rq = blockIdx.y * RC, rc = min(RC, R - rq);
+      int           mode[RC];
+      bool          one = COMBINED, two = false; // layers that some column takes
+#pragma unroll
+      for (int rr = 0; rr < RC; ++rr)
+        {
+          mode[rr] = COMBINED ? int(MODE_KER1) : (rr < rc ? int(modes[rq + rr]) : int(MODE_KER1));
+          if (!COMBINED && rr < rc)
+            {
+              one = one || mode[rr] != MODE_KER2;
+              two = two || mode[rr] != MODE_KER1;
+            }
+        }
+      double acc[RC][NPL];
+#pragma unroll
+      for (int rr = 0; rr < RC; ++rr)
+#pragma unroll
+        for (int c = 0; c < NPL; ++c)
+          acc[rr][c] = 0.0;
+      for (int64_t b0 = rb; b0 < re; b0 += 32)
+        {
+          const int nb = re - b0 < 32 ? int(re - b0) : 32;
+          double    w1[RC], w2[RC];
+#pragma unroll
+          for (int rr = 0; rr < RC; ++rr)
+            w1[rr] = w2[rr] = 0.0;
+          if (lane < nb)
+            {
+              const int  dof = prow_dof[b0 + lane];
+              const bool d   = !COMBINED && dir[dof] != 0;
+#pragma unroll
+              for (int rr = 0; rr < RC; ++rr)
+                if (rr < rc)
+                  {
+                    const double xv = x[int64_t(rq + rr) * N + dof];
+                    if constexpr (COMBINED)
+                      w1[rr] = xv;
+                    else
+                      {
+                        const bool dd = mode[rr] == MODE_SWAPPED ? !d : d;
+                        w1[rr] = mode[rr] == MODE_KER2 ? 0.0 : (mode[rr] == MODE_KER1 ? xv : (dd ? 0.0 : xv));
+                        w2[rr] = mode[rr] == MODE_KER1 ? 0.0 : (mode[rr] == MODE_KER2 ? xv : (dd ? -xv : 0.0));
+                      }
+                  }
+            }
+          for (int j0 = 0; j0 < nb; j0 += 8)
+            {
+              double t1[8][NPL], t2[COMBINED ? 1 : 8][NPL];
+#pragma unroll
+              for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int c = 0; c < NPL; ++c)
+                  {
+                    const bool   in = j0 + u < nb && lane + 32 * c < K4;
+                    const int64_t o = (b0 + j0 + u) * K4 + lane + 32 * c;
+                    t1[u][c]        = in && one ? T1[o] : 0.0;
+                    if constexpr (!COMBINED)
+                      t2[u][c] = in && two ? T2[o] : 0.0;
+                  }
+#pragma unroll
+              for (int u = 0; u < 8; ++u)
+                if (j0 + u < nb)
+#pragma unroll
+                  for (int rr = 0; rr < RC; ++rr)
+                    if (rr < rc)
+                      {
+                        const double a1 = __shfl_sync(0xffffffffu, w1[rr], j0 + u);
+                        if (COMBINED || mode[rr] != MODE_KER2)
+#pragma unroll
+                          for (int c = 0; c < NPL; ++c)
+                            acc[rr][c] = fma_rn(a1, t1[u][c], acc[rr][c]);
+                        if constexpr (!COMBINED)
+                          {
+                            const double a2 = __shfl_sync(0xffffffffu, w2[rr], j0 + u);
+                            if (mode[rr] != MODE_KER1)
+#pragma unroll
+                              for (int c = 0; c < NPL; ++c)
+                                acc[rr][c] = fma_rn(a2, t2[u][c], acc[rr][c]);
+                          }
+                      }
+            }
+        }
+#pragma unroll
+      for (int rr = 0; rr < RC; ++rr)
+        if (rr < rc)
+#pragma unroll
+          for (int c = 0; c < NPL; ++c)
+            if (lane + 32 * c < K)
+              M[(box * R + rq + rr) * K + lane + 32 * c] = acc[rr][c];
+    }
+
+    // L2P in FP64: lane l multiplies coefficients l, l + 32, ...; RR rows x RC columns are
+    // summed together by the butterfly's reduce-scatter (RR RC + 4 - log2(RR RC) additions
+    // instead of 5 RR RC, on a pipe where each takes as long as an FMA).  GB300, two columns
+    // at 386 nodes: 23 us as in FP32 -> 8.4.
+    template <int RC, int RR, int NPL>
+    __global__ void __launch_bounds__(256)
+      l2p64_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ row_ptr,
+                   const int32_t *__restrict__ lleaf_box, const int32_t *__restrict__ nrows,
+                   const double *__restrict__ W, const double *__restrict__ Lx, double *__restrict__ y)
+    {
+      pdl_entry();
+      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      if (leaf >= n_leaves)
+        return;
+      const int     K4  = (K + 3) / 4 * 4;
+      const int64_t box = lleaf_box[leaf];
+      const int64_t i0 = row_ptr[leaf], i1 = row_ptr[leaf + 1];
+      const int     ra = blockIdx.y * RC, rc = min(RC, R - ra);
+      double        l[RC][NPL];
+#pragma unroll
+      for (int r = 0; r < RC; ++r)
+#pragma unroll
+        for (int c = 0; c < NPL; ++c)
+          l[r][c] = r < rc && lane + 32 * c < K ? Lx[(box * R + ra + r) * K + lane + 32 * c] : 0.0;
+      for (int64_t i = i0; i < i1; i += RR)
+        {
+          double w[RR][NPL], v[RR * RC];
+#pragma unroll
+          for (int u = 0; u < RR; ++u)
+#pragma unroll
+            for (int c = 0; c < NPL; ++c)
+              w[u][c] = i + u < i1 && lane + 32 * c < K ? W[(i + u) * K4 + lane + 32 * c] : 0.0;
+#pragma unroll
+          for (int u = 0; u < RR; ++u)
+#pragma unroll
+            for (int r = 0; r < RC; ++r)
+              {
+                double s = mul_rn(w[u][0], l[r][0]);
+#pragma unroll
+                for (int c = 1; c < NPL; ++c)
+                  s = fma_rn(w[u][c], l[r][c], s);
+                v[u * RC + r] = s;
+              }
+          const double  t  = warp_sums<RR * RC>(v, [](double p, double q) { return p + q; });
+          constexpr int Wn = 32 / (RR * RC); // lanes per value
+          const int     u = lane / (Wn * RC), r = (lane / Wn) % RC;
+          if (lane % Wn == 0 && i + u < i1 && r < rc)
+            y[int64_t(ra + r) * N + nrows[i + u]] += t;
         }
     }
 
@@ -1209,7 +1373,7 @@ namespace pibem
                      const T *__restrict__ scratch, T *__restrict__ y)
     {
       pdl_entry();
-      const int ti = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int ti = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
       if (ti >= n_tgt)
         return;
       const int64_t  nn = tnode_ptr[ti + 1] - tnode_ptr[ti];
@@ -1251,14 +1415,15 @@ namespace pibem
     // column) value has the same roundings for every RC and RR.
     // One column: 8 rows (16-byte loads) in flight.  Several: a row of W is read once
     // for RC columns.
-    template <typename T, int RC, int RR>
+    template <int RC, int RR>
     __global__ void __launch_bounds__(256)
       l2p_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ row_ptr,
                  const int32_t *__restrict__ lleaf_box, const int32_t *__restrict__ nrows,
-                 const T *__restrict__ W, const T *__restrict__ Lx, T *__restrict__ y)
+                 const float *__restrict__ W, const float *__restrict__ Lx, float *__restrict__ y)
     {
+      using T = float;
       pdl_entry();
-      const int leaf = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
       if (leaf >= n_leaves)
         return;
       const int     K4  = (K + 3) / 4 * 4;
@@ -1325,7 +1490,7 @@ namespace pibem
                     const float2 *__restrict__ W, const float2 *__restrict__ Lx,
                     double *__restrict__ y)
     {
-      const int leaf = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
       if (leaf >= n_leaves)
         return;
       const int     K4  = (K + 3) / 4 * 4;
@@ -1396,12 +1561,25 @@ namespace pibem
 
   } // namespace
 
+  // Warps per block of the kernels that give a warp to each leaf or target box: at
+  // most 8, fewer while that leaves SMs without a block (a mesh of 1.5k nodes has some
+  // hundred leaves).  FMM product at 386 nodes with eight 218 us, so 178 (with the FP64
+  // P2M and L2P kernels)
+  static int leaf_warps(int64_t warps)
+  {
+    int w = 8;
+    while (w > 1 && warps < int64_t(w) * 2 * near_sm_count())
+      w /= 2;
+    return w;
+  }
+
   void launch_l2p_ff(const OperatorDev<double> &op, int R, int N, const float2 *Lff, double *y,
                      cudaStream_t s)
   {
     if (op.n_rows == 0 || op.n_near_leaves == 0)
       return;
-    l2p_ff_kernel<<<dim3(unsigned((op.n_near_leaves + 7) / 8), unsigned(R)), 256, 0, s>>>(
+    const int w = leaf_warps(int64_t(op.n_near_leaves) * R);
+    l2p_ff_kernel<<<dim3(unsigned((op.n_near_leaves + w - 1) / w), unsigned(R)), 32 * w, 0, s>>>(
       op.n_near_leaves, R, op.K, N, op.nrow_ptr, op.lleaf_box, op.nrows, op.Wff, Lff, y);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
@@ -1525,16 +1703,34 @@ namespace pibem
   {
     if (op.n_p2m_leaves == 0)
       return;
-    const dim3 grid(unsigned((op.n_p2m_leaves + 7) / 8), unsigned(R == 1 ? 1 : (R + 3) / 4));
     const bool comb = combined && op.Tc;
-    auto launch = [&](auto kern) {
-      launch_pdl(kern, grid, 256, 0, s, op.n_p2m_leaves, R, op.K, N, op.prow_ptr, op.pleaf_box, op.prow_dof,
-                                comb ? op.Tc : op.T1, op.T2, dir, modes, x, M);
+    auto launch = [&](auto kern, int rc) {
+      const int groups = (R + rc - 1) / rc, w = leaf_warps(int64_t(op.n_p2m_leaves) * groups);
+      launch_pdl(kern, dim3(unsigned((op.n_p2m_leaves + w - 1) / w), unsigned(groups)), 32 * w, 0, s,
+                 op.n_p2m_leaves, R, op.K, N, op.prow_ptr, op.pleaf_box, op.prow_dof,
+                 comb ? op.Tc : op.T1, op.T2, dir, modes, x, M);
     };
-    if (comb)
-      R == 1 ? launch(p2m_apply_kernel<T, true, 1>) : launch(p2m_apply_kernel<T, true, 4>);
+    if constexpr (std::is_same<T, double>::value)
+      {
+        auto by_k = [&](auto npl) {
+          constexpr int NPL = decltype(npl)::value;
+          if (comb)
+            R == 1 ? launch(p2m_apply64_kernel<true, 1, NPL>, 1) : launch(p2m_apply64_kernel<true, 4, NPL>, 4);
+          else
+            R == 1 ? launch(p2m_apply64_kernel<false, 1, NPL>, 1) : launch(p2m_apply64_kernel<false, 2, NPL>, 2);
+        };
+        switch ((op.K + 31) / 32)
+          {
+            case 1: by_k(std::integral_constant<int, 1>()); break;
+            case 2: by_k(std::integral_constant<int, 2>()); break;
+            case 3: by_k(std::integral_constant<int, 3>()); break;
+            default: by_k(std::integral_constant<int, 4>()); break;
+          }
+      }
+    else if (comb)
+      R == 1 ? launch(p2m_apply_kernel<true, 1>, 1) : launch(p2m_apply_kernel<true, 4>, 4);
     else
-      R == 1 ? launch(p2m_apply_kernel<T, false, 1>) : launch(p2m_apply_kernel<T, false, 4>);
+      R == 1 ? launch(p2m_apply_kernel<false, 1>, 1) : launch(p2m_apply_kernel<false, 4>, 4);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
@@ -1759,7 +1955,8 @@ namespace pibem
       eval(m2p_eval_kernel<T, 8>, 8);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
-    launch_pdl(m2p_sum_kernel<T>, dim3(unsigned((op.n_m2p_tgt + 7) / 8), unsigned(R)), 256, 0, s, 
+    const int w = leaf_warps(int64_t(op.n_m2p_tgt) * R);
+    launch_pdl(m2p_sum_kernel<T>, dim3(unsigned((op.n_m2p_tgt + w - 1) / w), unsigned(R)), 32 * w, 0, s,
       op.n_m2p_tgt, N, op.n_m2p_items, op.m2p_tnode_ptr, op.m2p_src_ptr, op.m2p_item_ptr,
       op.m2p_tnodes, op.m2p_scratch, y);
     PIBEM_CUDA(cudaGetLastError());
@@ -1782,7 +1979,8 @@ namespace pibem
       eval(m2p_eval_ff_kernel<4>, 4);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
-    m2p_sum_kernel<double><<<dim3(unsigned((op.n_m2p_tgt + 7) / 8), unsigned(R)), 256, 0, s>>>(
+    const int w = leaf_warps(int64_t(op.n_m2p_tgt) * R);
+    m2p_sum_kernel<double><<<dim3(unsigned((op.n_m2p_tgt + w - 1) / w), unsigned(R)), 32 * w, 0, s>>>(
       op.n_m2p_tgt, N, op.n_m2p_items, op.m2p_tnode_ptr, op.m2p_src_ptr, op.m2p_item_ptr,
       op.m2p_tnodes, op.m2p_scratch, y);
     PIBEM_CUDA(cudaGetLastError());
@@ -1809,13 +2007,33 @@ namespace pibem
     if (op.n_rows == 0 || op.n_near_leaves == 0)
       return;
     auto launch = [&](auto kern, int rc) {
-      launch_pdl(kern, dim3(unsigned((op.n_near_leaves + 7) / 8), unsigned((R + rc - 1) / rc)), 256, 0, s,
+      const int groups = (R + rc - 1) / rc, w = leaf_warps(int64_t(op.n_near_leaves) * groups);
+      launch_pdl(kern, dim3(unsigned((op.n_near_leaves + w - 1) / w), unsigned(groups)), 32 * w, 0, s,
                  op.n_near_leaves, R, op.K, N, op.nrow_ptr, op.lleaf_box, op.nrows, op.W, Lx, y);
     };
-    if (R == 1)
-      launch(l2p_kernel<T, 1, 8>, 1);
+    if constexpr (std::is_same<T, double>::value)
+      {
+        auto by_k = [&](auto npl) {
+          constexpr int NPL = decltype(npl)::value;
+          if (R == 1)
+            launch(l2p64_kernel<1, 8, NPL>, 1);
+          else if (R <= 3)
+            launch(l2p64_kernel<2, 4, NPL>, 2);
+          else
+            launch(l2p64_kernel<4, 4, NPL>, 4);
+        };
+        switch ((op.K + 31) / 32)
+          {
+            case 1: by_k(std::integral_constant<int, 1>()); break;
+            case 2: by_k(std::integral_constant<int, 2>()); break;
+            case 3: by_k(std::integral_constant<int, 3>()); break;
+            default: by_k(std::integral_constant<int, 4>()); break;
+          }
+      }
+    else if (R == 1)
+      launch(l2p_kernel<1, 8>, 1);
     else
-      launch(l2p_kernel<T, 4, 4>, 4);
+      launch(l2p_kernel<4, 4>, 4);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }

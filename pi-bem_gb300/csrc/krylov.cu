@@ -1289,10 +1289,14 @@ namespace pibem
         // beside two blocks per SM; else one, with fewer warps for very large leaves
         const size_t one = size_t(bp.max_rows) * sizeof(P);
         const bool   big = 16 * one + head > 200 * 1024;
-        const int    nw  = big ? 8 : 16;
+        // 16 warps a block (a warp per column in the Givens step), fewer while SMs would
+        // go without a block
+        int nw = big ? 8 : 16;
+        while (nw > 4 && bp.n_leaves < int64_t(nw) * AR_MAX_BLOCKS && nw / 2 >= a.Ra)
+          nw /= 2;
         const int64_t nb = std::min<int64_t>(2 * AR_MAX_BLOCKS, (bp.n_leaves + nw - 1) / nw);
         if (a.Ra > 1 && 64 * one + head <= 100 * 1024)
-          launch(arnoldi_finish_kernel<P, OUT, true, 4, false>, AR_THREADS, nb, head + 64 * one);
+          launch(arnoldi_finish_kernel<P, OUT, true, 4, false>, 32 * nw, nb, head + 4 * nw * one);
         else
           launch(arnoldi_finish_kernel<P, OUT, true, 1, false>, 32 * nw, nb, head + nw * one);
       }

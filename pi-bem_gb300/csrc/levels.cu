@@ -467,7 +467,10 @@ namespace pibem
     if (b <= a)
       return;
     const int64_t ncols = int64_t(b - a) * R;
-    launch_pdl(m2l_sum_kernel, unsigned((ncols + 7) / 8), 256, 0, s,
+    int w = 8; // a warp per column, fewer per block while SMs would go without one
+    while (w > 1 && ncols < int64_t(w) * 2 * lv_n_sm())
+      w /= 2;
+    launch_pdl(m2l_sum_kernel, unsigned((ncols + w - 1) / w), 32 * w, 0, s,
       R, op.K, ncols, op.down_box + a, op.down_m2l_beg + a, op.down_m2l_end + a, Y, Lx);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
