@@ -14,6 +14,7 @@
 #include <array>
 #include <atomic>
 #include <chrono>
+#include <memory>
 #include <cmath>
 #include <cstdlib>
 #include <functional>
@@ -125,16 +126,6 @@ namespace
             }
       }
     return true;
-  }
-
-  template <typename T>
-  void transpose_ops(const std::vector<double> &src, int nops, int K, std::vector<T> &dst)
-  {
-    dst.resize(size_t(nops) * K * K);
-    for (int o = 0; o < nops; ++o)
-      for (int i = 0; i < K; ++i)
-        for (int j = 0; j < K; ++j)
-          dst[size_t(o) * K * K + size_t(j) * K + i] = T(src[size_t(o) * K * K + size_t(i) * K + j]);
   }
 } // namespace
 
@@ -2472,61 +2463,39 @@ namespace
     phase(5);
     // translation operators
     {
-      std::vector<double> m2m, l2l, m2l;
-      build_m2m_ops(pl.p, m2m);
-      build_l2l_ops(pl.p, l2l);
-      const int nof = int(pl.offsets.size() / 3);
-      m2l.assign(size_t(std::max(nof, 1)) * K * K, 0.0);
-#pragma omp parallel for schedule(dynamic, 4)
-      for (int o = 0; o < nof; ++o)
-        build_m2l_op(pl.p, pl.offsets[3 * o], pl.offsets[3 * o + 1], pl.offsets[3 * o + 2],
-                     &m2l[size_t(o) * K * K]);
-      // concatenated table [M2L offsets | 8 M2M | 8 L2L], [in][out] per operator
-      const int nops = nof + 16;
-      std::vector<double> all(size_t(nops) * K * K);
-      std::copy(m2l.begin(), m2l.begin() + size_t(nof) * K * K, all.begin());
-      std::copy(m2m.begin(), m2m.end(), all.begin() + size_t(nof) * K * K);
-      std::copy(l2l.begin(), l2l.end(), all.begin() + size_t(nof + 8) * K * K);
-      std::vector<double> td;
-      std::vector<float>  tf;
-      transpose_ops(all, nops, K, td);
-      h->d_ops.upload(td, s);
-      transpose_ops(all, nops, K, tf);
-      h->d_opsf.upload(tf, s);
-      {
-        // the 16 level operators (8 M2M, 8 L2L), each padded to 16 bytes
-        const size_t        kk = fused_level_ops_floats(K) / 16;
-        std::vector<float> lv(16 * kk, 0.0f);
-        for (int o = 0; o < 16; ++o)
-          std::copy(tf.begin() + size_t(nof + o) * K * K, tf.begin() + size_t(nof + o + 1) * K * K,
-                    lv.begin() + o * kk);
-        h->d_lvopsf.upload(lv, s);
-      }
-      {
-        std::vector<float2> ff(td.size());
-        for (size_t i = 0; i < td.size(); ++i)
-          {
-            const float hi = float(td[i]);
-            ff[i]          = make_float2(hi, float(td[i] - double(hi)));
-          }
-        h->d_opsff.upload(ff, s);
-      }
-      h->d_tcimg.release();
+      // concatenated table [M2L offsets | 8 M2M | 8 L2L], [in][out] per operator; the
+      // other forms of it are made on the device
+      const int    nof = int(pl.offsets.size() / 3), nops = nof + 16;
+      const size_t kk = size_t(K) * K, lvk = fused_level_ops_floats(K) / 16;
+      std::unique_ptr<double[]> td(new double[size_t(nops) * kk]);
+      build_ops(pl.p, nof, pl.offsets.data(), td.get());
+      h->d_ops.upload(td.get(), size_t(nops) * kk, s);
+      h->d_opsf.alloc(size_t(nops) * kk);
+      launch_convert_d2f(int64_t(nops) * int64_t(kk), h->d_ops.p, h->d_opsf.p, s);
+      h->d_opsff.alloc(size_t(nops) * kk);
+      launch_convert_d2ff(int64_t(nops) * int64_t(kk), h->d_ops.p, h->d_opsff.p, s);
+      // the 16 level operators (8 M2M, 8 L2L), each padded to 16 bytes
+      h->d_lvopsf.alloc(16 * lvk);
+      h->d_lvopsf.zero(s);
+      PIBEM_CUDA(cudaMemcpy2DAsync(h->d_lvopsf.p, lvk * sizeof(float), h->d_opsf.p + size_t(nof) * kk,
+                                   kk * sizeof(float), kk * sizeof(float), 16, cudaMemcpyDeviceToDevice, s));
       if (h->use_tc && tc_geometry(K).ok)
         {
-          std::vector<float> img;
-          build_tc_images(all, nops, K, img);
-          h->d_tcimg.upload(img, s);
+          h->d_tcimg.alloc(tc_image_floats(nops, K));
+          launch_tc_images(h->d_ops.p, nops, K, h->d_tcimg.p, s);
         }
-      h->d_ozimg.release();
-      h->d_ozecol.release();
+      else
+        h->d_tcimg.release();
       if (h->use_tc && h->prm.precision_mode != PIBEM_PRECISION_FP64 && ozaki_ok(K))
         {
-          std::vector<uint16_t> oimg;
-          std::vector<int16_t>  ecol;
-          build_ozaki_images(all, nops, K, oimg, ecol);
-          h->d_ozimg.upload(oimg, s);
-          h->d_ozecol.upload(ecol, s);
+          h->d_ozimg.alloc(ozaki_image_values(nops, K));
+          h->d_ozecol.alloc(ozaki_column_values(nops, K));
+          launch_ozaki_images(h->d_ops.p, nops, K, h->d_ozimg.p, h->d_ozecol.p, s);
+        }
+      else
+        {
+          h->d_ozimg.release();
+          h->d_ozecol.release();
         }
       h->d_err.alloc(1);
       h->d_err.zero(s);

@@ -166,11 +166,12 @@ namespace pibem
   void launch_m2p(const OperatorDev<T> &op, const TreeDev &td, int R, int N, const T *M, T *y,
                   cudaStream_t s);
   // FP64-accurate translation GEMM on the tensor cores (ozaki_tc.cu): digits of
-  // the operators (host, once) and of the expansions (device, per product),
+  // the operators ([in][out], at set-up) and of the expansions (per product),
   // then Y = T E as (hi, lo) pairs; for K <= 128 (p <= 10)
   bool ozaki_ok(int K);
-  void build_ozaki_images(const std::vector<double> &ops_out_in, int nops, int K,
-                          std::vector<uint16_t> &img, std::vector<int16_t> &e_col);
+  size_t ozaki_image_values(int nops, int K);
+  size_t ozaki_column_values(int nops, int K);
+  void   launch_ozaki_images(const double *ops, int nops, int K, uint16_t *img, int16_t *e_col, cudaStream_t s);
   void launch_ozaki_slices(int64_t nrows, int K, const float2 *E, uint16_t *slices, int *e_row,
                            cudaStream_t s);
   void launch_ozaki_gemm(const OperatorDev<double> &op, int R, int c0, int c1,
@@ -228,9 +229,9 @@ namespace pibem
     bool   ok   = false;
   };
   TcGeometry tc_geometry(int K);
-  // hi/lo TF32 images of row-major [out][in] operators in the MMA B layout
-  void build_tc_images(const std::vector<double> &ops_out_in, int nops, int K,
-                       std::vector<float> &img);
+  // hi/lo TF32 images of the FP64 operators ([in][out]) in the MMA B layout
+  size_t tc_image_floats(int nops, int K);
+  void   launch_tc_images(const double *ops, int nops, int K, float *img, cudaStream_t s);
   // Y row of (pair q, rhs r): (yslot ? yslot[q] : q) * R + r, rows of ldy
   // values (ldy a multiple of 4 when yslot is given)
   void launch_tc_gemm(const OperatorDev<float> &op, int R, int c0, int c1, const float *E, float *Y,

@@ -533,14 +533,31 @@ namespace pibem
                      : "memory");
     }
 
-    inline float tf32_round_host(float x)
+    // Operator images: hi + lo TF32 halves of the FP64 operators ([in][out] K x K), Kp / 32
+    // chunks of [Np rows][32 k] each in the swizzled K-major layout, zero beyond K.  One
+    // thread per image element, rows fastest (coalesced reads).  Built here rather than on
+    // the host: with the images and the other forms of the table made and uploaded by the
+    // host, the operators of p = 8 took 18 - 20 ms of each set-up, now 1.4.
+    __global__ void tc_image_kernel(int64_t n, int K, int Np, int Kp, const double *__restrict__ ops,
+                                    float *__restrict__ img)
     {
-      uint32_t b;
-      std::memcpy(&b, &x, 4);
-      b = (b + 0x1000u) & ~0x1FFFu; // round to nearest, ties away from zero, 10-bit mantissa
-      float r;
-      std::memcpy(&r, &b, 4);
-      return r;
+      const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+      if (i >= n)
+        return;
+      const int     row = int(i % Np), k = int(i / Np % Kp);
+      const int64_t o    = i / (int64_t(Np) * Kp);
+      const int64_t half = int64_t(Kp) * Np;
+      float         h = 0.f, l = 0.f;
+      if (row < K && k < K)
+        {
+          const double v = ops[(o * K + k) * K + row];
+          // to nearest, ties away from zero, 10-bit mantissa
+          h = __uint_as_float((__float_as_uint(float(v)) + 0x1000u) & ~0x1FFFu);
+          l = float(v - double(h));
+        }
+      const int64_t at = o * 2 * half + int64_t(k / TC_KC) * Np * TC_KC + sw128_off(row, k % TC_KC) / 4;
+      img[at]        = h;
+      img[at + half] = l;
     }
   } // namespace
 
@@ -561,30 +578,19 @@ namespace pibem
     return g;
   }
 
-  // Image of one operator half: Kp / 32 chunks of [Np rows][32 k] in the swizzled
-  // K-major layout, zero beyond K; the hi and lo halves one after the other.
-  void build_tc_images(const std::vector<double> &ops_out_in, int nops, int K,
-                       std::vector<float> &img)
+  size_t tc_image_floats(int nops, int K)
   {
-    const TcGeometry g     = tc_geometry(K);
-    const int        nkc   = g.Kp / TC_KC;
-    const size_t     chunk = size_t(g.Np) * TC_KC; // floats
-    const size_t     half  = size_t(nkc) * chunk;
-    img.assign(size_t(nops) * 2 * half, 0.0f);
-    for (int o = 0; o < nops; ++o)
-      {
-        float *hi = img.data() + size_t(o) * 2 * half, *lo = hi + half;
-        for (int n = 0; n < K; ++n)
-          for (int k = 0; k < K; ++k)
-            {
-              const double v  = ops_out_in[size_t(o) * K * K + size_t(n) * K + k];
-              const float  h  = tf32_round_host(float(v));
-              const float  l  = float(v - double(h));
-              const size_t at = size_t(k / TC_KC) * chunk + sw128_off(n, k % TC_KC) / 4;
-              hi[at]          = h;
-              lo[at]          = l;
-            }
-      }
+    const TcGeometry g = tc_geometry(K);
+    return size_t(nops) * 2 * g.Np * g.Kp;
+  }
+
+  void launch_tc_images(const double *ops, int nops, int K, float *img, cudaStream_t s)
+  {
+    const TcGeometry g = tc_geometry(K);
+    const int64_t    n = int64_t(nops) * g.Np * g.Kp;
+    tc_image_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(n, K, g.Np, g.Kp, ops, img);
+    PIBEM_CUDA(cudaGetLastError());
+    note_launch();
   }
 
   void launch_tc_gemm(const OperatorDev<float> &op, int R, int c0, int c1, const float *E, float *Y,

@@ -472,48 +472,65 @@ namespace pibem
                      : "r"(tmem), "r"(OZ_TMEM_COLS)
                      : "memory");
     }
+
+    // Digits of every operator row (output coefficient; operators [in][out] K x K): B images
+    // and column exponents, zero beyond K.  One warp per row of a part's 48.
+    __global__ void __launch_bounds__(256)
+      oz_image_kernel(int64_t rows, int K, const double *__restrict__ ops, uint16_t *__restrict__ img,
+                      int16_t *__restrict__ e_col)
+    {
+      const int64_t r    = int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
+      const int     lane = threadIdx.x & 31;
+      if (r >= rows)
+        return;
+      const int64_t part = r / OZ_NP; // of all operators
+      const int     row = int(r % OZ_NP), parts = oz_parts(K), n = int(part % parts) * OZ_NP + row;
+      const double *t   = ops + part / parts * K * K + n;
+      constexpr int NV  = OZ_NKC * OZ_KC / 32;
+      double        v[NV], mx = 0.0;
+#pragma unroll
+      for (int c = 0; c < NV; ++c)
+        {
+          const int k = lane + 32 * c;
+          v[c]        = n < K && k < K ? t[int64_t(k) * K] : 0.0;
+          mx          = fmax(mx, fabs(v[c]));
+        }
+      for (int o = 16; o > 0; o >>= 1)
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      int e = 0;
+      if (mx > 0.0)
+        frexp(mx, &e); // mx < 2^e
+      if (lane == 0)
+        e_col[r] = int16_t(e);
+      uint16_t *tile = img + part * (OZ_B_BYTES / 2);
+#pragma unroll
+      for (int c = 0; c < NV; ++c)
+        {
+          const int k = lane + 32 * c;
+          double    x = ldexp(v[c], -e);
+          for (int i = 0; i < OZ_S; ++i)
+            {
+              x *= (i == 0 ? 128.0 : 256.0);
+              const double d = rint(x);
+              x -= d;
+              tile[size_t(k / OZ_KC * OZ_S + i) * (OZ_BT_BYTES / 2) + sw128_off_b16(row, k % OZ_KC) / 2] =
+                bf16_bits(ldexpf(float(d), -(7 + 8 * i))); // exact
+            }
+        }
+    }
   } // namespace
 
   bool ozaki_ok(int K) { return K >= 1 && K <= OZ_NKC * OZ_KC; }
 
-  // Host: digits of every operator row (output coefficient), B images and
-  // column exponents.  ops_out_in: nops row-major [out][in] K x K operators.
-  void build_ozaki_images(const std::vector<double> &ops_out_in, int nops, int K,
-                          std::vector<uint16_t> &img, std::vector<int16_t> &e_col)
+  size_t ozaki_image_values(int nops, int K) { return size_t(nops) * oz_parts(K) * (OZ_B_BYTES / 2); }
+  size_t ozaki_column_values(int nops, int K) { return size_t(nops) * oz_parts(K) * OZ_NP; }
+
+  void launch_ozaki_images(const double *ops, int nops, int K, uint16_t *img, int16_t *e_col, cudaStream_t s)
   {
-    const int parts = oz_parts(K);
-    img.assign(size_t(nops) * parts * (OZ_B_BYTES / 2), 0);
-    e_col.assign(size_t(nops) * parts * OZ_NP, 0);
-    double weight[OZ_S]; // of digit i: 2^-(7 + 8 i)
-    for (int i = 0; i < OZ_S; ++i)
-      weight[i] = std::ldexp(1.0, -(7 + 8 * i));
-#pragma omp parallel for schedule(dynamic, 4)
-    for (int o = 0; o < nops; ++o)
-      for (int n = 0; n < K; ++n)
-        {
-          const double *t  = &ops_out_in[(size_t(o) * K + n) * K];
-          double        mx = 0.0;
-          for (int k = 0; k < K; ++k)
-            mx = std::max(mx, std::fabs(t[k]));
-          int e = 0;
-          if (mx > 0.0)
-            std::frexp(mx, &e); // mx < 2^e
-          e_col[size_t(o) * parts * OZ_NP + n] = int16_t(e);
-          uint16_t *tile = &img[(size_t(o) * parts + n / OZ_NP) * (OZ_B_BYTES / 2)];
-          const int row  = n % OZ_NP;
-          for (int k = 0; k < K; ++k)
-            {
-              double v = std::ldexp(t[k], -e);
-              for (int i = 0; i < OZ_S; ++i)
-                {
-                  v *= (i == 0 ? 128.0 : 256.0);
-                  const double d = std::nearbyint(v);
-                  v -= d;
-                  tile[size_t(k / OZ_KC * OZ_S + i) * (OZ_BT_BYTES / 2) + sw128_off_b16(row, k % OZ_KC) / 2] =
-                    bf16_bits(float(d * weight[i])); // exact
-                }
-            }
-        }
+    const int64_t rows = int64_t(ozaki_column_values(nops, K));
+    oz_image_kernel<<<unsigned((rows + 7) / 8), 256, 0, s>>>(rows, K, ops, img, e_col);
+    PIBEM_CUDA(cudaGetLastError());
+    note_launch();
   }
 
   void launch_ozaki_slices(int64_t nrows, int K, const float2 *E, uint16_t *slices, int *e_row,

@@ -261,9 +261,7 @@ namespace pibem
                   int chunk_pairs = 128);
 
   // Real-form translation operators (scaled expansions), row-major K x K.
-  void build_m2m_ops(int p, std::vector<double> &ops8);
-  void build_l2l_ops(int p, std::vector<double> &ops8);
-  void build_m2l_op(int p, int dx, int dy, int dz, double *T);
+  void build_ops(int p, int nof, const int32_t *offsets, double *ops); // (nof + 16) K K values
 
   // Gauss-Legendre and Telles rules on [0,1]^2 (x index fastest).
   void gauss_rule_2d(int n, std::vector<double> &pts, std::vector<double> &w);
