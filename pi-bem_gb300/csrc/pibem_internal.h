@@ -135,7 +135,7 @@ namespace pibem
     std::vector<int>    childless; // reference childlessList order
     std::vector<char>   is_childless;
     std::vector<std::vector<int>> dofs_filled; // per level: boxes with nodes
-    std::vector<int>    qbox; // (L+1) * Q: box of each quad point at each level (leaf if shallower)
+    std::vector<int>    qbox; // (L+1) * Q: box of each quad point at each level (leaf if shallower); host builder only
     // lists[box][sub] sorted unique
     std::vector<std::vector<std::vector<int>>> nn, il, nil;
     std::vector<int>    node_leaf; // childless box of each node

@@ -398,7 +398,6 @@ namespace pibem
     pl     = Plan();
     pl.p   = p;
     pl.K   = (p + 1) * (p + 1);
-    const int64_t Q = int64_t(t.qbox.size() / (t.L + 1));
     // Target boxes: boxes holding collocation nodes (every box with nodes for
     // one body; a double body's boxes of image nodes only are sources only).
     std::vector<char> tgt(t.nb, 0);
@@ -852,7 +851,6 @@ namespace pibem
             pl.l2l_box.push_back(b);
       }
     pl.l2l_ptr_level[t.L + 1] = int(pl.l2l_box.size());
-    (void)Q;
   }
 
   // ---------------------------------------------------------------------
