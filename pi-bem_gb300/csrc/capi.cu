@@ -2359,6 +2359,9 @@ namespace
           }
       h->d_diag_col.upload(dc, s);
     }
+    DBuf<double> qw; // weights of the near-field integrals and the P2M tables
+    qw.alloc(size_t(4) * Q);
+    launch_quad_weights(Q, h->d_qjxw.p, h->d_qshape.p, qw.p, s);
     // near-field integrals
     {
       const int            nl = int(pl.nleaf_box.size());
@@ -2403,8 +2406,7 @@ namespace
       a.nq            = h->nq;
       a.qpts          = h->d_qpts.p;
       a.qnrm          = h->d_qnrm.p;
-      a.qjxw          = h->d_qjxw.p;
-      a.qshape        = h->d_qshape.p;
+      a.qw            = qw.p;
       a.gather_ptr    = h->d_gather_ptr.p;
       a.gather_ids    = h->d_gather_ids.p;
       a.staging       = staging.p;
@@ -2437,8 +2439,7 @@ namespace
       h->d_T2.zero(s);
       launch_p2m_tables(nrows_p, K, pl.p, int(pl.pleaf_box.size()), h->d_prow_ptr.p,
                         h->d_pleaf_box.p, h->d_pcontrib_ptr.p, h->d_pcontrib_q.p, h->d_center.p,
-                        h->d_delta.p, h->d_qpts.p, h->d_qnrm.p, h->d_qjxw.p, h->d_qshape.p,
-                        h->d_T1.p, h->d_T2.p, s);
+                        h->d_delta.p, Q, h->d_qpts.p, h->d_qnrm.p, qw.p, h->d_T1.p, h->d_T2.p, s);
       h->d_T1f.alloc(nrows_p * K4);
       h->d_T2f.alloc(nrows_p * K4);
       launch_convert_d2f(nrows_p * K4, h->d_T1.p, h->d_T1f.p, s);

@@ -11,6 +11,8 @@
 namespace pibem
 {
   // ---- setup (FP64) -------------------------------------------------------
+  // qw[4 q + j] = N_j JxW / (4 pi) of point q
+  void launch_quad_weights(int64_t n_points, const double *qjxw, const double *qshape, double *qw, cudaStream_t s);
   struct NearAssemblyArgs
   {
     int64_t          n_items = 0; // sum over leaves of rows * entries
@@ -23,7 +25,7 @@ namespace pibem
     const double    *xyz = nullptr;
     const int32_t   *cells = nullptr, *dbl_off = nullptr, *dbl_ids = nullptr;
     int              nq = 0;
-    const double    *qpts = nullptr, *qnrm = nullptr, *qjxw = nullptr, *qshape = nullptr;
+    const double    *qpts = nullptr, *qnrm = nullptr, *qw = nullptr; // qw: launch_quad_weights
     const int32_t   *gather_ptr = nullptr, *gather_ids = nullptr;
     double          *staging = nullptr;
     int64_t          staging_items = 0;
@@ -41,9 +43,8 @@ namespace pibem
   void launch_p2m_tables(int64_t n_rows, int K, int p, int n_leaves, const int64_t *row_ptr,
                          const int32_t *leaf_box, const int64_t *contrib_ptr,
                          const int32_t *contrib_q, const double *box_center,
-                         const double *box_delta, const double *qpts, const double *qnrm,
-                         const double *qjxw, const double *qshape, double *T1, double *T2,
-                         cudaStream_t s);
+                         const double *box_delta, int64_t n_points, const double *qpts,
+                         const double *qnrm, const double *qw, double *T1, double *T2, cudaStream_t s);
   void launch_l2p_tables(int64_t n_pos, int K, int ldw, int n_leaves, const int64_t *pos_ptr,
                          const int32_t *leaf_box, const int32_t *nodes, const double *xyz,
                          const double *box_center, const double *box_delta, double *W,

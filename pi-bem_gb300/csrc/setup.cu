@@ -98,16 +98,25 @@ namespace pibem
     }
 
     // LaplaceKernel::kernels (include/laplace_kernel.h:55-74) contracted with
-    // the normal: s = 1 / (4 pi r), dn = D.n with D = R / (-4 pi r^3), from one
+    // the normal, times 4 pi: s = 1 / r, dn = D.n with D = -R / r^3, from one
     // reciprocal square root (FP64 division and square root are
-    // multi-instruction sequences on the FP64 pipe, which bounds this kernel)
+    // multi-instruction sequences on the FP64 pipe, which bounds this kernel);
+    // the 1 / (4 pi) is in the quadrature weights
+    constexpr double C4PI = 1.0 / (4 * kPi);
     __device__ inline void kernel_pair(const double *R, const double *n, double &dn, double &s)
     {
-      constexpr double c4pi = 1.0 / (4 * kPi);
-      const double     r2   = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
-      const double     rinv = rsqrt(r2);
-      s                     = rinv * c4pi;
-      dn                    = -(R[0] * n[0] + R[1] * n[1] + R[2] * n[2]) * (rinv * rinv * rinv) * c4pi;
+      const double r2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
+      s               = rsqrt(r2);
+      dn              = -(R[0] * n[0] + R[1] * n[1] + R[2] * n[2]) * (s * s * s);
+    }
+
+    // weight of each quadrature point for each vertex of its cell: N_j JxW / (4 pi)
+    __global__ void quad_weight_kernel(int64_t n, const double *__restrict__ qjxw,
+                                       const double *__restrict__ qshape, double *__restrict__ qw)
+    {
+      const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+      if (i < n)
+        qw[i] = qshape[i] * qjxw[i >> 2] * C4PI;
     }
 
     // One (leaf row, entry) integral: 4 N values and 4 D values.  PASS 0 takes
@@ -115,7 +124,9 @@ namespace pibem
     // lists the singular ones (the cell holds the row's node or a double of
     // it); PASS 1 integrates the listed items (Telles rule), so that a warp's
     // threads run the same rule (a singular item costs several times a regular
-    // one).  Every item's values depend on the item alone.
+    // one).  Every item's values depend on the item alone.  The weights N_j JxW / (4 pi) are
+    // formed once per point, not once per item: 10.1 -> 7.0 ms at 23.8k nodes, bounded by
+    // the FP64 pipe (some 30 operations per item and point).
     template <int PASS>
     __global__ void near_entries_kernel(int64_t n_items, int n_leaves,
                                         const int64_t *__restrict__ item_ptr,
@@ -129,8 +140,7 @@ namespace pibem
                                         const int32_t *__restrict__ dbl_ids, int nq,
                                         const double *__restrict__ qpts,
                                         const double *__restrict__ qnrm,
-                                        const double *__restrict__ qjxw,
-                                        const double *__restrict__ qshape, int64_t item_base,
+                                        const double *__restrict__ qw, int64_t item_base,
                                         double *__restrict__ staging,
                                         int64_t *__restrict__ sing_list,
                                         unsigned long long *__restrict__ sing_count)
@@ -185,11 +195,11 @@ namespace pibem
                 double  n[3] = {qnrm[3 * k], qnrm[3 * k + 1], qnrm[3 * k + 2]};
                 double  dn, s;
                 kernel_pair(R, n, dn, s);
-                double w = qjxw[k];
                 for (int j = 0; j < 4; ++j)
                   {
-                    Nv[j] += dn * qshape[4 * k + j] * w;
-                    Dv[j] += s * qshape[4 * k + j] * w;
+                    const double w = qw[4 * k + j];
+                    Nv[j] += dn * w;
+                    Dv[j] += s * w;
                   }
               }
           }
@@ -207,11 +217,12 @@ namespace pibem
                 double R[3] = {g.x[0] - xi[0], g.x[1] - xi[1], g.x[2] - xi[2]};
                 double dn, s;
                 kernel_pair(R, g.n, dn, s);
-                double w = g.J * c_tel_w[sv][q];
+                const double w = g.J * c_tel_w[sv][q] * C4PI;
                 for (int j = 0; j < 4; ++j)
                   {
-                    Nv[j] += dn * g.N[j] * w;
-                    Dv[j] += s * g.N[j] * w;
+                    const double wj = g.N[j] * w;
+                    Nv[j] += dn * wj;
+                    Dv[j] += s * wj;
                   }
               }
           }
@@ -290,12 +301,15 @@ namespace pibem
     // dipole layer (Ker1, MultipoleExpansion::AddNormDer multipole_expansion.cc:125-181)
     // and of the single layer (Ker2, MultipoleExpansion::Add multipole_expansion.cc:94-122)
     // of the dof's shape function over the leaf's quadrature points, strengths
-    // N_j JxW / (4 pi) (bem_fma.cc:1722-1734).  One block per row: the row's
-    // contributions are taken P2M_CHUNK at a time; per contribution one thread
-    // computes its geometry (scaled offset, angles, normal derivatives of rho,
-    // alpha, beta), rho^n, cos / sin (m beta) and the tables of P~_n^m and
-    // dP~_n^m/dtheta into shared memory, then thread k adds the contributions'
-    // terms of coefficient k in contribution order.
+    // N_j JxW / (4 pi) (bem_fma.cc:1722-1734).  A quadrature point is in one leaf and
+    // the four rows of its cell's dofs take the same two expansions of it, each times
+    // N_j JxW / (4 pi): p2m_point_kernel forms the expansions of unit strength once per
+    // point, p2m_row_kernel adds a row's contributions to them in contribution order.
+    //   Bounded by FP64 arithmetic, nearly all of it the angles, powers and Legendre tables
+    // of a point (about 1,500 FP64 instructions however many lanes have a point).  At 23.8k
+    // nodes, p = 8: one block per row with a point's tables in each of its rows and 16 of
+    // 32 lanes at work 10.5 ms, so 2.25 (1.7 for the points, 0.55 for the rows; the intermediate, 2 K values a
+    // point, is bounded by chunks of points).
     // P~_n^m(x) of every n <= p, m <= n into P[n (n + 1) / 2 + m] and, with dS,
     // legendre_dsin(n, m) into dS[...]: the recurrences of legendre_nm and
     // legendre_dsin (devmath.cuh) at O(p^2), their square-root factors from
@@ -339,32 +353,23 @@ namespace pibem
           }
     }
 
-    constexpr int P2M_CHUNK = 32;
-    // doubles per contribution in shared memory for order p
+    constexpr int P2M_CHUNK = 32; // points per block
+    // doubles per point in shared memory for order p
     __host__ __device__ inline int p2m_geo_stride(int p)
     {
       const int npm = (p + 1) * (p + 2) / 2;
-      return 8 + 3 * (p + 1) + 2 * npm;
+      return 5 + 3 * (p + 1) + 2 * npm;
     }
-    __global__ void __launch_bounds__(128)
-      p2m_table_kernel(int64_t n_rows, int K, int p, int n_leaves,
-                       const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ leaf_box,
-                       const int64_t *__restrict__ contrib_ptr,
-                       const int32_t *__restrict__ contrib_q,
-                       const double *__restrict__ box_center,
-                       const double *__restrict__ box_delta, const double *__restrict__ qpts,
-                       const double *__restrict__ qnrm, const double *__restrict__ qjxw,
-                       const double *__restrict__ qshape, double *T1, double *T2)
+
+    // box of the leaf each quadrature point is in
+    __global__ void p2m_point_box_kernel(int64_t n_rows, int n_leaves, const int64_t *__restrict__ row_ptr,
+                                         const int32_t *__restrict__ leaf_box,
+                                         const int64_t *__restrict__ contrib_ptr,
+                                         const int32_t *__restrict__ contrib_q, int32_t *__restrict__ qbox)
     {
-      extern __shared__ double geo[]; // [P2M_CHUNK][stride]
-      const int64_t row = blockIdx.x;
+      const int64_t row = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
       if (row >= n_rows)
         return;
-      const int stride = p2m_geo_stride(p);
-      const int npm    = (p + 1) * (p + 2) / 2;
-      // layout of one contribution: 0 w, 1 ws, 2 rho, 3 dRhodN, 4 dBetadN,
-      // 5 dAlphadN, 6 ca, 7 sa, then rn[p+1], cos(m beta)[p+1], sin(m beta)[p+1],
-      // P[npm], dS[npm] (pair (n, m) at n (n+1) / 2 + m)
       int lo = 0, hi = n_leaves - 1;
       while (lo < hi)
         {
@@ -374,85 +379,130 @@ namespace pibem
           else
             hi = mid - 1;
         }
-      const int    box = leaf_box[lo];
-      const double h   = box_delta[box];
-      const double cx = box_center[3 * box], cy = box_center[3 * box + 1],
-                   cz = box_center[3 * box + 2];
-      const int k = threadIdx.x;
-      int       n = 0, m = 0, part = 0;
-      if (k < K)
-        real_index(k, n, m, part);
-      double        a1 = 0, a2 = 0;
-      const int64_t c0 = contrib_ptr[row], c1 = contrib_ptr[row + 1];
-      for (int64_t cb0 = c0; cb0 < c1; cb0 += P2M_CHUNK)
+      const int32_t box = leaf_box[lo];
+      for (int64_t c = contrib_ptr[row]; c < contrib_ptr[row + 1]; ++c)
+        if ((contrib_q[c] & 3) == 0) // one of the point's four
+          qbox[contrib_q[c] >> 2] = box;
+    }
+
+    // Unit-strength expansions of the points q0 ... q1 - 1: E[q - q0][2][K4], the dipole
+    // (per unit of 1 / h) and the monopole.  One warp forms the block's tables, a lane per
+    // point; then the threads take (point, coefficient).
+    __global__ void __launch_bounds__(128)
+      p2m_point_kernel(int64_t q0, int64_t q1, int K, int p, const int32_t *__restrict__ qbox,
+                       const double *__restrict__ box_center, const double *__restrict__ box_delta,
+                       const double *__restrict__ qpts, const double *__restrict__ qnrm,
+                       double *__restrict__ E)
+    {
+      extern __shared__ double geo[]; // [P2M_CHUNK][stride]
+      const int stride = p2m_geo_stride(p);
+      const int npm    = (p + 1) * (p + 2) / 2;
+      // layout of one point: 0 1 / h, 1 dRhodN, 2 dBetadN, 3 dAlphadN, then from 4 on
+      // rho^(n-1) for n = 0 (unused) ... p + 1, cos(m beta)[p+1], sin(m beta)[p+1], P[npm],
+      // dS[npm] (pair (n, m) at n (n+1) / 2 + m)
+      const int o_c = 4 + p + 2, o_s = o_c + p + 1, o_P = o_s + p + 1, o_d = o_P + npm;
+      const int64_t base = q0 + int64_t(blockIdx.x) * P2M_CHUNK;
+      const int     nc   = int(q1 - base < P2M_CHUNK ? q1 - base : int64_t(P2M_CHUNK));
+      if (threadIdx.x < nc)
         {
-          const int nc = int(c1 - cb0 < P2M_CHUNK ? c1 - cb0 : int64_t(P2M_CHUNK));
-          __syncthreads(); // the previous chunk's values are used up
-          if (threadIdx.x < nc)
+          double       *gq = geo + threadIdx.x * stride;
+          const int64_t q  = base + threadIdx.x;
+          const int     box = qbox[q];
+          const double  h   = box_delta[box];
+          const double  rx = (qpts[3 * q] - box_center[3 * box]) / h,
+                       ry = (qpts[3 * q + 1] - box_center[3 * box + 1]) / h,
+                       rz = (qpts[3 * q + 2] - box_center[3 * box + 2]) / h;
+          const double rho  = sqrt(rx * rx + ry * ry + rz * rz);
+          const double ca   = rz / rho;
+          const double sa   = sqrt(fmax(0.0, 1.0 - ca * ca));
+          const double beta = atan2(ry, rx);
+          double nn_ = sqrt(qnrm[3 * q] * qnrm[3 * q] + qnrm[3 * q + 1] * qnrm[3 * q + 1] +
+                            qnrm[3 * q + 2] * qnrm[3 * q + 2]);
+          double nx = qnrm[3 * q] / nn_, ny = qnrm[3 * q + 1] / nn_, nz = qnrm[3 * q + 2] / nn_;
+          double rxy2 = rx * rx + ry * ry;
+          double sb1, cb1;
+          sincos(beta, &sb1, &cb1);
+          gq[0]     = 1.0 / h;
+          gq[1]     = (rx / rho) * nx + (ry / rho) * ny + (rz / rho) * nz;
+          gq[2]     = (-ry / rxy2) * nx + (rx / rxy2) * ny;
+          gq[3]     = (ca * cb1 / rho) * nx + (ca * sb1 / rho) * ny + (-sa / rho) * nz;
+          gq[4]     = 0.0;
+          double rn = 1.0;
+          for (int i = 0; i <= p; ++i)
             {
-              double       *gq = geo + threadIdx.x * stride;
-              const int32_t qj = contrib_q[cb0 + threadIdx.x];
-              const int64_t q  = qj >> 2;
-              const int     j  = qj & 3;
-              const double  w  = qshape[4 * q + j] * qjxw[q] / 4 / kPi;
-              const double  rx = (qpts[3 * q] - cx) / h, ry = (qpts[3 * q + 1] - cy) / h,
-                           rz = (qpts[3 * q + 2] - cz) / h;
-              const double rho  = sqrt(rx * rx + ry * ry + rz * rz);
-              const double ca   = rz / rho;
-              const double sa   = sqrt(fmax(0.0, 1.0 - ca * ca));
-              const double beta = atan2(ry, rx);
-              double nn_ = sqrt(qnrm[3 * q] * qnrm[3 * q] + qnrm[3 * q + 1] * qnrm[3 * q + 1] +
-                                qnrm[3 * q + 2] * qnrm[3 * q + 2]);
-              double nx = qnrm[3 * q] / nn_, ny = qnrm[3 * q + 1] / nn_, nz = qnrm[3 * q + 2] / nn_;
-              double rxy2 = rx * rx + ry * ry;
-              gq[0]       = w;
-              gq[1]       = w / h;
-              gq[2]       = rho;
-              gq[3]       = (rx / rho) * nx + (ry / rho) * ny + (rz / rho) * nz;
-              gq[4]       = (-ry / rxy2) * nx + (rx / rxy2) * ny;
-              gq[5] = (ca * cos(beta) / rho) * nx + (ca * sin(beta) / rho) * ny + (-sa / rho) * nz;
-              gq[6] = ca;
-              gq[7] = sa;
-              double rn = 1.0;
-              for (int i = 0; i <= p; ++i)
-                {
-                  gq[8 + i] = rn;
-                  rn *= rho;
-                }
-              for (int mm = 0; mm <= p; ++mm)
-                {
-                  double sb, cb;
-                  sincos(mm * beta, &sb, &cb);
-                  gq[8 + (p + 1) + mm]     = cb;
-                  gq[8 + 2 * (p + 1) + mm] = sb;
-                }
-              legendre_table(p, ca, sa, gq + 8 + 3 * (p + 1), gq + 8 + 3 * (p + 1) + npm);
+              gq[5 + i] = rn;
+              rn *= rho;
             }
-          __syncthreads();
-          if (k < K)
-            for (int cq = 0; cq < nc; ++cq)
-              {
-                const double *gq  = geo + cq * stride;
-                const int     pmi = n * (n + 1) / 2 + m;
-                const double  cb = gq[8 + (p + 1) + m], sb = gq[8 + 2 * (p + 1) + m];
-                const double  P  = gq[8 + 3 * (p + 1) + pmi];
-                const double  rn = gq[8 + n];
-                // monopole: w P rho^n e^{-i m beta}
-                const double mono = gq[0] * P * rn;
-                a2 += part == 0 ? mono * cb : -mono * sb;
-                // dipole (scaled coordinates, strength w / h)
-                const double dS   = gq[8 + 3 * (p + 1) + npm + pmi];
-                const double rho  = gq[2];
-                const double rnm1 = n > 0 ? rn / rho : 0.0;
-                const double A    = double(n) * rnm1 * P * gq[3] - rn * dS * gq[5];
-                const double B    = -double(m) * rn * P * gq[4];
-                // e^{-i m beta} (A + i B)
-                a1 += gq[1] * (part == 0 ? (cb * A + sb * B) : (cb * B - sb * A));
-              }
+          gq[o_c] = 1.0;
+          gq[o_s] = 0.0;
+          for (int mm = 1; mm <= p; ++mm)
+            {
+              if (mm > 1)
+                sincos(mm * beta, &sb1, &cb1);
+              gq[o_c + mm] = cb1;
+              gq[o_s + mm] = sb1;
+            }
+          legendre_table(p, ca, sa, gq + o_P, gq + o_d);
         }
-      if (k < K)
+      __syncthreads();
+      const int K4 = (K + 3) / 4 * 4;
+      const int k  = threadIdx.x;
+      if (k >= K)
+        return;
+      int n, m, part;
+      real_index(k, n, m, part);
+      const int pmi = n * (n + 1) / 2 + m;
+      double   *out = E + (base - q0) * 2 * K4 + k;
+      for (int cq = 0; cq < nc; ++cq, out += 2 * K4)
         {
-          const int K4    = (K + 3) / 4 * 4; // padded row stride (16-byte vector loads)
+          const double *gq = geo + cq * stride;
+          const double  cb = gq[o_c + m], sb = gq[o_s + m], P = gq[o_P + pmi], rn = gq[5 + n];
+          // dipole (scaled coordinates): e^{-i m beta} (A + i B)
+          const double A = double(n) * gq[4 + n] * P * gq[1] - rn * gq[o_d + pmi] * gq[3];
+          const double B = -double(m) * rn * P * gq[2];
+          out[0]         = gq[0] * (part == 0 ? (cb * A + sb * B) : (cb * B - sb * A));
+          // monopole: P rho^n e^{-i m beta}
+          out[K4] = P * rn * (part == 0 ? cb : -sb);
+        }
+    }
+
+    // T1 / T2 of the rows: += the contributions of the points q0 ... q1 - 1 (the first
+    // chunk: =), a warp per row, contributions in order, P2M_AHEAD of them loaded together
+    constexpr int P2M_AHEAD = 4;
+    __global__ void __launch_bounds__(256)
+      p2m_row_kernel(int64_t n_rows, int64_t q0, int64_t q1, int K, const int64_t *__restrict__ contrib_ptr,
+                     const int32_t *__restrict__ contrib_q, const double *__restrict__ qw,
+                     const double *__restrict__ E, double *__restrict__ T1, double *__restrict__ T2)
+    {
+      const int64_t row  = int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
+      const int     lane = threadIdx.x & 31;
+      if (row >= n_rows)
+        return;
+      const int     K4 = (K + 3) / 4 * 4;
+      const int64_t c0 = contrib_ptr[row], c1 = contrib_ptr[row + 1];
+      for (int k = lane; k < K; k += 32)
+        {
+          double a1 = q0 ? T1[row * K4 + k] : 0.0, a2 = q0 ? T2[row * K4 + k] : 0.0;
+          for (int64_t c = c0; c < c1; c += P2M_AHEAD)
+            {
+              double w[P2M_AHEAD], e1[P2M_AHEAD], e2[P2M_AHEAD];
+#pragma unroll
+              for (int u = 0; u < P2M_AHEAD; ++u)
+                {
+                  const int32_t qj = c + u < c1 ? contrib_q[c + u] : -1;
+                  const int64_t q  = qj >> 2;
+                  const bool    in = qj >= 0 && q >= q0 && q < q1;
+                  w[u]             = in ? qw[qj] : 0.0;
+                  e1[u]            = in ? E[(q - q0) * 2 * K4 + k] : 0.0;
+                  e2[u]            = in ? E[(q - q0) * 2 * K4 + K4 + k] : 0.0;
+                }
+#pragma unroll
+              for (int u = 0; u < P2M_AHEAD; ++u)
+                {
+                  a1 += w[u] * e1[u];
+                  a2 += w[u] * e2[u];
+                }
+            }
           T1[row * K4 + k] = a1;
           T2[row * K4 + k] = a2;
         }
@@ -576,6 +626,13 @@ namespace pibem
     note_launch();
   }
 
+  void launch_quad_weights(int64_t n_points, const double *qjxw, const double *qshape, double *qw, cudaStream_t s)
+  {
+    quad_weight_kernel<<<unsigned((4 * n_points + 255) / 256), 256, 0, s>>>(4 * n_points, qjxw, qshape, qw);
+    PIBEM_CUDA(cudaGetLastError());
+    note_launch();
+  }
+
   void launch_near_assembly(const NearAssemblyArgs &a, cudaStream_t s)
   {
     // batches bounded by the staging buffer (items of 8 doubles)
@@ -607,14 +664,14 @@ namespace pibem
         PIBEM_CUDA(cudaMemsetAsync(a.sing_count, 0, sizeof(unsigned long long), s));
         near_entries_kernel<0><<<unsigned((cnt + 127) / 128), 128, 0, s>>>(
           end, a.n_leaves, a.item_ptr, a.row_ptr, a.ent_ptr, a.rows, a.ents, a.xyz, a.cells,
-          a.dbl_off, a.dbl_ids, a.nq, a.qpts, a.qnrm, a.qjxw, a.qshape, start, a.staging,
+          a.dbl_off, a.dbl_ids, a.nq, a.qpts, a.qnrm, a.qw, start, a.staging,
           a.sing_list, a.sing_count);
         PIBEM_CUDA(cudaGetLastError());
         note_launch();
         // the singular items of the batch (a grid-stride loop over the list)
         near_entries_kernel<1><<<unsigned(std::min<int64_t>((cnt + 127) / 128, 4096)), 128, 0, s>>>(
           end, a.n_leaves, a.item_ptr, a.row_ptr, a.ent_ptr, a.rows, a.ents, a.xyz, a.cells,
-          a.dbl_off, a.dbl_ids, a.nq, a.qpts, a.qnrm, a.qjxw, a.qshape, start, a.staging,
+          a.dbl_off, a.dbl_ids, a.nq, a.qpts, a.qnrm, a.qw, start, a.staging,
           a.sing_list, a.sing_count);
         PIBEM_CUDA(cudaGetLastError());
         note_launch();
@@ -694,24 +751,41 @@ namespace pibem
   void launch_p2m_tables(int64_t n_rows, int K, int p, int n_leaves, const int64_t *row_ptr,
                          const int32_t *leaf_box, const int64_t *contrib_ptr,
                          const int32_t *contrib_q, const double *box_center,
-                         const double *box_delta, const double *qpts, const double *qnrm,
-                         const double *qjxw, const double *qshape, double *T1, double *T2,
-                         cudaStream_t s)
+                         const double *box_delta, int64_t n_points, const double *qpts,
+                         const double *qnrm, const double *qw, double *T1, double *T2, cudaStream_t s)
   {
-    int64_t n = n_rows * K;
-    if (n == 0)
+    if (n_rows == 0)
       return;
     if (K > 128 || p > LEG_PMAX)
       throw Error(PIBEM_EINVAL, "P2M tables: more than 128 coefficients");
     set_legendre_coeffs(s);
     const size_t smem = size_t(P2M_CHUNK) * p2m_geo_stride(p) * sizeof(double);
     if (smem > 48 * 1024)
-      raise_smem_limit(reinterpret_cast<const void *>(p2m_table_kernel), smem);
-    p2m_table_kernel<<<unsigned(n_rows), 128, smem, s>>>(
-      n_rows, K, p, n_leaves, row_ptr, leaf_box, contrib_ptr, contrib_q, box_center, box_delta,
-      qpts, qnrm, qjxw, qshape, T1, T2);
+      raise_smem_limit(reinterpret_cast<const void *>(p2m_point_kernel), smem);
+    // at most 512 MB of expansions at a time
+    const int64_t K4 = (K + 3) / 4 * 4;
+    const int64_t chunk =
+      std::min<int64_t>(n_points, (int64_t(1) << 29) / int64_t(2 * K4 * sizeof(double)) / P2M_CHUNK * P2M_CHUNK);
+    DBuf<int32_t> qbox;
+    DBuf<double>  E;
+    qbox.alloc(size_t(n_points));
+    qbox.zero(s);
+    E.alloc(size_t(chunk) * 2 * K4);
+    p2m_point_box_kernel<<<unsigned((n_rows + 255) / 256), 256, 0, s>>>(n_rows, n_leaves, row_ptr, leaf_box,
+                                                                       contrib_ptr, contrib_q, qbox.p);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
+    for (int64_t q0 = 0; q0 < n_points; q0 += chunk)
+      {
+        const int64_t q1 = std::min(n_points, q0 + chunk);
+        p2m_point_kernel<<<unsigned((q1 - q0 + P2M_CHUNK - 1) / P2M_CHUNK), 128, smem, s>>>(
+          q0, q1, K, p, qbox.p, box_center, box_delta, qpts, qnrm, E.p);
+        p2m_row_kernel<<<unsigned((n_rows + 7) / 8), 256, 0, s>>>(n_rows, q0, q1, K, contrib_ptr, contrib_q,
+                                                                 qw, E.p, T1, T2);
+        PIBEM_CUDA(cudaGetLastError());
+        note_launch(2);
+      }
+    PIBEM_CUDA(cudaStreamSynchronize(s)); // before the buffers go
   }
 
   void launch_l2p_tables(int64_t n_pos, int K, int ldw, int n_leaves, const int64_t *pos_ptr,
