@@ -631,20 +631,48 @@ namespace pibem
         }
     }
 
+    // The P2M and L2P kernels give a leaf `split` warps, 1, 2 or LEAF_SPLIT: a leaf's rows
+    // are a serial chain of loads and sums, and one warp for each of a few hundred leaves
+    // leaves the SMs waiting for it.  L2P rows are dealt to the warps in groups; the P2M sums
+    // are formed over `split` runs of rows and added in run order.
+    constexpr int LEAF_SPLIT = 4;
+    __device__ __forceinline__ void p2m_part(const int64_t r0, const int64_t r1, int q, int split, int64_t &rb,
+                                             int64_t &re)
+    {
+      const int64_t per = ((r1 - r0 + split - 1) / split + 7) / 8 * 8; // whole load groups
+      rb                = min(r1, r0 + q * per);
+      re                = min(r1, rb + per);
+    }
+    template <int RC, typename T>
+    __device__ __forceinline__ void p2m_store(const T (*part)[RC][128], int w0, int split, int k, int rc, T *M,
+                                              int K)
+    {
+#pragma unroll
+      for (int rr = 0; rr < RC; ++rr)
+        if (rr < rc)
+          {
+            T t = part[w0][rr][k];
+            for (int q = 1; q < split; ++q)
+              t += part[w0 + q][rr][k];
+            M[int64_t(rr) * K + k] = t;
+          }
+    }
+
     // P2M apply: M^[leaf][r][k] = sum_rows w(row, r) T[row][k] x_r[dof(row)],
     // w selecting the double layer (Ker1), the single layer (Ker2) or the
-    // combined system strengths.  One warp per leaf, 8 leaves per block: lane l
-    // owns coefficients 4l..4l+3 (table rows padded to K4 values); the rows'
-    // weights are gathered 32 at a time (lane j: row j) and broadcast by
-    // shuffles; eight table rows in flight; the rows are summed in order.
+    // combined system strengths.  SPLIT: `split` > 1 warps per leaf, else one (without the
+    // code for the sum of the parts, 64 registers instead of 78: at 98k nodes 21 us against
+    // 25).  Lane l owns coefficients 4l..4l+3 (table rows padded to K4 values);
+    // the rows' weights are gathered 32 at a time (lane j: row j) and broadcast by
+    // shuffles; eight table rows in flight; a warp's rows are summed in order.
     // COMBINED: every column uses the combined strengths, read from the table
     // Tc = (Dirichlet dof ? -T2 : T1) made at set_bc (one table row per row
     // instead of two); T1 is then Tc and T2 is unused.
     // RC: columns per block (1 for one right-hand side, else 4; the groups of columns
     // over blockIdx.y: a few hundred leaves alone would leave most of the chip idle).
-    template <bool COMBINED, int RC>
+    template <bool COMBINED, int RC, bool SPLIT>
     __global__ void __launch_bounds__(256)
-      p2m_apply_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ prow_ptr,
+      p2m_apply_kernel(int n_leaves, int split, int R, int K, int N, const int64_t *__restrict__ prow_ptr,
                        const int32_t *__restrict__ pleaf_box, const int32_t *__restrict__ prow_dof,
                        const float *__restrict__ T1, const float *__restrict__ T2,
                        const uint8_t *__restrict__ dir, const uint8_t *__restrict__ modes,
@@ -652,12 +680,21 @@ namespace pibem
     {
       using T = float;
       pdl_entry();
-      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-      if (leaf >= n_leaves)
+      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      const int wi   = blockIdx.x * (blockDim.x >> 5) + warp;
+      const int leaf = SPLIT ? wi / split : wi;
+      const int K4   = (K + 3) / 4 * 4;
+      if (!SPLIT && leaf >= n_leaves)
         return;
-      const int     K4  = (K + 3) / 4 * 4;
-      const int64_t box = pleaf_box[leaf];
-      const int64_t rb = prow_ptr[leaf], re = prow_ptr[leaf + 1];
+      int64_t rb = 0, re = 0;
+      if (!SPLIT || leaf < n_leaves)
+        {
+          rb = prow_ptr[leaf];
+          re = prow_ptr[leaf + 1];
+          if constexpr (SPLIT)
+            p2m_part(rb, re, warp & (split - 1), split, rb, re);
+        }
+      const int64_t box = !SPLIT || leaf < n_leaves ? pleaf_box[leaf] : 0;
       const bool    act = 4 * lane < K4;
       const int rq = blockIdx.y * RC;
         {
@@ -730,18 +767,34 @@ namespace pibem
                           }
                 }
             }
-          if (act)
+          if constexpr (!SPLIT)
+            {
+              if (act)
 #pragma unroll
-            for (int rr = 0; rr < RC; ++rr)
-              if (rr < rc)
+                for (int rr = 0; rr < RC; ++rr)
+                  if (rr < rc)
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                  if (4 * lane + c < K)
-                    M[(box * R + rq + rr) * K + 4 * lane + c] = acc[rr][c];
+                    for (int c = 0; c < 4; ++c)
+                      if (4 * lane + c < K)
+                        M[(box * R + rq + rr) * K + 4 * lane + c] = acc[rr][c];
+            }
+          else
+            {
+              __shared__ __align__(16) float part[2 * LEAF_SPLIT][RC][128];
+              if (act)
+#pragma unroll
+                for (int rr = 0; rr < RC; ++rr)
+                  *reinterpret_cast<float4 *>(&part[warp][rr][4 * lane]) =
+                    make_float4(acc[rr][0], acc[rr][1], acc[rr][2], acc[rr][3]);
+              __syncthreads();
+              if (leaf < n_leaves)
+                for (int k = threadIdx.x & (32 * split - 1); k < K; k += 32 * split)
+                  p2m_store<RC>(part, warp & -split, split, k, rc, M + (box * R + rq) * K, K);
+            }
         }
     }
 
-    // P2M apply in FP64: the same sums (rows in order), but lane l owns coefficients l,
+    // P2M apply in FP64: the same sums, but lane l owns coefficients l,
     // l + 32, ... (NPL of them): the FP64 pipe takes a warp's FMA in the same time however
     // many lanes have work, and ceil(K / 32) FMA a row replace 4.  A column of one layer
     // only (KER1 / KER2) skips the other layer's table and products.  Bounded by those FMA and,
@@ -749,19 +802,20 @@ namespace pibem
     // four coefficients a lane and eight warps a block -> 11.8.
     template <bool COMBINED, int RC, int NPL>
     __global__ void __launch_bounds__(256)
-      p2m_apply64_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ prow_ptr,
+      p2m_apply64_kernel(int n_leaves, int split, int R, int K, int N, const int64_t *__restrict__ prow_ptr,
                          const int32_t *__restrict__ pleaf_box, const int32_t *__restrict__ prow_dof,
                          const double *__restrict__ T1, const double *__restrict__ T2,
                          const uint8_t *__restrict__ dir, const uint8_t *__restrict__ modes,
                          const double *__restrict__ x, double *__restrict__ M)
     {
       pdl_entry();
-      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-      if (leaf >= n_leaves)
-        return;
-      const int     K4  = (K + 3) / 4 * 4;
-      const int64_t box = pleaf_box[leaf];
-      const int64_t rb = prow_ptr[leaf], re = prow_ptr[leaf + 1];
+      __shared__ double part[2 * LEAF_SPLIT][RC][128];
+      const int         warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      const int         leaf = (blockIdx.x * (blockDim.x >> 5) + warp) / split;
+      const int         K4   = (K + 3) / 4 * 4;
+      int64_t           rb = 0, re = 0;
+      if (leaf < n_leaves)
+        p2m_part(prow_ptr[leaf], prow_ptr[leaf + 1], warp & (split - 1), split, rb, re);
       const int     rq = blockIdx.y * RC, rc = min(RC, R - rq);
       int           mode[RC];
       bool          one = COMBINED, two = false; // layers that some column takes
@@ -844,13 +898,27 @@ namespace pibem
                       }
             }
         }
+      if (split == 1)
+        {
+          if (leaf < n_leaves)
+#pragma unroll
+            for (int rr = 0; rr < RC; ++rr)
+              if (rr < rc)
+#pragma unroll
+                for (int c = 0; c < NPL; ++c)
+                  if (lane + 32 * c < K)
+                    M[(int64_t(pleaf_box[leaf]) * R + rq + rr) * K + lane + 32 * c] = acc[rr][c];
+          return;
+        }
 #pragma unroll
       for (int rr = 0; rr < RC; ++rr)
-        if (rr < rc)
 #pragma unroll
-          for (int c = 0; c < NPL; ++c)
-            if (lane + 32 * c < K)
-              M[(box * R + rq + rr) * K + lane + 32 * c] = acc[rr][c];
+        for (int c = 0; c < NPL; ++c)
+          part[warp][rr][lane + 32 * c] = acc[rr][c];
+      __syncthreads();
+      if (leaf < n_leaves)
+        for (int k = threadIdx.x & (32 * split - 1); k < K; k += 32 * split)
+          p2m_store<RC>(part, warp & -split, split, k, rc, M + (int64_t(pleaf_box[leaf]) * R + rq) * K, K);
     }
 
     // L2P in FP64: lane l multiplies coefficients l, l + 32, ...; RR rows x RC columns are
@@ -859,12 +927,13 @@ namespace pibem
     // at 386 nodes: 23 us as in FP32 -> 8.4.
     template <int RC, int RR, int NPL>
     __global__ void __launch_bounds__(256)
-      l2p64_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ row_ptr,
+      l2p64_kernel(int n_leaves, int split, int R, int K, int N, const int64_t *__restrict__ row_ptr,
                    const int32_t *__restrict__ lleaf_box, const int32_t *__restrict__ nrows,
                    const double *__restrict__ W, const double *__restrict__ Lx, double *__restrict__ y)
     {
       pdl_entry();
-      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int wi   = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int leaf = wi / split, part = wi & (split - 1);
       if (leaf >= n_leaves)
         return;
       const int     K4  = (K + 3) / 4 * 4;
@@ -877,7 +946,7 @@ namespace pibem
 #pragma unroll
         for (int c = 0; c < NPL; ++c)
           l[r][c] = r < rc && lane + 32 * c < K ? Lx[(box * R + ra + r) * K + lane + 32 * c] : 0.0;
-      for (int64_t i = i0; i < i1; i += RR)
+      for (int64_t i = i0 + part * RR; i < i1; i += split * RR)
         {
           double w[RR][NPL], v[RR * RC];
 #pragma unroll
@@ -1409,7 +1478,7 @@ namespace pibem
     }
 
     // L2P: y[r][node] += W[row] . L^[leaf][r] for every row (node of a
-    // childless box).  One warp per leaf and RC columns (blockIdx.y): lane l
+    // childless box).  `split` warps per leaf and RC columns (blockIdx.y): lane l
     // multiplies coefficients 4l..4l+3 (W rows padded to K4 values) of RR rows and
     // the columns; the lanes' products are added by warp_sum's butterfly.  A (row,
     // column) value has the same roundings for every RC and RR.
@@ -1417,13 +1486,14 @@ namespace pibem
     // for RC columns.
     template <int RC, int RR>
     __global__ void __launch_bounds__(256)
-      l2p_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ row_ptr,
+      l2p_kernel(int n_leaves, int split, int R, int K, int N, const int64_t *__restrict__ row_ptr,
                  const int32_t *__restrict__ lleaf_box, const int32_t *__restrict__ nrows,
                  const float *__restrict__ W, const float *__restrict__ Lx, float *__restrict__ y)
     {
       using T = float;
       pdl_entry();
-      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int wi   = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int leaf = wi / split, part = wi & (split - 1);
       if (leaf >= n_leaves)
         return;
       const int     K4  = (K + 3) / 4 * 4;
@@ -1437,7 +1507,7 @@ namespace pibem
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           l[r][c] = r < rc && 4 * lane + c < K ? Lx[(box * R + ra + r) * K + 4 * lane + c] : T(0);
-      for (int64_t i = i0; i < i1; i += RR)
+      for (int64_t i = i0 + part * RR; i < i1; i += split * RR)
         {
           T w[RR][4];
 #pragma unroll
@@ -1485,12 +1555,13 @@ namespace pibem
     // row sums carried with TwoSum and reduced by the same butterfly; y += the
     // sum in FP64.
     __global__ void __launch_bounds__(256)
-      l2p_ff_kernel(int n_leaves, int R, int K, int N, const int64_t *__restrict__ row_ptr,
+      l2p_ff_kernel(int n_leaves, int split, int R, int K, int N, const int64_t *__restrict__ row_ptr,
                     const int32_t *__restrict__ lleaf_box, const int32_t *__restrict__ nrows,
                     const float2 *__restrict__ W, const float2 *__restrict__ Lx,
                     double *__restrict__ y)
     {
-      const int leaf = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int wi   = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      const int leaf = wi / split, part = wi & (split - 1);
       if (leaf >= n_leaves)
         return;
       const int     K4  = (K + 3) / 4 * 4;
@@ -1511,7 +1582,7 @@ namespace pibem
                 if (4 * lane + c < K)
                   l[c] = lp[4 * lane + c];
             }
-          for (int64_t i0 = r0; i0 < r1; i0 += 8)
+          for (int64_t i0 = r0 + part * 8; i0 < r1; i0 += split * 8)
             {
               float2 w[8][4];
 #pragma unroll
@@ -1573,14 +1644,28 @@ namespace pibem
     return w;
   }
 
+  // Warps per leaf: as many as keep the warps of the launch (leaves x column groups) within
+  // what the SMs hold at once.  One warp -> four (GB300, us): P2M / L2P of a 1.5k-node mesh
+  // 6.5 / 5.8 -> 4.1 / 3.6, four columns at 6.1k nodes 13.5 / 11.8 -> 6.6 / 4.8; at 98k nodes
+  // (6,710 leaves) it would be 21 / 17 -> 27 / 23, every warp loading its leaf's expansion.
+  static int leaf_split(int64_t warps)
+  {
+    int w = LEAF_SPLIT;
+    while (w > 1 && warps * w > int64_t(32) * near_sm_count())
+      w /= 2;
+    return w;
+  }
+
   void launch_l2p_ff(const OperatorDev<double> &op, int R, int N, const float2 *Lff, double *y,
                      cudaStream_t s)
   {
     if (op.n_rows == 0 || op.n_near_leaves == 0)
       return;
-    const int w = leaf_warps(int64_t(op.n_near_leaves) * R);
-    l2p_ff_kernel<<<dim3(unsigned((op.n_near_leaves + w - 1) / w), unsigned(R)), 32 * w, 0, s>>>(
-      op.n_near_leaves, R, op.K, N, op.nrow_ptr, op.lleaf_box, op.nrows, op.Wff, Lff, y);
+    const int     split = leaf_split(int64_t(op.n_near_leaves) * R);
+    const int64_t nw    = int64_t(op.n_near_leaves) * split;
+    const int     w     = leaf_warps(nw * R);
+    l2p_ff_kernel<<<dim3(unsigned((nw + w - 1) / w), unsigned(R)), 32 * w, 0, s>>>(
+      op.n_near_leaves, split, R, op.K, N, op.nrow_ptr, op.lleaf_box, op.nrows, op.Wff, Lff, y);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
@@ -1705,9 +1790,12 @@ namespace pibem
       return;
     const bool comb = combined && op.Tc;
     auto launch = [&](auto kern, int rc) {
-      const int groups = (R + rc - 1) / rc, w = leaf_warps(int64_t(op.n_p2m_leaves) * groups);
-      launch_pdl(kern, dim3(unsigned((op.n_p2m_leaves + w - 1) / w), unsigned(groups)), 32 * w, 0, s,
-                 op.n_p2m_leaves, R, op.K, N, op.prow_ptr, op.pleaf_box, op.prow_dof,
+      const int groups = (R + rc - 1) / rc;
+      const int split  = leaf_split(op.n_p2m_leaves); // the same for every R: it orders the sums
+      const int w      = std::max(split, leaf_warps(int64_t(op.n_p2m_leaves) * split * groups));
+      const int per    = w / split; // leaves per block
+      launch_pdl(kern, dim3(unsigned((op.n_p2m_leaves + per - 1) / per), unsigned(groups)), 32 * w, 0, s,
+                 op.n_p2m_leaves, split, R, op.K, N, op.prow_ptr, op.pleaf_box, op.prow_dof,
                  comb ? op.Tc : op.T1, op.T2, dir, modes, x, M);
     };
     if constexpr (std::is_same<T, double>::value)
@@ -1727,10 +1815,17 @@ namespace pibem
             default: by_k(std::integral_constant<int, 4>()); break;
           }
       }
-    else if (comb)
-      R == 1 ? launch(p2m_apply_kernel<true, 1>, 1) : launch(p2m_apply_kernel<true, 4>, 4);
     else
-      R == 1 ? launch(p2m_apply_kernel<false, 1>, 1) : launch(p2m_apply_kernel<false, 4>, 4);
+      {
+        auto by_split = [&](auto sp) {
+          constexpr bool SP = decltype(sp)::value;
+          if (comb)
+            R == 1 ? launch(p2m_apply_kernel<true, 1, SP>, 1) : launch(p2m_apply_kernel<true, 4, SP>, 4);
+          else
+            R == 1 ? launch(p2m_apply_kernel<false, 1, SP>, 1) : launch(p2m_apply_kernel<false, 4, SP>, 4);
+        };
+        leaf_split(op.n_p2m_leaves) > 1 ? by_split(std::true_type()) : by_split(std::false_type());
+      }
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
   }
@@ -2007,9 +2102,11 @@ namespace pibem
     if (op.n_rows == 0 || op.n_near_leaves == 0)
       return;
     auto launch = [&](auto kern, int rc) {
-      const int groups = (R + rc - 1) / rc, w = leaf_warps(int64_t(op.n_near_leaves) * groups);
-      launch_pdl(kern, dim3(unsigned((op.n_near_leaves + w - 1) / w), unsigned(groups)), 32 * w, 0, s,
-                 op.n_near_leaves, R, op.K, N, op.nrow_ptr, op.lleaf_box, op.nrows, op.W, Lx, y);
+      const int     groups = (R + rc - 1) / rc, split = leaf_split(int64_t(op.n_near_leaves) * groups);
+      const int64_t nw = int64_t(op.n_near_leaves) * split;
+      const int     w  = leaf_warps(nw * groups);
+      launch_pdl(kern, dim3(unsigned((nw + w - 1) / w), unsigned(groups)), 32 * w, 0, s,
+                 op.n_near_leaves, split, R, op.K, N, op.nrow_ptr, op.lleaf_box, op.nrows, op.W, Lx, y);
     };
     if constexpr (std::is_same<T, double>::value)
       {
