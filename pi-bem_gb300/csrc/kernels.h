@@ -198,7 +198,7 @@ namespace pibem
                      double *y, cudaStream_t s);
   // whether the leaf blocks' x pairs (two buffers) fit in shared memory
   bool near_ff_fits(const OperatorDev<double> &op);
-  // FP64-accurate near SpMV on (hi, lo) FP32 pairs, one launch per column:
+  // FP64-accurate near SpMV on (hi, lo) FP32 pairs, columns in groups over the grid:
   // y[r] (=|+=) vals x[r], x given as pairs, y in FP64
   void launch_near_spmv_ff(const OperatorDev<double> &op, int R, int N, const float2 *vals,
                            const float2 *xff, double *y, bool accumulate, cudaStream_t s);

@@ -40,3 +40,32 @@ def test_column_counts(p, pibem_mod, oracle_mod, synthetic, monkeypatch):
             oN, oD = o.fmm_matvec(X[0], X[5])
             assert rel(N3[0], oN) < 1e-10 and rel(D3[0], oD) < 1e-10
         g.close()
+
+
+@pytest.mark.parametrize("leaf,leaves", [(40, (200, 1216)), (12, (1217, 2432)), (4, (2433, 9000))])
+def test_warps_per_leaf(leaf, leaves, pibem_mod, oracle_mod, synthetic, monkeypatch):
+    """P2M and L2P with four, two and one warps per leaf (by the number of leaves): FP64 products
+    against the oracle (1e-10), the FP32 operator against the FP64 one (2e-5, the bound of the level
+    passes' tests) and a column alone against the batch (bitwise)."""
+    mesh, mask = synthetic.spheroid_mixed_case(40, seed=6)[:2]
+    X = np.random.Generator(np.random.PCG64(leaf)).normal(size=(5, mesh.n_nodes))
+    o = oracle_mod.Oracle(p=4, levels=10, max_nodes=leaf, external=True)
+    o.set_mesh(mesh.xyz, mesh.cells)
+    o.set_bc(mask)
+    monkeypatch.setenv("PIBEM_MATVEC_FP32", "1")
+    y = {}
+    for mode in (pibem_mod.PRECISION_FP64, pibem_mod.PRECISION_MIXED):
+        g = pibem_mod.BEMSolver(fma_truncation_order=4, max_nodes_per_childless_block=leaf,
+                                is_external_flow=1, precision_mode=mode)
+        g.set_mesh(mesh.xyz, mesh.cells)
+        g.set_bc(mask)
+        assert leaves[0] <= g.tree_info()["n_leaves"] <= leaves[1]
+        y[mode] = g.system_matvec(X)
+        np.testing.assert_array_equal(np.stack([g.system_matvec(x) for x in X]), y[mode])
+        if mode == pibem_mod.PRECISION_FP64:
+            N, D = g.fmm_matvec(X[0], X[1])
+        g.close()
+    oN, oD = o.fmm_matvec(X[0], X[1])
+    assert rel(N, oN) < 1e-10 and rel(D, oD) < 1e-10
+    for r in range(5):
+        assert rel(y[pibem_mod.PRECISION_MIXED][r], y[pibem_mod.PRECISION_FP64][r]) < 2e-5
