@@ -2615,7 +2615,7 @@ namespace
     h->bc_ok = true;
   }
 
-  // A bounded device wait that gave up (tensor-core translations) is reported
+  // A bounded device wait that gave up (translations, ILU substitutions) is reported
   // as PIBEM_ETIMEDOUT; the flag is cleared for the next call.
   void check_device_error(pibem_handle *h)
   {
