@@ -485,7 +485,7 @@ namespace
             {
               // tensor-core FP64-accurate M2L from the digits of the multipoles
               const int64_t rows = int64_t(h->tree.nb) * R;
-              h->d_ozslc.alloc(size_t(6) * rows * 128);
+              h->d_ozslc.alloc(ozaki_slice_values(rows, op.K));
               h->d_ozerow.alloc(size_t(rows));
               launch_ozaki_slices(rows, op.K, Mff, h->d_ozslc.p, h->d_ozerow.p, s);
               launch_ozaki_gemm(op, R, 0, op.m2l_chunk_end, h->d_ozslc.p, h->d_ozerow.p, rows, Yff,

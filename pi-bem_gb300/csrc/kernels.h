@@ -172,6 +172,7 @@ namespace pibem
   bool ozaki_ok(int K);
   size_t ozaki_image_values(int nops, int K);
   size_t ozaki_column_values(int nops, int K);
+  size_t ozaki_slice_values(int64_t nrows, int K);
   void   launch_ozaki_images(const double *ops, int nops, int K, uint16_t *img, int16_t *e_col, cudaStream_t s);
   void launch_ozaki_slices(int64_t nrows, int K, const float2 *E, uint16_t *slices, int *e_row,
                            cudaStream_t s);
