@@ -14,8 +14,9 @@
 // Threads: LV_G groups of KT = 32 ceil(K/32) (at most 128) threads; thread t of a
 // group owns output coefficient t of the group's columns g, g + LV_G, ...  Every
 // column's result is computed by a fixed sequence of operations that depends on
-// the column's own data only (a K-term chain with k ascending per operator; M2M:
-// the eight octants' products added in a fixed order; M2L sums: one warp per 32
+// the column's own data only (a K-term chain with k ascending per operator, in L2L
+// beyond K = 81 four chains of a quarter each, added pairwise; M2M: the eight
+// octants' products added in a fixed order; M2L sums: one warp per 32
 // coefficients, pairs in list order): the same bits whatever the number of
 // columns, their grouping into blocks or the other columns of the batch.
 //
@@ -26,6 +27,7 @@
 // leaves room for the next level's blocks beside the running ones.
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "async_copy.cuh"
 #include "kernels.h"
@@ -38,6 +40,7 @@ namespace pibem
     __host__ __device__ inline int lv_kx(int K) { return (K + 3) / 4 * 4; }
 
     constexpr int  LV_G          = 4; // column groups per block
+    constexpr int  LV_ONE_CHAIN  = 81; // L2L: most terms in one chain (rounding grows with its length)
     constexpr long LV_SPIN_LIMIT = 1L << 24;
 
     __host__ __device__ inline int lv_kk(int K) { return (K * K + 3) / 4 * 4; } // padded operator
@@ -76,6 +79,62 @@ namespace pibem
           for (int i = 0; i < C; ++i)
             acc[i] = fmaf(tv, X[i * LV_G * Kx + k], acc[i]);
         }
+    }
+
+    // L2L: the chains CH of a sum (chain c: the terms [K c / CH, K (c + 1) / CH)), the row
+    // stride of X (each chain's terms from a 16-byte boundary on) and the place of term k
+    __host__ __device__ inline int lv_chains(int K) { return K <= LV_ONE_CHAIN ? 1 : 4; }
+    __host__ __device__ inline int lv_chain_stride(int K, int CH) { return lv_kx((K + CH - 1) / CH); }
+    __device__ inline int lv_chain_place(int K, int CH, int k)
+    {
+      const int c = CH == 1 ? 0 : (CH * k + CH - 1) / K;
+      return c * lv_chain_stride(K, CH) + k - K * c / CH;
+    }
+
+    // As lv_dot in four chains side by side, added pairwise; X rows of four chains
+    template <int C>
+    __device__ __forceinline__ void lv_dot4(float (&acc)[C], const float *T, const float *X, int K, int ko)
+    {
+      const int cs = lv_chain_stride(K, 4), stride = 4 * cs, n = K / 4; // n: the shortest chain
+      float     s[4][C];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < C; ++i)
+          s[c][i] = 0.0f;
+      int k = 0;
+      for (; k + 4 <= n; k += 4)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          {
+            float        tv[4];
+            const float *Tc = T + (K * c / 4 + k) * K + ko;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              tv[u] = Tc[u * K];
+#pragma unroll
+            for (int i = 0; i < C; ++i)
+              {
+                const float4 xv = *reinterpret_cast<const float4 *>(X + i * LV_G * stride + c * cs + k);
+                s[c][i]         = fmaf(tv[0], xv.x, s[c][i]);
+                s[c][i]         = fmaf(tv[1], xv.y, s[c][i]);
+                s[c][i]         = fmaf(tv[2], xv.z, s[c][i]);
+                s[c][i]         = fmaf(tv[3], xv.w, s[c][i]);
+              }
+          }
+      for (; k < (K + 3) / 4; ++k) // at most four more terms, one more in some chains
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (K * c / 4 + k < K * (c + 1) / 4)
+            {
+              const float tv = T[(K * c / 4 + k) * K + ko];
+#pragma unroll
+              for (int i = 0; i < C; ++i)
+                s[c][i] = fmaf(tv, X[i * LV_G * stride + c * cs + k], s[c][i]);
+            }
+#pragma unroll
+      for (int i = 0; i < C; ++i)
+        acc[i] = __fadd_rn(__fadd_rn(s[0][i], s[1][i]), __fadd_rn(s[2][i], s[3][i]));
     }
 
     // Thread 0 starts the bulk copy of one operator (lv_kk(K) floats, 16-byte
@@ -293,11 +352,14 @@ namespace pibem
     // and most blocks copy one only.  What does not depend on the launch ahead
     // (the operator, the box ids) is fetched before waiting for it.  Measured (as
     // above; one block per SM with up to eight operators before): 98k spheroid
-    // 43 -> 33 us over five levels; 55k hull, p = 10, 76 -> 49 us over seven.  A
+    // 43 -> 33 us over five levels; 55k hull, p = 10, 76 -> 52 us over seven.  A
     // mixed solve to 1e-12: 50.8 -> 47.2 ms (98k), 67.9 -> 58.6 ms (hull).
-    // Shared memory: T[lv_kk], X[LV_G C][Kx].
-    template <int C>
-    __global__ void __launch_bounds__(LV_G * 128)
+    //   CH: the chains of a sum.  One chain of 121 terms would take 49 us on the hull but
+    // double the rounding error of the four it had before; 64 registers keep two blocks
+    // per SM with four (82 registers, one block: 54 us).
+    // Shared memory: T[lv_kk], X[LV_G C][CH lv_chain_stride].
+    template <int C, int CH>
+    __global__ void __launch_bounds__(LV_G * 128, CH == 1 ? 0 : (C <= 4 ? 2 : 1))
       l2l_level_kernel(int R, int K, LevelOctants oct, int n_batches, const int32_t *__restrict__ box,
                        const int32_t *__restrict__ par, const float *__restrict__ lvops,
                        float *__restrict__ Lx, int *__restrict__ err)
@@ -305,10 +367,10 @@ namespace pibem
       extern __shared__ __align__(16) float lv_sm[];
       __shared__ uint64_t op_bar;
       constexpr int NB = LV_G * C; // columns of a batch
-      const int Kx = lv_kx(K);
+      const int Xs = CH * lv_chain_stride(K, CH); // row stride of X
       float    *T = lv_sm, *X = T + lv_kk(K);
       const int KT = blockDim.x / LV_G;
-      const int g = threadIdx.x / KT, ko = threadIdx.x - g * KT;
+      const int g = threadIdx.x / KT, ko = threadIdx.x - g * KT, place = lv_chain_place(K, CH, ko);
       int       b_lo = int(int64_t(n_batches) * blockIdx.x / gridDim.x);
       const int b_hi = int(int64_t(n_batches) * (blockIdx.x + 1) / gridDim.x);
       if (b_lo >= b_hi)
@@ -369,10 +431,10 @@ namespace pibem
                   sum[i] = *l[i];
                 }
             }
-          if (ko < Kx)
+          if (ko < (CH == 1 ? Xs : K))
 #pragma unroll
             for (int i = 0; i < C; ++i)
-              X[(g + LV_G * i) * Kx + ko] = v[i];
+              X[(g + LV_G * i) * Xs + place] = v[i];
           __syncthreads();
           if (waited < loads)
             {
@@ -384,7 +446,10 @@ namespace pibem
           if (ko < K && ops_ok)
             {
               float acc[C];
-              lv_dot<C>(acc, T, X + g * Kx, K, Kx, ko);
+              if constexpr (CH == 1)
+                lv_dot<C>(acc, T, X + g * Xs, K, Xs, ko);
+              else
+                lv_dot4<C>(acc, T, X + g * Xs, K, ko);
 #pragma unroll
               for (int i = 0; i < C; ++i)
                 if (l[i])
@@ -495,23 +560,27 @@ namespace pibem
       return;
     const int K     = op.K;
     const int max_b = 2 * lv_n_sm();
-    const int C     = lv_cols(ncols, max_b);
+    const int C     = lv_cols(ncols, max_b), CH = lv_chains(K);
     int       nb    = 0;
     for (int o = 0; o < 8; ++o)
       nb += ((oct.p[o + 1] - oct.p[o]) * R + LV_G * C - 1) / (LV_G * C);
-    const size_t smem = (size_t(lv_kk(K)) + size_t(LV_G) * C * lv_kx(K)) * sizeof(float);
+    const size_t smem = (size_t(lv_kk(K)) + size_t(LV_G) * C * CH * lv_chain_stride(K, CH)) * sizeof(float);
     auto launch = [&](auto kern) {
       if (smem > 48 * 1024)
         raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
       launch_pdl(kern, unsigned(std::min(nb, max_b)), LV_G * lv_kt(K), smem, s, R, K, oct, nb,
                  op.down_box, op.down_par, op.lv_ops + size_t(8) * lv_kk(K), Lx, op.dev_err);
     };
+    auto by_chains = [&](auto c) {
+      constexpr int Cc = decltype(c)::value;
+      CH == 1 ? launch(l2l_level_kernel<Cc, 1>) : launch(l2l_level_kernel<Cc, 4>);
+    };
     switch (C)
       {
-        case 8: launch(l2l_level_kernel<8>); break;
-        case 4: launch(l2l_level_kernel<4>); break;
-        case 2: launch(l2l_level_kernel<2>); break;
-        default: launch(l2l_level_kernel<1>); break;
+        case 8: by_chains(std::integral_constant<int, 8>()); break;
+        case 4: by_chains(std::integral_constant<int, 4>()); break;
+        case 2: by_chains(std::integral_constant<int, 2>()); break;
+        default: by_chains(std::integral_constant<int, 1>()); break;
       }
     PIBEM_CUDA(cudaGetLastError());
     note_launch();

@@ -2,6 +2,7 @@
 // what the C ABI shows only through whole operators.  Host arrays in and out; every function
 // returns the device error flag (0: none) or -1 after an exception.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <exception>
 #include <vector>
@@ -101,6 +102,62 @@ extern "C" int kh_m2l(int p, int nof, const int32_t *offsets, int n_rows, const 
     else
       launch_ff_gemm<float2>(o, 1, 0, int(cnt.size()), d_E.p, d_Y.p, nullptr);
     down(d_Y, reinterpret_cast<float2 *>(Y), size_t(n_pairs) * K);
+    int e = 0;
+    down(err, &e, 1);
+    return e;
+  });
+}
+
+// One L2L level of the FP32 operator: L[box] += T_octant L[par] for n boxes listed by octant (oct:
+// the nine bounds), R columns.  ref != 0: the same sums on the host, chain by chain.
+extern "C" int kh_l2l(int p, int R, int n_all, int n, const int32_t *box, const int32_t *par, const int32_t *oct,
+                      int ref, float *L)
+{
+  return guarded([&] {
+    const int           K = (p + 1) * (p + 1);
+    std::vector<double> ops(size_t(16) * K * K);
+    build_ops(p, 0, nullptr, ops.data());
+    const size_t       lvk = fused_level_ops_floats(K) / 16;
+    std::vector<float> lv(16 * lvk, 0.0f);
+    for (int o = 0; o < 16; ++o)
+      for (int i = 0; i < K * K; ++i)
+        lv[o * lvk + i] = float(ops[size_t(o) * K * K + i]);
+    if (ref)
+      {
+        for (int o = 0; o < 8; ++o)
+          for (int i = oct[o]; i < oct[o + 1]; ++i)
+            for (int r = 0; r < R; ++r)
+              for (int k = 0; k < K; ++k)
+                {
+                  const float *T = &lv[(8 + o) * lvk], *x = L + (size_t(par[i]) * R + r) * K;
+                  auto         chain = [&](int a, int b) {
+                    float s = 0.0f;
+                    for (int j = a; j < b; ++j)
+                      s = std::fmaf(T[j * K + k], x[j], s);
+                    return s;
+                  };
+                  L[(size_t(box[i]) * R + r) * K + k] +=
+                    K <= 81 ? chain(0, K) :
+                              (chain(0, K / 4) + chain(K / 4, K / 2)) + (chain(K / 2, 3 * K / 4) + chain(3 * K / 4, K));
+                }
+        return 0;
+      }
+    Up<float>   d_lv(lv), d_L(L, size_t(n_all) * R * K);
+    Up<int32_t> d_box(box, n), d_par(par, n);
+    DBuf<int>   err;
+    err.alloc(1);
+    err.zero(nullptr);
+    OperatorDev<float> o;
+    o.K        = K;
+    o.p        = p;
+    o.lv_ops   = d_lv.p;
+    o.down_box = d_box.p;
+    o.down_par = d_par.p;
+    o.dev_err  = err.p;
+    o.down_oct_ptr.resize(1);
+    std::copy(oct, oct + 9, o.down_oct_ptr[0].p);
+    launch_l2l_level_fused(o, R, 0, d_L.p, nullptr);
+    down(d_L, L, size_t(n_all) * R * K);
     int e = 0;
     down(err, &e, 1);
     return e;
