@@ -248,10 +248,12 @@ struct pibem_handle
   // order (values: L below the diagonal, unit diagonal implied; U from it),
   // the position of each row's diagonal, and the rows by level of the lower
   // and of the upper triangle (the rows of a level depend on earlier levels
-  // only)
+  // only), and the bounds of the levels where the substitutions run level by
+  // level (else empty)
   DBuf<int64_t> d_ilu_ptr, d_ilu_diag;
   DBuf<int32_t> d_ilu_col, d_ilu_rows_lo, d_ilu_rows_up;
   DBuf<double>  d_ilu_val, d_ilu_y; // d_ilu_y: work of the substitutions
+  std::vector<int64_t> ilu_lptr_lo, ilu_lptr_up;
   bool          ilu_on = false;
   bool          use_tc = true;
   std::vector<int64_t> blk_ptr;
@@ -908,6 +910,12 @@ namespace
 
   void ilu_apply(pibem_handle *h, int R, double *z, const int *sel, const int *jvec, cudaStream_t s)
   {
+    if (!h->ilu_lptr_lo.empty())
+      {
+        launch_ilu_levels(h->ilu_lptr_lo, h->d_ilu_rows_lo.p, h->ilu_lptr_up, h->d_ilu_rows_up.p, R, h->N(),
+                          h->d_ilu_ptr.p, h->d_ilu_col.p, h->d_ilu_val.p, h->d_ilu_diag.p, z, sel, jvec, s);
+        return;
+      }
     h->d_ilu_y.alloc(size_t(R) * h->N()); // sized by engine_open inside a capture
     launch_ilu_apply(h->N(), R, h->d_ilu_rows_lo.p, h->d_ilu_rows_up.p, h->d_ilu_ptr.p, h->d_ilu_col.p,
                      h->d_ilu_val.p, h->d_ilu_diag.p, z, h->d_ilu_y.p, sel, jvec, h->d_err.p, s);
@@ -981,7 +989,7 @@ namespace
     for (DBuf<int> *v : {&E.jcur, &E.kdone, &E.jvec, &E.its, &E.maxit, &E.sel})
       v->alloc(S);
     E.act.alloc(2 * S);
-    if (h->ilu_on)
+    if (h->ilu_on && h->ilu_lptr_lo.empty())
       h->d_ilu_y.alloc(size_t(S) * N);
     std::vector<int> minus(S, -1);
     E.jvec.upload(minus, h->stream);
@@ -1880,6 +1888,13 @@ namespace
     launch_ilu_factor(lptr_lo, h->d_ilu_rows_lo.p, h->d_ilu_ptr.p, h->d_ilu_col.p,
                       h->d_ilu_val.p, h->d_ilu_diag.p, max_row, s);
     PIBEM_CUDA(cudaStreamSynchronize(s));
+    if (!ilu_by_level(n, int64_t(lptr_lo.size() + lptr_up.size()) - 2))
+      {
+        lptr_lo.clear();
+        lptr_up.clear();
+      }
+    h->ilu_lptr_lo.swap(lptr_lo);
+    h->ilu_lptr_up.swap(lptr_up);
     h->ilu_on = true;
   }
 

@@ -949,6 +949,34 @@ namespace pibem
       z[idx] = v[r * ldv + t];
     }
 
+    // One level of a substitution (forward: lower triangle, unit diagonal; backward: upper),
+    // in place on the selected columns of z: a warp per (row, column), lanes over the row's
+    // entries, fixed butterfly.  For triangles of wide levels (launch_ilu_apply).
+    template <bool FWD>
+    __global__ void ilu_level_kernel(int nrows, const int32_t *__restrict__ rows, int R, int64_t n,
+                                     const int64_t *__restrict__ ptr, const int32_t *__restrict__ col,
+                                     const double *__restrict__ val, const int64_t *__restrict__ diag,
+                                     double *__restrict__ z, const int *__restrict__ sel,
+                                     const int *__restrict__ jvec)
+    {
+      const int64_t w    = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+      const int     lane = threadIdx.x & 31;
+      if (w >= int64_t(nrows) * R)
+        return;
+      const int r = int(w / nrows), i = rows[w - int64_t(r) * nrows];
+      if ((sel && !sel[r]) || (jvec && jvec[r] < 0))
+        return;
+      double       *zr = z + int64_t(r) * n;
+      const int64_t a0 = FWD ? ptr[i] : diag[i] + 1, a1 = FWD ? diag[i] : ptr[i + 1];
+      double        s  = 0;
+      for (int64_t e = a0 + lane; e < a1; e += 32)
+        s = fma(val[e], zr[col[e]], s);
+      for (int o = 16; o > 0; o >>= 1)
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0)
+        zr[i] = FWD ? zr[i] - s : (zr[i] - s) / val[diag[i]];
+    }
+
     // z = U^-1 L^-1 z in place: one block per column (blockIdx.x) runs both
     // substitutions.  Its warps take the rows in level order, one after another in
     // turn; a warp waits for the solution values of its row's columns in the vector
@@ -960,10 +988,10 @@ namespace pibem
     //   What bounds it: the chain of dependent rows (some 650 levels of 4 rows at 2.4k
     // nodes, 17,000 of 6 at 98k): no parallelism for more than an SM, so the
     // hand-over between rows decides.  Inside one block it goes through shared memory
-    // (SMEM: up to some 25,000 nodes) or the L1 cache, 1.2-1.6 us a level (FP64 latency:
+    // (SMEM: up to 25,600 nodes) or the L1 cache, 1.2-1.6 us a level (FP64 latency:
     // the last FMA, five shuffled additions, the pivot), where one launch per level
     // took 4.7 us.  The next row's indices are loaded a row ahead.  One application
-    // (p = 8, leaf 40): 2.4k nodes 13.4 -> 3.3 ms, 13.8k 29 -> 7.0, 31k 65 -> 21.
+    // (leaf 40): 2.4k nodes 13.4 -> 3.3 ms, 13.8k 29 -> 7.0, 31k 65 -> 21.
     constexpr int                ILU_THREADS = 512;
     constexpr int                ILU_E       = 16; // entries per lane loaded at once
     constexpr unsigned long long ILU_UNSET   = ~0ull;
@@ -1555,6 +1583,48 @@ namespace pibem
     note_launch();
   }
 
+  // Bytes of a column's solution up to which it is handed on in shared memory
+  static constexpr size_t ILU_SMEM = 200 * 1024;
+
+  // One block per column (ilu_apply_kernel) costs a latency per level while the levels hold
+  // a few rows, and then a time per row that one SM sets: 0.13 - 0.17 us in shared memory,
+  // 0.23 - 0.25 through L1.  A launch per level costs 6 us (200 entries a row) to 10 (500)
+  // whatever its width.  So triangles of wide levels (few long chains: nodes numbered at
+  // random or by colour; along a surface a level holds 2 - 10 rows) run level by level.
+  // Measured, ms an application, block / level launches, by rows per level:
+  //   shared memory (13.8k, 24.6k nodes)   21: 4.5 / 9.4   33: 8.2 / 13.0   47: 3.5 / 3.5   75: 5.9 / 4.2
+  //   L1 (38k, 65k nodes)   18: 18.5 / 27.2   21: 30.7 / 37.3   25: 25 / 39   51: 18.7 / 14.8   73: 33.7 / 19.6
+  //                        114: 17.3 / 4.8   231: 29.3 / 4.3
+  bool ilu_by_level(int64_t n, int64_t levels)
+  {
+    const int64_t wide = size_t(n) * sizeof(double) <= ILU_SMEM ? 46 : 32; // rows per level
+    return 2 * n > wide * levels;
+  }
+
+  void launch_ilu_levels(const std::vector<int64_t> &lptr_lo, const int32_t *rows_lo,
+                         const std::vector<int64_t> &lptr_up, const int32_t *rows_up, int R, int64_t n,
+                         const int64_t *ptr, const int32_t *col, const double *val,
+                         const int64_t *diag, double *z, const int *sel, const int *jvec,
+                         cudaStream_t s)
+  {
+    if (n == 0 || R == 0)
+      return;
+    auto sweep = [&](auto kern, const std::vector<int64_t> &lptr, const int32_t *rows) {
+      for (size_t l = 0; l + 1 < lptr.size(); ++l)
+        {
+          const int nr = int(lptr[l + 1] - lptr[l]);
+          if (nr == 0)
+            continue;
+          kern<<<nblocks(int64_t(nr) * R * 32), 256, 0, s>>>(nr, rows + lptr[l], R, n, ptr, col, val, diag, z,
+                                                             sel, jvec);
+          note_launch();
+        }
+    };
+    sweep(ilu_level_kernel<true>, lptr_lo, rows_lo);
+    sweep(ilu_level_kernel<false>, lptr_up, rows_up);
+    PIBEM_CUDA(cudaGetLastError());
+  }
+
   void launch_ilu_apply(int64_t n, int R, const int32_t *rows_lo, const int32_t *rows_up,
                         const int64_t *ptr, const int32_t *col, const double *val,
                         const int64_t *diag, double *z, double *y, const int *sel, const int *jvec,
@@ -1563,7 +1633,7 @@ namespace pibem
     if (n == 0 || R == 0)
       return;
     const size_t smem = size_t(n) * sizeof(double);
-    if (smem <= 200 * 1024)
+    if (smem <= ILU_SMEM)
       {
         if (smem > 40 * 1024)
           raise_smem_limit(reinterpret_cast<const void *>(ilu_apply_kernel<true>), smem);

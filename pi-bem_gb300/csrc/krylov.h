@@ -93,6 +93,13 @@ namespace pibem
   void launch_ilu_factor(const std::vector<int64_t> &lptr, const int32_t *rows, const int64_t *ptr,
                          const int32_t *col, double *val, const int64_t *diag, int64_t max_row,
                          cudaStream_t s);
+  // whether the substitutions run level by level (levels: of both triangles), and so
+  bool ilu_by_level(int64_t n, int64_t levels);
+  void launch_ilu_levels(const std::vector<int64_t> &lptr_lo, const int32_t *rows_lo,
+                         const std::vector<int64_t> &lptr_up, const int32_t *rows_up, int R, int64_t n,
+                         const int64_t *ptr, const int32_t *col, const double *val,
+                         const int64_t *diag, double *z, const int *sel, const int *jvec,
+                         cudaStream_t s);
   void launch_ilu_apply(int64_t n, int R, const int32_t *rows_lo, const int32_t *rows_up,
                         const int64_t *ptr, const int32_t *col, const double *val,
                         const int64_t *diag, double *z, double *y, const int *sel, const int *jvec,

@@ -1,0 +1,69 @@
+"""ILU(0) substitutions by the shape of the triangles' levels (krylov.cu): meshes numbered at random,
+whose levels are few and wide, run a launch per level; meshes numbered along the surface, whose levels
+hold a few rows, run one block per column, with the solution in shared memory up to 25,600 nodes (200 KB)
+and in global memory beyond.  All against the oracle's preconditioner at the bound of the other ILU
+tests, 1e-10 relative, two columns at once."""
+import numpy as np
+import pytest
+
+from conftest import rel
+
+pytestmark = pytest.mark.gpu
+
+
+def renumbered(synthetic, mesh, seed):
+    rng = np.random.Generator(np.random.PCG64(seed))
+    new = rng.permutation(mesh.n_nodes)
+    old = np.argsort(new)
+    return synthetic.Mesh(mesh.xyz[old], new[mesh.cells].astype(mesh.cells.dtype), mesh.normals[old])
+
+
+def solver(pibem_mod, mesh, mask, leaf, **kw):
+    g = pibem_mod.BEMSolver(fma_truncation_order=2, max_nodes_per_childless_block=leaf, is_external_flow=1,
+                            precision_mode=pibem_mod.PRECISION_FP64, **kw)
+    g.set_mesh(mesh.xyz, mesh.cells)
+    g.set_bc(mask)
+    return g
+
+
+# (resolution, random numbering, most launches of an application or None: a launch per level)
+@pytest.mark.parametrize("n,shuffled,launches", [(65, False, 4), (66, False, 4), (48, True, None), (66, True, None)])
+def test_apply(n, shuffled, launches, pibem_mod, oracle_mod, synthetic):
+    mesh = synthetic.spheroid(n)
+    if shuffled:
+        mesh = renumbered(synthetic, mesh, 1)
+    mask = synthetic.mixed_bc_by_cell_centroid(mesh)
+    o = oracle_mod.Oracle(p=2, levels=10, max_nodes=4, external=True)
+    o.set_mesh(mesh.xyz, mesh.cells)
+    o.set_bc(mask)
+    apply, _ = o.preconditioner(2)
+    g = solver(pibem_mod, mesh, mask, 4, preconditioner=2)
+    V = np.random.Generator(np.random.PCG64(n)).normal(size=(2, mesh.n_nodes))
+    l0 = pibem_mod.launch_count()
+    Z = g.apply_preconditioner(V)
+    count = pibem_mod.launch_count() - l0
+    assert count <= launches if launches else count > 100
+    for r in range(2):
+        assert rel(Z[r], apply(V[r])) < 1e-10
+    g.close()
+
+
+def test_solve_with_wide_levels(pibem_mod, synthetic):
+    """The level launches inside the GMRES cycle graph: the same bits step by step (profiling on),
+    and the solution of the leaf-block Jacobi solve to 1e-8 at a tolerance of 1e-11."""
+    mesh = renumbered(synthetic, synthetic.spheroid(48), 2)
+    mask = synthetic.mixed_bc_by_cell_centroid(mesh)
+    src = synthetic.sources_in_ball(np.random.Generator(np.random.PCG64(3)), 4)
+    tmp = synthetic.point_source_data(mesh, mask, src, np.array([1.0, -0.5, 0.7, 0.2]))[0]
+    out = {}
+    for prec in (1, 2):
+        g = solver(pibem_mod, mesh, mask, 4, preconditioner=prec, solver_tolerance=1e-11)
+        phi, dphi, _ = g.solve(tmp)
+        out[prec] = np.concatenate([phi, dphi])
+        if prec == 2:
+            g.set_profiling(1)
+            phi1, dphi1, _ = g.solve(tmp)
+            np.testing.assert_array_equal(phi1, phi)
+            np.testing.assert_array_equal(dphi1, dphi)
+        g.close()
+    assert rel(out[2], out[1]) < 1e-8
