@@ -984,14 +984,15 @@ namespace pibem
     // so a value is its own flag.  A row only waits for rows before it in the list
     // and each warp takes its rows in order, so the first unfinished row can always
     // proceed; every wait is bounded.  A row's sum: lanes stride over its entries,
-    // fixed butterfly.
+    // fixed butterfly, with the bits of ilu_level_kernel.
     //   What bounds it: the chain of dependent rows (some 650 levels of 4 rows at 2.4k
     // nodes, 17,000 of 6 at 98k): no parallelism for more than an SM, so the
     // hand-over between rows decides.  Inside one block it goes through shared memory
-    // (SMEM: up to 25,600 nodes) or the L1 cache, 1.2-1.6 us a level (FP64 latency:
-    // the last FMA, five shuffled additions, the pivot), where one launch per level
-    // took 4.7 us.  The next row's indices are loaded a row ahead.  One application
-    // (leaf 40): 2.4k nodes 13.4 -> 3.3 ms, 13.8k 29 -> 7.0, 31k 65 -> 21.
+    // (SMEM: up to 25,600 nodes) or the L1 cache, 1.2-1.7 us a level (FP64 latency:
+    // the last FMA, five shuffled additions, the division by the pivot, which takes 4 %
+    // more than a product with its reciprocal but rounds once), where one launch per
+    // level took 4.7 us.  The next row's indices are loaded a row ahead.  One application
+    // (leaf 40): 2.4k nodes 13.4 -> 3.5 ms, 13.8k 29 -> 7.3, 31k 65 -> 21.
     constexpr int                ILU_THREADS = 512;
     constexpr int                ILU_E       = 16; // entries per lane loaded at once
     constexpr unsigned long long ILU_UNSET   = ~0ull;
@@ -1040,7 +1041,7 @@ namespace pibem
           const int     i2 = row_at(k + 2 * nw);
           const int64_t n0 = begin(i1), n1 = end(i1);
           const double  nb = right(i1), nd = pivot(i1);
-          double        s = 0, di = 1.0 / d;
+          double        s = 0;
           for (int64_t e0 = a0; e0 < a1; e0 += 32 * ILU_E)
             {
               int    c[ILU_E];
@@ -1135,7 +1136,7 @@ namespace pibem
           for (int o = 16; o > 0; o >>= 1)
             s += __shfl_xor_sync(0xffffffffu, s, o);
           if (lane == 0)
-            ilu_put<SMEM>(out + i, FWD ? b - s : (b - s) * di);
+            ilu_put<SMEM>(out + i, FWD ? b - s : (b - s) / d);
           i  = i1;
           i1 = i2;
           a0 = n0;

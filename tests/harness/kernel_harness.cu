@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../pi-bem_gb300/csrc/kernels.h"
+#include "../../pi-bem_gb300/csrc/krylov.h"
 
 using namespace pibem;
 
@@ -158,6 +159,35 @@ extern "C" int kh_l2l(int p, int R, int n_all, int n, const int32_t *box, const 
     std::copy(oct, oct + 9, o.down_oct_ptr[0].p);
     launch_l2l_level_fused(o, R, 0, d_L.p, nullptr);
     down(d_L, L, size_t(n_all) * R * K);
+    int e = 0;
+    down(err, &e, 1);
+    return e;
+  });
+}
+
+// ILU(0) substitutions of R columns of z (n values each) with given factors (CSR, the diagonal's
+// positions) and rows by level: a launch per level, else one block per column.
+extern "C" int kh_ilu(int n, int R, const int64_t *ptr, const int32_t *col, const double *val, const int64_t *diag,
+                      int n_lo, const int64_t *lptr_lo, const int32_t *rows_lo, int n_up, const int64_t *lptr_up,
+                      const int32_t *rows_up, int by_level, double *z)
+{
+  return guarded([&] {
+    Up<int64_t>  d_ptr(ptr, n + 1), d_diag(diag, n);
+    Up<int32_t>  d_col(col, ptr[n]), d_lo(rows_lo, n), d_up(rows_up, n);
+    Up<double>   d_val(val, ptr[n]), d_z(z, size_t(n) * R);
+    DBuf<double> y;
+    DBuf<int>    err;
+    y.alloc(size_t(n) * R);
+    err.alloc(1);
+    err.zero(nullptr);
+    if (by_level)
+      launch_ilu_levels(std::vector<int64_t>(lptr_lo, lptr_lo + n_lo + 1), d_lo.p,
+                        std::vector<int64_t>(lptr_up, lptr_up + n_up + 1), d_up.p, R, n, d_ptr.p, d_col.p, d_val.p,
+                        d_diag.p, d_z.p, nullptr, nullptr, nullptr);
+    else
+      launch_ilu_apply(n, R, d_lo.p, d_up.p, d_ptr.p, d_col.p, d_val.p, d_diag.p, d_z.p, y.p, nullptr, nullptr,
+                       err.p, nullptr);
+    down(d_z, z, size_t(n) * R);
     int e = 0;
     down(err, &e, 1);
     return e;

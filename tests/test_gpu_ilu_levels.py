@@ -2,10 +2,13 @@
 whose levels are few and wide, run a launch per level; meshes numbered along the surface, whose levels
 hold a few rows, run one block per column, with the solution in shared memory up to 25,600 nodes (200 KB)
 and in global memory beyond.  All against the oracle's preconditioner at the bound of the other ILU
-tests, 1e-10 relative, two columns at once."""
+tests, 1e-10 relative, two columns at once; and the two forms against each other, bit for bit."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
+import kernel_harness as kh
 from conftest import rel
 
 pytestmark = pytest.mark.gpu
@@ -67,3 +70,40 @@ def test_solve_with_wide_levels(pibem_mod, synthetic):
             np.testing.assert_array_equal(dphi1, dphi)
         g.close()
     assert rel(out[2], out[1]) < 1e-8
+
+
+@pytest.mark.parametrize("n", [3, 700, 25600, 25601])
+def test_both_forms_round_alike(n):
+    """Random factors, rows of 1 to 600 entries (more than the 512 that a warp loads at once), pivots
+    without short reciprocals: the two forms' sums and quotients are the same."""
+    lib = kh.load()
+    rng = np.random.Generator(np.random.PCG64(n))
+    cols = []
+    for i in range(n):
+        k = int(rng.choice([0, 3, 9, 40])) if n > 1000 else int(rng.choice([0, 3, 40, 600]))
+        cols.append(np.unique(np.append(rng.integers(0, n, k), i)))
+    ptr = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int64)
+    col = np.concatenate(cols).astype(np.int32)
+    diag = np.array([ptr[i] + np.searchsorted(cols[i], i) for i in range(n)], np.int64)
+    val = rng.normal(size=len(col)) / 40.0
+    val[diag] = rng.uniform(0.5, 2.0, n)
+
+    def by_level(lower):
+        lev = np.zeros(n, int)
+        for i in range(n) if lower else range(n - 1, -1, -1):
+            c = cols[i][cols[i] < i] if lower else cols[i][cols[i] > i]
+            if len(c):
+                lev[i] = lev[c].max() + 1
+        count = np.bincount(lev)
+        return np.concatenate([[0], np.cumsum(count)]).astype(np.int64), np.argsort(lev, kind="stable").astype(np.int32)
+
+    lo, up = by_level(True), by_level(False)
+    z0 = rng.normal(size=(2, n))
+    z = {}
+    for levels in (0, 1):
+        z[levels] = z0.copy()
+        assert lib.kh_ilu(n, 2, kh.ptr(ptr, C.c_int64), kh.ptr(col, C.c_int32), kh.ptr(val, C.c_double),
+                          kh.ptr(diag, C.c_int64), len(lo[0]) - 1, kh.ptr(lo[0], C.c_int64), kh.ptr(lo[1], C.c_int32),
+                          len(up[0]) - 1, kh.ptr(up[0], C.c_int64), kh.ptr(up[1], C.c_int32), levels,
+                          kh.ptr(z[levels], C.c_double)) == 0
+    np.testing.assert_array_equal(z[0], z[1])
