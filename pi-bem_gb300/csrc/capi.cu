@@ -2377,6 +2377,7 @@ namespace
     DBuf<double> qw; // weights of the near-field integrals and the P2M tables
     qw.alloc(size_t(4) * Q);
     launch_quad_weights(Q, h->d_qjxw.p, h->d_qshape.p, qw.p, s);
+    size_t p2m_work = size_t(128) << 20; // work of the P2M tables: at most what the near field gave back
     // near-field integrals
     {
       const int            nl = int(pl.nleaf_box.size());
@@ -2397,6 +2398,7 @@ namespace
         maxrow = std::max<int64_t>(maxrow, pl.nent_ptr[k + 1] - pl.nent_ptr[k]);
       st_items = std::max(st_items, maxrow);
       staging.alloc(8 * std::max<int64_t>(st_items, 1));
+      p2m_work = std::min(p2m_work, staging.bytes());
       DBuf<int64_t>            sing_list;
       DBuf<unsigned long long> sing_count;
       sing_list.alloc(std::max<int64_t>(st_items, 1));
@@ -2452,9 +2454,27 @@ namespace
       h->d_T2.alloc(nrows_p * K4);
       h->d_T1.zero(s);
       h->d_T2.zero(s);
-      launch_p2m_tables(nrows_p, K, pl.p, int(pl.pleaf_box.size()), h->d_prow_ptr.p,
-                        h->d_pleaf_box.p, h->d_pcontrib_ptr.p, h->d_pcontrib_q.p, h->d_center.p,
-                        h->d_delta.p, Q, h->d_qpts.p, h->d_qnrm.p, qw.p, h->d_T1.p, h->d_T2.p, s);
+      P2mTableArgs a;
+      a.K             = K;
+      a.p             = pl.p;
+      a.n_leaves      = int(pl.pleaf_box.size());
+      a.row_ptr       = h->d_prow_ptr.p;
+      a.contrib_ptr   = h->d_pcontrib_ptr.p;
+      a.h_row_ptr     = pl.prow_ptr.data();
+      a.h_contrib_ptr = pl.pcontrib_ptr.data();
+      a.leaf_box      = h->d_pleaf_box.p;
+      a.contrib_q     = h->d_pcontrib_q.p;
+      a.box_center    = h->d_center.p;
+      a.box_delta     = h->d_delta.p;
+      a.n_points      = Q;
+      a.qpts          = h->d_qpts.p;
+      a.qnrm          = h->d_qnrm.p;
+      a.qw            = qw.p;
+      a.work_bytes    = p2m_work;
+      a.T1            = h->d_T1.p;
+      a.T2            = h->d_T2.p;
+      launch_p2m_tables(a, s);
+      qw.release();
       h->d_T1f.alloc(nrows_p * K4);
       h->d_T2f.alloc(nrows_p * K4);
       launch_convert_d2f(nrows_p * K4, h->d_T1.p, h->d_T1f.p, s);

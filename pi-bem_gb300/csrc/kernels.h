@@ -40,11 +40,20 @@ namespace pibem
                         const double *gpts, const double *gw, double *qpts, double *qnrm,
                         double *qjxw, double *qshape, cudaStream_t s);
   void launch_near_assembly(const NearAssemblyArgs &a, cudaStream_t s);
-  void launch_p2m_tables(int64_t n_rows, int K, int p, int n_leaves, const int64_t *row_ptr,
-                         const int32_t *leaf_box, const int64_t *contrib_ptr,
-                         const int32_t *contrib_q, const double *box_center,
-                         const double *box_delta, int64_t n_points, const double *qpts,
-                         const double *qnrm, const double *qw, double *T1, double *T2, cudaStream_t s);
+  // P2M tables T1, T2 (rows of K values padded to a multiple of 4): the leaves' rows, each
+  // row's contributions (point * 4 + vertex, by point), both pointers on the host too
+  struct P2mTableArgs
+  {
+    int            K = 0, p = 0, n_leaves = 0;
+    const int64_t *row_ptr = nullptr, *contrib_ptr = nullptr, *h_row_ptr = nullptr, *h_contrib_ptr = nullptr;
+    const int32_t *leaf_box = nullptr, *contrib_q = nullptr;
+    const double  *box_center = nullptr, *box_delta = nullptr;
+    int64_t        n_points = 0;
+    const double  *qpts = nullptr, *qnrm = nullptr, *qw = nullptr; // qw: launch_quad_weights
+    size_t         work_bytes = 0; // of the points' expansions held at a time
+    double        *T1 = nullptr, *T2 = nullptr;
+  };
+  void launch_p2m_tables(const P2mTableArgs &a, cudaStream_t s);
   void launch_l2p_tables(int64_t n_pos, int K, int ldw, int n_leaves, const int64_t *pos_ptr,
                          const int32_t *leaf_box, const int32_t *nodes, const double *xyz,
                          const double *box_center, const double *box_delta, double *W,

@@ -304,12 +304,16 @@ namespace pibem
     // N_j JxW / (4 pi) (bem_fma.cc:1722-1734).  A quadrature point is in one leaf and
     // the four rows of its cell's dofs take the same two expansions of it, each times
     // N_j JxW / (4 pi): p2m_point_kernel forms the expansions of unit strength once per
-    // point, p2m_row_kernel adds a row's contributions to them in contribution order.
+    // point, p2m_row_kernel adds a row's contributions to them in contribution order.  The
+    // leaves are taken in runs whose points' expansions (2 K values each) fit the work
+    // buffer, the points numbered leaf after leaf, so that every row and every point has
+    // its turn once.
     //   Bounded by FP64 arithmetic, nearly all of it the angles, powers and Legendre tables
     // of a point (about 1,500 FP64 instructions however many lanes have a point).  At 23.8k
     // nodes, p = 8: one block per row with a point's tables in each of its rows and 16 of
-    // 32 lanes at work 10.5 ms, so 2.25 (1.7 for the points, 0.55 for the rows; the intermediate, 2 K values a
-    // point, is bounded by chunks of points).
+    // 32 lanes at work 10.5 ms, so 2.4 (1.75 for the points, 0.67 for the rows).  P2M and
+    // L2P tables at 400k nodes, p = 10: 237 ms -> 69 (319 where a run was a range of point
+    // ids, each walking every row).
     // P~_n^m(x) of every n <= p, m <= n into P[n (n + 1) / 2 + m] and, with dS,
     // legendre_dsin(n, m) into dS[...]: the recurrences of legendre_nm and
     // legendre_dsin (devmath.cuh) at O(p^2), their square-root factors from
@@ -361,35 +365,41 @@ namespace pibem
       return 5 + 3 * (p + 1) + 2 * npm;
     }
 
-    // box of the leaf each quadrature point is in
-    __global__ void p2m_point_box_kernel(int64_t n_rows, int n_leaves, const int64_t *__restrict__ row_ptr,
-                                         const int32_t *__restrict__ leaf_box,
-                                         const int64_t *__restrict__ contrib_ptr,
-                                         const int32_t *__restrict__ contrib_q, int32_t *__restrict__ qbox)
+    // A number for each quadrature point, leaf after leaf and in contribution order within
+    // the leaf (a warp per leaf; a point has four contributions in its leaf, j = 0 .. 3):
+    // num[q], and of each number its point and the leaf's box
+    __global__ void __launch_bounds__(128)
+      p2m_number_kernel(int n_leaves, const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ leaf_box,
+                        const int64_t *__restrict__ contrib_ptr, const int32_t *__restrict__ contrib_q,
+                        int32_t *__restrict__ num, int32_t *__restrict__ point, int32_t *__restrict__ box)
     {
-      const int64_t row = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-      if (row >= n_rows)
+      const int leaf = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+      if (leaf >= n_leaves)
         return;
-      int lo = 0, hi = n_leaves - 1;
-      while (lo < hi)
+      const int64_t c0 = contrib_ptr[row_ptr[leaf]], c1 = contrib_ptr[row_ptr[leaf + 1]];
+      int64_t       at = c0 / 4;
+      for (int64_t c = c0; c < c1; c += 32)
         {
-          int mid = (lo + hi + 1) >> 1;
-          if (row_ptr[mid] <= row)
-            lo = mid;
-          else
-            hi = mid - 1;
+          const int32_t  qj   = c + lane < c1 ? contrib_q[c + lane] : -1;
+          const bool     mine = qj >= 0 && (qj & 3) == 0;
+          const unsigned all  = __ballot_sync(0xffffffffu, mine);
+          if (mine)
+            {
+              const int64_t n = at + __popc(all & ((1u << lane) - 1u));
+              num[qj >> 2]    = int32_t(n);
+              point[n]        = qj >> 2;
+              box[n]          = leaf_box[leaf];
+            }
+          at += __popc(all);
         }
-      const int32_t box = leaf_box[lo];
-      for (int64_t c = contrib_ptr[row]; c < contrib_ptr[row + 1]; ++c)
-        if ((contrib_q[c] & 3) == 0) // one of the point's four
-          qbox[contrib_q[c] >> 2] = box;
     }
 
-    // Unit-strength expansions of the points q0 ... q1 - 1: E[q - q0][2][K4], the dipole
-    // (per unit of 1 / h) and the monopole.  One warp forms the block's tables, a lane per
-    // point; then the threads take (point, coefficient).
+    // Unit-strength expansions of the points of numbers n0 ... n1 - 1: E[n - n0][2][K4], the
+    // dipole (per unit of 1 / h) and the monopole.  One warp forms the block's tables, a lane
+    // per point; then the threads take (point, coefficient).
     __global__ void __launch_bounds__(128)
-      p2m_point_kernel(int64_t q0, int64_t q1, int K, int p, const int32_t *__restrict__ qbox,
+      p2m_point_kernel(int64_t n0, int64_t n1, int K, int p, const int32_t *__restrict__ point,
+                       const int32_t *__restrict__ point_box,
                        const double *__restrict__ box_center, const double *__restrict__ box_delta,
                        const double *__restrict__ qpts, const double *__restrict__ qnrm,
                        double *__restrict__ E)
@@ -401,13 +411,13 @@ namespace pibem
       // rho^(n-1) for n = 0 (unused) ... p + 1, cos(m beta)[p+1], sin(m beta)[p+1], P[npm],
       // dS[npm] (pair (n, m) at n (n+1) / 2 + m)
       const int o_c = 4 + p + 2, o_s = o_c + p + 1, o_P = o_s + p + 1, o_d = o_P + npm;
-      const int64_t base = q0 + int64_t(blockIdx.x) * P2M_CHUNK;
-      const int     nc   = int(q1 - base < P2M_CHUNK ? q1 - base : int64_t(P2M_CHUNK));
+      const int64_t base = n0 + int64_t(blockIdx.x) * P2M_CHUNK;
+      const int     nc   = int(n1 - base < P2M_CHUNK ? n1 - base : int64_t(P2M_CHUNK));
       if (threadIdx.x < nc)
         {
           double       *gq = geo + threadIdx.x * stride;
-          const int64_t q  = base + threadIdx.x;
-          const int     box = qbox[q];
+          const int64_t q   = point[base + threadIdx.x];
+          const int     box = point_box[base + threadIdx.x];
           const double  h   = box_delta[box];
           const double  rx = (qpts[3 * q] - box_center[3 * box]) / h,
                        ry = (qpts[3 * q + 1] - box_center[3 * box + 1]) / h,
@@ -452,7 +462,7 @@ namespace pibem
       int n, m, part;
       real_index(k, n, m, part);
       const int pmi = n * (n + 1) / 2 + m;
-      double   *out = E + (base - q0) * 2 * K4 + k;
+      double   *out = E + (base - n0) * 2 * K4 + k;
       for (int cq = 0; cq < nc; ++cq, out += 2 * K4)
         {
           const double *gq = geo + cq * stride;
@@ -466,35 +476,36 @@ namespace pibem
         }
     }
 
-    // T1 / T2 of the rows: += the contributions of the points q0 ... q1 - 1 (the first
-    // chunk: =), a warp per row, contributions in order, P2M_AHEAD of them loaded together
+    // T1 / T2 of the rows row0 ... row1 - 1, whose points' numbers begin at n0: a warp per
+    // row, contributions in order, P2M_AHEAD of them loaded together
     constexpr int P2M_AHEAD = 4;
     __global__ void __launch_bounds__(256)
-      p2m_row_kernel(int64_t n_rows, int64_t q0, int64_t q1, int K, const int64_t *__restrict__ contrib_ptr,
-                     const int32_t *__restrict__ contrib_q, const double *__restrict__ qw,
-                     const double *__restrict__ E, double *__restrict__ T1, double *__restrict__ T2)
+      p2m_row_kernel(int64_t row0, int64_t row1, int64_t n0, int K, const int64_t *__restrict__ contrib_ptr,
+                     const int32_t *__restrict__ contrib_q, const int32_t *__restrict__ num,
+                     const double *__restrict__ qw, const double *__restrict__ E, double *__restrict__ T1,
+                     double *__restrict__ T2)
     {
-      const int64_t row  = int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
+      const int64_t row  = row0 + int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
       const int     lane = threadIdx.x & 31;
-      if (row >= n_rows)
+      if (row >= row1)
         return;
       const int     K4 = (K + 3) / 4 * 4;
       const int64_t c0 = contrib_ptr[row], c1 = contrib_ptr[row + 1];
       for (int k = lane; k < K; k += 32)
         {
-          double a1 = q0 ? T1[row * K4 + k] : 0.0, a2 = q0 ? T2[row * K4 + k] : 0.0;
+          double a1 = 0.0, a2 = 0.0;
           for (int64_t c = c0; c < c1; c += P2M_AHEAD)
             {
               double w[P2M_AHEAD], e1[P2M_AHEAD], e2[P2M_AHEAD];
 #pragma unroll
               for (int u = 0; u < P2M_AHEAD; ++u)
                 {
-                  const int32_t qj = c + u < c1 ? contrib_q[c + u] : -1;
-                  const int64_t q  = qj >> 2;
-                  const bool    in = qj >= 0 && q >= q0 && q < q1;
+                  const bool    in = c + u < c1;
+                  const int32_t qj = in ? contrib_q[c + u] : 0;
+                  const int64_t e  = in ? (num[qj >> 2] - n0) * 2 * K4 + k : 0;
                   w[u]             = in ? qw[qj] : 0.0;
-                  e1[u]            = in ? E[(q - q0) * 2 * K4 + k] : 0.0;
-                  e2[u]            = in ? E[(q - q0) * 2 * K4 + K4 + k] : 0.0;
+                  e1[u]            = in ? E[e] : 0.0;
+                  e2[u]            = in ? E[e + K4] : 0.0;
                 }
 #pragma unroll
               for (int u = 0; u < P2M_AHEAD; ++u)
@@ -748,40 +759,50 @@ namespace pibem
       done[dev] = true;
   }
 
-  void launch_p2m_tables(int64_t n_rows, int K, int p, int n_leaves, const int64_t *row_ptr,
-                         const int32_t *leaf_box, const int64_t *contrib_ptr,
-                         const int32_t *contrib_q, const double *box_center,
-                         const double *box_delta, int64_t n_points, const double *qpts,
-                         const double *qnrm, const double *qw, double *T1, double *T2, cudaStream_t s)
+  void launch_p2m_tables(const P2mTableArgs &a, cudaStream_t s)
   {
-    if (n_rows == 0)
+    if (a.n_leaves == 0)
       return;
-    if (K > 128 || p > LEG_PMAX)
+    if (a.K > 128 || a.p > LEG_PMAX)
       throw Error(PIBEM_EINVAL, "P2M tables: more than 128 coefficients");
     set_legendre_coeffs(s);
-    const size_t smem = size_t(P2M_CHUNK) * p2m_geo_stride(p) * sizeof(double);
+    const size_t smem = size_t(P2M_CHUNK) * p2m_geo_stride(a.p) * sizeof(double);
     if (smem > 48 * 1024)
       raise_smem_limit(reinterpret_cast<const void *>(p2m_point_kernel), smem);
-    // at most 512 MB of expansions at a time
-    const int64_t K4 = (K + 3) / 4 * 4;
-    const int64_t chunk =
-      std::min<int64_t>(n_points, (int64_t(1) << 29) / int64_t(2 * K4 * sizeof(double)) / P2M_CHUNK * P2M_CHUNK);
-    DBuf<int32_t> qbox;
+    // the runs of leaves: [run[i], run[i + 1]), a single leaf where that has more points
+    const int64_t K4    = (a.K + 3) / 4 * 4;
+    const int64_t most  = int64_t(a.work_bytes / (2 * K4 * sizeof(double)));
+    auto          first = [&](int leaf) { return a.h_contrib_ptr[a.h_row_ptr[leaf]] / 4; }; // number
+    std::vector<int> run(1, 0);
+    int64_t          longest = 0;
+    while (run.back() < a.n_leaves)
+      {
+        const int l0 = run.back();
+        int       l1 = l0 + 1;
+        while (l1 < a.n_leaves && first(l1 + 1) - first(l0) <= most)
+          ++l1;
+        longest = std::max(longest, first(l1) - first(l0));
+        run.push_back(l1);
+      }
+    const size_t  n_listed = size_t(first(a.n_leaves));
+    DBuf<int32_t> num, point, box;
     DBuf<double>  E;
-    qbox.alloc(size_t(n_points));
-    qbox.zero(s);
-    E.alloc(size_t(chunk) * 2 * K4);
-    p2m_point_box_kernel<<<unsigned((n_rows + 255) / 256), 256, 0, s>>>(n_rows, n_leaves, row_ptr, leaf_box,
-                                                                       contrib_ptr, contrib_q, qbox.p);
+    num.alloc(size_t(a.n_points));
+    point.alloc(n_listed);
+    box.alloc(n_listed);
+    E.alloc(size_t(longest) * 2 * K4);
+    p2m_number_kernel<<<unsigned((a.n_leaves + 3) / 4), 128, 0, s>>>(
+      a.n_leaves, a.row_ptr, a.leaf_box, a.contrib_ptr, a.contrib_q, num.p, point.p, box.p);
     PIBEM_CUDA(cudaGetLastError());
     note_launch();
-    for (int64_t q0 = 0; q0 < n_points; q0 += chunk)
+    for (size_t i = 0; i + 1 < run.size(); ++i)
       {
-        const int64_t q1 = std::min(n_points, q0 + chunk);
-        p2m_point_kernel<<<unsigned((q1 - q0 + P2M_CHUNK - 1) / P2M_CHUNK), 128, smem, s>>>(
-          q0, q1, K, p, qbox.p, box_center, box_delta, qpts, qnrm, E.p);
-        p2m_row_kernel<<<unsigned((n_rows + 7) / 8), 256, 0, s>>>(n_rows, q0, q1, K, contrib_ptr, contrib_q,
-                                                                 qw, E.p, T1, T2);
+        const int64_t n0 = first(run[i]), n1 = first(run[i + 1]);
+        const int64_t row0 = a.h_row_ptr[run[i]], row1 = a.h_row_ptr[run[i + 1]];
+        p2m_point_kernel<<<unsigned((n1 - n0 + P2M_CHUNK - 1) / P2M_CHUNK), 128, smem, s>>>(
+          n0, n1, a.K, a.p, point.p, box.p, a.box_center, a.box_delta, a.qpts, a.qnrm, E.p);
+        p2m_row_kernel<<<unsigned((row1 - row0 + 7) / 8), 256, 0, s>>>(
+          row0, row1, n0, a.K, a.contrib_ptr, a.contrib_q, num.p, a.qw, E.p, a.T1, a.T2);
         PIBEM_CUDA(cudaGetLastError());
         note_launch(2);
       }

@@ -193,3 +193,38 @@ extern "C" int kh_ilu(int n, int R, const int64_t *ptr, const int32_t *col, cons
     return e;
   });
 }
+
+// P2M tables T1, T2 (rows of K4 values) of n_leaves leaves, the boxes 0 ... n_leaves - 1, with work
+// for the points' expansions of work_bytes
+extern "C" int kh_p2m_tables(int p, int n_leaves, const int64_t *row_ptr, const int64_t *contrib_ptr,
+                             const int32_t *contrib_q, const double *center, const double *delta, int n_points,
+                             const double *qpts, const double *qnrm, const double *qw, int64_t work_bytes,
+                             double *T1, double *T2)
+{
+  return guarded([&] {
+    const int            K = (p + 1) * (p + 1), K4 = (K + 3) / 4 * 4;
+    const int64_t        rows = row_ptr[n_leaves];
+    std::vector<int32_t> box(n_leaves);
+    for (int i = 0; i < n_leaves; ++i)
+      box[i] = i;
+    Up<int64_t>  d_row(row_ptr, n_leaves + 1), d_cp(contrib_ptr, rows + 1);
+    Up<int32_t>  d_cq(contrib_q, contrib_ptr[rows]), d_box(box);
+    Up<double>   d_c(center, 3 * n_leaves), d_d(delta, n_leaves), d_p(qpts, 3 * n_points), d_n(qnrm, 3 * n_points),
+      d_w(qw, 4 * n_points);
+    DBuf<double> t1, t2;
+    t1.alloc(rows * K4);
+    t2.alloc(rows * K4);
+    t1.zero(nullptr);
+    t2.zero(nullptr);
+    P2mTableArgs a;
+    a.K = K, a.p = p, a.n_leaves = n_leaves;
+    a.row_ptr = d_row.p, a.contrib_ptr = d_cp.p, a.h_row_ptr = row_ptr, a.h_contrib_ptr = contrib_ptr;
+    a.leaf_box = d_box.p, a.contrib_q = d_cq.p, a.box_center = d_c.p, a.box_delta = d_d.p;
+    a.n_points = n_points, a.qpts = d_p.p, a.qnrm = d_n.p, a.qw = d_w.p;
+    a.work_bytes = size_t(work_bytes), a.T1 = t1.p, a.T2 = t2.p;
+    launch_p2m_tables(a, nullptr);
+    down(t1, T1, size_t(rows) * K4);
+    down(t2, T2, size_t(rows) * K4);
+    return 0;
+  });
+}
