@@ -2662,7 +2662,7 @@ namespace
     if (e)
       {
         h->d_err.zero(h->stream);
-        throw Error(PIBEM_ETIMEDOUT, "a bounded device wait timed out in the translations");
+        throw Error(PIBEM_ETIMEDOUT, device_error_text(e));
       }
   }
 

@@ -1067,7 +1067,7 @@ namespace pibem
                 if (!*abort)
                   {
                     *abort = 1;
-                    atomicExch(err, 1);
+                    atomicOr(err, int(DEV_TIMEOUT_ILU));
                   }
                 next = cnt;
               };

@@ -152,7 +152,7 @@ namespace pibem
     {
       if (mbar_wait_bounded(bar, parity, LV_SPIN_LIMIT))
         return true;
-      atomicExch(err, 1);
+      atomicOr(err, int(DEV_TIMEOUT_TRANSLATIONS));
       return false;
     }
 

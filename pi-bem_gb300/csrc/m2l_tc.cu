@@ -216,7 +216,7 @@ namespace pibem
           {
             ok         = false;
             abort_flag = 1;
-            atomicExch(err, 1);
+            atomicOr(err, int(DEV_TIMEOUT_TRANSLATIONS));
           }
       };
 

@@ -123,7 +123,7 @@ namespace pibem
             return false;
         }
       *abort = 1;
-      atomicExch(err, 1);
+      atomicOr(err, int(DEV_TIMEOUT_TRANSLATIONS));
       return false;
     }
 

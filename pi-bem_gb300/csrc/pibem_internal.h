@@ -30,6 +30,22 @@ namespace pibem
     }                                                                                          \
   while (0)
 
+  // A handle's device error flag (or-ed together): which bounded device wait gave up
+  enum : int
+  {
+    DEV_TIMEOUT_TRANSLATIONS = 1, // tensor-core translations and fused level passes
+    DEV_TIMEOUT_ILU          = 2  // ILU(0) substitutions
+  };
+  inline const char *device_error_text(int e)
+  {
+    switch (e & (DEV_TIMEOUT_TRANSLATIONS | DEV_TIMEOUT_ILU))
+      {
+        case DEV_TIMEOUT_TRANSLATIONS: return "a bounded device wait timed out in the translations";
+        case DEV_TIMEOUT_ILU: return "a bounded device wait timed out in the ILU(0) substitutions";
+        default: return "bounded device waits timed out in the translations and the ILU(0) substitutions";
+      }
+  }
+
   // Counts kernel launches of this library (all handles, all streams).
   void    note_launch(int64_t n = 1);
   int64_t launch_count();

@@ -107,3 +107,23 @@ def test_both_forms_round_alike(n):
                           len(up[0]) - 1, kh.ptr(up[0], C.c_int64), kh.ptr(up[1], C.c_int32), levels,
                           kh.ptr(z[levels], C.c_double)) == 0
     np.testing.assert_array_equal(z[0], z[1])
+
+
+def test_wait_that_gives_up_has_its_own_code():
+    """Row 0 of the forward order waits for a row that its own warp only takes later (16 warps): the
+    bounded wait runs out, the kernel returns and the error flag is the substitutions' own."""
+    lib = kh.load()
+    n = 40
+    ptr = np.arange(n + 1, dtype=np.int64)
+    ptr[18:] += 1  # row 17 = [16, 17], the others their diagonal
+    col = np.insert(np.arange(n), 17, 16).astype(np.int32)
+    diag = np.array([ptr[i] + (i == 17) for i in range(n)], np.int64)
+    val = np.ones(n + 1)
+    rows = np.arange(n, dtype=np.int32)
+    rows[[0, 17]] = rows[[17, 0]]  # row 17 first, row 16 at place 16: both of warp 0
+    lptr = np.array([0, n], np.int64)
+    z = np.ones((1, n))
+    assert lib.kh_ilu(n, 1, kh.ptr(ptr, C.c_int64), kh.ptr(col, C.c_int32), kh.ptr(val, C.c_double),
+                      kh.ptr(diag, C.c_int64), 1, kh.ptr(lptr, C.c_int64), kh.ptr(rows, C.c_int32),
+                      1, kh.ptr(lptr, C.c_int64), kh.ptr(np.arange(n, dtype=np.int32), C.c_int32), 0,
+                      kh.ptr(z, C.c_double)) == 2
