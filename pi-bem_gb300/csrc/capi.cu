@@ -879,21 +879,13 @@ namespace
   // gathered into one contiguous batch), and the Arnoldi steps of every column
   // inside a GMRES cycle run on the device -- CGS2 in FP64, the Hessenberg
   // column's Givens rotation and the stopping test (arnoldi_finish_kernel) -- as
-  // one CUDA graph, a conditional while node around one step, until some column
-  // ends its cycle (it met its tolerance, took m steps or reached its iteration
+  // one CUDA graph, a conditional while node around one step, until every column
+  // has ended its cycle (it met its tolerance, took m steps or reached its iteration
   // limit).  While phase timing is on, or the caller's stream is itself being
   // captured, the same launches are issued step by step.  A column's arithmetic
   // never depends on the other columns, so its result is the same alone, in a
   // batch, or admitted while other columns are in the middle of their solves.
   // ---------------------------------------------------------------------
-
-  // R columns of n doubles from src (column stride lds) to dst (column stride ldd)
-  void copy_cols(double *dst, int64_t ldd, const double *src, int64_t lds, int64_t n, int R,
-                 cudaStream_t s)
-  {
-    PIBEM_CUDA(cudaMemcpy2DAsync(dst, size_t(ldd) * sizeof(double), src, size_t(lds) * sizeof(double),
-                                 size_t(n) * sizeof(double), size_t(R), cudaMemcpyDeviceToDevice, s));
-  }
 
   template <typename P>
   BlockPrec<P> block_prec(pibem_handle *h, const P *Pinv)
@@ -993,7 +985,7 @@ namespace
       h->d_ilu_y.alloc(size_t(S) * N);
     std::vector<int> minus(S, -1);
     E.jvec.upload(minus, h->stream);
-    E.ctl.alloc(4);
+    E.ctl.alloc(3);
     E.ipin.alloc(size_t(3) * S + 4);
     E.h_bn.assign(S, 1.0);
     E.h_tol.assign(S, 0.0);
@@ -1176,8 +1168,8 @@ namespace
       launch_arnoldi_finish(a, block_prec(h, E.prec ? h->d_Pinv.p : nullptr), E.cz.p, false, s);
   }
 
-  // Runs the Arnoldi steps of the columns in a cycle until one of them ends its
-  // cycle or quantum steps have run; returns the steps run.
+  // Runs the Arnoldi steps of the columns in a cycle until all of them have ended it
+  // or quantum steps have run; returns the steps run.
   int eng_cycle(pibem_handle *h, const std::vector<int> &act, int quantum)
   {
     Engine      &E  = h->eng;
@@ -1200,7 +1192,7 @@ namespace
     // waits, frozen, and the columns' next operator applications stay
     // batched) or for at most a quantum of steps (serving: new submissions
     // join, and finished columns leave, at the next call)
-    E.h_ctl = {0, 0, quantum > 0 ? quantum : std::numeric_limits<int>::max(), 0};
+    E.h_ctl = {0, 0, quantum > 0 ? quantum : std::numeric_limits<int>::max()};
     E.ctl.upload(E.h_ctl, s);
     PIBEM_CUDA(cudaMemsetAsync(E.jcur.p, 0xff, sizeof(int) * E.S, s)); // -1: not in a cycle
     if (eng_direct32(h))
@@ -1352,7 +1344,7 @@ namespace
   }
 
   // Advances every column from event to event until each has finished or waits
-  // in a GMRES cycle, then runs the cycle graph once (until some column ends
+  // in a GMRES cycle, then runs the cycle graph once (until every column has ended
   // its cycle, or for at most quantum steps when quantum > 0).  Returns the
   // number of columns that finished.
   int engine_advance(pibem_handle *h, int quantum = 0)

@@ -22,8 +22,6 @@ namespace pibem
 {
   namespace
   {
-    constexpr int RC = 4; // rhs columns handled per register block in the SpMVs
-
     template <typename T>
     __device__ inline T warp_sum(T v)
     {

@@ -323,8 +323,7 @@ namespace pibem
     // bn <= tol).  hb: [h1 (R x L) | h2 (R x L)], L = m + 1, the two Gram-Schmidt
     // passes' coefficients of a step.  ctl[0]: 1 while
     // the steps go on; ctl[1]: steps run; ctl[2]: most steps before the host is
-    // back (a quantum); ctl[3]: 1 to stop at the first column that ends its
-    // cycle, 0 to go on until every column has ended its cycle.
+    // back (a quantum).
 
     // cycle start of the selected columns: g[r] = (beta_r, 0, ...) with beta_r =
     // sqrt(nrm2[r]), jvec[r] = 0, kdone[r] = -1
@@ -647,9 +646,9 @@ namespace pibem
     __device__ __forceinline__ void givens_step(const GivensArgs &a, int Ra, int S, const int *act,
                                                 const int *sj, const double *snr)
     {
-      __shared__ int ended, alive;
+      __shared__ int alive;
       if (threadIdx.x == 0)
-        ended = alive = 0;
+        alive = 0;
       __syncthreads();
       const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
       const int m = a.m, L = m + 1;
@@ -700,10 +699,7 @@ namespace pibem
               if (fabs(g1) / a.bn[r] <= a.tol[r] || bb == 0.0)
                 a.kdone[r] = done = j + 1;
               if (done >= 0 || j + 1 >= m || it >= a.maxit[r])
-                {
-                  a.jvec[r] = -2 - (j + 1);
-                  ended     = 1;
-                }
+                a.jvec[r] = -2 - (j + 1);
               else
                 {
                   a.jvec[r] = j + 1;
@@ -715,10 +711,9 @@ namespace pibem
       if (threadIdx.x == 0)
         {
           const int steps = a.ctl[1] + 1; // steps run since the host set ctl
-          // the steps go on while some column is in its cycle, for at most
-          // ctl[2] steps, and with ctl[3] set only until the first column ends
-          // its cycle (every active column ends its cycle within m steps)
-          const int stop = !alive || (ended && a.ctl[3]) || steps >= a.ctl[2];
+          // the steps go on while some column is in its cycle (every one ends it within
+          // m steps), for at most ctl[2] steps
+          const int stop = !alive || steps >= a.ctl[2];
           a.ctl[0]       = !stop;
           a.ctl[1]       = steps;
           if (a.use_cond && stop)

@@ -315,11 +315,11 @@ namespace pibem
     // L2P tables at 400k nodes, p = 10: 237 ms -> 69 (319 where a run was a range of point
     // ids, each walking every row).
     // P~_n^m(x) of every n <= p, m <= n into P[n (n + 1) / 2 + m] and, with dS,
-    // legendre_dsin(n, m) into dS[...]: the recurrences of legendre_nm and
-    // legendre_dsin (devmath.cuh) at O(p^2), their square-root factors from
-    // the constant tables (the same values) and the division of the
-    // three-term recurrence as a product with the reciprocal (the values agree
-    // with theirs to a few ulp).
+    // sqrt(1-x^2) dP~_n^m/dx = -dP~_n^m/dtheta into dS[...]:
+    //   dP~_n^m/dtheta = (sqrt((n-m)(n+m+1)) P~_n^{m+1} - sqrt((n+m)(n-m+1)) P~_n^{m-1}) / 2,
+    //   dP~_n^0/dtheta = sqrt(n (n+1)) P~_n^1,
+    // the recurrences at O(p^2) with their square-root factors from the constant tables and
+    // the division of the three-term recurrence as a product with the reciprocal.
     __device__ inline void legendre_table(int p, double x, double s, double *P, double *dS)
     {
       double pmm = 1.0;
