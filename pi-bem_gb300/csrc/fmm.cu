@@ -797,7 +797,7 @@ namespace pibem
     // many lanes have work, and ceil(K / 32) FMA a row replace 4.  A column of one layer
     // only (KER1 / KER2) skips the other layer's table and products.  Bounded by those FMA and,
     // on small meshes, by the rows' serial chain.  GB300, two columns at 386 nodes: 36 us with
-    // four coefficients a lane and eight warps a block -> 11.8.
+    // four coefficients a lane and eight warps a block -> 11.8, with four warps a leaf 7.5.
     template <bool COMBINED, int RC, int NPL>
     __global__ void __launch_bounds__(256)
       p2m_apply64_kernel(int n_leaves, int split, int R, int K, int N, const int64_t *__restrict__ prow_ptr,
@@ -922,7 +922,7 @@ namespace pibem
     // L2P in FP64: lane l multiplies coefficients l, l + 32, ...; RR rows x RC columns are
     // summed together by the butterfly's reduce-scatter (RR RC + 4 - log2(RR RC) additions
     // instead of 5 RR RC, on a pipe where each takes as long as an FMA).  GB300, two columns
-    // at 386 nodes: 23 us as in FP32 -> 8.4.
+    // at 386 nodes: 23 us as in FP32 -> 8.4, with four warps a leaf 4.1.
     template <int RC, int RR, int NPL>
     __global__ void __launch_bounds__(256)
       l2p64_kernel(int n_leaves, int split, int R, int K, int N, const int64_t *__restrict__ row_ptr,
@@ -1646,6 +1646,9 @@ namespace pibem
   // what the SMs hold at once.  One warp -> four (GB300, us): P2M / L2P of a 1.5k-node mesh
   // 6.5 / 5.8 -> 4.1 / 3.6, four columns at 6.1k nodes 13.5 / 11.8 -> 6.6 / 4.8; at 98k nodes
   // (6,710 leaves) it would be 21 / 17 -> 27 / 23, every warp loading its leaf's expansion.
+  // The line in between is flat: FP32 products of one and four columns at 1.5k to 55k nodes
+  // (128 to 14,900 leaves) with 64 warps per SM within 4 % of 32 either way, with 16 up to 5 %
+  // slower (four columns, 1,616 leaves 241 -> 254 us).
   static int leaf_split(int64_t warps)
   {
     int w = LEAF_SPLIT;
@@ -1843,7 +1846,11 @@ namespace pibem
   // 4, and eight threads across 64 columns (32 in FP64, whose blocks take so long that
   // the last wave of 64-column ones left a third of the chip idle).  A launch with fewer
   // than 256 blocks of 64 columns (the tree's small levels) splits the rows over
-  // blockIdx.z, 16 per block, and takes 16 (FP64) or 32 columns per block.
+  // blockIdx.z, 16 per block, and takes 16 (FP64) or 32 columns per block.  Whole products,
+  // us, with the line at 64 / 256 / 1,024 blocks: float-float, four columns, p = 8 at 6.1k
+  // nodes 701 / 528 / 530, p = 10 at 24.6k 1,987 / 1,622 / 1,622; FP64, four columns, p = 8 at
+  // 6.1k 1,957 / 1,744 / 1,745; FP64, one column, p = 8 at 1.5k 309 / 307 / 236, at 6.1k 628 / 625 /
+  // 612, at 13.8k alike: only one-column FP64 products of small meshes would want it higher.
   template <typename IO, typename OP>
   static void launch_cuda_core_gemm(int K, int max_chunk_pairs, int R, int c0,
                                     int c1, const int32_t *ch_start, const int32_t *ch_cnt,

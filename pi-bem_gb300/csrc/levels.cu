@@ -9,7 +9,7 @@
 // level are small (a few thousand K x K matrix-vector products); as batched
 // GEMMs followed by a gather they cost two dependent launches per level and a
 // round trip of the products through HBM.  Here a block computes complete
-// expansions of up to CPB columns (column = (box, right-hand side)).
+// expansions of a batch of columns (column = (box, right-hand side)).
 //
 // Threads: LV_G groups of KT = 32 ceil(K/32) (at most 128) threads; thread t of a
 // group owns output coefficient t of the group's columns g, g + LV_G, ...  Every
@@ -196,7 +196,7 @@ namespace pibem
     // Shared memory: T[lv_kk], X[LV_G C][Kx], P[2][LV_G C][Kx].
     // What bounds it: latency (a level's arithmetic is below a microsecond).  Measured
     // (kernel times, warm caches, GB300), against one block per SM holding all
-    // eight operators: 98k spheroid, p = 8, five levels 50 -> 46 us, and less in the
+    // eight operators: 98k spheroid, p = 8, five levels 50 -> 43 us, and less in the
     // step, where the copies overlap the launch ahead; 55k hull, p = 10, seven
     // levels 85 -> 65 us (the operators read through L1 before).
     template <int C>
@@ -502,7 +502,8 @@ namespace pibem
       return;
     const int K     = op.K;
     const int ncols = (b - a) * R;
-    // three blocks per SM where they fit, else two, in clusters of eight (the deepest
+    // three blocks per SM where they fit (220 KB of the SM's 228 for them with 2 KB each
+    // for static and reserved shared memory), else two, in clusters of eight (the deepest
     // level of a 98k-node mesh, 1,700 parents, with two: 14.7 us, with three 11.5)
     int    max_cl, C;
     size_t smem;

@@ -45,14 +45,14 @@
 //              memory and coalesced row segments;
 //   warp 12    copies the part's 2 S operator slice tiles (pre-swizzled at set-up) with
 //              one bulk copy when operator or part change, and issues the MMAs.
-// What bounds it: the tensor unit's operand reads (six digits: sm__pipe_tc 42 %
-// active, the products themselves 23 %), the epilogue's FP32 instructions and the
-// hand-overs between the roles.  Measured (GB300; before: one accumulator set of 96 columns, the
-// epilogue after the MMAs, a row loaded and stored by one thread, and the CUDA-core
-// float-float GEMM beyond K = 96): 98k spheroid (p = 8, 272,776 pairs) 441 -> 281 us,
-// 198k hull (p = 10) 5,920 -> 1,090 us, 16 columns at 23,816 nodes 1,754 -> 814 us.
-// (One MMA per slice pair 426 us for the first, four epilogue warps 318; six digits for
-// the second 840.)
+// What bounds it: the tensor unit's operand reads (sm__pipe_tc 34 - 35 % active, the
+// products themselves 18 % with six digits, 21 % with seven), the epilogue's FP32
+// instructions and the hand-overs between the roles.  Measured (GB300; before: one
+// accumulator set of 96 columns, the epilogue after the MMAs, a row loaded and stored by
+// one thread, and the CUDA-core float-float GEMM beyond K = 96): 98k spheroid (p = 8,
+// 272,776 pairs) 441 -> 281 us, 198k hull (p = 10) 5,920 -> 1,095 us, 16 columns at 23,816
+// nodes 1,754 -> 814 us.  (One MMA per slice pair 426 us for the first, four epilogue
+// warps 318; six digits for the second 840.)
 // All waits are bounded; a timeout is recorded in *err and the host reports
 // PIBEM_ETIMEDOUT.
 #include <algorithm>
