@@ -2856,6 +2856,18 @@ namespace
                                    std::to_string(worst) + ")");
   }
 
+  // Columns of one pass of the calls with host arrays: launches put column groups into grid
+  // dimensions of 65,535 blocks, the finest of them (FP64 translations of 2 R columns in
+  // groups of 16 pairs' columns) for up to 8,191 columns.  A column's result does not depend
+  // on the others of its pass.
+  constexpr int32_t CALL_COLUMNS = 4096;
+  template <typename F>
+  void column_groups(int32_t R, F f)
+  {
+    for (int64_t r0 = 0; r0 == 0 || r0 < R; r0 += CALL_COLUMNS)
+      f(int32_t(r0), int32_t(std::min<int64_t>(CALL_COLUMNS, R - r0)));
+  }
+
   // host <-> device staging of the host-pointer entry points, in the handle's
   // grow-only slots
   struct HostIO
@@ -2980,19 +2992,21 @@ extern "C"
         throw Error(PIBEM_EINVAL, "pibem_fmm_matvec before pibem_set_mesh");
       if (R < 1 || !phi || !dphi || !oN || !oD)
         throw Error(PIBEM_EINVAL, "bad arguments");
-      const size_t n = size_t(R) * h->N();
-      HostIO       io{h};
-      double      *dp = io.in(phi, n), *dd = io.in(dphi, n);
-      double      *on = io.scratch(n), *od = io.scratch(n);
       if (h->d_dir.n == 0)
         {
           std::vector<uint8_t> z(h->N(), 0);
           h->d_dir.upload(z, h->stream);
         }
-      fmm_apply64(h, R, dp, dd, on, od);
-      PIBEM_CUDA(cudaMemcpyAsync(oN, on, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-      PIBEM_CUDA(cudaMemcpyAsync(oD, od, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-      PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      column_groups(R, [&](int32_t r0, int32_t Rg) {
+        const size_t o = size_t(r0) * h->N(), n = size_t(Rg) * h->N();
+        HostIO       io{h};
+        double      *dp = io.in(phi + o, n), *dd = io.in(dphi + o, n);
+        double      *on = io.scratch(n), *od = io.scratch(n);
+        fmm_apply64(h, Rg, dp, dd, on, od);
+        PIBEM_CUDA(cudaMemcpyAsync(oN + o, on, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        PIBEM_CUDA(cudaMemcpyAsync(oD + o, od, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      });
     });
   }
 
@@ -3013,17 +3027,19 @@ extern "C"
         throw Error(PIBEM_EINVAL, "pibem_apply_preconditioner before pibem_set_bc");
       if (R < 1 || !v || !z)
         throw Error(PIBEM_EINVAL, "bad arguments");
-      const int64_t N  = h->N();
-      const size_t  n  = size_t(R) * N;
-      HostIO        io{h};
-      double       *dv = io.in(v, n), *dz = io.scratch(n);
-      if (h->prm.preconditioner == 0)
-        PIBEM_CUDA(cudaMemcpyAsync(dz, dv, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-      else
-        apply_prec(h, R, dv, N, dz, h->stream);
-      check_device_error(h);
-      PIBEM_CUDA(cudaMemcpyAsync(z, dz, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-      PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      const int64_t N = h->N();
+      column_groups(R, [&](int32_t r0, int32_t Rg) {
+        const size_t o = size_t(r0) * N, n = size_t(Rg) * N;
+        HostIO       io{h};
+        double      *dv = io.in(v + o, n), *dz = io.scratch(n);
+        if (h->prm.preconditioner == 0)
+          PIBEM_CUDA(cudaMemcpyAsync(dz, dv, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+        else
+          apply_prec(h, Rg, dv, N, dz, h->stream);
+        check_device_error(h);
+        PIBEM_CUDA(cudaMemcpyAsync(z + o, dz, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      });
     });
   }
 
@@ -3034,16 +3050,18 @@ extern "C"
         throw Error(PIBEM_EINVAL, "pibem_system_matvec before pibem_set_bc");
       if (R < 1 || !x || !y)
         throw Error(PIBEM_EINVAL, "bad arguments");
-      const size_t n  = size_t(R) * h->N();
-      HostIO       io{h};
-      double      *dx = io.in(x, n), *dy = io.scratch(n);
-      if (h->prm.precision_mode == PIBEM_PRECISION_MIXED && std::getenv("PIBEM_MATVEC_FP32"))
-        system_apply32(h, R, dx, dy);
-      else
-        system_apply64(h, R, dx, dy);
-      check_device_error(h);
-      PIBEM_CUDA(cudaMemcpyAsync(y, dy, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-      PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      column_groups(R, [&](int32_t r0, int32_t Rg) {
+        const size_t o = size_t(r0) * h->N(), n = size_t(Rg) * h->N();
+        HostIO       io{h};
+        double      *dx = io.in(x + o, n), *dy = io.scratch(n);
+        if (h->prm.precision_mode == PIBEM_PRECISION_MIXED && std::getenv("PIBEM_MATVEC_FP32"))
+          system_apply32(h, Rg, dx, dy);
+        else
+          system_apply64(h, Rg, dx, dy);
+        check_device_error(h);
+        PIBEM_CUDA(cudaMemcpyAsync(y + o, dy, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      });
     });
   }
 
@@ -3052,12 +3070,14 @@ extern "C"
     return guarded(h, [&] {
       if (!h->bc_ok)
         throw Error(PIBEM_EINVAL, "pibem_compute_rhs before pibem_set_bc");
-      const size_t n  = size_t(R) * h->N();
-      HostIO       io{h};
-      double      *dt = io.in(tmp, n), *db = io.scratch(n);
-      compute_rhs_dev(h, R, dt, db);
-      PIBEM_CUDA(cudaMemcpyAsync(rhs, db, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-      PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      column_groups(R, [&](int32_t r0, int32_t Rg) {
+        const size_t o = size_t(r0) * h->N(), n = size_t(Rg) * h->N();
+        HostIO       io{h};
+        double      *dt = io.in(tmp + o, n), *db = io.scratch(n);
+        compute_rhs_dev(h, Rg, dt, db);
+        PIBEM_CUDA(cudaMemcpyAsync(rhs + o, db, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      });
     });
   }
 
@@ -3232,15 +3252,17 @@ extern "C"
         throw Error(PIBEM_EINVAL, "L2 projection before pibem_set_mesh");
       if (R < 1 || !out || (mode > 0 && !u) || (mode == 2 && !dudn))
         throw Error(PIBEM_EINVAL, "bad arguments");
-      const int64_t N = h->N(), n = size_t(R) * N;
-      HostIO        io{h};
-      const double *du = mode > 0 ? io.in(u, n) : nullptr;
-      const double *dd = mode == 2 ? io.in(dudn, n) : nullptr;
-      double       *dout = io.scratch(size_t(3) * n);
-      projection_dev(h, mode, R, du, dd, dout);
-      PIBEM_CUDA(cudaMemcpyAsync(out, dout, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost,
-                                 h->stream));
-      PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      column_groups(R, [&](int32_t r0, int32_t Rg) {
+        const size_t  o = size_t(r0) * h->N(), n = size_t(Rg) * h->N();
+        HostIO        io{h};
+        const double *du = mode > 0 ? io.in(u + o, n) : nullptr;
+        const double *dd = mode == 2 ? io.in(dudn + o, n) : nullptr;
+        double       *dout = io.scratch(size_t(3) * n);
+        projection_dev(h, mode, Rg, du, dd, dout);
+        PIBEM_CUDA(cudaMemcpyAsync(out + 3 * o, dout, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost,
+                                   h->stream));
+        PIBEM_CUDA(cudaStreamSynchronize(h->stream));
+      });
     });
   }
 
