@@ -355,8 +355,11 @@ struct pibem_handle
 
 namespace
 {
+  // A failed launch leaves its error for the next cudaGetLastError(), which may be that
+  // of another handle's call: taken here.
   int fail(pibem_handle *h, const Error &e)
   {
+    (void)cudaGetLastError();
     if (h)
       h->err = e.what();
     return e.code;
@@ -2931,7 +2934,7 @@ extern "C"
       }
     catch (const Error &e)
       {
-        int c = e.code;
+        int c = fail(nullptr, e);
         delete h;
         return c;
       }

@@ -1,5 +1,6 @@
 """The calls with host arrays at column counts beyond what one launch's grid takes (65,535 blocks a
-dimension): every column has the bits it has alone."""
+dimension): every column has the bits it has alone.  And a call that fails leaves nothing behind for
+the next one."""
 import numpy as np
 import pytest
 
@@ -25,4 +26,13 @@ def test_many_columns(mode, leaf, pibem_mod, synthetic, monkeypatch):
         Y = f(X)
         for r in some:
             np.testing.assert_array_equal(np.asarray(f(X[r:r + 1]))[0], Y[r], err_msg=f"{name} {r}")
+    g.close()
+
+
+def test_failed_call_leaves_no_error(pibem_mod, synthetic):
+    mesh = synthetic.spheroid(3)
+    with pytest.raises(pibem_mod.PibemError):
+        pibem_mod.BEMSolver(device=99)
+    g = pibem_mod.BEMSolver(fma_truncation_order=2)
+    g.set_mesh(mesh.xyz, mesh.cells)
     g.close()
