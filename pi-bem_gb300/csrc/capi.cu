@@ -2387,7 +2387,9 @@ namespace
       h->d_N.zero(s);
       h->d_D.zero(s);
       DBuf<double> staging;
-      int64_t      st_items = std::min<int64_t>(item_ptr[nl], int64_t(1) << 24);
+      // at most 1.2 GB of staging (72 bytes an item) and weights together
+      const int64_t st_most  = std::max<int64_t>((int64_t(1) << 24) - int64_t(qw.bytes() / 72), int64_t(1) << 22);
+      int64_t       st_items = std::min<int64_t>(item_ptr[nl], st_most);
       int64_t      maxrow   = 0;
       for (int k = 0; k < nl; ++k)
         maxrow = std::max<int64_t>(maxrow, pl.nent_ptr[k + 1] - pl.nent_ptr[k]);
