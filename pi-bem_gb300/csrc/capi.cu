@@ -359,7 +359,8 @@ namespace
   // of another handle's call: taken here.
   int fail(pibem_handle *h, const Error &e)
   {
-    (void)cudaGetLastError();
+    if (e.code == PIBEM_ECUDA || e.code == PIBEM_ENOMEM_HBM)
+      (void)cudaGetLastError();
     if (h)
       h->err = e.what();
     return e.code;
